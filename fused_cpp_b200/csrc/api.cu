@@ -85,7 +85,7 @@ int make_layout(bool int8, int64_t tokens, int top_k, int experts, int hidden, i
   layout->sorted_routes = take(sizeof(int) * rows);
   layout->row_expert = take(sizeof(int) * rows);
   layout->items = take(sizeof(int) * 4 * max_items * 4);  // four work-item lists (see fmoe::ItemLists)
-  layout->scratch = take(fmoe::route_scratch_bytes(routes, experts));
+  layout->scratch = take(0);
   layout->a_rows = take(with_route_out ? rows * hidden * (int8 ? 1 : 2) : 256);
   layout->a_scale = take(sizeof(float) * rows);
   layout->y = take(rows * inter * 2);
@@ -275,7 +275,6 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   int* items_dn_big = items_gu_big + 4 * static_cast<size_t>(max_items);
   const fmoe::ItemLists lists{item_rows_gu, item_rows_dn, items_gu, items_dn, max_items, split ? kSplitRows : 0, split ? pair_item_rows : 0,
                               items_gu_big, items_dn_big};
-  int* scratch = reinterpret_cast<int*>(base + layout.scratch);
   float* a_scale = reinterpret_cast<float*>(base + layout.a_scale);
   uint16_t* y = reinterpret_cast<uint16_t*>(base + layout.y);
   float* y_scale = reinterpret_cast<float*>(base + layout.y_scale);
@@ -291,12 +290,12 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
     if (marks != nullptr) cudaEventRecord(marks[index], stream);
   };
   mark(0);
-  cudaError_t error = cudaMemsetAsync(status_block, 0, sizeof(int) * fmoe::kStatusWords, stream);
-  if (error != cudaSuccess) return cuda_fail(error, "cudaMemsetAsync(status)");
+  cudaError_t error = cudaSuccess;
   uint64_t* row_out_ptrs = nullptr;
   if (peer) {
     // The rows arrived in expert order: only the work items and the output addresses remain to be made.
-    error = fmoe::launch_items_from_counts(f.experts, f.sorted_counts, f.sorted_offsets, lists, scratch, status_block, stream);
+    error = cudaMemsetAsync(status_block, 0, sizeof(int) * fmoe::kStatusWords, stream);
+    if (error == cudaSuccess) error = fmoe::launch_items_from_counts(f.experts, f.sorted_counts, f.sorted_offsets, lists, status_block, stream);
     if (error != cudaSuccess) return cuda_fail(error, "work items");
     row_out_ptrs = reinterpret_cast<uint64_t*>(base + layout.route_out);
     error = fmoe::launch_peer_row_ptrs(f.sorted_offsets + f.experts, routes, f.rows_source, f.peer_slabs, f.peer_route_out_offset,
@@ -304,8 +303,8 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
                                        f.peer_scrap_row, status_block, stream);
     if (error != cudaSuccess) return cuda_fail(error, "peer output addresses");
   } else {
-    error = fmoe::launch_route_build(f.topk_ids, routes, f.experts, lists, status_block, counts, offsets, sorted_routes, row_expert, scratch,
-                                     stream, reinterpret_cast<int*>(base + layout.route_pos));
+    error = fmoe::launch_route_build(f.topk_ids, routes, f.experts, lists, status_block, counts, offsets, sorted_routes, row_expert, stream,
+                                     reinterpret_cast<int*>(base + layout.route_pos));
     if (error != cudaSuccess) return cuda_fail(error, "route build");
   }
   mark(FMOE_STAGE_ROUTE + 1);
@@ -588,8 +587,7 @@ size_t fmoe_ep_dispatch_workspace_bytes(int64_t tokens, int32_t top_k, int32_t w
   if (tokens < 0 || top_k <= 0 || world <= 0) return 0;
   const size_t routes = static_cast<size_t>(tokens) * top_k;
   return align_up(sizeof(int) * fmoe::kStatusWords, 256) + align_up(sizeof(int64_t) * (routes > 0 ? routes : 1), 256) +
-         align_up(sizeof(int) * (world + 1), 256) + align_up(sizeof(int) * (routes > 0 ? routes : 1), 256) +
-         align_up(fmoe::route_scratch_bytes(routes, world), 256) + 256;
+         align_up(sizeof(int) * (world + 1), 256) + align_up(sizeof(int) * (routes > 0 ? routes : 1), 256) + 256;
 }
 
 int fmoe_ep_dispatch_prepare(const void* x, const int64_t* topk_ids, int64_t tokens, int32_t top_k, int32_t experts_global,
@@ -617,11 +615,10 @@ int fmoe_ep_dispatch_prepare(const void* x, const int64_t* topk_ids, int64_t tok
   int64_t* dest = reinterpret_cast<int64_t*>(take(sizeof(int64_t) * (routes > 0 ? routes : 1)));
   int* offsets = reinterpret_cast<int*>(take(sizeof(int) * (world + 1)));
   int* row_rank = reinterpret_cast<int*>(take(sizeof(int) * (routes > 0 ? routes : 1)));
-  int* scratch = reinterpret_cast<int*>(take(fmoe::route_scratch_bytes(routes, world)));
-  cudaError_t error = cudaMemsetAsync(status_block, 0, sizeof(int) * fmoe::kStatusWords, stream);
-  if (error != cudaSuccess) return cuda_fail(error, "cudaMemsetAsync(status)");
+  cudaError_t error = cudaSuccess;
   if (routes == 0) {
-    error = cudaMemsetAsync(dest_counts, 0, sizeof(int) * world, stream);
+    error = cudaMemsetAsync(status_block, 0, sizeof(int) * fmoe::kStatusWords, stream);
+    if (error == cudaSuccess) error = cudaMemsetAsync(dest_counts, 0, sizeof(int) * world, stream);
     return error == cudaSuccess ? FMOE_OK : cuda_fail(error, "cudaMemsetAsync(counts)");
   }
   if (x == nullptr || topk_ids == nullptr || send_order == nullptr || send_rows == nullptr || send_expert == nullptr ||
@@ -632,7 +629,7 @@ int fmoe_ep_dispatch_prepare(const void* x, const int64_t* topk_ids, int64_t tok
   if (error == cudaSuccess) {
     // A stable counting sort of the routes by destination rank: the same kernels as the per-expert route build.
     error = fmoe::launch_route_build(dest, routes, world, fmoe::no_item_lists(), status_block, dest_counts, offsets, send_order, row_rank,
-                                     scratch, stream);
+                                     stream);
   }
   const int* valid_rows = offsets + world;
   if (error == cudaSuccess) {
@@ -944,14 +941,12 @@ struct DispatchScratch {
   int* send_order;  // [routes] flat route ids in expert order
   int* row_expert;  // [routes]
   int* route_pos;   // [routes] position of every flat route in that order, -1 = dropped
-  int* scratch;
 };
 
 size_t dispatch_scratch_bytes(int64_t routes, int experts_total) {
   const size_t r = static_cast<size_t>(routes > 0 ? routes : 1);
   return align_up(sizeof(int) * fmoe::kStatusWords, 256) + align_up(sizeof(int) * experts_total, 256) +
-         align_up(sizeof(int) * (experts_total + 1), 256) + 3 * align_up(sizeof(int) * r, 256) +
-         align_up(fmoe::route_scratch_bytes(routes, experts_total), 256);
+         align_up(sizeof(int) * (experts_total + 1), 256) + 3 * align_up(sizeof(int) * r, 256);
 }
 
 DispatchScratch carve_dispatch(char* base, int64_t routes, int experts_total) {
@@ -969,7 +964,6 @@ DispatchScratch carve_dispatch(char* base, int64_t routes, int experts_total) {
   d.send_order = reinterpret_cast<int*>(take(sizeof(int) * r));
   d.row_expert = reinterpret_cast<int*>(take(sizeof(int) * r));
   d.route_pos = reinterpret_cast<int*>(take(sizeof(int) * r));
-  d.scratch = reinterpret_cast<int*>(take(fmoe::route_scratch_bytes(routes, experts_total)));
   return d;
 }
 
@@ -1139,13 +1133,16 @@ int fmoe_ep_peer_dispatch(fmoe_ep_peer_context* ctx, const void* x, const int64_
   const int experts_total = experts_global + has_shared;
   const int per_rank = experts_global / ctx->world;
   const DispatchScratch d = carve_dispatch(ctx->dispatch_ws, ctx->tokens_max * ctx->top_k, ctx->experts_total_max);
-  cudaError_t error = cudaMemsetAsync(d.status, 0, sizeof(int) * fmoe::kStatusWords, stream);
-  if (error == cudaSuccess && routes == 0) error = cudaMemsetAsync(d.counts, 0, sizeof(int) * experts_total, stream);
+  cudaError_t error = cudaSuccess;
+  if (routes == 0) {
+    error = cudaMemsetAsync(d.status, 0, sizeof(int) * fmoe::kStatusWords, stream);
+    if (error == cudaSuccess) error = cudaMemsetAsync(d.counts, 0, sizeof(int) * experts_total, stream);
+  }
   if (error == cudaSuccess && routes > 0) {
     // Stable counting sort of this rank's routes by global expert id (the shared expert is id experts_global):
     // expert order is destination-rank order, and inside a destination its local expert order.
     error = fmoe::launch_route_build(topk_ids, routes, experts_total, fmoe::no_item_lists(), d.status, d.counts, d.offsets, d.send_order,
-                                     d.row_expert, d.scratch, stream, d.route_pos);
+                                     d.row_expert, stream, d.route_pos);
   }
   if (error == cudaSuccess) {
     // Every rank learns every rank's counts per expert (row `rank` of the table in each slab) ...

@@ -7,14 +7,12 @@
 
 namespace fmoe {
 
-constexpr int kUnitRoutes = 512;   // routes per warp in the route-build kernels
 constexpr int kMaxExperts = 2048;  // bound of the per-warp shared-memory histograms
 
 // ---- api.cu
 int report_error(int code, const char* text);
 
 // ---- route.cu
-size_t route_scratch_bytes(int64_t routes, int experts);
 // The work-item lists a route build fills: a and b for the gate_up and the down GEMM (tile heights tile_a,
 // tile_b).  With split_rows > 0, a and b hold only the experts with at most split_rows rows and c and d
 // (tile big_tile) the experts with more; every list has room for max_items items of four ints.
@@ -29,12 +27,12 @@ struct ItemLists {
   int* items_d;
 };
 inline ItemLists no_item_lists() { return ItemLists{16, 16, nullptr, nullptr, 0, 0, 0, nullptr, nullptr}; }
+// One launch; clears the status block, then raises FMOE_ERR_EXPERT_ID_RANGE in it for ids outside [0, experts).
 cudaError_t launch_route_build(const int64_t* topk_ids, int64_t routes, int experts, const ItemLists& lists, int* status, int* counts,
-                               int* offsets, int* sorted_routes, int* row_expert, int* scratch, cudaStream_t stream,
-                               int* route_pos = nullptr);
+                               int* offsets, int* sorted_routes, int* row_expert, cudaStream_t stream, int* route_pos = nullptr);
 
-// Work items from per-expert counts / offsets of rows that are already in expert order (scratch: 2 * experts + 1 ints).
-cudaError_t launch_items_from_counts(int experts, const int* counts, const int* offsets, const ItemLists& lists, int* scratch, int* status,
+// Work items from per-expert counts / offsets of rows that are already in expert order.
+cudaError_t launch_items_from_counts(int experts, const int* counts, const int* offsets, const ItemLists& lists, int* status,
                                      cudaStream_t stream);
 
 // ---- quant.cu

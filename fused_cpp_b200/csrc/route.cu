@@ -3,13 +3,20 @@
 // The reference walks topk_ids once on the calling thread and pushes each flat route id t*K+slot
 // onto its expert's vector (csrc/moe/arm/i8mm_w8a8/kernels.cpp:583-592;
 // csrc/moe/arm/common/fused_moe_bf16_tiled.cpp:6455-6469), i.e. a stable counting sort by expert.
-// Here the same order is produced by three small kernels built on warp primitives:
-//   1. route_hist:    every warp owns a unit of kUnitRoutes consecutive routes and histograms it;
-//   2. route_scan:    one block turns the unit histograms into per-(unit, expert) cursors, the
-//                     per-expert offsets and the (expert, row-tile) work items;
-//   3. route_scatter: every warp replays its unit in order; __match_any_sync ranks equal ids inside
-//                     a 32-route round, so positions are assigned in ascending flat-id order.
+// Here one launch of one thread-block cluster (1 to 8 CTAs) produces the same order:
+//   1. every warp owns a run of consecutive routes and histograms it in its own shared-memory row;
+//   2. the CTA turns the rows into exclusive counts over its warps, the cluster exchanges the CTA totals through
+//      distributed shared memory, and every CTA scans the totals over the experts;
+//   3. every warp replays its run in order; ballots rank equal ids inside a 32-route round, so positions are
+//      assigned in ascending flat-id order.  Meanwhile one warp per list writes the (expert, row tile) work items.
 // Ids outside [0, E) raise FMOE_ERR_EXPERT_ID_RANGE in the status block and are dropped.
+//
+// The work is a few KB per CTA: what bounds it is latency - launches, barriers and dependent loads - so the form that
+// counts is the one with the fewest of them.  Back to back on one stream: 8 routes 6.2 us, 4072 routes 10.3 us, 65536
+// routes 18.5 us, 147456 routes 31 us (256 experts).  The form before it (a memset of the status block and one block up
+// to 1024 routes, three launches - histogram, one-block scan, scatter - above) took, by the stage timer, 14 / 35 / 60 /
+// 105 us, where this one takes 9 / 13 / 28 / 54 us.
+#include <cooperative_groups.h>
 #include <cstdio>
 #include <mutex>
 
@@ -20,39 +27,88 @@ namespace fmoe {
 
 namespace {
 
-constexpr int kWarpsPerBlock = 4;
+constexpr int kRouteThreads = 1024;
+constexpr int kRouteWarps = kRouteThreads / 32;
+constexpr int kMaxRouteCluster = 8;         // portable cluster size
+constexpr int kRoutesPerCta = 1024;         // one 32-route round per warp; more routes take more CTAs first, then more rounds
+constexpr int kHistogramInts = 32 * 1024;   // shared-memory histogram rows: 32 warps up to 1024 experts, 16 up to 2048
 
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-route_hist_kernel(const int64_t* __restrict__ topk_ids, int64_t routes, int experts, int units, int* unit_hist, int* status) {
-  extern __shared__ int smem_hist[];
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int unit = blockIdx.x * kWarpsPerBlock + warp;
-  int* hist = smem_hist + warp * experts;
-  for (int e = lane; e < experts; e += 32) hist[e] = 0;
-  __syncwarp();
-  if (unit >= units) return;
-  const int64_t begin = static_cast<int64_t>(unit) * kUnitRoutes;
-  for (int round = 0; round < kUnitRoutes / 32; ++round) {
-    const int64_t route = begin + round * 32 + lane;
-    if (route < routes) {
-      const int64_t id = topk_ids[route];
-      if (id < 0 || id >= experts) {
-        raise_error(status, FMOE_ERR_EXPERT_ID_RANGE, static_cast<int>(route));
-      } else {
-        atomicAdd(hist + id, 1);
+// The work items of one list: (expert, first sorted row, rows, group key) for every row tile of every expert that
+// belongs to it.  Lists a and b (gate_up and down GEMM) have independent tile heights.  With split_rows > 0 they
+// hold only the experts with at most split_rows rows, and lists c and d (tile big_tile) the experts with more: the
+// batch's routing decides on the device, expert by expert, whether an expert's rows go to the weight-streaming kernel
+// or to the two-SM kernel, with no host-side guess about the distribution.  Called by one whole warp.
+__device__ void build_item_list(int list, int experts, const int* counts, const int* offsets, const ItemLists& lists, int* status, int lane) {
+  const int split_rows = lists.split_rows;
+  const int max_items = lists.max_items;
+  const bool big = list >= 2;
+  const int word = list == 0 ? kStatusItems : list == 1 ? kStatusItemsB : list == 2 ? kStatusItemsC : kStatusItemsD;
+  if (big && split_rows <= 0) {
+    if (lane == 0) status[word] = 0;
+    return;
+  }
+  const int tile = list == 0 ? lists.tile_a : list == 1 ? lists.tile_b : lists.big_tile;
+  int* items = list == 0 ? lists.items_a : list == 1 ? lists.items_b : list == 2 ? lists.items_c : lists.items_d;
+  const int shift = __ffs(tile) - 1;  // row tiles are powers of two
+  int carry = 0;
+  int active = 0;
+  constexpr int kBatch = 8;  // groups of 32 experts whose scans are interleaved: a scan is a chain of dependent shuffles
+  for (int base = 0; base < experts; base += 32 * kBatch) {
+    int count[kBatch], inclusive[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int e = base + 32 * i + lane;
+      count[i] = e < experts ? counts[e] : 0;
+      active += __popc(__ballot_sync(0xffffffffu, count[i] > 0));
+      if (split_rows > 0 && big != (count[i] > split_rows)) count[i] = 0;  // belongs to the other list
+      inclusive[i] = (count[i] + tile - 1) >> shift;
+    }
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) {
+        const int other = __shfl_up_sync(0xffffffffu, inclusive[i], offset);
+        if (lane >= offset) inclusive[i] += other;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int tiles = (count[i] + tile - 1) >> shift;
+      const int first = carry + inclusive[i] - tiles;
+      carry += __shfl_sync(0xffffffffu, inclusive[i], 31);
+      if (tiles == 0) continue;
+      const int e = base + 32 * i + lane;
+      const int row0 = offsets[e];
+      // The expert's rows are spread evenly over its tiles (in steps of 32 rows, the granularity of the MMA's N):
+      // 290 rows become 160 + 130, not 256 + 34.
+      int rows_per = tile;
+      if (tiles > 1) {
+        const int step = tile < 32 ? tile : 32;
+        const int even = ((count[i] + tiles - 1) / tiles + step - 1) & ~(step - 1);
+        if (even <= tile && (tiles - 1) * even < count[i]) rows_per = even;
+      }
+      for (int t = 0; t < tiles && first + t < max_items; ++t) {
+        // Group key for the unit order of the grouped GEMM: first item of this expert and its tile count, so that the
+        // row tiles of one (expert, channel block) are consecutive work units (see decode_unit).
+        reinterpret_cast<int4*>(items)[first + t] = make_int4(e, row0 + t * rows_per, min(rows_per, count[i] - t * rows_per),
+                                                              tiles < 2048 ? (first | (tiles << 20)) : ((first + t) | (1 << 20)));
       }
     }
   }
-  __syncwarp();
-  for (int e = lane; e < experts; e += 32) unit_hist[static_cast<int64_t>(unit) * experts + e] = hist[e];
+  if (lane == 0) {
+    status[word] = carry < max_items ? carry : max_items;
+    if (list == 0) status[kStatusActive] = active;
+  }
 }
 
-// Exclusive scan of `values[0..n)` by one warp, 32 entries per step; returns the total.
-__device__ int warp_exclusive_scan(const int* values, int* out, int n, int lane) {
-  int carry = 0;
-  for (int base = 0; base < n; base += 32) {
-    const int index = base + lane;
+// Exclusive scan of values[0..n) into out[0..n], out[n] = total.  Called by the whole block; chunk_sums has room for
+// (n + 31) / 32 ints.  Every 32 values are scanned by one warp, the chunk totals by warp 0.
+__device__ void block_exclusive_scan(const int* values, int* out, int n, int* chunk_sums) {
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int chunks = (n + 31) >> 5;
+  for (int chunk = warp; chunk < chunks; chunk += static_cast<int>(blockDim.x >> 5)) {
+    const int index = chunk * 32 + lane;
     const int value = index < n ? values[index] : 0;
     int inclusive = value;
 #pragma unroll
@@ -60,242 +116,246 @@ __device__ int warp_exclusive_scan(const int* values, int* out, int n, int lane)
       const int other = __shfl_up_sync(0xffffffffu, inclusive, offset);
       if (lane >= offset) inclusive += other;
     }
-    if (index < n) out[index] = carry + inclusive - value;
-    carry += __shfl_sync(0xffffffffu, inclusive, 31);
+    if (index < n) out[index] = inclusive - value;
+    if (lane == 31) chunk_sums[chunk] = inclusive;
   }
-  return carry;
-}
-
-// Work items: (expert, first sorted row, rows, group key) for every row tile of every active expert, and the
-// number of active experts.  Lists a and b (gate_up and down GEMM) have independent tile heights.  With
-// split_rows > 0 they hold only the experts with at most split_rows rows, and lists c and d (tile big_tile) the
-// experts with more: the batch's routing decides on the device, expert by expert, whether an expert's rows go to
-// the weight-streaming kernel or to the two-SM kernel, with no host-side guess about the distribution.
-// Called by a whole block; scan_tmp has room for 2 * experts + 1 ints (global or shared).
-__device__ void build_items(int experts, const int* counts, const int* offsets, const ItemLists& lists, int* scan_tmp, int* status) {
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int split_rows = lists.split_rows;
-  const int max_items = lists.max_items;
-  for (int list = 0; list < 4; ++list) {
-    const bool big = list >= 2;
-    const int word = list == 0 ? kStatusItems : list == 1 ? kStatusItemsB : list == 2 ? kStatusItemsC : kStatusItemsD;
-    if (big && split_rows <= 0) {
-      if (threadIdx.x == 0) status[word] = 0;
-      continue;
-    }
-    const int tile = list == 0 ? lists.tile_a : list == 1 ? lists.tile_b : lists.big_tile;
-    int* items = list == 0 ? lists.items_a : list == 1 ? lists.items_b : list == 2 ? lists.items_c : lists.items_d;
-    for (int e = threadIdx.x; e < experts; e += blockDim.x) {
-      const bool mine = split_rows <= 0 || (big ? counts[e] > split_rows : counts[e] <= split_rows);
-      scan_tmp[e] = mine ? (counts[e] + tile - 1) / tile : 0;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      const int total = warp_exclusive_scan(scan_tmp, scan_tmp + experts, experts, lane);
-      if (lane == 0) status[word] = total < max_items ? total : max_items;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < experts; e += blockDim.x) {
-      const int tiles = scan_tmp[e];
-      const int first = scan_tmp[experts + e];
-      // The expert's rows are spread evenly over its tiles (in steps of 32 rows, the granularity of the MMA's N):
-      // 290 rows become 160 + 130, not 256 + 34.
-      int rows_per = tile;
-      if (tiles > 1) {
-        const int step = tile < 32 ? tile : 32;
-        const int even = ((counts[e] + tiles - 1) / tiles + step - 1) / step * step;
-        if (even <= tile && (tiles - 1) * even < counts[e]) rows_per = even;
-      }
-      for (int t = 0; t < tiles && first + t < max_items; ++t) {
-        int* item = items + 4 * static_cast<int64_t>(first + t);
-        item[0] = e;
-        item[1] = offsets[e] + t * rows_per;
-        item[2] = min(rows_per, counts[e] - t * rows_per);
-        // Group key for the unit order of the grouped GEMM: first item of this expert and its tile count, so
-        // that the row tiles of one (expert, channel block) are consecutive work units (see decode_unit).
-        item[3] = tiles < 2048 ? (first | (tiles << 20)) : ((first + t) | (1 << 20));
-      }
-    }
-    __syncthreads();
-  }
+  __syncthreads();
   if (warp == 0) {
-    int active = 0;
-    for (int e = lane; e < experts; e += 32) active += counts[e] > 0;
-    active = warp_sum(active);
-    if (lane == 0) status[kStatusActive] = active;
+    int carry = 0;
+    for (int base = 0; base < chunks; base += 32) {
+      const int index = base + lane;
+      const int value = index < chunks ? chunk_sums[index] : 0;
+      int inclusive = value;
+#pragma unroll
+      for (int offset = 1; offset < 32; offset <<= 1) {
+        const int other = __shfl_up_sync(0xffffffffu, inclusive, offset);
+        if (lane >= offset) inclusive += other;
+      }
+      if (index < chunks) chunk_sums[index] = carry + inclusive - value;
+      carry += __shfl_sync(0xffffffffu, inclusive, 31);
+    }
+    if (lane == 0) out[n] = carry;
   }
+  __syncthreads();
+  for (int index = threadIdx.x; index < n; index += blockDim.x) out[index] += chunk_sums[index >> 5];
+  __syncthreads();
 }
 
-// The whole route build in one block for lists of at most kSmallRoutes entries (decode batches, and the
-// expert-parallel lists at decode): ids and histogram in shared memory, the stable position of a route is its
-// expert's offset plus the number of earlier routes with the same id (a scan of the shared ids, at most
-// kSmallRoutes steps).  Same outputs as the three-kernel form.
-constexpr int kSmallRoutes = 1024;
+// The lanes of the warp that hold the same `id` as this one.  One ballot per bit of the id: `__match_any_sync`, which
+// answers the same, costs about 80 clocks of the SM per call (65536 routes: 22 us with it, 18.5 us with ballots).
+__device__ __forceinline__ unsigned lanes_with_same(int id, int bits) {
+  unsigned same = 0xffffffffu;
+  for (int bit = 0; bit < bits; ++bit) {
+    const bool set = (id >> bit) & 1;
+    const unsigned with_bit = __ballot_sync(0xffffffffu, set);
+    same &= set ? with_bit : ~with_bit;
+  }
+  return same;
+}
 
-__global__ void __launch_bounds__(kSmallRoutes)
-route_small_kernel(const int64_t* __restrict__ topk_ids, int routes, int experts, ItemLists lists, int* status, int* counts, int* offsets,
-                   int* sorted_routes, int* row_expert, int* route_pos) {
-  extern __shared__ int small_smem[];
-  int* s_id = small_smem;
-  int* s_counts = s_id + kSmallRoutes;
+// Shared memory: hist[warps][experts] | counts[experts] | offsets[experts + 1] | chunk sums | kCluster: totals[experts],
+// base[experts].  `run` routes per warp (a multiple of 32); warp w of CTA c owns the run number c * warps + w.
+template <bool kCluster>
+__global__ void __launch_bounds__(kRouteThreads)
+route_build_kernel(const int64_t* __restrict__ topk_ids, int64_t routes, int experts, int warps, int64_t run, ItemLists lists, int* status,
+                   int* counts, int* offsets, int* sorted_routes, int* row_expert, int* route_pos) {
+  namespace cg = cooperative_groups;
+  extern __shared__ int route_smem[];
+  int* hist = route_smem;
+  int* s_counts = hist + warps * experts;  // routes per expert
   int* s_offsets = s_counts + experts;
-  int* s_tmp = s_offsets + experts + 1;
+  int* chunk_sums = s_offsets + experts + 1;
+  int* totals = kCluster ? chunk_sums + (experts + 31) / 32 : s_counts;  // this CTA's routes per expert (read by the other CTAs)
+  int* base = kCluster ? totals + experts : s_offsets;                   // first sorted position of this CTA's routes of an expert
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  for (int e = threadIdx.x; e < experts; e += blockDim.x) s_counts[e] = 0;
+  const int rank = kCluster ? static_cast<int>(cg::this_cluster().block_rank()) : 0;
+  const int ctas = kCluster ? static_cast<int>(cg::this_cluster().num_blocks()) : 1;
+
+  for (int i = threadIdx.x; i < warps * experts; i += blockDim.x) hist[i] = 0;
+  if (rank == 0 && threadIdx.x < kStatusWords) status[threadIdx.x] = 0;
   __syncthreads();
-  const int r = threadIdx.x;
-  int id = -1;
-  if (r < routes) {
-    const int64_t value = topk_ids[r];
-    if (value >= 0 && value < experts) {
-      id = static_cast<int>(value);
-      atomicAdd(s_counts + id, 1);
-    } else {
-      raise_error(status, FMOE_ERR_EXPERT_ID_RANGE, r);
+
+  const int64_t begin = (static_cast<int64_t>(rank) * warps + warp) * run;
+  const int64_t end = warp < warps ? min(begin + run, routes) : begin;
+  int* row = hist + warp * experts;
+  int64_t bad_route = -1;  // reported below, once the status block is known to be clear
+  constexpr int kBatch = kCluster ? 4 : 1;  // rounds whose loads are in flight together (one CTA: a warp has one round)
+  for (int64_t r0 = begin; r0 < end; r0 += 32 * kBatch) {
+    int64_t ids[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) ids[i] = r0 + 32 * i + lane < end ? topk_ids[r0 + 32 * i + lane] : -1;
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      if (r0 + 32 * i + lane >= end) continue;
+      if (ids[i] >= 0 && ids[i] < experts) {
+        atomicAdd(row + ids[i], 1);
+      } else {
+        bad_route = r0 + 32 * i + lane;
+      }
     }
   }
-  s_id[r] = id;
   __syncthreads();
-  if (warp == 0) {
-    const int total = warp_exclusive_scan(s_counts, s_offsets, experts, lane);
-    if (lane == 0) s_offsets[experts] = total;
-  }
-  __syncthreads();
-  int position = -1;
-  if (id >= 0) {
-    int rank = 0;
-    for (int j = 0; j < r; ++j) rank += s_id[j] == id;
-    position = s_offsets[id] + rank;
-    sorted_routes[position] = r;
-    row_expert[position] = id;
-  }
-  if (route_pos != nullptr && r < routes) route_pos[r] = position;
-  for (int e = threadIdx.x; e <= experts; e += blockDim.x) {
-    if (e < experts) counts[e] = s_counts[e];
-    offsets[e] = s_offsets[e];
-  }
-  build_items(experts, s_counts, s_offsets, lists, s_tmp, status);
-}
-
-__global__ void __launch_bounds__(1024)
-route_scan_kernel(int experts, int units, int* unit_hist, int* counts, int* offsets, ItemLists lists, int* scan_tmp, int* status) {
-  // Pass 1: per expert, exclusive scan over units (unit_hist becomes the unit's cursor relative to the
-  // expert's first row) and the expert total.  One thread per expert (adjacent threads read adjacent words);
-  // the units are taken sixteen at a time, all loads of a batch issued before the first store, so the
-  // sweep costs one memory round trip per batch and not one per unit.
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  constexpr int kBatch = 16;
   for (int e = threadIdx.x; e < experts; e += blockDim.x) {
     int running = 0;
-    for (int base = 0; base < units; base += kBatch) {
-      int values[kBatch];
+#pragma unroll 8
+    for (int w = 0; w < warps; ++w) {
+      const int value = hist[w * experts + e];
+      hist[w * experts + e] = running;
+      running += value;
+    }
+    totals[e] = running;
+  }
+  if constexpr (kCluster) {
+    cg::this_cluster().sync();  // totals of every CTA and the cleared status block are visible
+    for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+      int values[kMaxRouteCluster];
 #pragma unroll
-      for (int i = 0; i < kBatch; ++i) {
-        const int u = base + i;
-        values[i] = u < units ? unit_hist[static_cast<int64_t>(u) * experts + e] : 0;
+      for (int c = 0; c < kMaxRouteCluster; ++c) values[c] = c < ctas ? cg::this_cluster().map_shared_rank(totals, c)[e] : 0;
+      int before = 0, all = 0;
+#pragma unroll
+      for (int c = 0; c < kMaxRouteCluster; ++c) {
+        if (c < rank) before += values[c];
+        all += values[c];
       }
+      base[e] = before;
+      s_counts[e] = all;
+    }
+    // This CTA reads no other CTA's totals after this.  (Nothing was written for the others: no release is needed.)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  }
+  __syncthreads();
+  if (bad_route >= 0) raise_error(status, FMOE_ERR_EXPERT_ID_RANGE, static_cast<int>(bad_route));
+  block_exclusive_scan(s_counts, s_offsets, experts, chunk_sums);
+  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+    const int offset = s_offsets[e];
+    if (kCluster) base[e] += offset;
+    if (rank == 0) {
+      counts[e] = s_counts[e];
+      offsets[e] = offset;
+    }
+  }
+  if (rank == 0 && threadIdx.x == 0) offsets[experts] = s_offsets[experts];
+  if (kCluster) __syncthreads();
+
+  // One warp per work-item list, in different CTAs where there are several (the last warps: they have the shortest runs).
+  const int list = (static_cast<int>(blockDim.x >> 5) - 1 - warp) * ctas + rank;
+  if (list < 4) build_item_list(list, experts, s_counts, s_offsets, lists, status, lane);
+
+  const unsigned lanes_below = (1u << lane) - 1u;
+  const int bits = 32 - __clz(experts);  // of the ids 0 .. experts, where `experts` stands for a dropped route
+  for (int64_t r0 = begin; r0 < end; r0 += 32 * kBatch) {
+    int ids[kBatch];
 #pragma unroll
-      for (int i = 0; i < kBatch; ++i) {
-        const int u = base + i;
-        if (u < units) unit_hist[static_cast<int64_t>(u) * experts + e] = running;
-        running += values[i];
+    for (int i = 0; i < kBatch; ++i) {
+      ids[i] = experts;
+      if (r0 + 32 * i + lane < end) {
+        const int64_t value = topk_ids[r0 + 32 * i + lane];
+        if (value >= 0 && value < experts) ids[i] = static_cast<int>(value);
       }
     }
-    counts[e] = running;
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      if (r0 + 32 * i >= end) break;  // warp-uniform
+      const int64_t route = r0 + 32 * i + lane;
+      const int id = ids[i];
+      const bool valid = id < experts;
+      const unsigned peers = lanes_with_same(id, bits);
+      int position = -1;
+      if (valid) position = base[id] + row[id] + __popc(peers & lanes_below);
+      __syncwarp();
+      if (valid && (peers & lanes_below) == 0) row[id] += __popc(peers);
+      __syncwarp();
+      if (valid) {
+        sorted_routes[position] = static_cast<int>(route);
+        if (!kCluster) row_expert[position] = id;
+      }
+      // Inverse permutation: sorted position of every flat route (-1 for a dropped route).
+      if (route_pos != nullptr && route < end) route_pos[route] = position;
+    }
   }
-  __syncthreads();
-  if (warp == 0) {
-    const int total = warp_exclusive_scan(counts, offsets, experts, lane);
-    if (lane == 0) offsets[experts] = total;
+  if (kCluster) {
+    // The expert of every sorted row, a run of consecutive positions per warp: a scattered store takes 32 clocks of the
+    // SM, so with a longer list the rows are not written where their routes are found.  Each lane looks the expert of
+    // its first position up and walks the offsets from there.
+    const int64_t rows_end = min(end, static_cast<int64_t>(s_offsets[experts]));
+    int low = 0;
+    for (int high = experts; low < high;) {
+      const int middle = (low + high) >> 1;
+      if (s_offsets[middle + 1] > begin + lane) {
+        high = middle;
+      } else {
+        low = middle + 1;
+      }
+    }
+    for (int64_t p = begin + lane; p < rows_end; p += 32) {
+      while (s_offsets[low + 1] <= p) ++low;
+      row_expert[p] = low;
+    }
   }
-  __syncthreads();
-  build_items(experts, counts, offsets, lists, scan_tmp, status);
+  if (kCluster) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // no CTA leaves while another may still read its totals
 }
 
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-route_scatter_kernel(const int64_t* __restrict__ topk_ids, int64_t routes, int experts, int units,
-                     const int* __restrict__ unit_hist, const int* __restrict__ offsets, int* sorted_routes,
-                     int* row_expert, int* route_pos) {
-  extern __shared__ int smem_cursor[];
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int unit = blockIdx.x * kWarpsPerBlock + warp;
-  if (unit >= units) return;
-  int* cursor = smem_cursor + warp * experts;
-  for (int e = lane; e < experts; e += 32) cursor[e] = offsets[e] + unit_hist[static_cast<int64_t>(unit) * experts + e];
-  __syncwarp();
-  const int64_t begin = static_cast<int64_t>(unit) * kUnitRoutes;
-  const unsigned lanes_below = (1u << lane) - 1u;
-  for (int round = 0; round < kUnitRoutes / 32; ++round) {
-    const int64_t route = begin + round * 32 + lane;
-    int id = -1;
-    if (route < routes) {
-      const int64_t value = topk_ids[route];
-      if (value >= 0 && value < experts) id = static_cast<int>(value);
-    }
-    const unsigned peers = __match_any_sync(0xffffffffu, id);
-    int position = -1;
-    if (id >= 0) position = cursor[id] + __popc(peers & lanes_below);
-    __syncwarp();
-    if (id >= 0 && (peers & lanes_below) == 0) cursor[id] += __popc(peers);
-    __syncwarp();
-    if (id >= 0) {
-      sorted_routes[position] = static_cast<int>(route);
-      row_expert[position] = id;
-    }
-    // Inverse permutation: sorted position of every flat route (-1 for a dropped route).
-    if (route_pos != nullptr && route < routes) route_pos[route] = position;
-  }
+// Work items from given per-expert counts and offsets (rows that already lie in expert order: nothing to sort).
+__global__ void __launch_bounds__(128)
+items_from_counts_kernel(int experts, const int* __restrict__ counts, const int* __restrict__ offsets, ItemLists lists, int* status) {
+  build_item_list(threadIdx.x >> 5, experts, counts, offsets, lists, status, threadIdx.x & 31);
 }
 
 }  // namespace
 
-size_t route_scratch_bytes(int64_t routes, int experts) {
-  const int64_t units = (routes + kUnitRoutes - 1) / kUnitRoutes;
-  return static_cast<size_t>((units > 0 ? units : 1) * experts + 2 * (experts + 1)) * sizeof(int);
-}
-
+// The status block is cleared by the build.
 cudaError_t launch_route_build(const int64_t* topk_ids, int64_t routes, int experts, const ItemLists& lists, int* status, int* counts,
-                               int* offsets, int* sorted_routes, int* row_expert, int* scratch, cudaStream_t stream, int* route_pos) {
-  if (routes <= kSmallRoutes) {
-    const size_t small_bytes = (static_cast<size_t>(kSmallRoutes) + 4 * static_cast<size_t>(experts) + 4) * sizeof(int);
-    route_small_kernel<<<1, kSmallRoutes, small_bytes, stream>>>(topk_ids, static_cast<int>(routes), experts, lists, status, counts, offsets,
-                                                                 sorted_routes, row_expert, route_pos);
+                               int* offsets, int* sorted_routes, int* row_expert, cudaStream_t stream, int* route_pos) {
+  static_assert(kMaxExperts * 16 <= kHistogramInts, "the histogram rows of kMaxExperts experts need at least 16 warps");
+  int64_t ctas = 1;
+  while (ctas < kMaxRouteCluster && ctas * kRoutesPerCta < routes) ctas *= 2;
+  int warps = kHistogramInts / experts < kRouteWarps ? kHistogramInts / experts : kRouteWarps;
+  const int64_t rounds = (routes + 32 * ctas * warps - 1) / (32 * ctas * warps);
+  const int64_t run = 32 * (rounds > 0 ? rounds : 1);
+  int threads = kRouteThreads;
+  if (ctas == 1) {
+    // A short list: fewer rows to clear and to scan, and no more warps than there is work for.
+    const int64_t used = (routes + run - 1) / run;
+    warps = static_cast<int>(used > 0 ? used : 1);
+    const int wanted = warps * 32 > experts ? warps * 32 : experts;
+    threads = wanted <= 128 ? 128 : wanted <= 256 ? 256 : wanted <= 512 ? 512 : kRouteThreads;
+  }
+  const size_t smem = (static_cast<size_t>(warps) * experts + 2 * static_cast<size_t>(experts) + 1 + (experts + 31) / 32 +
+                       (ctas > 1 ? 2 * static_cast<size_t>(experts) : 0)) * sizeof(int);
+  static PerDeviceOnce configured;
+  const int device = current_device_ordinal();
+  if (configured.needed(device)) {
+    constexpr int kMostBytes = static_cast<int>((kHistogramInts + 4 * kMaxExperts + 1 + kMaxExperts / 32) * sizeof(int));
+    cudaError_t error = cudaFuncSetAttribute(route_build_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostBytes);
+    if (error == cudaSuccess) error = cudaFuncSetAttribute(route_build_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostBytes);
+    if (error != cudaSuccess) return error;
+    configured.mark(device);
+  }
+  if (ctas == 1) {
+    route_build_kernel<false><<<1, threads, smem, stream>>>(topk_ids, routes, experts, warps, run, lists, status, counts, offsets, sorted_routes,
+                                                            row_expert, route_pos);
     return cudaGetLastError();
   }
-  const int units = static_cast<int>((routes + kUnitRoutes - 1) / kUnitRoutes);
-  int* unit_hist = scratch;
-  int* scan_tmp = scratch + static_cast<int64_t>(units > 0 ? units : 1) * experts;
-  const size_t smem = static_cast<size_t>(kWarpsPerBlock) * experts * sizeof(int);
-  const int blocks = (units + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  if (blocks > 0) {
-    route_hist_kernel<<<blocks, kWarpsPerBlock * 32, smem, stream>>>(topk_ids, routes, experts, units, unit_hist, status);
-  }
-  route_scan_kernel<<<1, 1024, 0, stream>>>(experts, units, unit_hist, counts, offsets, lists, scan_tmp, status);
-  if (blocks > 0) {
-    route_scatter_kernel<<<blocks, kWarpsPerBlock * 32, smem, stream>>>(topk_ids, routes, experts, units, unit_hist,
-                                                                        offsets, sorted_routes, row_expert, route_pos);
-  }
-  return cudaGetLastError();
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(static_cast<unsigned>(ctas));
+  config.blockDim = dim3(kRouteThreads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = static_cast<unsigned>(ctas);
+  attribute.val.clusterDim.y = 1;
+  attribute.val.clusterDim.z = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, route_build_kernel<true>, topk_ids, routes, experts, warps, run, lists, status, counts, offsets,
+                            sorted_routes, row_expert, route_pos);
 }
 
-namespace {
-// Work items and the status words of the grouped GEMMs from given per-expert counts and offsets (rows that
-// already lie in expert order: nothing to sort).
-__global__ void __launch_bounds__(1024)
-items_from_counts_kernel(int experts, const int* __restrict__ counts, const int* __restrict__ offsets, ItemLists lists, int* scan_tmp,
-                         int* status) {
-  build_items(experts, counts, offsets, lists, scan_tmp, status);
-}
-
-}  // namespace
-
-cudaError_t launch_items_from_counts(int experts, const int* counts, const int* offsets, const ItemLists& lists, int* scratch, int* status,
+cudaError_t launch_items_from_counts(int experts, const int* counts, const int* offsets, const ItemLists& lists, int* status,
                                      cudaStream_t stream) {
-  items_from_counts_kernel<<<1, 1024, 0, stream>>>(experts, counts, offsets, lists, scratch, status);
+  items_from_counts_kernel<<<1, 128, 0, stream>>>(experts, counts, offsets, lists, status);
   return cudaGetLastError();
 }
 
@@ -305,25 +365,23 @@ cudaError_t launch_items_from_counts(int experts, const int* counts, const int* 
 // Some hosts of this library must not allocate device memory once they are serving: an inference
 // server that handed the whole HBM budget to its KV-cache pool at start-up has nothing left for a
 // cudaMalloc to take, and a runtime whose memory plan is frozen after warm-up treats any later
-// allocation as a bug.  For them the route build is also offered with its scratch (the per-unit
-// histograms, the scan temporaries and the status block) in a fixed array that lives in the
-// library's device image, so the call needs no workspace and performs no allocation of any kind.
-// The price is a fixed ceiling on the problem size and one array shared by every call.
+// allocation as a bug.  For them the route build is also offered with its status block in a fixed array that
+// lives in the library's device image (everything else the build needs is shared memory), so the call needs no
+// workspace and performs no allocation of any kind.  The price is a fixed ceiling on the problem size and one
+// status block shared by every call.
 
 namespace {
 
 constexpr int64_t kStaticMaxRoutes = 131072;  // tokens * top_k
 constexpr int kStaticMaxExperts = 512;
-constexpr size_t kStaticScratchInts = fmoe::kStatusWords + static_cast<size_t>(kStaticMaxRoutes / fmoe::kUnitRoutes) * kStaticMaxExperts +
-                                      2 * (kStaticMaxExperts + 1);
 constexpr int kStaticMaxDevices = 64;
 
-// 528 KB per GPU, held from the moment the library is loaded on that GPU until the process exits.
-static __device__ __align__(256) int g_static_route_scratch[kStaticScratchInts];
+// Held from the moment the library is loaded on a GPU until the process exits.
+static __device__ __align__(256) int g_static_route_status[kStatusWords];
 
 // In host code the array's name only stands for the symbol; the address a kernel can use has to be
 // asked for, per device, with that device current.
-int* static_scratch_for_current_device(cudaError_t* error) {
+int* static_status_for_current_device(cudaError_t* error) {
   static std::mutex guard;
   static int* address[kStaticMaxDevices] = {};
   int device = 0;
@@ -336,7 +394,7 @@ int* static_scratch_for_current_device(cudaError_t* error) {
   std::lock_guard<std::mutex> lock(guard);
   if (address[device] == nullptr) {
     int* pointer = nullptr;
-    *error = cudaGetSymbolAddress(reinterpret_cast<void**>(&pointer), g_static_route_scratch);
+    *error = cudaGetSymbolAddress(reinterpret_cast<void**>(&pointer), g_static_route_status);
     if (*error != cudaSuccess) return nullptr;
     address[device] = pointer;
   }
@@ -369,19 +427,13 @@ extern "C" int fmoe_route_build_noalloc(const int64_t* topk_ids, int64_t tokens,
     return fmoe::report_error(FMOE_ERR_UNSUPPORTED_DEVICE, "fmoe_route_build_noalloc: the current device is not a compute capability 10.x GPU");
   }
   cudaError_t error = cudaSuccess;
-  int* scratch = fmoe::static_scratch_for_current_device(&error);
-  if (scratch == nullptr) {
+  int* status = fmoe::static_status_for_current_device(&error);
+  if (status == nullptr) {
     snprintf(text, sizeof(text), "fmoe_route_build_noalloc: cudaGetSymbolAddress failed: %s", cudaGetErrorString(error));
     return fmoe::report_error(FMOE_ERR_CUDA, text);
   }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  int* status = scratch;                       // kStatusWords ints: must start at zero, the kernels only ever raise it
-  int* work = scratch + fmoe::kStatusWords;    // histograms + scan temporaries: fully rewritten by every call
-  error = cudaMemsetAsync(status, 0, sizeof(int) * fmoe::kStatusWords, stream);
-  if (error == cudaSuccess) {
-    error = fmoe::launch_route_build(topk_ids, routes, experts, fmoe::no_item_lists(), status, counts, offsets, sorted_routes, row_expert, work,
-                                     stream);
-  }
+  error = fmoe::launch_route_build(topk_ids, routes, experts, fmoe::no_item_lists(), status, counts, offsets, sorted_routes, row_expert, stream);
   if (error == cudaSuccess) error = cudaMemcpyAsync(status_out, status, 2 * sizeof(int), cudaMemcpyDeviceToDevice, stream);
   if (error != cudaSuccess) {
     snprintf(text, sizeof(text), "fmoe_route_build_noalloc: %s", cudaGetErrorString(error));

@@ -117,7 +117,7 @@ typedef struct fmoe_workspace_layout {
   size_t sorted_routes;  /* int32[T*K] flat route ids t*K+slot grouped by expert, ascending inside an expert */
   size_t row_expert;     /* int32[T*K] expert of each sorted row */
   size_t items;          /* int32[4*max_items] (expert, first row, rows, reserved) per work item; two lists */
-  size_t scratch;        /* route-build scratch */
+  size_t scratch;        /* empty (the route build needs no memory of its own) */
   size_t a_rows;         /* W8A8: int8[T*K,H] quantised token rows; BF16: bf16[T*K,H] gathered rows */
   size_t a_scale;        /* W8A8: fp32[T*K] activation scales */
   size_t y;              /* bf16[T*K,I] SiLU(gate)*up */
@@ -194,12 +194,12 @@ FMOE_API int fmoe_quantize_rows(const void* x, int64_t rows, int32_t cols, int32
 /* Route build without any allocation or caller workspace.  It has no counterpart in the reference, whose
  * route lists are std::vectors grown on the calling thread.  It exists for hosts that must not allocate
  * device memory while serving -- a server that gave all of HBM to its KV-cache pool, a runtime with a frozen
- * memory plan -- and so cannot provide the forward calls' workspace: the histograms and scan temporaries
- * live in a 528 KB array inside the library's device image (one per GPU that loads the library, held until
- * the process exits).  Limits: tokens * top_k <= 131072 and experts <= 512; larger requests are refused
- * with FMOE_ERR_INVALID_ARGUMENT.  The first call on each device looks the array's device address up
+ * memory plan -- and so cannot provide the forward calls' workspace: the histograms live in shared memory
+ * and the status block in the library's device image (one per GPU that loads the library, held until the
+ * process exits).  Limits: tokens * top_k <= 131072 and experts <= 512; larger requests are refused
+ * with FMOE_ERR_INVALID_ARGUMENT.  The first call on each device looks the block's device address up
  * (cudaGetSymbolAddress); make that first call during start-up, before any stream capture.  Every call
- * uses the same array, so two calls that overlap on the GPU (different streams, or threads) race: issue
+ * uses the same block, so two calls that overlap on the GPU (different streams, or threads) race: issue
  * them on one stream.  Inputs and outputs are the caller's: counts[E], offsets[E+1], sorted_routes[T*K],
  * row_expert[T*K] as in fmoe_workspace_layout, status_out[2] = (error code, detail) as fmoe_read_status
  * would report them.  No cudaMalloc, cudaFree or other allocating call is made. */
