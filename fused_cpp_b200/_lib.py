@@ -28,6 +28,8 @@ GEMM_UMMA = 2
 ACTIVATION_SILU = 0
 ACTIVATION_GELU = 2
 ACTIVATION_SWIGLUOAI = 3
+W13_INTERLEAVED = 0x100  # or-ed into the activation: gate and up rows of w13 alternate
+BIAS_BF16 = 0x200        # or-ed into the activation: w13_bias / w2_bias are bf16
 
 LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libfused_moe_b200.so")
 DIAG_LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libfused_moe_b200_diag.so")
@@ -332,13 +334,18 @@ def moe_forward(x, w13, w2, topk_weights, topk_ids, *, s13=None, s2=None, numeri
     config.activation = int(activation)
     config.route_rows_bf16 = 1 if route_rows_bf16 else 0
     config.w8a16_form = w8a16_form_from_env() if w8a16_form is None else int(w8a16_form)
+    bias_dtype = torch.float32
+    if w13_bias is not None or w2_bias is not None:
+        if all(bias is None or bias.dtype == torch.bfloat16 for bias in (w13_bias, w2_bias)):
+            bias_dtype = torch.bfloat16
+            config.activation |= BIAS_BF16
     if w13_bias is not None:
-        w13_bias = _require_cuda("w13_bias", w13_bias, torch.float32)
+        w13_bias = _require_cuda("w13_bias", w13_bias, bias_dtype)
         if tuple(w13_bias.shape) != (experts, two_i):
             raise ValueError("w13_bias must be [E, 2I]")
         config.w13_bias = w13_bias.data_ptr()
     if w2_bias is not None:
-        w2_bias = _require_cuda("w2_bias", w2_bias, torch.float32)
+        w2_bias = _require_cuda("w2_bias", w2_bias, bias_dtype)
         if tuple(w2_bias.shape) != (experts, hidden):
             raise ValueError("w2_bias must be [E, H]")
         config.w2_bias = w2_bias.data_ptr()

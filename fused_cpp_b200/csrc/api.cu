@@ -191,7 +191,10 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   fmoe_config defaults;
   memset(&defaults, 0, sizeof(defaults));
   defaults.swiglu_limit = f.int8 ? 10.0f : 0.0f;
-  const fmoe_config cfg = config ? *config : defaults;
+  fmoe_config cfg = config ? *config : defaults;
+  const bool interleaved = (cfg.activation & FMOE_W13_INTERLEAVED) != 0;
+  const bool bias_bf16 = (cfg.activation & FMOE_BIAS_BF16) != 0;
+  cfg.activation &= ~(FMOE_W13_INTERLEAVED | FMOE_BIAS_BF16);
   if (f.int8 && cfg.swiglu_limit != 10.0f) {
     return fail(FMOE_ERR_INVALID_ARGUMENT, "W8A8 supports only clamped SwiGLU limit 10.0");
   }
@@ -228,6 +231,7 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   }
   const bool umma = true;
 #endif
+  if (interleaved && !umma) return fail(FMOE_ERR_INVALID_ARGUMENT, "interleaved w13 rows run on the tensor-core GEMMs only");
   const int64_t routes = f.tokens * f.top_k;
   // Above 64 tokens an expert can hold anything from one row to all of them, and the host does not know the routing.
   // Unless the caller fixed the tiles, the experts are then split on the device: those with at most 64 rows
@@ -355,6 +359,8 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   gu.swiglu_limit = cfg.swiglu_limit;
   gu.activation = cfg.activation;
   gu.expert_bias = cfg.w13_bias;
+  gu.bias_bf16 = bias_bf16 ? 1 : 0;
+  gu.interleaved = interleaved ? 1 : 0;
   gu.y = y;
   gu.route_out = nullptr;
   gu.dump_acc = cfg.dump_acc1;

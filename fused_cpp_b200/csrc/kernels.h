@@ -153,8 +153,13 @@ struct GroupedGemmArgs {
   // BF16 path only: per-expert bias added to the fp32 accumulators before the activation (gate_up: [E, 2I], gate
   // channels then up channels) or before the store (down: [E, H]); null = none.  `activation` selects the gated
   // activation of the gate_up epilogue: FMOE_ACT_SILU (with swiglu_limit), FMOE_ACT_GELU, FMOE_ACT_SWIGLUOAI.
-  const float* expert_bias;
+  const void* expert_bias;   // fp32, or bf16 with bias_bf16
+  int bias_bf16;
   int activation;
+  // gate_up: the gate and up rows of w13 (and their scales and biases) alternate, channel n = rows 2n and 2n + 1, as a
+  // swigluoai checkpoint stores them, instead of gate rows [0, I) then up rows [I, 2I).  Only the tensor map's strides
+  // and the index of a channel's scale and bias differ.
+  int interleaved;
   int w8a16;                 // int8 weights with w_scale and 16-bit activations: 1 = bf16 rows, the one-SM kernel widens the weight
                              // tile to bf16; 2 = two int8 planes per route (a_rows holds 2 * total_rows rows, a_scale one
                              // scale per route, row_tile counts plane rows), the int8 one-SM kernel pairs accumulator columns
@@ -171,6 +176,16 @@ struct GroupedGemmArgs {
   // ignores the field): bit 0 = epilogue does no work, bit 1 = producer loads nothing, bit 2 = no MMA is issued.
   int diag;
 };
+
+// Index of channel n's gate / up row in the [2I] rows of w13, its scales and its bias.
+#ifdef __CUDACC__
+__device__ __forceinline__ int gate_channel(const GroupedGemmArgs& args, int n) { return args.interleaved ? 2 * n : n; }
+__device__ __forceinline__ int up_channel(const GroupedGemmArgs& args, int n) { return args.interleaved ? 2 * n + 1 : n + args.n_out; }
+__device__ __forceinline__ float load_expert_bias(const GroupedGemmArgs& args, int64_t index) {
+  if (!args.bias_bf16) return static_cast<const float*>(args.expert_bias)[index];
+  return __uint_as_float(static_cast<uint32_t>(static_cast<const uint16_t*>(args.expert_bias)[index]) << 16);
+}
+#endif
 
 // The stage switches above exist only in the diagnostic build; in the product build the tests fold to `false`.
 #ifdef FMOE_DIAG

@@ -452,15 +452,15 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
       if (n < n_out) {
         if (kInt8) {
           const float* s = args.w_scale + static_cast<int64_t>(info.expert) * n_total;
-          t.scale_gate = s[n];
-          if (kGateUp) t.scale_up = s[n + n_out];
+          t.scale_gate = s[kGateUp ? gate_channel(args, n) : n];
+          if (kGateUp) t.scale_up = s[up_channel(args, n)];
         }
         if (kDense && args.bias != nullptr) t.bias = args.bias[n];
         if (!kInt8 && !kDense && args.expert_bias != nullptr) {
           // BF16 path: the per-expert bias rides in the scale slots (unused without int8) and is ADDED.
-          const float* b = args.expert_bias + static_cast<int64_t>(info.expert) * n_total;
-          t.scale_gate = b[n];
-          if (kGateUp) t.scale_up = b[n + n_out];
+          const int64_t first = static_cast<int64_t>(info.expert) * n_total;
+          t.scale_gate = load_expert_bias(args, first + (kGateUp ? gate_channel(args, n) : n));
+          if (kGateUp) t.scale_up = load_expert_bias(args, first + up_channel(args, n));
         }
       }
       return t;
@@ -709,25 +709,31 @@ bool make_tensor_map(CUtensorMap* map, const void* base, bool int8, uint64_t row
 // operation per stage; the gate|up stride is larger than the group stride that follows it).  Otherwise
 // {K, 16 rows, I/16 groups, gate|up, E} with strides in ascending order and a box of one group (4 KB, four
 // operations per stage): the fallback if the driver refuses the first encoding.
-bool make_gate_up_map(CUtensorMap* map, const void* base, bool int8, uint64_t experts, uint64_t inter, uint64_t k, bool one_box) {
+// The layout of w13 (gate rows then up rows, or alternating: args.interleaved) is in the strides of the first row
+// dimension and of gate|up.
+bool make_gate_up_map(CUtensorMap* map, const GroupedGemmArgs& args, bool int8, bool one_box) {
   EncodeTiledFn encode = encode_tiled_fn();
   if (encode == nullptr) return false;
   const uint64_t elem_bytes = int8 ? 1 : 2;
+  const uint64_t k = static_cast<uint64_t>(args.k), inter = static_cast<uint64_t>(args.n_out), experts = static_cast<uint64_t>(args.experts);
   const uint64_t row_bytes = k * elem_bytes;
+  const uint64_t channel_bytes = args.interleaved ? 2 * row_bytes : row_bytes;  // from a channel's row to the next channel's
+  const uint64_t up_bytes = args.interleaved ? row_bytes : inter * row_bytes;   // from a channel's gate row to its up row
+  void* const base = const_cast<void*>(args.weights);
   const cuuint32_t inner = static_cast<cuuint32_t>(kBlockKBytes / elem_bytes);
   const cuuint32_t elem_strides[5] = {1, 1, 1, 1, 1};
   const CUtensorMapDataType type = int8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   if (one_box) {
     const cuuint64_t dims[5] = {k, 16, 2, inter / 16, experts};
-    const cuuint64_t strides[4] = {row_bytes, inter * row_bytes, 16 * row_bytes, 2 * inter * row_bytes};
+    const cuuint64_t strides[4] = {channel_bytes, up_bytes, 16 * channel_bytes, 2 * inter * row_bytes};
     const cuuint32_t box[5] = {inner, 16, 2, 4, 1};
-    return encode(map, type, 5, const_cast<void*>(base), dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    return encode(map, type, 5, base, dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   }
   const cuuint64_t dims[5] = {k, 16, inter / 16, 2, experts};
-  const cuuint64_t strides[4] = {row_bytes, 16 * row_bytes, inter * row_bytes, 2 * inter * row_bytes};
+  const cuuint64_t strides[4] = {channel_bytes, 16 * channel_bytes, up_bytes, 2 * inter * row_bytes};
   const cuuint32_t box[5] = {inner, 16, 1, 2, 1};
-  return encode(map, type, 5, const_cast<void*>(base), dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  return encode(map, type, 5, base, dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -741,7 +747,6 @@ cudaError_t launch_pair(const GroupedGemmArgs& args, cudaStream_t stream) {
     if (err != cudaSuccess) return err;
     configured.mark(device);
   }
-  const int n_total = kGateUp ? 2 * args.n_out : args.n_out;
   CUtensorMap weight_map, token_map;
   GroupedGemmArgs launch_args = args;
   bool weights_ok;
@@ -751,10 +756,10 @@ cudaError_t launch_pair(const GroupedGemmArgs& args, cudaStream_t stream) {
     const char* forced = getenv("FUSED_CPP_MOE_GATE_UP_BOXES");  // diagnostic library only: "4" forces the four-box encoding
     if (forced != nullptr && forced[0] == '4') try_one = false;
 #endif
-    launch_args.gate_up_one_box = try_one && make_gate_up_map(&weight_map, args.weights, kInt8, args.experts, args.n_out, args.k, true);
-    weights_ok = launch_args.gate_up_one_box || make_gate_up_map(&weight_map, args.weights, kInt8, args.experts, args.n_out, args.k, false);
+    launch_args.gate_up_one_box = try_one && make_gate_up_map(&weight_map, args, kInt8, true);
+    weights_ok = launch_args.gate_up_one_box || make_gate_up_map(&weight_map, args, kInt8, false);
   } else {
-    weights_ok = make_tensor_map(&weight_map, args.weights, kInt8, static_cast<uint64_t>(args.experts) * n_total, args.k, kRowsPerCta);
+    weights_ok = make_tensor_map(&weight_map, args.weights, kInt8, static_cast<uint64_t>(args.experts) * args.n_out, args.k, kRowsPerCta);
   }
   const uint64_t token_rows = static_cast<uint64_t>(args.total_rows) * (kPlanes ? 2 : 1);
   if (!weights_ok || !make_tensor_map(&token_map, args.a_rows, kInt8, token_rows, args.k, kRowsPerCta)) {

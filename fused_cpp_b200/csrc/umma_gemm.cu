@@ -232,7 +232,8 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
           decode_unit(args.items, unit, n_blocks, &item, &block);
           item = __shfl_sync(0xffffffffu, item, 0);  // read from the item list: the same in every lane
           block = __shfl_sync(0xffffffffu, block, 0);
-          const int weight_row = __shfl_sync(0xffffffffu, args.items[4 * item + 0], 0) * n_total + block * kBlockM;
+          const int expert = __shfl_sync(0xffffffffu, args.items[4 * item + 0], 0);
+          const int n0 = block * kBlockM;
           const int row0 = __shfl_sync(0xffffffffu, args.items[4 * item + 1], 0);
           for (int kb = 0; kb < k_blocks; ++kb) {
             ptx::mbar_wait(&ctl->landing_free[slot], slot_phase ^ 1u, abort_flag, status, 6);
@@ -241,10 +242,12 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
               const int x = kb * kBlockKElems;
               ptx::mbar_arrive_expect_tx(&ctl->landed[slot], Cfg::kTokenBytes + Cfg::kInt8TileBytes);
               ptx::tma_load_2d(landing, &token_map, &ctl->landed[slot], x, row0);
-              ptx::tma_load_2d(landing + Cfg::kTokenRegionBytes, &weight_map, &ctl->landed[slot], x, weight_row);
               if (kGateUp) {
-                ptx::tma_load_2d(landing + Cfg::kTokenRegionBytes + kBlockM * kLandingRowBytes, &weight_map, &ctl->landed[slot], x,
-                                 weight_row + args.n_out);
+                ptx::tma_load_4d(landing + Cfg::kTokenRegionBytes, &weight_map, &ctl->landed[slot], x, n0, 0, expert);
+                ptx::tma_load_4d(landing + Cfg::kTokenRegionBytes + kBlockM * kLandingRowBytes, &weight_map, &ctl->landed[slot], x, n0, 1,
+                                 expert);
+              } else {
+                ptx::tma_load_2d(landing + Cfg::kTokenRegionBytes, &weight_map, &ctl->landed[slot], x, expert * n_total + n0);
               }
             }
             ++landed_issued;
@@ -291,8 +294,12 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
           } else {
             ptx::mbar_arrive_expect_tx(&ctl->full[stage], Cfg::kStageBytes);
             const int x = kb * kBlockKElems;
-            ptx::tma_load_2d(stage_base, &weight_map, &ctl->full[stage], x, weight_row);
-            if (kGateUp) ptx::tma_load_2d(stage_base + kBlockM * kBlockKBytes, &weight_map, &ctl->full[stage], x, weight_row + args.n_out);
+            if (kGateUp) {
+              ptx::tma_load_4d(stage_base, &weight_map, &ctl->full[stage], x, n0, 0, expert);
+              ptx::tma_load_4d(stage_base + kBlockM * kBlockKBytes, &weight_map, &ctl->full[stage], x, n0, 1, expert);
+            } else {
+              ptx::tma_load_2d(stage_base, &weight_map, &ctl->full[stage], x, weight_row);
+            }
             ptx::tma_load_2d(stage_base + Cfg::kWeightBytes, &token_map, &ctl->full[stage], x, row0);
           }
           ++issued;
@@ -474,8 +481,9 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
         const int n0 = block * kBlockM;
         {
           const float* s = args.w_scale + static_cast<int64_t>(expert) * n_total;
-          meta->scale[epilogue_thread] = n0 + epilogue_thread < n_out ? s[n0 + epilogue_thread] : 0.0f;
-          if (kGateUp) meta->scale[kBlockM + epilogue_thread] = n0 + epilogue_thread < n_out ? s[n_out + n0 + epilogue_thread] : 0.0f;
+          const int c = n0 + epilogue_thread;
+          meta->scale[epilogue_thread] = c < n_out ? s[kGateUp ? gate_channel(args, c) : c] : 0.0f;
+          if (kGateUp) meta->scale[kBlockM + epilogue_thread] = c < n_out ? s[up_channel(args, c)] : 0.0f;
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
         ptx::mbar_wait(&ctl->acc_full[buffer], use & 1u, abort_flag, status, 4);
@@ -556,16 +564,16 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
       float scale_gate = 1.0f, scale_up = 1.0f;
       if ((kInt8 || kW8A16) && channel_ok) {
         const float* s = args.w_scale + static_cast<int64_t>(expert) * n_total;
-        scale_gate = s[n];
-        if (kGateUp) scale_up = s[n + n_out];
+        scale_gate = s[kGateUp ? gate_channel(args, n) : n];
+        if (kGateUp) scale_up = s[up_channel(args, n)];
       }
       float bias = 0.0f;
       if (kDense && channel_ok && args.bias != nullptr) bias = args.bias[n];
       float bias_gate = 0.0f, bias_up = 0.0f;  // per-expert bias of the BF16 path (gate_up: gate / up; down: bias_gate)
       if (!kInt8 && !kDense && channel_ok && args.expert_bias != nullptr) {
-        const float* b = args.expert_bias + static_cast<int64_t>(expert) * n_total;
-        bias_gate = b[n];
-        if (kGateUp) bias_up = b[n + n_out];
+        const int64_t first = static_cast<int64_t>(expert) * n_total;
+        bias_gate = load_expert_bias(args, first + (kGateUp ? gate_channel(args, n) : n));
+        if (kGateUp) bias_up = load_expert_bias(args, first + up_channel(args, n));
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");  // metadata visible to the four epilogue warps
       ptx::mbar_wait(&ctl->acc_full[buffer], use & 1u, abort_flag, status, 4);
@@ -762,6 +770,28 @@ bool make_landing_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// gate_up weights [E, 2I, K] as dimensions {K, channel, gate|up, expert}, boxes of 128 channels of either kind; the
+// layout of w13 (gate rows then up rows, or alternating) is in the strides, so an interleaved checkpoint costs nothing
+// (re-ordering it in front of the kernels cost a pass over w13: 200 tokens of a 16-expert 2048 x 1024 layer 459 us
+// against 159 us; decode of the plain layout is the same with four coordinates as with two: 917 us at 64 tokens).
+// landing: W8A16's unswizzled 64-byte rows.
+bool make_gate_up_map(CUtensorMap* map, const GroupedGemmArgs& args, bool int8, bool landing) {
+  EncodeTiledFn encode = encode_tiled_fn();
+  if (encode == nullptr) return false;
+  const uint64_t elem_bytes = int8 ? 1 : 2;
+  const uint64_t row_bytes = static_cast<uint64_t>(args.k) * elem_bytes;
+  const uint64_t inter = static_cast<uint64_t>(args.n_out);
+  const cuuint64_t dims[4] = {static_cast<cuuint64_t>(args.k), inter, 2, static_cast<cuuint64_t>(args.experts)};
+  const cuuint64_t strides[3] = {args.interleaved ? 2 * row_bytes : row_bytes, args.interleaved ? row_bytes : inter * row_bytes,
+                                 2 * inter * row_bytes};
+  const cuuint32_t box[4] = {static_cast<cuuint32_t>(landing ? kLandingRowBytes : kBlockKBytes / elem_bytes), kBlockM, 1, 1};
+  const cuuint32_t elem_strides[4] = {1, 1, 1, 1};
+  return encode(map, int8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(args.weights), dims,
+                strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                landing ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <bool kInt8, bool kGateUp, int kRowTile, bool kDense, bool kW8A16 = false, bool kPlanes = false>
 cudaError_t launch_config(const GroupedGemmArgs& args, cudaStream_t stream) {
   using Cfg = TileConfig<kGateUp, kRowTile, kW8A16>;
@@ -773,10 +803,11 @@ cudaError_t launch_config(const GroupedGemmArgs& args, cudaStream_t stream) {
     if (err != cudaSuccess) return err;
     configured.mark(device);
   }
-  const int n_total = kGateUp ? 2 * args.n_out : args.n_out;
   CUtensorMap weight_map, token_map;
-  const bool weights_ok = kW8A16 ? make_landing_map(&weight_map, args.weights, static_cast<uint64_t>(args.experts) * n_total, args.k)
-                                 : make_tensor_map(&weight_map, args.weights, kInt8, static_cast<uint64_t>(args.experts) * n_total, args.k, kBlockM);
+  const uint64_t weight_rows = static_cast<uint64_t>(args.experts) * args.n_out;  // down / dense
+  const bool weights_ok = kGateUp   ? make_gate_up_map(&weight_map, args, kInt8 || kW8A16, kW8A16)
+                          : kW8A16 ? make_landing_map(&weight_map, args.weights, weight_rows, args.k)
+                                   : make_tensor_map(&weight_map, args.weights, kInt8, weight_rows, args.k, kBlockM);
   const uint64_t token_rows = static_cast<uint64_t>(args.total_rows) * (kPlanes ? 2 : 1);
   if (!weights_ok || !make_tensor_map(&token_map, args.a_rows, kInt8, token_rows, args.k, kRowTile)) {
     return cudaErrorInvalidValue;

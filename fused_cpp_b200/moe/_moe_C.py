@@ -220,40 +220,21 @@ def fused_moe_w8a8_tiled_async_plan_v2(
 def _native_activation(activation: str) -> tuple[int, float]:
     """Activation string of the op -> (activation id of the C ABI, swiglu_limit)."""
     table = {"silu": (_lib.ACTIVATION_SILU, 0.0), "silu_clamp10": (_lib.ACTIVATION_SILU, 10.0),
-             "gelu": (_lib.ACTIVATION_GELU, 0.0), "swigluoai": (_lib.ACTIVATION_SWIGLUOAI, 0.0)}
+             "gelu": (_lib.ACTIVATION_GELU, 0.0),
+             # swigluoai checkpoints interleave gate and up channels (row 2j = gate j, row 2j + 1 = up j; naive.py:39-47)
+             "swigluoai": (_lib.ACTIVATION_SWIGLUOAI | _lib.W13_INTERLEAVED, 0.0)}
     if activation not in table:
         raise RuntimeError(f"unsupported MoE activation: {activation}")
     return table[activation]
 
 
-def _check_bias(bias, experts: int, channels: int, name: str):
+def _check_bias(bias, experts: int, channels: int, name: str, dtype: torch.dtype):
     """check_optional_bias of the reference (fused_moe_bf16_tiled.cpp:6420-6421): [E, N] of a floating dtype."""
     if bias is None:
         return None
     if bias.dim() != 2 or tuple(bias.shape) != (experts, channels) or not bias.dtype.is_floating_point:
         raise RuntimeError(f"{name} must be a floating [E, N] = [{experts}, {channels}] tensor")
-    return bias.to(device=_device(), dtype=torch.float32).contiguous()
-
-
-# swigluoai checkpoints interleave gate and up channels (row 2j = gate j, row 2j + 1 = up j; naive.py:39-47); the
-# kernels take gate rows then up rows.  The reordered copy is made once per weight tensor and kept while it lives.
-_DEINTERLEAVED: dict = {}
-
-
-def _gate_then_up(tensor: torch.Tensor, dim: int) -> torch.Tensor:
-    key = (tensor.data_ptr(), tuple(tensor.shape), tensor.dtype, dim)
-    cached = _DEINTERLEAVED.get(key)
-    if cached is not None and cached[0]() is tensor:
-        return cached[1]
-    import weakref
-
-    count = tensor.shape[dim]
-    order = torch.cat((torch.arange(0, count, 2), torch.arange(1, count, 2))).to(tensor.device)
-    result = tensor.index_select(dim, order).contiguous()
-    for stale in [k for k, v in _DEINTERLEAVED.items() if v[0]() is None]:
-        del _DEINTERLEAVED[stale]
-    _DEINTERLEAVED[key] = (weakref.ref(tensor), result)
-    return result
+    return bias.to(device=_device(), dtype=dtype).contiguous()
 
 
 def _bf16_forward(input, w13_packed, w13_k, w13_n, w2_packed, w2_k, w2_n, topk_weights, topk_ids, w13_bias, w2_bias,
@@ -273,14 +254,12 @@ def _bf16_forward(input, w13_packed, w13_k, w13_n, w2_packed, w2_k, w2_n, topk_w
         raise RuntimeError("skip_weighted is only valid when top_k == 1")
     _check_out(input, out, (input, w13_packed, w2_packed, topk_weights, topk_ids))
     activation_id, limit = _native_activation(activation)
-    w13_bias = _check_bias(w13_bias, experts, w13_n, "w13_bias")
-    w2_bias = _check_bias(w2_bias, experts, w2_n, "w2_bias")
+    # bf16 biases go to the kernels as they are (they widen them), anything else as fp32.
+    bias_dtype = torch.bfloat16 if all(b is None or b.dtype == torch.bfloat16 for b in (w13_bias, w2_bias)) else torch.float32
+    w13_bias = _check_bias(w13_bias, experts, w13_n, "w13_bias", bias_dtype)
+    w2_bias = _check_bias(w2_bias, experts, w2_n, "w2_bias", bias_dtype)
     w13 = w13_packed.reshape(experts, w13_n, w13_k)
     w2 = w2_packed.reshape(experts, w2_n, w2_k)
-    if activation_id == _lib.ACTIVATION_SWIGLUOAI:
-        w13 = _gate_then_up(w13, 1)
-        if w13_bias is not None:
-            w13_bias = _gate_then_up(w13_bias, 1)
     # The reference narrows the valid id range to [0, global_num_experts) and raises on ids beyond it
     # (fused_moe_bf16_tiled.cpp:6439-6458): the route build sees only that many experts, so such ids are reported as
     # out of range instead of being routed to the trailing prepared experts.
@@ -587,8 +566,6 @@ def fused_moe_w8a16_tiled_async_plan_v2(
     w13 = w13_packed.reshape(experts, w13_N, w13_K)
     w2 = w2_packed.reshape(experts, w2_N, w2_K)
     s13, s2 = w13_scales, w2_scales
-    if activation_id == _lib.ACTIVATION_SWIGLUOAI:
-        w13, s13 = _gate_then_up(w13, 1), _gate_then_up(s13, 1)
     if global_num_experts != -1 and global_num_experts < experts:
         experts = int(global_num_experts)
         w13, w2, s13, s2 = w13[:experts], w2[:experts], s13[:experts], s2[:experts]

@@ -101,11 +101,15 @@ typedef struct fmoe_config {
 /* Gated activations of the BF16 op (activation_to_bf16, csrc/moe/arm/common/fused_moe_bf16_tiled.cpp:1911-1936):
  * SILU = gate * up / (1 + exp(-gate)) with the optional clamp of swiglu_limit; GELU = gelu_erf(gate) * up;
  * SWIGLUOAI = (clamp(up, +-7) + 1) * g * sigmoid(1.702 g) with g = min(gate, 7).  The kernels take gate channels
- * [0, I) and up channels [I, 2I) of w13 for every activation (callers holding the interleaved SWIGLUOAI layout
- * de-interleave once at preparation). */
+ * [0, I) and up channels [I, 2I) of w13 for every activation unless FMOE_W13_INTERLEAVED is or-ed into `activation`:
+ * then channel n's gate and up rows are rows 2n and 2n + 1 of w13, as SWIGLUOAI checkpoints store them, and its scales
+ * and w13_bias values lie at 2n and 2n + 1 as well.  FMOE_BIAS_BF16, or-ed in too: w13_bias and w2_bias point to bf16
+ * values instead of fp32 ones (widened exactly). */
 #define FMOE_ACTIVATION_SILU 0
 #define FMOE_ACTIVATION_GELU 2
 #define FMOE_ACTIVATION_SWIGLUOAI 3
+#define FMOE_W13_INTERLEAVED 0x100
+#define FMOE_BIAS_BF16 0x200
 
 /* Byte offsets of the regions of a forward workspace (all 256-byte aligned).  Rows of the
  * per-route regions are in SORTED order: position p holds flat route sorted_routes[p]. */
