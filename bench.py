@@ -892,7 +892,7 @@ def run_dense_point(rows: int, k: int, n: int, device: torch.device, steps: int,
     bound = "hbm" if t_hbm >= t_tensor else "tensor"
     return {"workload": f"i8gemm_dense_M{rows}_K{k}_N{n}", "tokens": rows, "dtype": "int8(w8a8)", "ms_per_step": ms,
             "value": rows / (ms * 1e-3), "eager_ms_per_step": eager_ms,
-            "launch_mode": ("cuda_graph_replay" if graph is not None else "eager") + " (row quantiser + GEMM, two launches; three with the K split of at most 16 rows)",
+            "launch_mode": ("cuda_graph_replay" if graph is not None else "eager") + " (row quantiser + GEMM, two launches)",
             "l2": "flushed between steps (a buffer of twice the L2 is written)" if flush is not None else "inputs larger than L2",
             "roofline": {"bound": bound, "achieved": nbytes / (ms * 1e-3) / 1e9 if bound == "hbm" else ops / (ms * 1e-3) / 1e12,
                          "peak": peaks["hbm_gbs"] if bound == "hbm" else tensor_peak, "unit": "GB/s" if bound == "hbm" else "TOP/s",

@@ -717,80 +717,67 @@ DenseLayout dense_layout(int64_t rows, int k) {
   return d;
 }
 
-// Row tile of the dense GEMM: the smallest one-SM tile that holds a decode batch, the two-SM kernel (256-row work
-// items) for anything taller than one 128-row tile.
-int dense_row_tile(int64_t rows) {
-  if (rows <= 16) return 16;
-  if (rows <= 32) return 32;
-  if (rows <= 64) return 64;
-  if (rows <= 128) return 128;
-  return fmoe::kPairRowTile;
-}
+// One or two int8 products over the rows that dense_prologue quantised: up to kDenseMaxRows rows one launch of the
+// split-K kernel, above that one launch of the two-SM kernel (256-row work items) per matrix.
+// FUSED_CPP_MOE_DENSE_SPLIT=0 keeps the K range of a channel block in one CTA.
+struct DenseProduct {
+  const int8_t* w;
+  const float* scale;
+  const float* bias;
+  int n;
+  void* out;
+};
 
-// Split-K for products with very few rows: how many parts the K range of a channel block is cut into so that the work
-// units fill the SMs (every part at least two 128-byte K blocks), and the bytes its table of partial sums and its
-// counters take behind the base layout.  Such a product is latency-bound (a 7168 x 1536 projection streams 11 MB: 2 us
-// of HBM time inside 20 us of launches, prologue and one CTA's 0.9 MB stream); measured in a CUDA graph, per op:
-// 1 row 20.2 -> 14.7 us, 16 rows 19.5 -> 15.7 us, but 64 rows 22.4 -> 24.9 us and 128 rows x 16384 x 7168 48.7 -> 64.3 us
-// (8192 atomic additions per work unit), hence the row limit.  FUSED_CPP_MOE_DENSE_SPLIT=0 switches it off.
-constexpr int kDenseSplitMaxRows = 16;
-
-int dense_split_parts(int64_t rows, int k_padded, int n) {
-  if (rows <= 0 || rows > kDenseSplitMaxRows) return 1;
-  const char* text = getenv("FUSED_CPP_MOE_DENSE_SPLIT");
-  if (text != nullptr && text[0] == '0') return 1;
-  const int n_blocks = (n + 127) / 128;
-  const int k_blocks = (k_padded + 127) / 128;
-  int parts = fmoe::sm_count_of_current_device() / n_blocks;
-  if (parts > k_blocks / 2) parts = k_blocks / 2;
-  if (parts > 16) parts = 16;
-  return parts >= 2 ? parts : 1;
-}
-
-size_t dense_split_bytes(int64_t rows, int n, int max_items) {
-  if (rows <= 0 || rows > kDenseSplitMaxRows || n <= 0) return 0;
-  const size_t n_blocks = static_cast<size_t>((n + 127) / 128);
-  return align_up(static_cast<size_t>(rows) * n * sizeof(int), 256) + align_up(sizeof(int) * n_blocks * static_cast<size_t>(max_items), 256);
-}
-
-// One int8 GEMM with the dense epilogue over already-quantised rows.
-cudaError_t dense_gemm(const DenseLayout& d, char* base, size_t workspace_bytes, int64_t rows, const int8_t* w, const float* w_scale,
-                       const float* bias, int n, void* out, int out_is_bf16, int row_tile, cudaStream_t stream) {
-  fmoe::GroupedGemmArgs args;
-  memset(&args, 0, sizeof(args));
-  const int parts = dense_split_parts(rows, d.k_padded, n);
-  const size_t split_bytes = dense_split_bytes(rows, n, d.max_items);
-  if (parts > 1 && workspace_bytes >= d.total + split_bytes) {
-    // Partial sums and counters start at zero (one memset: the two regions are adjacent).
-    const cudaError_t error = cudaMemsetAsync(base + d.total, 0, split_bytes, stream);
-    if (error != cudaSuccess) return error;
-    args.dense_splits = parts;
-    args.dense_partial = reinterpret_cast<int*>(base + d.total);
-    args.dense_counters = reinterpret_cast<int*>(base + d.total + align_up(static_cast<size_t>(rows) * n * sizeof(int), 256));
+cudaError_t dense_gemm(const DenseLayout& d, char* base, int64_t rows, const DenseProduct* products, int count, int out_is_bf16,
+                       cudaStream_t stream) {
+  if (rows <= fmoe::kDenseMaxRows) {
+    fmoe::DenseGemmArgs args;
+    memset(&args, 0, sizeof(args));
+    const int8_t* weights[2] = {nullptr, nullptr};
+    for (int i = 0; i < count; ++i) {
+      weights[i] = products[i].w;
+      args.w_scale[i] = products[i].scale;
+      args.out[i] = products[i].out;
+      args.n[i] = products[i].n;
+    }
+    args.a_scale = reinterpret_cast<const float*>(base + d.scale);
+    args.bias = products[0].bias;
+    args.out_bf16 = out_is_bf16;
+    args.rows = static_cast<int>(rows);
+    args.k_padded = d.k_padded;
+    args.status = reinterpret_cast<int*>(base + d.status);
+    const char* text = getenv("FUSED_CPP_MOE_DENSE_SPLIT");
+    return fmoe::launch_dense_gemm(args, base + d.xq, weights, text == nullptr || text[0] != '0', stream);
   }
-  args.a_rows = base + d.xq;
-  args.weights = w;
-  args.a_scale = reinterpret_cast<const float*>(base + d.scale);
-  args.w_scale = w_scale;
-  args.items = reinterpret_cast<const int*>(base + d.items);
-  args.status = reinterpret_cast<const int*>(base + d.status);
-  args.status_rw = reinterpret_cast<int*>(base + d.status);
-  args.item_count_word = fmoe::kStatusItems;
-  args.max_items = d.max_items;
-  args.experts = 1;
-  args.k = d.k_padded;
-  args.n_out = n;
-  args.numerics = FMOE_NUMERICS_TORCHREF;  // (acc * x_scale) * w_scale, csrc/i8gemm.cpp:157
-  args.total_rows = rows;
-  args.row_tile = row_tile;
-  args.dense_out = out;
-  args.dense_out_bf16 = out_is_bf16;
-  args.bias = bias;
-  return fmoe::launch_umma_grouped_gemm(args, true, false, stream);
+  cudaError_t error = cudaSuccess;
+  for (int i = 0; i < count && error == cudaSuccess; ++i) {
+    fmoe::GroupedGemmArgs args;
+    memset(&args, 0, sizeof(args));
+    args.a_rows = base + d.xq;
+    args.weights = products[i].w;
+    args.a_scale = reinterpret_cast<const float*>(base + d.scale);
+    args.w_scale = products[i].scale;
+    args.items = reinterpret_cast<const int*>(base + d.items);
+    args.status = reinterpret_cast<const int*>(base + d.status);
+    args.status_rw = reinterpret_cast<int*>(base + d.status);
+    args.item_count_word = fmoe::kStatusItems;
+    args.max_items = d.max_items;
+    args.experts = 1;
+    args.k = d.k_padded;
+    args.n_out = products[i].n;
+    args.numerics = FMOE_NUMERICS_TORCHREF;  // (acc * x_scale) * w_scale, csrc/i8gemm.cpp:157
+    args.total_rows = rows;
+    args.row_tile = fmoe::kPairRowTile;
+    args.dense_out = products[i].out;
+    args.dense_out_bf16 = out_is_bf16;
+    args.bias = products[i].bias;
+    error = fmoe::launch_umma_grouped_gemm(args, true, false, stream);
+  }
+  return error;
 }
 
 int dense_prologue(const void* x, int x_is_bf16, int64_t rows, int k, int clamp_low, void* workspace, size_t workspace_bytes,
-                   DenseLayout* layout, int* row_tile, cudaStream_t stream) {
+                   DenseLayout* layout, cudaStream_t stream) {
   int status = check_device();
   if (status != FMOE_OK) return status;
   if (rows < 0 || k <= 0) return fail(FMOE_ERR_INVALID_ARGUMENT, "i8gemm: rows must be >= 0 and K positive");
@@ -801,11 +788,10 @@ int dense_prologue(const void* x, int x_is_bf16, int64_t rows, int k, int clamp_
     return fail(FMOE_ERR_WORKSPACE, "i8gemm: workspace missing, misaligned or too small (%zu bytes needed)", layout->total);
   }
   char* base = static_cast<char*>(workspace);
-  *row_tile = dense_row_tile(rows);
-  // One launch: the quantiser's first block also resets the status block and writes the GEMM's work items.
+  // One launch: the quantiser's first block also resets the status block and writes the two-SM kernel's work items.
   const cudaError_t error = fmoe::launch_quantize_rows_dense(
       x, x_is_bf16, rows, k, layout->k_padded, clamp_low, reinterpret_cast<int8_t*>(base + layout->xq),
-      reinterpret_cast<float*>(base + layout->scale), *row_tile == fmoe::kPairRowTile ? 256 : *row_tile, layout->max_items,
+      reinterpret_cast<float*>(base + layout->scale), 256, layout->max_items,
       reinterpret_cast<int*>(base + layout->items), reinterpret_cast<int*>(base + layout->status), stream);
   return error == cudaSuccess ? FMOE_OK : cuda_fail(error, "i8gemm activation quantisation");
 }
@@ -813,8 +799,8 @@ int dense_prologue(const void* x, int x_is_bf16, int64_t rows, int k, int clamp_
 
 size_t fmoe_i8gemm_workspace_bytes(int64_t rows, int32_t k, int32_t n) {
   if (rows < 0 || k <= 0) return 0;
-  const DenseLayout layout = dense_layout(rows, k);
-  return layout.total + dense_split_bytes(rows, n, layout.max_items);  // n = the widest product that will use the workspace
+  (void)n;
+  return dense_layout(rows, k).total;
 }
 
 int fmoe_i8gemm_dynamic_scaled_mm(const void* x, int32_t x_is_bf16, int64_t rows, int32_t k, const int8_t* w,
@@ -822,12 +808,12 @@ int fmoe_i8gemm_dynamic_scaled_mm(const void* x, int32_t x_is_bf16, int64_t rows
                                   void* workspace, size_t workspace_bytes, void* stream_ptr) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   DenseLayout layout;
-  int row_tile = 16;
   if (n <= 0) return fail(FMOE_ERR_INVALID_ARGUMENT, "i8gemm: N must be positive");
-  const int status = dense_prologue(x, x_is_bf16, rows, k, -128, workspace, workspace_bytes, &layout, &row_tile, stream);
+  const int status = dense_prologue(x, x_is_bf16, rows, k, -128, workspace, workspace_bytes, &layout, stream);
   if (status != FMOE_OK || rows == 0) return status;
   if (w == nullptr || w_scale == nullptr || out == nullptr) return fail(FMOE_ERR_INVALID_ARGUMENT, "i8gemm: null pointer");
-  const cudaError_t error = dense_gemm(layout, static_cast<char*>(workspace), workspace_bytes, rows, w, w_scale, bias, n, out, out_is_bf16, row_tile, stream);
+  const DenseProduct product = {w, w_scale, bias, n, out};
+  const cudaError_t error = dense_gemm(layout, static_cast<char*>(workspace), rows, &product, 1, out_is_bf16, stream);
   return error == cudaSuccess ? FMOE_OK : cuda_fail(error, "i8gemm GEMM");
 }
 
@@ -837,17 +823,15 @@ int fmoe_i8gemm_dynamic_scaled_mm_pair(const void* x_bf16, int64_t rows, int32_t
                                        void* stream_ptr) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   DenseLayout layout;
-  int row_tile = 16;
   if (first_n <= 0 || second_n <= 0) return fail(FMOE_ERR_INVALID_ARGUMENT, "i8gemm pair: N must be positive");
-  const int status = dense_prologue(x_bf16, 1, rows, k, -127, workspace, workspace_bytes, &layout, &row_tile, stream);
+  const int status = dense_prologue(x_bf16, 1, rows, k, -127, workspace, workspace_bytes, &layout, stream);
   if (status != FMOE_OK || rows == 0) return status;
   if (first_w == nullptr || second_w == nullptr || first_scale == nullptr || second_scale == nullptr || first_out == nullptr ||
       second_out == nullptr) {
     return fail(FMOE_ERR_INVALID_ARGUMENT, "i8gemm pair: null pointer");
   }
-  char* base = static_cast<char*>(workspace);
-  cudaError_t error = dense_gemm(layout, base, workspace_bytes, rows, first_w, first_scale, nullptr, first_n, first_out, 1, row_tile, stream);
-  if (error == cudaSuccess) error = dense_gemm(layout, base, workspace_bytes, rows, second_w, second_scale, nullptr, second_n, second_out, 1, row_tile, stream);
+  const DenseProduct products[2] = {{first_w, first_scale, nullptr, first_n, first_out}, {second_w, second_scale, nullptr, second_n, second_out}};
+  const cudaError_t error = dense_gemm(layout, static_cast<char*>(workspace), rows, products, 2, 1, stream);
   return error == cudaSuccess ? FMOE_OK : cuda_fail(error, "i8gemm pair GEMM");
 }
 

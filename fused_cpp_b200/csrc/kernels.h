@@ -1,6 +1,7 @@
 // Launchers of the individual kernels; the C ABI in api.cu sequences them.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -164,13 +165,6 @@ struct GroupedGemmArgs {
                              // tile to bf16; 2 = two int8 planes per route (a_rows holds 2 * total_rows rows, a_scale one
                              // scale per route, row_tile counts plane rows), the int8 one-SM kernel pairs accumulator columns
   int gate_up_one_box;       // two-SM gate_up: the weight rows of a stage arrive as one 16 KB TMA box (set by the launcher)
-  // Dense GEMM over few rows (one-SM kernel): the K range of every (row tile, channel block) is cut into dense_splits
-  // parts that run as work units of their own, so that a product with few channel blocks still fills the SMs.  The
-  // parts add their int32 accumulators into dense_partial[rows, n_out] (zero on entry) and count themselves in
-  // dense_counters[unit] (zero on entry); the part that arrives last dequantises and stores.  0 or 1 = no split.
-  int dense_splits;
-  int* dense_partial;
-  int* dense_counters;
   int route_out_bf16;        // the result rows are stored as bf16 (2 bytes per channel, rows 2 * n_out bytes apart) instead of fp32
   // Diagnostic build only (compiled with -DFMOE_DIAG, the separate libfused_moe_b200_diag.so; the product library
   // ignores the field): bit 0 = epilogue does no work, bit 1 = producer loads nothing, bit 2 = no MMA is issued.
@@ -220,6 +214,26 @@ inline int sm_count_of_current_device() {
   if (device >= 0 && device < kMaxDevices) counts[device] = count;
   return count;
 }
+
+// 2-D K-major tensor [rows, k] with 128-byte-swizzled boxes of {128 bytes of K, box_rows} (umma_gemm.cu).
+bool make_sw128_map(CUtensorMap* map, const void* base, bool int8, uint64_t rows, uint64_t k, uint32_t box_rows);
+
+// ---- dense_gemm.cu: dense W8A8 linear over at most kDenseMaxRows rows, one or two weight matrices in one launch.
+// Programmatic dependent of the kernel in front of it in the stream (the row quantiser that writes a_rows / a_scale).
+constexpr int kDenseMaxRows = 128;
+struct DenseGemmArgs {
+  const float* a_scale;      // [rows]
+  const float* w_scale[2];   // [n[i]]
+  const float* bias;         // [n[0]] or null
+  void* out[2];              // [rows, n[i]]
+  int n[2];                  // n[1] = 0: one matrix
+  int out_bf16;
+  int rows;
+  int k_padded;
+  int* status;
+  int first_blocks, k_blocks, parts;  // set by the launcher
+};
+cudaError_t launch_dense_gemm(const DenseGemmArgs& args, const void* a_rows, const int8_t* const* weights, bool split, cudaStream_t stream);
 
 // ---- simt_gemm.cu: CUDA-core grouped GEMM of the diagnostic library only (work items of at most 8 rows)
 constexpr int kSimtRowTile = 8;

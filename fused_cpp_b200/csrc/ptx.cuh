@@ -147,6 +147,12 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// Programmatic dependent launch.  A kernel launched with the programmatic-serialisation attribute starts once every CTA
+// of the kernel before it has called launch_dependents (or ended); grid_dependency_wait then holds until that kernel has
+// completed and its stores are visible.  Both do nothing in a launch without the attribute.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- tensor memory ---------------------------------------------------------------------------
 
 // Whole-warp calls.  `columns` is a power of two in [32, 512].

@@ -8,6 +8,7 @@
 // the output is already in expert-sorted order for the grouped GEMM (gather and quantise fused).
 #include "common.cuh"
 #include "kernels.h"
+#include "ptx.cuh"
 
 namespace fmoe {
 
@@ -308,6 +309,7 @@ __device__ __forceinline__ void write_dense_items(const DenseItems& d) {
 __global__ void __launch_bounds__(kQuantThreads)
 quantize_rows_dense_kernel(const void* __restrict__ x, int x_is_bf16, int cols, int cols_padded, float clamp_low,
                            int8_t* __restrict__ q, float* __restrict__ scale_out, DenseItems dense_items) {
+  ptx::launch_dependents();
   if (blockIdx.x == 0) write_dense_items(dense_items);
   __shared__ float smem[32];
   const int64_t row = blockIdx.x;
@@ -412,35 +414,57 @@ cudaError_t launch_quantize_tokens_scatter(const uint16_t* x, int64_t tokens, in
   return cudaGetLastError();
 }
 
-// The same quantiser for bf16 rows whose length is a multiple of 8: 16-byte loads, 8-byte stores, and the division
-// replaced as in quantize4_torchref_fast (the statement is the same clamp(rint(x / scale)); with scale = amax / 127 of
-// the same row no quotient rounds below -127, so the lower clamp of -128 some callers ask for never binds).
-__global__ void __launch_bounds__(kQuantThreads)
-quantize_rows_dense_bf16x8_kernel(const uint16_t* __restrict__ x, int cols, int cols_padded, int8_t* __restrict__ q,
-                                  float* __restrict__ scale_out, DenseItems dense_items) {
+// The same quantiser for rows whose length is a multiple of 8 and at most 16 * 1024: the row is read once, into registers
+// (two groups of eight values per thread: a 512-thread CTA holds a 7168-column row), and the division is replaced as in
+// quantize4_torchref_fast (the statement is the same clamp(rint(x / scale)); with scale = amax / 127 of the same row no
+// quotient rounds below -127, so the lower clamp of -128 some callers ask for never binds).  Latency-bound for a decode
+// batch: one memory round trip instead of two, and the GEMM behind it fetches weights meanwhile (dense_gemm.cu has the
+// figures of the op); HBM-bound above.
+constexpr int kDenseVectors = 2;
+
+template <bool kBf16>
+__global__ void __launch_bounds__(1024)
+quantize_rows_dense_vec8_kernel(const void* __restrict__ x, int cols, int cols_padded, int8_t* __restrict__ q, float* __restrict__ scale_out,
+                                DenseItems dense_items) {
+  ptx::launch_dependents();  // the GEMM behind this kernel may start fetching its weights
   __shared__ float smem[32];
   if (blockIdx.x == 0) write_dense_items(dense_items);
   const int64_t row = blockIdx.x;
-  const uint4* src = reinterpret_cast<const uint4*>(x + row * cols);
   const int vec8 = cols >> 3;
+  float values[kDenseVectors][8];
   float local = 0.0f;
-  for (int v = threadIdx.x; v < vec8; v += kQuantThreads) local = fmaxf(local, amax8(src[v]));
+#pragma unroll
+  for (int i = 0; i < kDenseVectors; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
+    if (v < vec8) {
+      if constexpr (kBf16) {
+        unpack8(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(x) + row * cols)[v], values[i]);
+      } else {
+        const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(x) + row * cols) + 2 * v;
+        *reinterpret_cast<float4*>(values[i]) = src[0];
+        *reinterpret_cast<float4*>(values[i] + 4) = src[1];
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) values[i][j] = 0.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) local = fmaxf(local, fabsf(values[i][j]));
+  }
   const float amax = block_max(local, smem);
   const float scale = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 1.0f;
   if (threadIdx.x == 0) scale_out[row] = scale;
   const float inverse = __fdiv_rn(1.0f, scale);
   uint2* dst = reinterpret_cast<uint2*>(q + row * cols_padded);
-  const int vec8_padded = cols_padded >> 3;
-  for (int v = threadIdx.x; v < vec8_padded; v += kQuantThreads) {
-    uint2 out = make_uint2(0u, 0u);
+#pragma unroll
+  for (int i = 0; i < kDenseVectors; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
     if (v < vec8) {
-      float values[8];
-      unpack8(src[v], values);
-      out.x = quantize4_torchref_fast(values, scale, inverse);
-      out.y = quantize4_torchref_fast(values + 4, scale, inverse);
+      dst[v] = make_uint2(quantize4_torchref_fast(values[i], scale, inverse), quantize4_torchref_fast(values[i] + 4, scale, inverse));
     }
-    dst[v] = out;
   }
+  // cols_padded is cols or cols + 8 (a multiple of 16).
+  if (threadIdx.x == 0 && cols_padded > cols) dst[vec8] = make_uint2(0u, 0u);
 }
 
 cudaError_t launch_quantize_rows_dense(const void* x, int x_is_bf16, int64_t rows, int cols, int cols_padded, int clamp_low,
@@ -448,11 +472,14 @@ cudaError_t launch_quantize_rows_dense(const void* x, int x_is_bf16, int64_t row
                                        cudaStream_t stream) {
   if (rows <= 0) return cudaSuccess;
   const DenseItems dense_items = {rows, row_tile, max_items, items, status};
-  const bool vector_form = x_is_bf16 && cols % 8 == 0 && cols_padded % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
-                           (reinterpret_cast<uintptr_t>(q) & 7u) == 0;
+  const int vec8 = cols >> 3;
+  const bool vector_form = cols % 8 == 0 && vec8 <= 1024 * kDenseVectors && cols_padded - cols <= 8 && cols_padded % 8 == 0 &&
+                           (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(q) & 7u) == 0;
   if (vector_form) {
-    quantize_rows_dense_bf16x8_kernel<<<static_cast<unsigned>(rows), kQuantThreads, 0, stream>>>(static_cast<const uint16_t*>(x), cols,
-                                                                                                cols_padded, q, scale, dense_items);
+    int threads = 64;
+    while (threads * kDenseVectors < vec8) threads *= 2;
+    auto kernel = x_is_bf16 ? quantize_rows_dense_vec8_kernel<true> : quantize_rows_dense_vec8_kernel<false>;
+    kernel<<<static_cast<unsigned>(rows), threads, 0, stream>>>(x, cols, cols_padded, q, scale, dense_items);
   } else {
     quantize_rows_dense_kernel<<<static_cast<unsigned>(rows), kQuantThreads, 0, stream>>>(
         x, x_is_bf16, cols, cols_padded, static_cast<float>(clamp_low), q, scale, dense_items);

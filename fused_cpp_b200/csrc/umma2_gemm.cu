@@ -690,20 +690,6 @@ EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-// 2-D K-major tensor [rows, k] with 128-byte-swizzled boxes of {128 bytes of K, box_rows}.
-bool make_tensor_map(CUtensorMap* map, const void* base, bool int8, uint64_t rows, uint64_t k, uint32_t box_rows) {
-  EncodeTiledFn encode = encode_tiled_fn();
-  if (encode == nullptr) return false;
-  const uint32_t elem_bytes = int8 ? 1 : 2;
-  const cuuint64_t dims[2] = {k, rows};
-  const cuuint64_t strides[1] = {k * elem_bytes};
-  const cuuint32_t box[2] = {kBlockKBytes / elem_bytes, box_rows};
-  const cuuint32_t elem_strides[2] = {1, 1};
-  return encode(map, int8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides,
-                box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // gate_up weights [E, 2I, K] as a 5-D tensor whose boxes put the 16 gate rows of a channel group next to its 16
 // up rows.  one_box: dimensions {K, 16 rows, gate|up, I/16 groups, E} and a box of four groups (16 KB, one TMA
 // operation per stage; the gate|up stride is larger than the group stride that follows it).  Otherwise
@@ -759,10 +745,10 @@ cudaError_t launch_pair(const GroupedGemmArgs& args, cudaStream_t stream) {
     launch_args.gate_up_one_box = try_one && make_gate_up_map(&weight_map, args, kInt8, true);
     weights_ok = launch_args.gate_up_one_box || make_gate_up_map(&weight_map, args, kInt8, false);
   } else {
-    weights_ok = make_tensor_map(&weight_map, args.weights, kInt8, static_cast<uint64_t>(args.experts) * args.n_out, args.k, kRowsPerCta);
+    weights_ok = make_sw128_map(&weight_map, args.weights, kInt8, static_cast<uint64_t>(args.experts) * args.n_out, args.k, kRowsPerCta);
   }
   const uint64_t token_rows = static_cast<uint64_t>(args.total_rows) * (kPlanes ? 2 : 1);
-  if (!weights_ok || !make_tensor_map(&token_map, args.a_rows, kInt8, token_rows, args.k, kRowsPerCta)) {
+  if (!weights_ok || !make_sw128_map(&token_map, args.a_rows, kInt8, token_rows, args.k, kRowsPerCta)) {
     return cudaErrorInvalidValue;
   }
   const int sms = sm_count_of_current_device();

@@ -122,7 +122,6 @@ struct SmemControl {
   uint64_t acc_empty[2];
   uint32_t tmem_base;
   volatile int abort_flag;
-  int last_part;           // dense split-K: this CTA holds the last part of its unit and finishes it
   uint32_t exp_table[64];  // copy of kExp2Table: divergent lookups are served by 32 banks
   ColumnMeta meta[2];
 };
@@ -150,12 +149,12 @@ __device__ __forceinline__ void widen_int8x4(uint32_t word, uint32_t* low_pair, 
 // X = 256 * high + low, so a work item of r routes has 2r token rows and its accumulator columns come in pairs:
 // the exact integer dot product of route p with a channel is 256 * column(2p) + column(2p + 1).  Work items are
 // given in routes; loads, the MMA's N and the epilogue count plane rows.
-template <bool kInt8, bool kGateUp, int kRowTile, bool kDense, bool kW8A16 = false, bool kPlanes = false>
+template <bool kInt8, bool kGateUp, int kRowTile, bool kW8A16 = false, bool kPlanes = false>
 __global__ void __launch_bounds__(kW8A16 ? kThreadsW8A16 : kThreads, 1)
 umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_constant__ CUtensorMap token_map,
                          GroupedGemmArgs args) {
-  static_assert(!kW8A16 || (!kInt8 && !kDense), "W8A16 is an instance of the bf16 grouped kernel");
-  static_assert(!kPlanes || (kInt8 && !kDense && !kW8A16), "the two-plane form is an instance of the int8 grouped kernel");
+  static_assert(!kW8A16 || !kInt8, "W8A16 is an instance of the bf16 grouped kernel");
+  static_assert(!kPlanes || (kInt8 && !kW8A16), "the two-plane form is an instance of the int8 grouped kernel");
   constexpr int kRowsPerRoute = kPlanes ? 2 : 1;
   using Cfg = TileConfig<kGateUp, kRowTile, kW8A16>;
   constexpr int kElemBytes = kInt8 ? 1 : 2;
@@ -176,10 +175,6 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
   const int n_total = kGateUp ? 2 * args.n_out : args.n_out;
   const int64_t units = static_cast<int64_t>(items) * n_blocks;
   const int k_blocks = (args.k + kBlockKElems - 1) / kBlockKElems;
-  // Dense split-K: `parts` work units per (row tile, channel block), part p over K blocks [p k_blocks / parts,
-  // (p + 1) k_blocks / parts).  Everything else runs with parts == 1.
-  const int parts = kDense ? (args.dense_splits > 1 ? args.dense_splits : 1) : 1;
-  const int64_t part_units = units * parts;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::kStages; ++s) {
@@ -272,10 +267,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
           }
         }
       }
-      for (int64_t part_unit = blockIdx.x; !kW8A16 && part_unit < part_units; part_unit += gridDim.x) {
-        const int64_t unit = part_unit / parts;
-        const int part = static_cast<int>(part_unit - unit * parts);
-        const int kb_begin = part * k_blocks / parts, kb_end = (part + 1) * k_blocks / parts;
+      for (int64_t unit = blockIdx.x; !kW8A16 && unit < units; unit += gridDim.x) {
         int item, block;
         decode_unit(args.items, unit, n_blocks, &item, &block);
         item = __shfl_sync(0xffffffffu, item, 0);  // read from the item list: the same in every lane
@@ -284,7 +276,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
         const int expert = __shfl_sync(0xffffffffu, args.items[4 * item + 0], 0);
         const int row0 = __shfl_sync(0xffffffffu, args.items[4 * item + 1], 0) * kRowsPerRoute;
         const int weight_row = expert * n_total + n0;
-        for (int kb = kb_begin; kb < kb_end; ++kb) {
+        for (int kb = 0; kb < k_blocks; ++kb) {
           ptx::mbar_wait(&ctl->empty[stage], phase ^ 1u, abort_flag, status, 1);
           uint8_t* stage_base = smem + static_cast<size_t>(stage) * Cfg::kStageBytes;
           if (!issuer) {
@@ -393,10 +385,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
       uint32_t phase = 0;
       int slot = 0;  // W8A16: landing slot of the K block (its token tile is the MMA's B operand)
       int local = 0;
-      for (int64_t part_unit = blockIdx.x; part_unit < part_units; part_unit += gridDim.x, ++local) {
-        const int64_t unit = part_unit / parts;
-        const int part = static_cast<int>(part_unit - unit * parts);
-        const int kb_begin = part * k_blocks / parts, kb_end = (part + 1) * k_blocks / parts;
+      for (int64_t unit = blockIdx.x; unit < units; unit += gridDim.x, ++local) {
         const int buffer = local % Cfg::kAccBuffers;
         const uint32_t use = static_cast<uint32_t>(local / Cfg::kAccBuffers);
         // The MMA's N follows the rows this unit really has (multiple of 16): a tail item of a few rows costs a
@@ -413,7 +402,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
         ptx::mbar_wait(&ctl->acc_empty[buffer], (use & 1u) ^ 1u, abort_flag, status, 2);
         ptx::tcgen05_fence_after();
         const uint32_t acc = tmem_base + static_cast<uint32_t>(buffer * Cfg::kAccColumns);
-        for (int kb = kb_begin; kb < kb_end; ++kb) {
+        for (int kb = 0; kb < k_blocks; ++kb) {
           ptx::mbar_wait(&ctl->full[stage], phase, abort_flag, status, 3);
           ptx::tcgen05_fence_after();
           const uint32_t stage_addr = ptx::smem_u32(smem + static_cast<size_t>(stage) * Cfg::kStageBytes);
@@ -425,7 +414,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
             if (FMOE_DIAG_BIT(args, 4) || !issuer) break;
             const uint64_t desc_gate = ptx::make_smem_desc_sw128(stage_addr + ks * kUmmaKBytes);
             const uint64_t desc_tok = ptx::make_smem_desc_sw128(token_addr + ks * kUmmaKBytes);
-            const uint32_t accumulate = (kb > kb_begin || ks > 0) ? 1u : 0u;
+            const uint32_t accumulate = (kb > 0 || ks > 0) ? 1u : 0u;
             if constexpr (kW8A16) {
               ptx::umma_ss<false>(acc, desc_tok, desc_gate, idesc, accumulate);  // A = tokens, B = gate (+ up) channels
               continue;
@@ -460,8 +449,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
     const int activation = args.activation;
     uint32_t* const dump = kPlanes ? nullptr : static_cast<uint32_t*>(args.dump_acc);  // the dump holds one row per route
     int local = 0;
-    for (int64_t part_unit = blockIdx.x; part_unit < part_units; part_unit += gridDim.x, ++local) {
-      const int64_t unit = part_unit / parts;
+    for (int64_t unit = blockIdx.x; unit < units; unit += gridDim.x, ++local) {
       const int buffer = local % Cfg::kAccBuffers;
       const uint32_t use = static_cast<uint32_t>(local / Cfg::kAccBuffers);
       int item, block;
@@ -552,9 +540,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
       for (int c = epilogue_thread; c < rows; c += 128) {
         const int route_row = (row0 + c) / kRowsPerRoute;  // sorted position of the column's route
         if (kInt8) meta->scale[c] = args.a_scale[route_row];
-        if constexpr (kDense) {
-          meta->rowptr[c] = reinterpret_cast<uint64_t>(args.dense_out) + static_cast<uint64_t>(row0 + c) * n_out * (args.dense_out_bf16 ? 2 : 4);
-        } else if constexpr (!kGateUp) {
+        if constexpr (!kGateUp) {
           meta->rowptr[c] = args.row_out_ptrs != nullptr
                                 ? args.row_out_ptrs[route_row]
                                 : reinterpret_cast<uint64_t>(args.route_out) +
@@ -567,10 +553,8 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
         scale_gate = s[kGateUp ? gate_channel(args, n) : n];
         if (kGateUp) scale_up = s[up_channel(args, n)];
       }
-      float bias = 0.0f;
-      if (kDense && channel_ok && args.bias != nullptr) bias = args.bias[n];
       float bias_gate = 0.0f, bias_up = 0.0f;  // per-expert bias of the BF16 path (gate_up: gate / up; down: bias_gate)
-      if (!kInt8 && !kDense && channel_ok && args.expert_bias != nullptr) {
+      if (!kInt8 && channel_ok && args.expert_bias != nullptr) {
         const int64_t first = static_cast<int64_t>(expert) * n_total;
         bias_gate = load_expert_bias(args, first + (kGateUp ? gate_channel(args, n) : n));
         if (kGateUp) bias_up = load_expert_bias(args, first + up_channel(args, n));
@@ -579,55 +563,6 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
       ptx::mbar_wait(&ctl->acc_full[buffer], use & 1u, abort_flag, status, 4);
       ptx::tcgen05_fence_after();
       const uint32_t acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buffer * Cfg::kAccColumns);
-      if constexpr (kDense) {
-        if (parts > 1) {
-          // This part's int32 sums go into the shared table; the part that finds the other parts' counts complete reads
-          // the totals back and finishes the unit (integer addition: the order of the parts changes nothing).
-          for (int c0 = 0; c0 < rows; c0 += 8) {
-            uint32_t bits[8];
-            ptx::tmem_ld_x8(acc + c0, bits);
-            ptx::tmem_ld_wait();
-            if (channel_ok) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                if (c0 + j < rows) atomicAdd(args.dense_partial + static_cast<int64_t>(row0 + c0 + j) * n_out + n, static_cast<int>(bits[j]));
-              }
-            }
-          }
-          ptx::tcgen05_fence_before();
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&ctl->acc_empty[buffer]);
-          __threadfence();  // this thread's additions are visible before the count below
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          if (epilogue_thread == 0) ctl->last_part = atomicAdd(args.dense_counters + unit, 1) == parts - 1 ? 1 : 0;
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          if (ctl->last_part) {
-            __threadfence();  // the other parts' additions, published before their counts, are visible after ours
-            if (channel_ok) {
-              // Sixteen rows at a time: the loads of a batch are in flight together.
-              for (int c0 = 0; c0 < rows; c0 += 16) {
-                int totals[16];
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  totals[j] = c0 + j < rows ? __ldcg(args.dense_partial + static_cast<int64_t>(row0 + c0 + j) * n_out + n) : 0;
-                }
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  if (c0 + j >= rows) break;
-                  const float value = __fadd_rn(dequantize(totals[j], meta->scale[c0 + j], scale_gate, numerics), bias);
-                  const uint64_t rowptr = meta->rowptr[c0 + j];
-                  if (args.dense_out_bf16) {
-                    reinterpret_cast<uint16_t*>(rowptr)[n] = f32_to_bf16_bits(value);
-                  } else {
-                    reinterpret_cast<float*>(rowptr)[n] = value;
-                  }
-                }
-              }
-            }
-          }
-          continue;
-        }
-      }
       for (int c0 = 0; c0 < (FMOE_DIAG_BIT(args, 1) ? 0 : rows); c0 += 8) {
         uint32_t gate_bits[8];
         uint32_t up_bits[8];
@@ -691,14 +626,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
                   value = __fadd_rn(__uint_as_float(gate_bits[j]), bias_gate);
                 }
                 const uint64_t rowptr = meta->rowptr[c0 + j];
-                if constexpr (kDense) {
-                  value = __fadd_rn(value, bias);
-                  if (args.dense_out_bf16) {
-                    reinterpret_cast<uint16_t*>(rowptr)[n] = f32_to_bf16_bits(value);
-                  } else {
-                    reinterpret_cast<float*>(rowptr)[n] = value;
-                  }
-                } else if (args.route_out_bf16) {
+                if (args.route_out_bf16) {
                   reinterpret_cast<uint16_t*>(rowptr)[n] = f32_to_bf16_bits(value);
                 } else {
                   reinterpret_cast<float*>(rowptr)[n] = value;
@@ -742,8 +670,9 @@ EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-// 2-D K-major tensor [rows, k] with 128-byte-swizzled boxes of {128 bytes of K, box_rows}.
-bool make_tensor_map(CUtensorMap* map, const void* base, bool int8, uint64_t rows, uint64_t k, uint32_t box_rows) {
+}  // namespace
+
+bool make_sw128_map(CUtensorMap* map, const void* base, bool int8, uint64_t rows, uint64_t k, uint32_t box_rows) {
   EncodeTiledFn encode = encode_tiled_fn();
   if (encode == nullptr) return false;
   const uint32_t elem_bytes = int8 ? 1 : 2;
@@ -756,6 +685,8 @@ bool make_tensor_map(CUtensorMap* map, const void* base, bool int8, uint64_t row
                                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return result == CUDA_SUCCESS;
 }
+
+namespace {
 
 // W8A16 landing loads: int8 weight rows [rows, k] as plain (unswizzled) boxes of {64 bytes of K, 128 rows}.
 bool make_landing_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t k) {
@@ -792,10 +723,10 @@ bool make_gate_up_map(CUtensorMap* map, const GroupedGemmArgs& args, bool int8, 
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <bool kInt8, bool kGateUp, int kRowTile, bool kDense, bool kW8A16 = false, bool kPlanes = false>
+template <bool kInt8, bool kGateUp, int kRowTile, bool kW8A16 = false, bool kPlanes = false>
 cudaError_t launch_config(const GroupedGemmArgs& args, cudaStream_t stream) {
   using Cfg = TileConfig<kGateUp, kRowTile, kW8A16>;
-  auto kernel = umma_grouped_gemm_kernel<kInt8, kGateUp, kRowTile, kDense, kW8A16, kPlanes>;
+  auto kernel = umma_grouped_gemm_kernel<kInt8, kGateUp, kRowTile, kW8A16, kPlanes>;
   static PerDeviceOnce configured;
   const int device = current_device_ordinal();
   if (configured.needed(device)) {
@@ -807,13 +738,13 @@ cudaError_t launch_config(const GroupedGemmArgs& args, cudaStream_t stream) {
   const uint64_t weight_rows = static_cast<uint64_t>(args.experts) * args.n_out;  // down / dense
   const bool weights_ok = kGateUp   ? make_gate_up_map(&weight_map, args, kInt8 || kW8A16, kW8A16)
                           : kW8A16 ? make_landing_map(&weight_map, args.weights, weight_rows, args.k)
-                                   : make_tensor_map(&weight_map, args.weights, kInt8, weight_rows, args.k, kBlockM);
+                                   : make_sw128_map(&weight_map, args.weights, kInt8, weight_rows, args.k, kBlockM);
   const uint64_t token_rows = static_cast<uint64_t>(args.total_rows) * (kPlanes ? 2 : 1);
-  if (!weights_ok || !make_tensor_map(&token_map, args.a_rows, kInt8, token_rows, args.k, kRowTile)) {
+  if (!weights_ok || !make_sw128_map(&token_map, args.a_rows, kInt8, token_rows, args.k, kRowTile)) {
     return cudaErrorInvalidValue;
   }
   const int n_blocks = (args.n_out + kBlockM - 1) / kBlockM;
-  int64_t grid = static_cast<int64_t>(args.max_items) * n_blocks * (kDense && args.dense_splits > 1 ? args.dense_splits : 1);
+  int64_t grid = static_cast<int64_t>(args.max_items) * n_blocks;
   const int sms = sm_count_of_current_device();
   if (grid > sms) grid = sms;
   if (grid <= 0) return cudaSuccess;
@@ -821,19 +752,19 @@ cudaError_t launch_config(const GroupedGemmArgs& args, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-template <bool kInt8, bool kGateUp, bool kDense, bool kW8A16 = false, bool kPlanes = false>
+template <bool kInt8, bool kGateUp, bool kW8A16 = false, bool kPlanes = false>
 cudaError_t launch_tile(const GroupedGemmArgs& args, cudaStream_t stream) {
   switch (args.row_tile) {
-    case 16: return launch_config<kInt8, kGateUp, 16, kDense, kW8A16, kPlanes>(args, stream);
-    case 32: return launch_config<kInt8, kGateUp, 32, kDense, kW8A16, kPlanes>(args, stream);
-    case 64: return launch_config<kInt8, kGateUp, 64, kDense, kW8A16, kPlanes>(args, stream);
-    case 128: return launch_config<kInt8, kGateUp, 128, kDense, kW8A16, kPlanes>(args, stream);
+    case 16: return launch_config<kInt8, kGateUp, 16, kW8A16, kPlanes>(args, stream);
+    case 32: return launch_config<kInt8, kGateUp, 32, kW8A16, kPlanes>(args, stream);
+    case 64: return launch_config<kInt8, kGateUp, 64, kW8A16, kPlanes>(args, stream);
+    case 128: return launch_config<kInt8, kGateUp, 128, kW8A16, kPlanes>(args, stream);
     case 256:
       // Token-major W8A16 holds an item in the 128 lanes of one accumulator: no 256-row tile.
       if constexpr (kW8A16) {
         return cudaErrorInvalidValue;
       } else {
-        return launch_config<kInt8, kGateUp, 256, kDense, kW8A16, kPlanes>(args, stream);
+        return launch_config<kInt8, kGateUp, 256, kW8A16, kPlanes>(args, stream);
       }
     default: return cudaErrorInvalidValue;
   }
@@ -859,24 +790,21 @@ cudaError_t launch_umma_grouped_gemm(const GroupedGemmArgs& caller_args, bool in
     // row_tile counts plane rows (two per route).
     if (!int8 || args.dense_out != nullptr || args.w_scale == nullptr || args.a_scale == nullptr) return cudaErrorInvalidValue;
     if (args.row_tile == kPairRowTile) return launch_umma_pair_grouped_gemm(args, true, gate_up, stream);  // items of at most 128 routes
-    return gate_up ? launch_tile<true, true, false, false, true>(args, stream) : launch_tile<true, false, false, false, true>(args, stream);
+    return gate_up ? launch_tile<true, true, false, true>(args, stream) : launch_tile<true, false, false, true>(args, stream);
   }
   if (args.w8a16) {
     // int8 weights with bf16 activations: the one-SM kernel with its widening warps, for every row tile.
     if (int8 || args.dense_out != nullptr || args.w_scale == nullptr) return cudaErrorInvalidValue;
     if (args.row_tile > 128) return cudaErrorInvalidValue;  // the caller caps W8A16 work items at 128 rows
-    return gate_up ? launch_tile<false, true, false, true>(args, stream) : launch_tile<false, false, false, true>(args, stream);
+    return gate_up ? launch_tile<false, true, true>(args, stream) : launch_tile<false, false, true>(args, stream);
   }
   if (args.row_tile == kPairRowTile) {
     if (umma_pair_supported(gate_up, args.n_out, args.total_rows)) return launch_umma_pair_grouped_gemm(args, int8, gate_up, stream);
     args.row_tile = 256;  // same 256-row work items, one-SM kernel
   }
-  if (args.dense_out != nullptr) {
-    if (!int8 || gate_up) return cudaErrorInvalidValue;  // the dense epilogue exists for the int8 single-stage GEMM
-    return launch_tile<true, false, true>(args, stream);
-  }
-  if (int8) return gate_up ? launch_tile<true, true, false>(args, stream) : launch_tile<true, false, false>(args, stream);
-  return gate_up ? launch_tile<false, true, false>(args, stream) : launch_tile<false, false, false>(args, stream);
+  if (args.dense_out != nullptr) return cudaErrorInvalidValue;  // dense products: the two-SM kernel or dense_gemm.cu
+  if (int8) return gate_up ? launch_tile<true, true>(args, stream) : launch_tile<true, false>(args, stream);
+  return gate_up ? launch_tile<false, true>(args, stream) : launch_tile<false, false>(args, stream);
 }
 
 }  // namespace fmoe

@@ -1,0 +1,43 @@
+"""Dense W8A8 linear at the sizes where its kernels change: row tiles of 16 to 128 rows and the two-SM kernel above, K
+ranges of one 128-byte block up to several per part of the cluster split, K and N off every vector and tile width, rows
+too long for the register-held quantiser (16384 columns), one and two weight matrices.  Bit for bit against the oracle."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from fused_cpp_b200 import i8gemm
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _weight(n, k, generator):
+    return torch.randint(-127, 128, (n, k), dtype=torch.int8, generator=generator), torch.rand(n, generator=generator) * 0.01 + 1e-3
+
+
+@pytest.mark.parametrize("rows,k,n,x_dtype,out_dtype,with_bias", [
+    (1, 8, 1, torch.bfloat16, torch.float32, True), (16, 128, 128, torch.bfloat16, torch.bfloat16, False),
+    (17, 264, 129, torch.float32, torch.bfloat16, True), (32, 2056, 520, torch.bfloat16, torch.float32, False),
+    (33, 1000, 130, torch.float32, torch.float32, True), (64, 4096, 1536, torch.bfloat16, torch.bfloat16, True),
+    (65, 777, 300, torch.bfloat16, torch.bfloat16, False), (128, 1536, 4000, torch.bfloat16, torch.bfloat16, True),
+    (129, 1536, 300, torch.float32, torch.bfloat16, True), (3, 16384, 136, torch.bfloat16, torch.bfloat16, False),
+    (5, 16400, 200, torch.bfloat16, torch.float32, True), (2, 16392, 64, torch.float32, torch.float32, False),
+])
+def test_product(cuda_device, rows, k, n, x_dtype, out_dtype, with_bias):
+    generator = torch.Generator().manual_seed(rows + k + n)
+    weight, scale = _weight(n, k, generator)
+    x = torch.randn((rows, k), generator=generator).to(x_dtype)
+    bias = torch.randn(n, generator=generator) if with_bias else None
+    got = i8gemm.dynamic_scaled_mm(x.to(cuda_device), i8gemm.prepare(weight, scale), bias=None if bias is None else bias.to(cuda_device), out_dtype=out_dtype)
+    torch.testing.assert_close(got.cpu(), oracle.i8gemm_dynamic(x, weight, scale, bias, out_dtype), atol=0, rtol=0)
+
+
+@pytest.mark.parametrize("rows,k,first_n,second_n", [(1, 1536, 4000, 72), (40, 512, 130, 129), (128, 300, 64, 700), (200, 512, 300, 130)])
+def test_pair(cuda_device, rows, k, first_n, second_n):
+    generator = torch.Generator().manual_seed(rows + k)
+    first, second = _weight(first_n, k, generator), _weight(second_n, k, generator)
+    x = torch.randn((rows, k), generator=generator).to(torch.bfloat16)
+    got = i8gemm.dynamic_scaled_mm_pair(x.to(cuda_device), i8gemm.prepare(*first), i8gemm.prepare(*second))
+    for out, (weight, scale) in zip(got, (first, second)):
+        torch.testing.assert_close(out.cpu(), oracle.i8gemm_dynamic(x, weight, scale, None, torch.bfloat16, clamp_low=-127), atol=0, rtol=0)
