@@ -236,11 +236,11 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   // Above 64 tokens an expert can hold anything from one row to all of them, and the host does not know the routing.
   // Unless the caller fixed the tiles, the experts are then split on the device: those with at most 64 rows
   // go through the one-SM kernel (64-row tile, every weight byte streamed once), the others through the
-  // two-SM kernel (256-row work items).  Up to 64 tokens no expert can exceed 64 rows and the tile follows
+  // two-SM kernel (320-row work items).  Up to 64 tokens no expert can exceed 64 rows and the tile follows
   // the batch size (pick_row_tile).
   // W8A16.  Its fixed-point form runs on the int8 kernels with two token rows (planes) per route: the kernel's row
   // tile is twice the routes of a work item, so an item holds at most 128 routes; above 64 tokens the experts are
-  // split like W8A8's (thin ones to the one-SM kernel, the others to the two-SM kernel in 128-route items).  Its
+  // split like W8A8's (thin ones to the one-SM kernel, the others to the two-SM kernel in 160-route items).  Its
   // bf16-activation form runs every expert through the one-SM kernel (the int8 -> bf16 widening lives there): no
   // split, and a 128-row tile above 64 tokens.
   const bool planes = f.w8a16 && umma && cfg.w8a16_form == FMOE_W8A16_FIXED_POINT;
@@ -260,8 +260,8 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   if (umma && (!fmoe::umma_row_tile_supported(tile_gu) || !fmoe::umma_row_tile_supported(tile_dn))) {
     return fail(FMOE_ERR_INVALID_ARGUMENT, "row tiles must be 16, 32, 64, 128, 256 or 512 = two-SM pairs (got %d, %d)", tile_gu, tile_dn);
   }
-  // Tile 512 selects the two-SM kernel, whose work items hold up to 256 rows.
-  const int pair_item_rows = planes ? 128 : 256;  // routes of a two-SM work item (256 token rows either way)
+  // Tile 512 selects the two-SM kernel, whatever its work items hold.
+  const int pair_item_rows = planes ? fmoe::kPairItemRows / 2 : fmoe::kPairItemRows;  // in routes (two token rows each with planes)
   const int item_rows_gu = tile_gu == fmoe::kPairRowTile ? pair_item_rows : tile_gu;
   const int item_rows_dn = tile_dn == fmoe::kPairRowTile ? pair_item_rows : tile_dn;
 

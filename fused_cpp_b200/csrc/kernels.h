@@ -243,9 +243,9 @@ cudaError_t launch_simt_grouped_gemm(const GroupedGemmArgs& args, bool int8, boo
 bool umma_row_tile_supported(int row_tile);
 cudaError_t launch_umma_grouped_gemm(const GroupedGemmArgs& args, bool int8, bool gate_up, cudaStream_t stream);
 
-// ---- umma2_gemm.cu: two-SM (cta_group::2) grouped GEMM, 256-row work items.  Selected by row tile 512.
+// ---- umma2_gemm.cu: two-SM (cta_group::2) grouped GEMM.  Selected by row tile 512.
 constexpr int kPairRowTile = 512;
-bool umma_pair_supported(bool gate_up, int n_out, int64_t output_rows);  // else callers use the one-SM kernel on the same items
+constexpr int kPairItemRows = 320;  // token rows of a work item at most (umma2_gemm.cu says why)
 cudaError_t launch_umma_pair_grouped_gemm(const GroupedGemmArgs& args, bool int8, bool gate_up, cudaStream_t stream);
 
 // ---- probe.cu (diagnostic library only): tcgen05.mma issue-rate probe (128 x n x 32-byte MMAs back to back on every CTA)

@@ -49,7 +49,14 @@ __device__ void build_item_list(int list, int experts, const int* counts, const 
   }
   const int tile = list == 0 ? lists.tile_a : list == 1 ? lists.tile_b : lists.big_tile;
   int* items = list == 0 ? lists.items_a : list == 1 ? lists.items_b : list == 2 ? lists.items_c : lists.items_d;
-  const int shift = __ffs(tile) - 1;  // row tiles are powers of two
+  // Row tiles are powers of two but for the two-SM kernel's, 5/4 of one (320 token rows): its full height spares an expert a
+  // second pass over its weights for a few rows; longer lists are cut at the power of two, whose accumulators double-buffer
+  // without sharing columns.  About 256 rows per expert (int8, 8192 tokens): 4228 -> 3877 us.  Lists of thousands of rows,
+  // bf16, took 3312 us cut at 256 and 3367 us cut at 320; about 512 rows (int8, 16384 tokens) are the same either way.
+  const bool tall = (tile & (tile - 1)) != 0;
+  const int cut = tall ? tile / 5 * 4 : tile;
+  const int shift = __ffs(cut) - 1;
+  auto tiles_of = [&](int rows) { return tall && rows > cut && rows <= tile ? 1 : (rows + cut - 1) >> shift; };
   int carry = 0;
   int active = 0;
   constexpr int kBatch = 8;  // groups of 32 experts whose scans are interleaved: a scan is a chain of dependent shuffles
@@ -61,7 +68,7 @@ __device__ void build_item_list(int list, int experts, const int* counts, const 
       count[i] = e < experts ? counts[e] : 0;
       active += __popc(__ballot_sync(0xffffffffu, count[i] > 0));
       if (split_rows > 0 && big != (count[i] > split_rows)) count[i] = 0;  // belongs to the other list
-      inclusive[i] = (count[i] + tile - 1) >> shift;
+      inclusive[i] = tiles_of(count[i]);
     }
 #pragma unroll
     for (int offset = 1; offset < 32; offset <<= 1) {
@@ -73,14 +80,14 @@ __device__ void build_item_list(int list, int experts, const int* counts, const 
     }
 #pragma unroll
     for (int i = 0; i < kBatch; ++i) {
-      const int tiles = (count[i] + tile - 1) >> shift;
+      const int tiles = tiles_of(count[i]);
       const int first = carry + inclusive[i] - tiles;
       carry += __shfl_sync(0xffffffffu, inclusive[i], 31);
       if (tiles == 0) continue;
       const int e = base + 32 * i + lane;
       const int row0 = offsets[e];
       // The expert's rows are spread evenly over its tiles (in steps of 32 rows, the granularity of the MMA's N):
-      // 290 rows become 160 + 130, not 256 + 34.
+      // 330 rows become 192 + 138, not 256 + 74.
       int rows_per = tile;
       if (tiles > 1) {
         const int step = tile < 32 ? tile : 32;

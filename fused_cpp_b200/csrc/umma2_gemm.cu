@@ -19,6 +19,10 @@
 //   gate_up: A rows of CTA r = channels c0 + 64 r .. + 63 as four groups of [16 gate rows | 16 up rows]
 //            (one 5-D TMA box: {K bytes, 16 rows, gate/up, 4 groups, expert}), so lanes l and l + 16 of every
 //            epilogue warp hold gate and up of the same channel and swap them with one shuffle.
+// Work units.  Up to 256 token rows are one MMA per K step; an expert with 257 to 320 rows is one unit of two MMAs that share
+// the weight tile, where two units of about 144 rows would each bring 32 KB of weights per K block for 20 KB of rows and
+// wait for L2 (route.cu makes the items).  About 256 rows per expert, 8192 tokens of the 256-expert 7168 x 2048 int8 layer:
+// gate_up 1969 -> 1770 us, down 1086 -> 1012 us.
 // Barriers.  Both producers signal the leader's "full" barrier (TMA complete_tx through the cluster
 // address), the leader's single MMA thread commits to the "empty" and "accumulator full" barriers of
 // both CTAs, and the follower's epilogue warps arrive on the leader's "accumulator empty" barrier
@@ -34,8 +38,13 @@ namespace fmoe {
 
 namespace {
 
-constexpr int kRowsPerCta = 128;    // A rows and B rows staged by one CTA
-constexpr int kPairTokens = 256;    // MMA N
+constexpr int kRowsPerCta = 128;    // A rows staged by one CTA
+constexpr int kMmaTokens = 256;     // largest N of one MMA
+constexpr int kMaxTokenRows = kPairItemRows;         // token rows of a work unit
+constexpr int kTokensPerCta = kMaxTokenRows / 2;     // B rows staged by one CTA
+constexpr int kBoxTokens = 16;                       // token rows of a block in one CTA, and of the smallest TMA box
+constexpr int kMidBox = 4;                           // blocks of the middle box
+constexpr int kFullBox = 8;                          // blocks of the largest
 constexpr int kBlockKBytes = 128;
 constexpr int kUmmaKBytes = 32;
 #ifndef FMOE_PAIR_EPILOGUE_WARPS
@@ -45,15 +54,19 @@ constexpr int kEpilogueWarps = FMOE_PAIR_EPILOGUE_WARPS;  // a multiple of 4: ev
 constexpr int kEpilogueThreads = kEpilogueWarps * 32;
 constexpr int kThreads = 64 + kEpilogueThreads;
 constexpr int kStages = 6;
-constexpr int kStageBytes = 2 * kRowsPerCta * kBlockKBytes;  // 32 KB
-constexpr int kAccColumns = kPairTokens;                     // one accumulator: 256 columns
-constexpr int kTmemColumns = 512;                            // two accumulators
-constexpr size_t kSmemBytes = 1024 + static_cast<size_t>(kStages) * kStageBytes + 8192;
+constexpr int kWeightBytes = kRowsPerCta * kBlockKBytes;                // 16 KB
+constexpr int kStageBytes = kWeightBytes + kTokensPerCta * kBlockKBytes;  // 36 KB
+constexpr int kTmemColumns = 512;                                         // a ring of 32-column blocks (AccSlot)
+constexpr int kRingBlocks = kTmemColumns / 32;
+constexpr int kMmaBlocks = kMmaTokens / 32;
+constexpr size_t kControlBytes = 9216;
+constexpr size_t kSmemBytes = 1024 + static_cast<size_t>(kStages) * kStageBytes + kControlBytes;
+static_assert(kSmemBytes <= 227 * 1024, "a CTA has 227 KB of shared memory");
 
 // Per-column values of a work unit, staged one unit ahead so that the element loop reads shared memory.
 struct ColumnMeta {
-  float scale[256];      // activation scale of the row (int8)
-  uint64_t rowptr[256];  // byte address of the output row (down / dense; may be peer memory)
+  float scale[kMaxTokenRows];      // activation scale of the row (int8)
+  uint64_t rowptr[kMaxTokenRows];  // byte address of the output row (down / dense; may be peer memory)
 };
 
 struct PairControl {
@@ -61,12 +74,13 @@ struct PairControl {
   uint64_t full[kStages];
   uint64_t empty[kStages];
   uint64_t acc_full[2];
+  uint64_t acc_part[2];   // the blocks of the unit that the next unit's accumulator takes over have been read
   uint64_t acc_empty[2];
   uint32_t tmem_base;
   volatile int abort_flag;
   uint32_t exp_table[64];  // copy of kExp2Table: divergent lookups are served by 32 banks
 };
-static_assert(sizeof(PairControl) <= 8192, "control block exceeds its shared-memory reservation");
+static_assert(sizeof(PairControl) <= kControlBytes, "control block exceeds its shared-memory reservation");
 
 __device__ __forceinline__ uint32_t cluster_cta_rank() {
   uint32_t rank;
@@ -203,6 +217,41 @@ __device__ __forceinline__ UnitInfo load_unit(const int* __restrict__ items, int
   return info;
 }
 
+// Where a unit's accumulator lies.  Tensor memory is a ring of sixteen 32-column blocks; a unit of up to 320 rows takes
+// one block per 32 rows, behind the unit before it, so that its main loop runs while that unit's accumulator is still
+// being read: two units of up to 256 rows never share a block, and of two larger ones the second waits only for the
+// blocks it takes over (blocks_shared, barrier acc_part), not for the whole accumulator.
+// Up to 256 rows are one MMA over consecutive columns; above that two MMAs share the staged weight tile, the first over
+// `head` blocks.  Where the ring ends inside the accumulator the split lies there, and each MMA gets at least 64
+// columns (a 32-column MMA takes as long as a 64-column one: it reads the same weight rows).
+struct AccSlot {
+  int start;   // running block number; its place in the ring is start mod 16
+  int blocks;
+  int head;
+};
+
+__device__ __forceinline__ AccSlot place_unit(int start, int rows) {
+  AccSlot slot = {start, (rows + 31) >> 5, 0};
+  const int place = start & (kRingBlocks - 1);
+  const int room = kRingBlocks - place;
+  if (slot.blocks <= kMmaBlocks) {
+    if (slot.blocks > room) slot.start += room;
+    slot.head = slot.blocks;
+  } else if (slot.blocks <= room || room < 2) {
+    if (room < 2) slot.start += room;
+    slot.head = (slot.blocks + 1) >> 1;
+  } else {
+    slot.head = min(room, min(kMmaBlocks, slot.blocks - 2));
+    slot.start += room - slot.head;
+  }
+  return slot;
+}
+
+// Leading blocks of `before` that lie where `slot`, the unit after it, has its accumulator.
+__device__ __forceinline__ int blocks_shared(const AccSlot& before, const AccSlot& slot) {
+  return max(0, slot.start + slot.blocks - kRingBlocks - before.start);
+}
+
 // The same unit with every field taken from lane 0 (all lanes hold the same values already).
 __device__ __forceinline__ UnitInfo warp_uniform(UnitInfo info) {
   info.expert = __shfl_sync(0xffffffffu, info.expert, 0);
@@ -214,12 +263,13 @@ __device__ __forceinline__ UnitInfo warp_uniform(UnitInfo info) {
 
 // kPlanes (an instance of the int8 kernel; W8A16 in its fixed-point form): every route arrives as two int8 token rows,
 // the high plane at row 2p and the low plane at row 2p + 1 of its 16-bit fixed-point activations, so a work item of r
-// routes has 2r token rows (at most 128 routes) and accumulator columns (2j, 2j + 1) belong to route j: the exact
+// routes has 2r token rows (at most 160 routes) and accumulator columns (2j, 2j + 1) belong to route j: the exact
 // integer dot product is 256 * column(2j) + column(2j + 1) (common.cuh: dequantize_planes).  Work items are given in
 // routes; loads, the MMA's N and the epilogue count plane rows.
 template <bool kInt8, bool kGateUp, bool kDense, bool kPlanes = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_constant__ CUtensorMap token_map,
+                              const __grid_constant__ CUtensorMap token_map_mid, const __grid_constant__ CUtensorMap token_map_full,
                               GroupedGemmArgs args) {
   static_assert(!kPlanes || (kInt8 && !kDense), "the two-plane form is an instance of the int8 grouped kernel");
   constexpr int kElemBytes = kInt8 ? 1 : 2;
@@ -254,7 +304,8 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
     }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(&ctl->acc_full[b], 1);
-      ptx::mbar_init(&ctl->acc_empty[b], 2 * kEpilogueWarps);  // the epilogue warps of both CTAs
+      ptx::mbar_init(&ctl->acc_part[b], 2 * kEpilogueWarps);  // the epilogue warps of both CTAs
+      ptx::mbar_init(&ctl->acc_empty[b], 2 * kEpilogueWarps);
     }
     ctl->abort_flag = 0;
     ptx::fence_barrier_init();
@@ -280,17 +331,28 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
       if (issuer) {
         ptx::prefetch_tensormap(&weight_map);
         ptx::prefetch_tensormap(&token_map);
+        ptx::prefetch_tensormap(&token_map_mid);
+        ptx::prefetch_tensormap(&token_map_full);
       }
       const uint32_t full_leader0 = map_to_cta(ptx::smem_u32(&ctl->full[0]), 0);
       int stage = 0;
       uint32_t phase = 0;
       int issued = 0;
       UnitInfo cur = warp_uniform(load_unit(args.items, first_unit, units, n_blocks, kRowsPerRoute));
+      int ring_end = 0;
       for (int64_t unit = first_unit; unit < units; unit += unit_stride) {
         const UnitInfo next = warp_uniform(load_unit(args.items, unit + unit_stride, units, n_blocks, kRowsPerRoute));  // in flight during this unit
-        // The MMA takes the first N/2 token rows from the leader's tile and the other N/2 from the follower's.
-        const int mma_n = min(kPairTokens, (cur.rows + 31) & ~31);
-        const int token_row = cur.row0 + (mma_n / 2) * static_cast<int>(cta);
+        // An MMA of N columns takes its first N/2 token rows from the leader's tile and the other N/2 from the follower's:
+        // 16 rows per CTA and block.  One box brings the rows of a one-MMA unit, up to the next box size (a few
+        // boxes of exactly its rows move less and take longer: about 512 rows per expert, 16384 tokens, 8087 -> 8216 us);
+        // the two halves of a larger unit are laid out by boxes of 64 and 16 rows.
+        const AccSlot slot = place_unit(ring_end, cur.rows);
+        ring_end = slot.start + slot.blocks;
+        const int tail = slot.blocks - slot.head;
+        const int head_row = cur.row0 + slot.head * kBoxTokens * static_cast<int>(cta);
+        const int tail_row = cur.row0 + slot.head * 32 + tail * kBoxTokens * static_cast<int>(cta);
+        const int loaded = tail > 0 ? slot.blocks : slot.head <= kMidBox ? kMidBox : kFullBox;
+        const uint32_t stage_tx = 2u * (kWeightBytes + static_cast<uint32_t>(loaded) * kBoxTokens * kBlockKBytes);
         const int channel0 = cur.block * kChannelsPerUnit + (kChannelsPerUnit / 2) * static_cast<int>(cta);
         const int weight_row = cur.expert * n_total + channel0;  // down
         const int group = channel0 >> 4;                         // gate_up: 16-channel group
@@ -303,7 +365,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
           } else {
             const uint32_t dst = smem_base + static_cast<uint32_t>(stage) * kStageBytes;
             const uint32_t bar = full_leader0 + 8u * static_cast<uint32_t>(stage);
-            if (leader) ptx::mbar_arrive_expect_tx(&ctl->full[stage], 2 * kStageBytes);
+            if (leader) ptx::mbar_arrive_expect_tx(&ctl->full[stage], stage_tx);
             const int x = kb * kBlockKElems;
             if constexpr (kGateUp) {
               if (args.gate_up_one_box) {
@@ -318,7 +380,20 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
             } else {
               tma_load_2d_pair(dst, &weight_map, bar, x, weight_row);
             }
-            tma_load_2d_pair(dst + kRowsPerCta * kBlockKBytes, &token_map, bar, x, token_row);
+            const uint32_t tokens = dst + kWeightBytes;
+            auto load_tokens = [&](uint32_t to, int blocks, int row) {
+              int b = 0;
+              for (; b + kMidBox <= blocks; b += kMidBox) {
+                tma_load_2d_pair(to + b * kBoxTokens * kBlockKBytes, &token_map_mid, bar, x, row + b * kBoxTokens);
+              }
+              for (; b < blocks; ++b) tma_load_2d_pair(to + b * kBoxTokens * kBlockKBytes, &token_map, bar, x, row + b * kBoxTokens);
+            };
+            if (tail == 0) {
+              tma_load_2d_pair(tokens, slot.head <= kMidBox ? &token_map_mid : &token_map_full, bar, x, head_row);
+            } else {
+              load_tokens(tokens, slot.head, head_row);
+              load_tokens(tokens + slot.head * kBoxTokens * kBlockKBytes, tail, tail_row);
+            }
           }
           ++issued;
           if (++stage == kStages) {
@@ -355,7 +430,8 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
       const uint32_t desc_hi = static_cast<uint32_t>(1024 >> 4) | (1u << 14) | (2u << 29);
       const uint32_t a_lo_stage0 = ((smem_base & 0x3ffffu) >> 4) | (1u << 16);
       constexpr uint32_t kStageStep = kStageBytes >> 4;
-      constexpr uint32_t kTokenStep = (kRowsPerCta * kBlockKBytes) >> 4;
+      constexpr uint32_t kTokenStep = kWeightBytes >> 4;
+      constexpr uint32_t kBlockStep = (kBoxTokens * kBlockKBytes) >> 4;  // one block's token rows in a CTA's tile
       const uint32_t empty_c0 = map_to_cta(ptx::smem_u32(&ctl->empty[0]), 0);
       const uint32_t empty_c1 = map_to_cta(ptx::smem_u32(&ctl->empty[0]), 1);
       const uint32_t accfull_c0 = map_to_cta(ptx::smem_u32(&ctl->acc_full[0]), 0);
@@ -365,6 +441,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
       uint32_t a_lo = a_lo_stage0;
       int local = 0;
       UnitInfo cur = load_unit(args.items, first_unit, units, n_blocks, kRowsPerRoute);
+      AccSlot before = {0, 0, 0};
       for (int64_t unit = first_unit; unit < units; unit += unit_stride, ++local) {
         const UnitInfo next = load_unit(args.items, unit + unit_stride, units, n_blocks, kRowsPerRoute);
         const uint32_t buffer = static_cast<uint32_t>(local) & 1u;
@@ -372,32 +449,56 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
         // N follows the rows this unit really has (a multiple of 32 for two-SM MMAs).  The row count comes from a global
         // load; the shuffle tells the compiler that every lane holds the same value.
         const int unit_rows = __shfl_sync(0xffffffffu, cur.rows, 0);
-        const int mma_n = min(kPairTokens, (unit_rows + 31) & ~31);
-        const uint32_t idesc = ptx::make_instr_desc(kInt8, 2 * kRowsPerCta, mma_n);
+        const AccSlot slot = place_unit(before.start + before.blocks, unit_rows);
+        const int tail = __shfl_sync(0xffffffffu, slot.blocks - slot.head, 0);
+        const uint32_t idesc_head = __shfl_sync(0xffffffffu, ptx::make_instr_desc(kInt8, 2 * kRowsPerCta, 32 * slot.head), 0);
+        const uint32_t idesc_tail = __shfl_sync(0xffffffffu, ptx::make_instr_desc(kInt8, 2 * kRowsPerCta, 32 * tail), 0);
+        // The unit two before this one has left tensor memory, and the one before it the blocks that this one takes over.
         ptx::mbar_wait(&ctl->acc_empty[buffer], (use & 1u) ^ 1u, abort_flag, status, 12);
+        if (local > 0 && blocks_shared(before, slot) > 0) {
+          ptx::mbar_wait(&ctl->acc_part[buffer ^ 1u], (static_cast<uint32_t>(local - 1) >> 1) & 1u, abort_flag, status, 15);
+        }
+        before = slot;
         ptx::tcgen05_fence_after();
-        const uint32_t acc = tmem_base + buffer * kAccColumns;
-        uint32_t accumulate = 0;
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          ptx::mbar_wait(&ctl->full[stage], phase, abort_flag, status, 13);
-          ptx::tcgen05_fence_after();
-          if (issuer) {
-            if (!FMOE_DIAG_BIT(args, 4)) {
+        const uint32_t acc_head = __shfl_sync(0xffffffffu, tmem_base + 32u * static_cast<uint32_t>(slot.start & (kRingBlocks - 1)), 0);
+        const uint32_t acc_tail =
+            __shfl_sync(0xffffffffu, tmem_base + 32u * static_cast<uint32_t>((slot.start + slot.head) & (kRingBlocks - 1)), 0);
+        const uint32_t tail_step = __shfl_sync(0xffffffffu, kTokenStep + kBlockStep * static_cast<uint32_t>(slot.head), 0);
+        // One loop per form: the usual one carries nothing of the other.
+        auto main_loop = [&](auto tail_tag) {
+          uint32_t accumulate = 0;
+          for (int kb = 0; kb < k_blocks; ++kb) {
+            ptx::mbar_wait(&ctl->full[stage], phase, abort_flag, status, 13);
+            ptx::tcgen05_fence_after();
+            if (issuer) {
+              if (!FMOE_DIAG_BIT(args, 4)) {
 #pragma unroll
-              for (uint32_t ks = 0; ks < kBlockKBytes / kUmmaKBytes; ++ks) {
-                umma_pair<kInt8>(acc, a_lo + 2u * ks, a_lo + kTokenStep + 2u * ks, desc_hi, idesc, ks == 0 ? accumulate : 1u);
+                for (uint32_t ks = 0; ks < kBlockKBytes / kUmmaKBytes; ++ks) {
+                  umma_pair<kInt8>(acc_head, a_lo + 2u * ks, a_lo + kTokenStep + 2u * ks, desc_hi, idesc_head, ks == 0 ? accumulate : 1u);
+                }
+                if constexpr (decltype(tail_tag)::value) {
+#pragma unroll
+                  for (uint32_t ks = 0; ks < kBlockKBytes / kUmmaKBytes; ++ks) {
+                    umma_pair<kInt8>(acc_tail, a_lo + 2u * ks, a_lo + tail_step + 2u * ks, desc_hi, idesc_tail, ks == 0 ? accumulate : 1u);
+                  }
+                }
               }
+              tcgen05_commit_pair(empty_c0 + 8u * static_cast<uint32_t>(stage));
+              tcgen05_commit_pair(empty_c1 + 8u * static_cast<uint32_t>(stage));
             }
-            tcgen05_commit_pair(empty_c0 + 8u * static_cast<uint32_t>(stage));
-            tcgen05_commit_pair(empty_c1 + 8u * static_cast<uint32_t>(stage));
+            accumulate = 1;
+            a_lo += kStageStep;
+            if (++stage == kStages) {
+              stage = 0;
+              phase ^= 1u;
+              a_lo = a_lo_stage0;
+            }
           }
-          accumulate = 1;
-          a_lo += kStageStep;
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1u;
-            a_lo = a_lo_stage0;
-          }
+        };
+        if (tail > 0) {
+          main_loop(TrueTag{});
+        } else {
+          main_loop(FalseTag{});
         }
         if (issuer) {
           tcgen05_commit_pair(accfull_c0 + 8u * buffer);
@@ -412,7 +513,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
     const int chunk_first = (warp - 2) >> 2;         // warps sharing a lane quarter take 32-column chunks round-robin
     constexpr int kChunkStep = kEpilogueWarps / 4;
     const int lane_in_tile = quarter * 32 + lane;    // TMEM lane = A row of this CTA
-    const int tid = static_cast<int>(threadIdx.x) - 64;  // threads 0..255 each stage the metadata of one column
+    const int tid = static_cast<int>(threadIdx.x) - 64;  // threads 0..255 stage the metadata of column tid and, below 64, of column 256 + tid
     const int n_out = args.n_out;
     const bool native = args.numerics == FMOE_NUMERICS_NATIVE;
     const float limit = args.swiglu_limit;
@@ -422,6 +523,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
     // Output channel of this thread inside the unit's channel block.
     const int channel_in_unit = kGateUp ? 64 * static_cast<int>(cta) + 16 * quarter + (lane & 15)
                                         : kRowsPerCta * static_cast<int>(cta) + lane_in_tile;
+    const uint32_t acc_part_leader = map_to_cta(ptx::smem_u32(&ctl->acc_part[0]), 0);
     const uint32_t acc_empty_leader = map_to_cta(ptx::smem_u32(&ctl->acc_empty[0]), 0);
     const uint32_t acc_lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t* exp_table = ctl->exp_table;
@@ -429,23 +531,26 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
     // Per-unit values: the column metadata in shared memory and this thread's weight scales in registers.  Both
     // are fetched while the previous unit is being finished.
     struct ThreadUnit {
-      float column_scale;      // of column `tid`
-      uint64_t column_rowptr;  // of column `tid`: byte address of its output row (down / dense)
+      float column_scale[2];      // of columns `tid` and `tid` + 256
+      uint64_t column_rowptr[2];  // of the same columns: byte address of the output row (down / dense)
       float scale_gate, scale_up, bias;
     };
     auto fetch = [&](const UnitInfo& info, bool valid) {
-      ThreadUnit t = {0.0f, 0ull, kInt8 ? 1.0f : 0.0f, kInt8 ? 1.0f : 0.0f, 0.0f};
+      ThreadUnit t = {{0.0f, 0.0f}, {0ull, 0ull}, kInt8 ? 1.0f : 0.0f, kInt8 ? 1.0f : 0.0f, 0.0f};
       if (!valid) return t;
-      if (tid < info.rows) {
-        const int row = (info.row0 + tid) / kRowsPerRoute;  // sorted position of the column's route
-        if (kInt8) t.column_scale = args.a_scale[row];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int column = tid + 256 * i;
+        if (column >= info.rows) break;
+        const int row = (info.row0 + column) / kRowsPerRoute;  // sorted position of the column's route
+        if (kInt8) t.column_scale[i] = args.a_scale[row];
         if constexpr (kDense) {
-          t.column_rowptr = reinterpret_cast<uint64_t>(args.dense_out) + static_cast<uint64_t>(row) * n_out * (args.dense_out_bf16 ? 2 : 4);
+          t.column_rowptr[i] = reinterpret_cast<uint64_t>(args.dense_out) + static_cast<uint64_t>(row) * n_out * (args.dense_out_bf16 ? 2 : 4);
         } else if constexpr (!kGateUp) {
-          t.column_rowptr = args.row_out_ptrs != nullptr
-                                ? args.row_out_ptrs[row]
-                                : reinterpret_cast<uint64_t>(args.route_out) +
-                                      static_cast<uint64_t>(args.sorted_routes[row]) * n_out * (args.route_out_bf16 ? 2 : 4);
+          t.column_rowptr[i] = args.row_out_ptrs != nullptr
+                                   ? args.row_out_ptrs[row]
+                                   : reinterpret_cast<uint64_t>(args.route_out) +
+                                         static_cast<uint64_t>(args.sorted_routes[row]) * n_out * (args.route_out_bf16 ? 2 : 4);
         }
       }
       const int n = info.block * kChannelsPerUnit + channel_in_unit;
@@ -499,13 +604,19 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
     UnitInfo cur = load_unit(args.items, first_unit, units, n_blocks, kRowsPerRoute);
     UnitInfo next = load_unit(args.items, first_unit + unit_stride, units, n_blocks, kRowsPerRoute);
     ThreadUnit mine = fetch(cur, first_unit < units);
-    if (tid < 256) {
-      ctl->meta[0].scale[tid] = mine.column_scale;
-      ctl->meta[0].rowptr[tid] = mine.column_rowptr;
-    }
+    auto publish = [&](ColumnMeta* meta, const ThreadUnit& t) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (tid >= (i == 0 ? 256 : kMaxTokenRows - 256)) break;
+        meta->scale[tid + 256 * i] = t.column_scale[i];
+        meta->rowptr[tid + 256 * i] = t.column_rowptr[i];
+      }
+    };
+    publish(&ctl->meta[0], mine);
     epilogue_bar_sync();
 
     int local = 0;
+    AccSlot slot = place_unit(0, cur.rows);
     for (int64_t unit = first_unit; unit < units; unit += unit_stride, ++local) {
       const uint32_t buffer = static_cast<uint32_t>(local) & 1u;
       const uint32_t use = static_cast<uint32_t>(local) >> 1;
@@ -523,10 +634,20 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
 
       ptx::mbar_wait(&ctl->acc_full[buffer], use & 1u, abort_flag, status, 14);
       ptx::tcgen05_fence_after();
-      const uint32_t acc = acc_lane_base + buffer * kAccColumns;
+      // The next unit's accumulator may start on this one's first blocks: they are released as soon as they are read.
+      const AccSlot next_slot = place_unit(slot.start + slot.blocks, next.rows);
+      const int handed_over = blocks_shared(slot, next_slot);
+      bool part_released = false;
+      auto release_part = [&]() {
+        part_released = true;
+        ptx::tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(acc_part_leader + 8u * buffer);
+      };
       for (int chunk = chunk_first; chunk < chunks; chunk += kChunkStep) {
+        if (!part_released && chunk >= handed_over) release_part();
         uint32_t v[32];
-        tmem_ld_x32(acc + static_cast<uint32_t>(chunk * 32), v);
+        tmem_ld_x32(acc_lane_base + 32u * static_cast<uint32_t>((slot.start + chunk) & (kRingBlocks - 1)), v);
         ptx::tmem_ld_wait();
         const int col0 = chunk * 32;
         const bool fast = block_full && col0 + 32 <= rows && dump == nullptr;  // warp-uniform
@@ -645,19 +766,17 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
           dispatch(fast, body);
         }
       }
+      if (!part_released) release_part();
       ptx::tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(acc_empty_leader + 8u * buffer);
 
       // Publish the next unit's column metadata.  Nobody still reads that buffer: it belonged to the previous
       // unit, which every warp left before the barrier at the end of the previous iteration.
-      if (tid < 256) {
-        ColumnMeta* meta_next = &ctl->meta[(local + 1) & 1];
-        meta_next->scale[tid] = upcoming.column_scale;
-        meta_next->rowptr[tid] = upcoming.column_rowptr;
-      }
+      publish(&ctl->meta[(local + 1) & 1], upcoming);
       epilogue_bar_sync();
       mine = upcoming;
+      slot = next_slot;
       cur = next;
       next = after;
     }
@@ -733,7 +852,7 @@ cudaError_t launch_pair(const GroupedGemmArgs& args, cudaStream_t stream) {
     if (err != cudaSuccess) return err;
     configured.mark(device);
   }
-  CUtensorMap weight_map, token_map;
+  CUtensorMap weight_map, token_map, token_map_mid, token_map_full;
   GroupedGemmArgs launch_args = args;
   bool weights_ok;
   if (kGateUp) {
@@ -748,7 +867,9 @@ cudaError_t launch_pair(const GroupedGemmArgs& args, cudaStream_t stream) {
     weights_ok = make_sw128_map(&weight_map, args.weights, kInt8, static_cast<uint64_t>(args.experts) * args.n_out, args.k, kRowsPerCta);
   }
   const uint64_t token_rows = static_cast<uint64_t>(args.total_rows) * (kPlanes ? 2 : 1);
-  if (!weights_ok || !make_sw128_map(&token_map, args.a_rows, kInt8, token_rows, args.k, kRowsPerCta)) {
+  if (!weights_ok || !make_sw128_map(&token_map, args.a_rows, kInt8, token_rows, args.k, kBoxTokens) ||
+      !make_sw128_map(&token_map_mid, args.a_rows, kInt8, token_rows, args.k, kMidBox * kBoxTokens) ||
+      !make_sw128_map(&token_map_full, args.a_rows, kInt8, token_rows, args.k, kFullBox * kBoxTokens)) {
     return cudaErrorInvalidValue;
   }
   const int sms = sm_count_of_current_device();
@@ -757,23 +878,17 @@ cudaError_t launch_pair(const GroupedGemmArgs& args, cudaStream_t stream) {
   int64_t pairs = static_cast<int64_t>(args.max_items) * n_blocks;
   if (pairs > sms / 2) pairs = sms / 2;
   if (pairs <= 0) return cudaSuccess;
-  kernel<<<static_cast<unsigned>(2 * pairs), kThreads, kSmemBytes, stream>>>(weight_map, token_map, launch_args);
+  kernel<<<static_cast<unsigned>(2 * pairs), kThreads, kSmemBytes, stream>>>(weight_map, token_map, token_map_mid, token_map_full, launch_args);
   return cudaGetLastError();
 }
 
 }  // namespace
 
-// gate_up stages 16-channel groups through its 5-D tensor map.
-bool umma_pair_supported(bool gate_up, int n_out, int64_t output_rows) {
-  (void)output_rows;
-  return !gate_up || n_out % 16 == 0;
-}
-
 cudaError_t launch_umma_pair_grouped_gemm(const GroupedGemmArgs& args, bool int8, bool gate_up, cudaStream_t stream) {
   if (args.max_items <= 0 || args.total_rows <= 0) return cudaSuccess;
-  if (!umma_pair_supported(gate_up, args.n_out, args.total_rows)) return cudaErrorInvalidValue;
+  if (gate_up && args.n_out % 16 != 0) return cudaErrorInvalidValue;  // gate_up stages 16-channel groups
   if (args.w8a16 == 2) {
-    // W8A16 in its fixed-point form: int8 kernel, two token rows per route, work items of at most 128 routes.
+    // W8A16 in its fixed-point form: int8 kernel, two token rows per route, work items of at most 160 routes.
     if (!int8 || args.dense_out != nullptr || args.a_scale == nullptr) return cudaErrorInvalidValue;
     return gate_up ? launch_pair<true, true, false, true>(args, stream) : launch_pair<true, false, false, true>(args, stream);
   }

@@ -789,7 +789,7 @@ cudaError_t launch_umma_grouped_gemm(const GroupedGemmArgs& caller_args, bool in
     // int8 weights, activations as two int8 planes per route: the int8 one-SM kernel with paired accumulator columns;
     // row_tile counts plane rows (two per route).
     if (!int8 || args.dense_out != nullptr || args.w_scale == nullptr || args.a_scale == nullptr) return cudaErrorInvalidValue;
-    if (args.row_tile == kPairRowTile) return launch_umma_pair_grouped_gemm(args, true, gate_up, stream);  // items of at most 128 routes
+    if (args.row_tile == kPairRowTile) return launch_umma_pair_grouped_gemm(args, true, gate_up, stream);  // items of at most 160 routes
     return gate_up ? launch_tile<true, true, false, true>(args, stream) : launch_tile<true, false, false, true>(args, stream);
   }
   if (args.w8a16) {
@@ -798,10 +798,7 @@ cudaError_t launch_umma_grouped_gemm(const GroupedGemmArgs& caller_args, bool in
     if (args.row_tile > 128) return cudaErrorInvalidValue;  // the caller caps W8A16 work items at 128 rows
     return gate_up ? launch_tile<false, true, true>(args, stream) : launch_tile<false, false, true>(args, stream);
   }
-  if (args.row_tile == kPairRowTile) {
-    if (umma_pair_supported(gate_up, args.n_out, args.total_rows)) return launch_umma_pair_grouped_gemm(args, int8, gate_up, stream);
-    args.row_tile = 256;  // same 256-row work items, one-SM kernel
-  }
+  if (args.row_tile == kPairRowTile) return launch_umma_pair_grouped_gemm(args, int8, gate_up, stream);
   if (args.dense_out != nullptr) return cudaErrorInvalidValue;  // dense products: the two-SM kernel or dense_gemm.cu
   if (int8) return gate_up ? launch_tile<true, true>(args, stream) : launch_tile<true, false>(args, stream);
   return gate_up ? launch_tile<false, true>(args, stream) : launch_tile<false, false>(args, stream);

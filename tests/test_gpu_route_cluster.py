@@ -11,7 +11,7 @@ from oracle import oracle
 
 pytestmark = pytest.mark.gpu
 
-SPLIT_ROWS, BIG_ROWS = 64, 256
+SPLIT_ROWS, BIG_ROWS = 64, 320
 
 
 def _covered_rows(items: torch.Tensor, rows_most: int) -> dict:
