@@ -322,8 +322,8 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   } else if (f.rows_mode && f.int8) {
     // int8 rows travel as H bytes: gather them as H/2 16-bit words, then their scales.
     error = fmoe::launch_gather_rows(static_cast<const uint16_t*>(f.x), routes, f.hidden / 2, sorted_routes, 1, valid_rows,
-                                     reinterpret_cast<uint16_t*>(base + layout.a_rows), stream);
-    if (error == cudaSuccess) error = fmoe::launch_gather_scalars(f.rows_scale, routes, sorted_routes, valid_rows, a_scale, stream);
+                                     reinterpret_cast<uint16_t*>(base + layout.a_rows), stream, true);
+    if (error == cudaSuccess) error = fmoe::launch_gather_scalars(f.rows_scale, routes, sorted_routes, valid_rows, a_scale, stream, true);
   } else if (planes) {
     error = fmoe::launch_split_tokens_scatter_planes(static_cast<const uint16_t*>(f.x), f.tokens, f.hidden, f.top_k,
                                                      reinterpret_cast<const int*>(base + layout.route_pos),
@@ -333,8 +333,9 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
                                                  reinterpret_cast<const int*>(base + layout.route_pos), cfg.numerics,
                                                  reinterpret_cast<int8_t*>(base + layout.a_rows), a_scale, stream);
   } else {
-    error = fmoe::launch_gather_rows(static_cast<const uint16_t*>(f.x), routes, f.hidden, sorted_routes, f.top_k, valid_rows,
-                                     reinterpret_cast<uint16_t*>(base + layout.a_rows), stream);
+    error = fmoe::launch_gather_tokens_scatter(static_cast<const uint16_t*>(f.x), f.tokens, f.hidden, f.top_k,
+                                               reinterpret_cast<const int*>(base + layout.route_pos),
+                                               reinterpret_cast<uint16_t*>(base + layout.a_rows), stream);
   }
   if (error != cudaSuccess) return cuda_fail(error, "activation quantise/gather");
   mark(FMOE_STAGE_QUANT_IN + 1);
@@ -376,6 +377,7 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
     fmoe::GroupedGemmArgs big = gu;
     big.items = items_gu_big;
     big.item_count_word = fmoe::kStatusItemsC;
+    big.beside = 1;
     big.row_tile = fmoe::kPairRowTile;
     error = fmoe::launch_umma_grouped_gemm(big, int8_gemm, true, stream);
   }
@@ -385,7 +387,7 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   const void* down_rows = y;
   if (f.int8) {
     int8_t* yq = reinterpret_cast<int8_t*>(base + layout.yq);
-    error = fmoe::launch_quantize_rows(y, routes, f.inter, nullptr, 1, valid_rows, cfg.numerics, 0, yq, y_scale, stream);
+    error = fmoe::launch_quantize_rows(y, routes, f.inter, nullptr, 1, valid_rows, cfg.numerics, 0, yq, y_scale, stream, true);
     if (error != cudaSuccess) return cuda_fail(error, "intermediate quantise");
     down_rows = yq;
   } else if (planes) {
@@ -423,6 +425,7 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
     fmoe::GroupedGemmArgs big = dn;
     big.items = items_dn_big;
     big.item_count_word = fmoe::kStatusItemsD;
+    big.beside = 1;
     big.row_tile = fmoe::kPairRowTile;
     error = fmoe::launch_umma_grouped_gemm(big, int8_gemm, false, stream);
   }
@@ -431,11 +434,12 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
 
   if (!f.rows_mode && compact_rows) {
     error = fmoe::launch_merge_bf16_rows(reinterpret_cast<const uint16_t*>(route_out), f.topk_weights, f.tokens, f.top_k, f.hidden,
-                                         f.int8 ? 0 : 1, static_cast<uint16_t*>(out), stream, reinterpret_cast<const int*>(base + layout.route_pos));
+                                         f.int8 ? 0 : 1, static_cast<uint16_t*>(out), stream, reinterpret_cast<const int*>(base + layout.route_pos),
+                                         true);
     if (error != cudaSuccess) return cuda_fail(error, "top-k merge");
   } else if (!f.rows_mode) {
     error = fmoe::launch_merge(route_out, f.topk_weights, f.tokens, f.top_k, f.hidden, f.int8 ? 0 : 1, static_cast<uint16_t*>(out), stream,
-                               reinterpret_cast<const int*>(base + layout.route_pos));
+                               reinterpret_cast<const int*>(base + layout.route_pos), true);
     if (error != cudaSuccess) return cuda_fail(error, "top-k merge");
   }
   mark(FMOE_STAGE_MERGE + 1);

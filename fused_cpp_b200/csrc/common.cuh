@@ -36,9 +36,9 @@ __device__ __forceinline__ void raise_error(int* status, int code, int detail) {
 // inside one expert, the row tiles of a channel block are adjacent: CTAs that run side by side then read the
 // same weight tile at the same time and the second read is served by L2 instead of HBM.  items[4*i+3] packs
 // the first item of the item's expert (20 bits) and that expert's tile count.
-__device__ __forceinline__ void decode_unit(const int* __restrict__ items, int64_t unit, int n_blocks, int* item, int* block) {
+__device__ __forceinline__ void decode_unit(const int* items, int64_t unit, int n_blocks, int* item, int* block) {
   const int guess = static_cast<int>(unit / n_blocks);
-  const int packed = items[4 * guess + 3];
+  const int packed = __ldcg(items + 4 * guess + 3);
   const int first = packed & 0xfffff;
   const int tiles = packed >> 20;
   const int64_t local = unit - static_cast<int64_t>(first) * n_blocks;

@@ -43,7 +43,7 @@ cudaError_t launch_items_from_counts(int experts, const int* counts, const int* 
 // valid_rows (nullable, device): rows at or beyond *valid_rows are skipped (routes dropped for a bad id).
 cudaError_t launch_quantize_rows(const uint16_t* x, int64_t out_rows, int cols, const int* sorted_routes, int top_k,
                                  const int* valid_rows, int numerics, int weight_mode, int8_t* q, float* scale,
-                                 cudaStream_t stream);
+                                 cudaStream_t stream, bool chained = false);
 // Quantise every token row once and write it to the sorted positions of its top_k routes
 // (route_pos[t*top_k+slot], -1 = dropped): same bits as quantising per route, one read of x per token.
 cudaError_t launch_quantize_tokens_scatter(const uint16_t* x, int64_t tokens, int cols, int top_k, const int* route_pos,
@@ -62,11 +62,15 @@ cudaError_t launch_quantize_rows_dense(const void* x, int x_is_bf16, int64_t row
                                        cudaStream_t stream);
 // Copy bf16 rows into expert-sorted order: out[p] = x[sorted_routes[p] / top_k].
 cudaError_t launch_gather_rows(const uint16_t* x, int64_t out_rows, int cols, const int* sorted_routes, int top_k,
-                               const int* valid_rows, uint16_t* out, cudaStream_t stream);
+                               const int* valid_rows, uint16_t* out, cudaStream_t stream, bool chained = false);
+
+// The same with one CTA per token, which stores its row to the sorted positions of its routes (route_pos, -1 = dropped).
+cudaError_t launch_gather_tokens_scatter(const uint16_t* x, int64_t tokens, int cols, int top_k, const int* route_pos, uint16_t* out,
+                                         cudaStream_t stream);
 
 // out[i] = in[index[i]] for fp32 scalars (activation scales following their rows).
 cudaError_t launch_gather_scalars(const float* in, int64_t n, const int* index, const int* valid_rows, float* out,
-                                  cudaStream_t stream);
+                                  cudaStream_t stream, bool chained = false);
 
 // ---- ep.cu: helpers of the expert-parallel dispatch / combine
 // dest[i] = ids[i] / experts_per_rank as int64 (ids outside [0, experts_global) become -1).  With
@@ -117,10 +121,10 @@ cudaError_t launch_router_topk(const float* logits, const float* selection_bias,
 // BF16: pairwise tree for K in {2,4,6,8}, chain otherwise.
 // route_pos (nullable): sorted position of every flat route, -1 = dropped by the route build; such rows count as zeros.
 cudaError_t launch_merge(const float* route_out, const float* topk_weights, int64_t tokens, int top_k, int hidden,
-                         int tree, uint16_t* out, cudaStream_t stream, const int* route_pos = nullptr);
+                         int tree, uint16_t* out, cudaStream_t stream, const int* route_pos = nullptr, bool chained = false);
 // Same with the route rows stored as bf16 (opt-in compact return of the expert-parallel path).
 cudaError_t launch_merge_bf16_rows(const uint16_t* route_out, const float* topk_weights, int64_t tokens, int top_k, int hidden,
-                                   int tree, uint16_t* out, cudaStream_t stream, const int* route_pos = nullptr);
+                                   int tree, uint16_t* out, cudaStream_t stream, const int* route_pos = nullptr, bool chained = false);
 
 // ---- grouped GEMM, shared argument block
 struct GroupedGemmArgs {
@@ -164,6 +168,9 @@ struct GroupedGemmArgs {
   int w8a16;                 // int8 weights with w_scale and 16-bit activations: 1 = bf16 rows, the one-SM kernel widens the weight
                              // tile to bf16; 2 = two int8 planes per route (a_rows holds 2 * total_rows rows, a_scale one
                              // scale per route, row_tile counts plane rows), the int8 one-SM kernel pairs accumulator columns
+  // Two-SM kernel: the kernel in front is the one-SM launch of the same stage (the thin experts' items), which waited for all
+  // that this one reads and writes other rows: no wait before the work, SM pairs are taken as they fall free, one at the end.
+  int beside;
   int gate_up_one_box;       // two-SM gate_up: the weight rows of a stage arrive as one 16 KB TMA box (set by the launcher)
   int route_out_bf16;        // the result rows are stored as bf16 (2 bytes per channel, rows 2 * n_out bytes apart) instead of fp32
   // Diagnostic build only (compiled with -DFMOE_DIAG, the separate libfused_moe_b200_diag.so; the product library
@@ -176,8 +183,8 @@ struct GroupedGemmArgs {
 __device__ __forceinline__ int gate_channel(const GroupedGemmArgs& args, int n) { return args.interleaved ? 2 * n : n; }
 __device__ __forceinline__ int up_channel(const GroupedGemmArgs& args, int n) { return args.interleaved ? 2 * n + 1 : n + args.n_out; }
 __device__ __forceinline__ float load_expert_bias(const GroupedGemmArgs& args, int64_t index) {
-  if (!args.bias_bf16) return static_cast<const float*>(args.expert_bias)[index];
-  return __uint_as_float(static_cast<uint32_t>(static_cast<const uint16_t*>(args.expert_bias)[index]) << 16);
+  if (!args.bias_bf16) return __ldcg(static_cast<const float*>(args.expert_bias) + index);
+  return __uint_as_float(static_cast<uint32_t>(__ldcg(static_cast<const unsigned short*>(args.expert_bias) + index)) << 16);
 }
 #endif
 
@@ -186,6 +193,47 @@ __device__ __forceinline__ float load_expert_bias(const GroupedGemmArgs& args, i
 #define FMOE_DIAG_BIT(args, bit) (((args).diag & (bit)) != 0)
 #else
 #define FMOE_DIAG_BIT(args, bit) false
+#endif
+
+#ifdef __CUDACC__
+// Launch, with `chained` as a programmatic dependent of the kernel before it in the stream.  The kernels of a forward pass
+// behind its first, an ordinary launch, are chained this way, under these rules (griddepcontrol, ptx.cuh):
+//   * every CTA calls grid_dependency_wait before it touches anything that the kernel before it reads or writes;
+//   * it calls launch_dependents (or ends) only after that.  A kernel that has started therefore knows that every kernel
+//     but the one right before it has completed: route lists and work items may be read before the wait by any kernel
+//     that is not the first behind the route build.  What is read before a wait
+//     is read through L2 (__ldcg): only the wait promises that an L1 line left by an earlier call is not found again;
+//   * what is read behind a wait is not reached through a const __restrict__ parameter: such loads count as invariant, and
+//     the compiler may move them in front of the wait;
+//   * a kernel that does not need the one before it (the second grouped GEMM of a split stage) waits before it ends.
+// Launch, prologue and the first weight loads of a kernel overlap the end of the one before it: one token of the 256-expert
+// layer 200 -> 181 us, 16 tokens of the 16-expert one 137 -> 119 us.  A kernel whose neighbour in front may be anybody's (the
+// first of a call, a stand-alone quantiser) is not chained.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, bool chained,
+                                  Args&&... args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
+// The same for the kernels that stream rows with a short-lived CTA per row; the last kernel parameter says whether the
+// launch is chained.  A grid of several waves is not: waiting costs every CTA of it about a microsecond (merge of 65536
+// rows: 302 us, chained 381 us) and hides one launch.
+constexpr uint64_t kChainedBlocks = 148 * 8;
+template <typename... Params, typename... Args>
+inline cudaError_t launch_streaming(void (*kernel)(Params...), dim3 grid, unsigned threads, cudaStream_t stream, bool chained, Args&&... args) {
+  const bool chain = chained && static_cast<uint64_t>(grid.x) * grid.y <= kChainedBlocks;
+  return launch_chained(kernel, grid, threads, 0, stream, chain, args..., chain);
+}
 #endif
 
 // Launch set-up that belongs to a device, not to the process: the opt-in to more than 48 KB of dynamic shared

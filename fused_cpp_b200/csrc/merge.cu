@@ -8,6 +8,7 @@
 // epilogue; this pass is a pure streaming read of fp32 rows with 16-byte loads.
 #include "common.cuh"
 #include "kernels.h"
+#include "ptx.cuh"
 
 namespace fmoe {
 
@@ -111,14 +112,18 @@ __device__ __forceinline__ void tree_merge8_bf16(const uint16_t* route_out, int6
 
 // The same merge over bf16 rows with eight channels per thread: one 16-byte load per slot, one 16-byte store.
 __global__ void __launch_bounds__(kMergeThreads)
-merge_bf16_rows8_kernel(const uint16_t* __restrict__ route_out, const float* __restrict__ topk_weights, const int* __restrict__ route_pos,
-                        int top_k, int hidden, int tree, uint16_t* __restrict__ out) {
+merge_bf16_rows8_kernel(const uint16_t* route_out, const float* topk_weights, const int* route_pos,
+                        int top_k, int hidden, int tree, uint16_t* __restrict__ out, bool chained) {
   __shared__ float weights[kMaxTopK];
   __shared__ bool present[kMaxTopK];
+  if (chained) {
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
+  }
   const int64_t token = blockIdx.x;
   if (threadIdx.x < top_k) {
-    weights[threadIdx.x] = topk_weights[token * top_k + threadIdx.x];
-    present[threadIdx.x] = route_pos == nullptr || route_pos[token * top_k + threadIdx.x] >= 0;
+    weights[threadIdx.x] = __ldcg(topk_weights + token * top_k + threadIdx.x);
+    present[threadIdx.x] = route_pos == nullptr || __ldcg(route_pos + token * top_k + threadIdx.x) >= 0;
   }
   __syncthreads();
   const int h = (blockIdx.y * kMergeThreads + threadIdx.x) * 8;
@@ -157,17 +162,21 @@ merge_bf16_rows8_kernel(const uint16_t* __restrict__ route_out, const float* __r
 
 template <bool kBf16Rows>
 __global__ void __launch_bounds__(kMergeThreads)
-merge_kernel(const void* __restrict__ route_out, const float* __restrict__ topk_weights, const int* __restrict__ route_pos, int top_k,
-             int hidden, int tree, uint16_t* __restrict__ out) {
+merge_kernel(const void* route_out, const float* topk_weights, const int* route_pos, int top_k,
+             int hidden, int tree, uint16_t* __restrict__ out, bool chained) {
   __shared__ float weights[kMaxTopK];
   __shared__ bool present[kMaxTopK];
+  if (chained) {
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
+  }
   // Tokens ride on grid.x (up to 2^31 - 1 blocks), the few chunks of a row on grid.y (at most 65535).
   const int64_t token = blockIdx.x;
   if (threadIdx.x < top_k) {
-    weights[threadIdx.x] = topk_weights[token * top_k + threadIdx.x];
+    weights[threadIdx.x] = __ldcg(topk_weights + token * top_k + threadIdx.x);
     // A route dropped by the route build (expert id out of range; reported in the status block) has no row: the
     // down GEMM never wrote it, so it counts as a row of zeros instead of whatever the workspace held.
-    present[threadIdx.x] = route_pos == nullptr || route_pos[token * top_k + threadIdx.x] >= 0;
+    present[threadIdx.x] = route_pos == nullptr || __ldcg(route_pos + token * top_k + threadIdx.x) >= 0;
   }
   __syncthreads();
   const int h = (blockIdx.y * kMergeThreads + threadIdx.x) * 4;
@@ -209,26 +218,23 @@ merge_kernel(const void* __restrict__ route_out, const float* __restrict__ topk_
 }  // namespace
 
 cudaError_t launch_merge(const float* route_out, const float* topk_weights, int64_t tokens, int top_k, int hidden,
-                         int tree, uint16_t* out, cudaStream_t stream, const int* route_pos) {
+                         int tree, uint16_t* out, cudaStream_t stream, const int* route_pos, bool chained) {
   if (tokens <= 0) return cudaSuccess;
   if (top_k > kMaxTopK) return cudaErrorInvalidValue;
   const dim3 grid(static_cast<unsigned>(tokens), (hidden / 4 + kMergeThreads - 1) / kMergeThreads);
-  merge_kernel<false><<<grid, kMergeThreads, 0, stream>>>(route_out, topk_weights, route_pos, top_k, hidden, tree, out);
-  return cudaGetLastError();
+  return launch_streaming(merge_kernel<false>, grid, kMergeThreads, stream, chained, route_out, topk_weights, route_pos, top_k, hidden, tree, out);
 }
 
 cudaError_t launch_merge_bf16_rows(const uint16_t* route_out, const float* topk_weights, int64_t tokens, int top_k, int hidden,
-                                   int tree, uint16_t* out, cudaStream_t stream, const int* route_pos) {
+                                   int tree, uint16_t* out, cudaStream_t stream, const int* route_pos, bool chained) {
   if (tokens <= 0) return cudaSuccess;
   if (top_k > kMaxTopK) return cudaErrorInvalidValue;
   if (hidden % 8 == 0) {
     const dim3 grid8(static_cast<unsigned>(tokens), (hidden / 8 + kMergeThreads - 1) / kMergeThreads);
-    merge_bf16_rows8_kernel<<<grid8, kMergeThreads, 0, stream>>>(route_out, topk_weights, route_pos, top_k, hidden, tree, out);
-    return cudaGetLastError();
+    return launch_streaming(merge_bf16_rows8_kernel, grid8, kMergeThreads, stream, chained, route_out, topk_weights, route_pos, top_k, hidden, tree, out);
   }
   const dim3 grid(static_cast<unsigned>(tokens), (hidden / 4 + kMergeThreads - 1) / kMergeThreads);
-  merge_kernel<true><<<grid, kMergeThreads, 0, stream>>>(route_out, topk_weights, route_pos, top_k, hidden, tree, out);
-  return cudaGetLastError();
+  return launch_streaming(merge_kernel<true>, grid, kMergeThreads, stream, chained, route_out, topk_weights, route_pos, top_k, hidden, tree, out);
 }
 
 }  // namespace fmoe

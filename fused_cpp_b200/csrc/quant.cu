@@ -59,13 +59,17 @@ __device__ __forceinline__ uint32_t pack4(const float* values, float operand, fl
 
 // cols % 16 == 0.  One CTA per output row.
 __global__ void __launch_bounds__(kQuantThreads)
-quantize_rows_kernel(const uint16_t* __restrict__ x, int cols, const int* __restrict__ sorted_routes, int top_k,
-                     const int* __restrict__ valid_rows, int numerics, int weight_mode, int8_t* __restrict__ q,
-                     float* __restrict__ scale_out) {
+quantize_rows_kernel(const uint16_t* x, int cols, const int* sorted_routes, int top_k,
+                     const int* valid_rows, int numerics, int weight_mode, int8_t* __restrict__ q,
+                     float* __restrict__ scale_out, bool chained) {
   __shared__ float smem[32];
+  if (chained) {
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
+  }
   const int64_t row = blockIdx.x;
-  if (valid_rows && row >= *valid_rows) return;  // rows of dropped (out-of-range) routes
-  const int64_t src_row = sorted_routes ? static_cast<int64_t>(sorted_routes[row] / top_k) : row;
+  if (valid_rows && row >= __ldcg(valid_rows)) return;  // rows of dropped (out-of-range) routes
+  const int64_t src_row = sorted_routes ? static_cast<int64_t>(__ldcg(sorted_routes + row) / top_k) : row;
   const uint4* src = reinterpret_cast<const uint4*>(x + src_row * cols);
   const int vec16 = cols >> 4;
   float local = 0.0f;
@@ -104,14 +108,18 @@ quantize_rows_kernel(const uint16_t* __restrict__ x, int cols, const int* __rest
 // Rows of a few KB (the 2048-column intermediate of the W8A8 layer) are too short to keep a 256-thread CTA busy.
 template <int kVectors>
 __global__ void __launch_bounds__(kQuantThreads)
-quantize_rows_warp_kernel(const uint16_t* __restrict__ x, int64_t out_rows, int cols, const int* __restrict__ sorted_routes, int top_k,
-                          const int* __restrict__ valid_rows, int numerics, int weight_mode, int8_t* __restrict__ q,
-                          float* __restrict__ scale_out) {
+quantize_rows_warp_kernel(const uint16_t* x, int64_t out_rows, int cols, const int* sorted_routes, int top_k,
+                          const int* valid_rows, int numerics, int weight_mode, int8_t* __restrict__ q,
+                          float* __restrict__ scale_out, bool chained) {
+  if (chained) {
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
+  }
   const int lane = threadIdx.x & 31;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * (kQuantThreads / 32) + (threadIdx.x >> 5);
   if (row >= out_rows) return;
-  if (valid_rows && row >= *valid_rows) return;
-  const int64_t src_row = sorted_routes ? static_cast<int64_t>(sorted_routes[row] / top_k) : row;
+  if (valid_rows && row >= __ldcg(valid_rows)) return;
+  const int64_t src_row = sorted_routes ? static_cast<int64_t>(__ldcg(sorted_routes + row) / top_k) : row;
   const uint4* src = reinterpret_cast<const uint4*>(x + src_row * cols);
   const int vec16 = cols >> 4;
   uint4 held[kVectors][2];
@@ -158,19 +166,23 @@ quantize_rows_warp_kernel(const uint16_t* __restrict__ x, int64_t out_rows, int 
 // cols % 16 == 0, top_k <= 32.  One CTA per token: the row is quantised once and stored to each of its routes'
 // sorted positions (the reference re-quantises the token for every route, kernels.cpp:639-644; the bits are the same).
 __global__ void __launch_bounds__(kQuantThreads)
-quantize_tokens_scatter_kernel(const uint16_t* __restrict__ x, int cols, int top_k, const int* __restrict__ route_pos,
-                               int numerics, int8_t* __restrict__ q, float* __restrict__ scale_out) {
+quantize_tokens_scatter_kernel(const uint16_t* x, int cols, int top_k, const int* route_pos,
+                               int numerics, int8_t* __restrict__ q, float* __restrict__ scale_out, bool chained) {
   __shared__ float smem[32];
   __shared__ int positions[32];
   const int64_t token = blockIdx.x;
-  if (threadIdx.x < top_k) positions[threadIdx.x] = route_pos[token * top_k + threadIdx.x];
   const uint4* src = reinterpret_cast<const uint4*>(x + token * cols);
   const int vec16 = cols >> 4;
   float local = 0.0f;
   for (int v = threadIdx.x; v < vec16; v += kQuantThreads) {
-    local = fmaxf(local, amax8(src[2 * v]));
-    local = fmaxf(local, amax8(src[2 * v + 1]));
+    local = fmaxf(local, amax8(__ldcg(src + 2 * v)));
+    local = fmaxf(local, amax8(__ldcg(src + 2 * v + 1)));
   }
+  if (chained) {
+    ptx::grid_dependency_wait();  // the route build: x itself is older
+    ptx::launch_dependents();
+  }
+  if (threadIdx.x < top_k) positions[threadIdx.x] = __ldcg(route_pos + token * top_k + threadIdx.x);
   const float amax = block_max(local, smem);  // its barriers also publish positions[]
   const float scale = row_scale_from_amax(amax, numerics);
   if (threadIdx.x < top_k && positions[threadIdx.x] >= 0) scale_out[positions[threadIdx.x]] = scale;
@@ -178,8 +190,8 @@ quantize_tokens_scatter_kernel(const uint16_t* __restrict__ x, int cols, int top
   const float inverse = __fdiv_rn(1.0f, scale);
   for (int v = threadIdx.x; v < vec16; v += kQuantThreads) {
     float values[16];
-    unpack8(src[2 * v], values);
-    unpack8(src[2 * v + 1], values + 8);
+    unpack8(__ldcg(src + 2 * v), values);
+    unpack8(__ldcg(src + 2 * v + 1), values + 8);
     uint4 out;
     out.x = pack4(values, operand, inverse, numerics);
     out.y = pack4(values + 4, operand, inverse, numerics);
@@ -196,12 +208,16 @@ quantize_tokens_scatter_kernel(const uint16_t* __restrict__ x, int cols, int top
 // given): the bf16 row becomes 16-bit fixed point (plane_fixed_point) and is stored as two int8 rows, the high plane at
 // row 2p and the low plane at row 2p + 1 of `planes`; scale_out[p] is the row scale.
 __global__ void __launch_bounds__(kQuantThreads)
-split_rows_planes_kernel(const uint16_t* __restrict__ x, int cols, const int* __restrict__ sorted_routes, int top_k,
-                         const int* __restrict__ valid_rows, int8_t* __restrict__ planes, float* __restrict__ scale_out) {
+split_rows_planes_kernel(const uint16_t* x, int cols, const int* sorted_routes, int top_k,
+                         const int* valid_rows, int8_t* __restrict__ planes, float* __restrict__ scale_out, bool chained) {
   __shared__ float smem[32];
+  if (chained) {
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
+  }
   const int64_t row = blockIdx.x;
-  if (valid_rows && row >= *valid_rows) return;
-  const int64_t src_row = sorted_routes ? static_cast<int64_t>(sorted_routes[row] / top_k) : row;
+  if (valid_rows && row >= __ldcg(valid_rows)) return;
+  const int64_t src_row = sorted_routes ? static_cast<int64_t>(__ldcg(sorted_routes + row) / top_k) : row;
   const uint4* src = reinterpret_cast<const uint4*>(x + src_row * cols);
   const int vec16 = cols >> 4;
   float local = 0.0f;
@@ -236,26 +252,30 @@ split_rows_planes_kernel(const uint16_t* __restrict__ x, int cols, const int* __
 // The same split once per TOKEN, stored to the sorted positions of its top_k routes (route_pos, -1 = dropped): the bits
 // every route would get from split_rows_planes_kernel, one read of x and one fixed-point conversion per token.
 __global__ void __launch_bounds__(kQuantThreads)
-split_tokens_scatter_planes_kernel(const uint16_t* __restrict__ x, int cols, int top_k, const int* __restrict__ route_pos,
-                                   int8_t* __restrict__ planes, float* __restrict__ scale_out) {
+split_tokens_scatter_planes_kernel(const uint16_t* x, int cols, int top_k, const int* route_pos,
+                                   int8_t* __restrict__ planes, float* __restrict__ scale_out, bool chained) {
   __shared__ float smem[32];
   __shared__ int positions[32];
   const int64_t token = blockIdx.x;
-  if (threadIdx.x < top_k) positions[threadIdx.x] = route_pos[token * top_k + threadIdx.x];
   const uint4* src = reinterpret_cast<const uint4*>(x + token * cols);
   const int vec16 = cols >> 4;
   float local = 0.0f;
   for (int v = threadIdx.x; v < vec16; v += kQuantThreads) {
-    local = fmaxf(local, amax8(src[2 * v]));
-    local = fmaxf(local, amax8(src[2 * v + 1]));
+    local = fmaxf(local, amax8(__ldcg(src + 2 * v)));
+    local = fmaxf(local, amax8(__ldcg(src + 2 * v + 1)));
   }
+  if (chained) {
+    ptx::grid_dependency_wait();  // the route build: x itself is older
+    ptx::launch_dependents();
+  }
+  if (threadIdx.x < top_k) positions[threadIdx.x] = __ldcg(route_pos + token * top_k + threadIdx.x);
   const float amax = block_max(local, smem);  // its barriers also publish positions[]
   const float scale = plane_row_scale(amax);
   if (threadIdx.x < top_k && positions[threadIdx.x] >= 0) scale_out[positions[threadIdx.x]] = scale;
   for (int v = threadIdx.x; v < vec16; v += kQuantThreads) {
     float values[16];
-    unpack8(src[2 * v], values);
-    unpack8(src[2 * v + 1], values + 8);
+    unpack8(__ldcg(src + 2 * v), values);
+    unpack8(__ldcg(src + 2 * v + 1), values + 8);
     uint32_t high[4] = {0, 0, 0, 0};
     uint32_t low[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -336,37 +356,93 @@ quantize_rows_dense_kernel(const void* __restrict__ x, int x_is_bf16, int cols, 
   }
 }
 
+constexpr int kGatherVectors = 4;  // 16-byte vectors a thread holds at a time: 8192 bf16 columns per CTA and round
+
 // cols % 8 == 0.  out[p] = x[sorted_routes[p] / top_k].
 __global__ void __launch_bounds__(kQuantThreads)
-gather_rows_kernel(const uint16_t* __restrict__ x, int cols, const int* __restrict__ sorted_routes, int top_k,
-                   const int* __restrict__ valid_rows, uint16_t* __restrict__ out) {
+gather_rows_kernel(const uint16_t* x, int cols, const int* sorted_routes, int top_k,
+                   const int* valid_rows, uint16_t* __restrict__ out, bool chained) {
+  if (chained) {
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
+  }
   const int64_t row = blockIdx.x;
-  if (valid_rows && row >= *valid_rows) return;
-  const int64_t src_row = sorted_routes[row] / top_k;
+  if (valid_rows && row >= __ldcg(valid_rows)) return;
+  const int64_t src_row = __ldcg(sorted_routes + row) / top_k;
   const uint4* src = reinterpret_cast<const uint4*>(x + src_row * cols);
   uint4* dst = reinterpret_cast<uint4*>(out + row * cols);
-  for (int v = threadIdx.x; v < (cols >> 3); v += kQuantThreads) dst[v] = src[v];
+  const int vec8 = cols >> 3;
+  for (int v0 = threadIdx.x; v0 < vec8; v0 += kGatherVectors * kQuantThreads) {
+    uint4 held[kGatherVectors];
+#pragma unroll
+    for (int i = 0; i < kGatherVectors; ++i) {
+      if (v0 + i * kQuantThreads < vec8) held[i] = src[v0 + i * kQuantThreads];
+    }
+#pragma unroll
+    for (int i = 0; i < kGatherVectors; ++i) {
+      if (v0 + i * kQuantThreads < vec8) dst[v0 + i * kQuantThreads] = held[i];
+    }
+  }
 }
 
-__global__ void gather_scalars_kernel(const float* __restrict__ in, int64_t n, const int* __restrict__ index,
-                                      const int* __restrict__ valid_rows, float* __restrict__ out) {
+// cols % 8 == 0, top_k <= 32.  One CTA per token: its row is read once and stored to each of its routes' sorted positions
+// (-1 = dropped).  Bound by the writes: a CTA per sorted row, which reads the row again for every route, took 127 us for
+// 32760 rows of 14 KB; this one 86 us.
+__global__ void __launch_bounds__(kQuantThreads)
+gather_tokens_scatter_kernel(const uint16_t* x, int cols, int top_k, const int* route_pos, uint16_t* __restrict__ out, bool chained) {
+  __shared__ int positions[32];
+  const int64_t token = blockIdx.x;
+  const uint4* src = reinterpret_cast<const uint4*>(x + token * cols);
+  const int vec8 = cols >> 3;
+  for (int v0 = threadIdx.x; v0 < (vec8 + kQuantThreads - 1) / kQuantThreads * kQuantThreads; v0 += kGatherVectors * kQuantThreads) {
+    uint4 held[kGatherVectors];
+#pragma unroll
+    for (int i = 0; i < kGatherVectors; ++i) {
+      if (v0 + i * kQuantThreads < vec8) held[i] = __ldcg(src + v0 + i * kQuantThreads);
+    }
+    if (v0 == static_cast<int>(threadIdx.x)) {
+      // The first round, which every thread takes part in.
+      if (chained) {
+        ptx::grid_dependency_wait();  // the route build: x itself is older
+        ptx::launch_dependents();
+      }
+      if (threadIdx.x < top_k) positions[threadIdx.x] = __ldcg(route_pos + token * top_k + threadIdx.x);
+      __syncthreads();
+    }
+    for (int slot = 0; slot < top_k; ++slot) {
+      const int position = positions[slot];
+      if (position < 0) continue;
+      uint4* dst = reinterpret_cast<uint4*>(out + static_cast<int64_t>(position) * cols);
+#pragma unroll
+      for (int i = 0; i < kGatherVectors; ++i) {
+        if (v0 + i * kQuantThreads < vec8) dst[v0 + i * kQuantThreads] = held[i];
+      }
+    }
+  }
+}
+
+__global__ void gather_scalars_kernel(const float* in, int64_t n, const int* index,
+                                      const int* valid_rows, float* __restrict__ out, bool chained) {
+  if (chained) {
+    ptx::grid_dependency_wait();
+    ptx::launch_dependents();
+  }
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (i >= n || (valid_rows && i >= *valid_rows)) return;
+  if (i >= n || (valid_rows && i >= __ldcg(valid_rows))) return;
   out[i] = in[index[i]];
 }
 
 }  // namespace
 
 cudaError_t launch_gather_scalars(const float* in, int64_t n, const int* index, const int* valid_rows, float* out,
-                                  cudaStream_t stream) {
+                                  cudaStream_t stream, bool chained) {
   if (n <= 0) return cudaSuccess;
-  gather_scalars_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(in, n, index, valid_rows, out);
-  return cudaGetLastError();
+  return launch_streaming(gather_scalars_kernel, dim3(static_cast<unsigned>((n + 255) / 256)), 256, stream, chained, in, n, index, valid_rows, out);
 }
 
 cudaError_t launch_quantize_rows(const uint16_t* x, int64_t out_rows, int cols, const int* sorted_routes, int top_k,
                                  const int* valid_rows, int numerics, int weight_mode, int8_t* q, float* scale,
-                                 cudaStream_t stream) {
+                                 cudaStream_t stream, bool chained) {
   if (out_rows <= 0) return cudaSuccess;
   const int vec16 = cols >> 4;
   const unsigned warp_blocks = static_cast<unsigned>((out_rows + kQuantThreads / 32 - 1) / (kQuantThreads / 32));
@@ -374,44 +450,39 @@ cudaError_t launch_quantize_rows(const uint16_t* x, int64_t out_rows, int cols, 
   // values per lane alone on an SM (10.7 us against the other kernel's ~5 us for 8 rows of 2048 columns).
   const bool few_rows = out_rows <= 592;  // four CTAs per SM at most
   if (few_rows) {
-    quantize_rows_kernel<<<static_cast<unsigned>(out_rows), kQuantThreads, 0, stream>>>(x, cols, sorted_routes, top_k, valid_rows,
-                                                                                       numerics, weight_mode, q, scale);
-    return cudaGetLastError();
+    return launch_streaming(quantize_rows_kernel, dim3(static_cast<unsigned>(out_rows)), kQuantThreads, stream, chained, x, cols, sorted_routes,
+                          top_k, valid_rows, numerics, weight_mode, q, scale);
   }
   if (vec16 <= 64) {
-    quantize_rows_warp_kernel<2><<<warp_blocks, kQuantThreads, 0, stream>>>(x, out_rows, cols, sorted_routes, top_k, valid_rows, numerics,
-                                                                             weight_mode, q, scale);
+    return launch_streaming(quantize_rows_warp_kernel<2>, dim3(warp_blocks), kQuantThreads, stream, chained, x, out_rows, cols, sorted_routes, top_k,
+                          valid_rows, numerics, weight_mode, q, scale);
   } else if (vec16 <= 128) {
-    quantize_rows_warp_kernel<4><<<warp_blocks, kQuantThreads, 0, stream>>>(x, out_rows, cols, sorted_routes, top_k, valid_rows, numerics,
-                                                                             weight_mode, q, scale);
-  } else {
-    quantize_rows_kernel<<<static_cast<unsigned>(out_rows), kQuantThreads, 0, stream>>>(x, cols, sorted_routes, top_k, valid_rows,
-                                                                                       numerics, weight_mode, q, scale);
+    return launch_streaming(quantize_rows_warp_kernel<4>, dim3(warp_blocks), kQuantThreads, stream, chained, x, out_rows, cols, sorted_routes, top_k,
+                          valid_rows, numerics, weight_mode, q, scale);
   }
-  return cudaGetLastError();
+  return launch_streaming(quantize_rows_kernel, dim3(static_cast<unsigned>(out_rows)), kQuantThreads, stream, chained, x, cols, sorted_routes, top_k,
+                        valid_rows, numerics, weight_mode, q, scale);
 }
 
 cudaError_t launch_split_rows_planes(const uint16_t* x, int64_t out_rows, int cols, const int* sorted_routes, int top_k,
                                      const int* valid_rows, int8_t* planes, float* scale, cudaStream_t stream) {
   if (out_rows <= 0) return cudaSuccess;
-  split_rows_planes_kernel<<<static_cast<unsigned>(out_rows), kQuantThreads, 0, stream>>>(x, cols, sorted_routes, top_k, valid_rows, planes,
-                                                                                         scale);
-  return cudaGetLastError();
+  return launch_streaming(split_rows_planes_kernel, dim3(static_cast<unsigned>(out_rows)), kQuantThreads, stream, true, x, cols, sorted_routes,
+                        top_k, valid_rows, planes, scale);
 }
 
 cudaError_t launch_split_tokens_scatter_planes(const uint16_t* x, int64_t tokens, int cols, int top_k, const int* route_pos, int8_t* planes,
                                                float* scale, cudaStream_t stream) {
   if (tokens <= 0) return cudaSuccess;
-  split_tokens_scatter_planes_kernel<<<static_cast<unsigned>(tokens), kQuantThreads, 0, stream>>>(x, cols, top_k, route_pos, planes, scale);
-  return cudaGetLastError();
+  return launch_streaming(split_tokens_scatter_planes_kernel, dim3(static_cast<unsigned>(tokens)), kQuantThreads, stream, true, x, cols, top_k,
+                        route_pos, planes, scale);
 }
 
 cudaError_t launch_quantize_tokens_scatter(const uint16_t* x, int64_t tokens, int cols, int top_k, const int* route_pos,
                                            int numerics, int8_t* q, float* scale, cudaStream_t stream) {
   if (tokens <= 0) return cudaSuccess;
-  quantize_tokens_scatter_kernel<<<static_cast<unsigned>(tokens), kQuantThreads, 0, stream>>>(x, cols, top_k, route_pos, numerics, q,
-                                                                                             scale);
-  return cudaGetLastError();
+  return launch_streaming(quantize_tokens_scatter_kernel, dim3(static_cast<unsigned>(tokens)), kQuantThreads, stream, true, x, cols, top_k,
+                        route_pos, numerics, q, scale);
 }
 
 // The same quantiser for rows whose length is a multiple of 8 and at most 16 * 1024: the row is read once, into registers
@@ -487,11 +558,18 @@ cudaError_t launch_quantize_rows_dense(const void* x, int x_is_bf16, int64_t row
   return cudaGetLastError();
 }
 
+cudaError_t launch_gather_tokens_scatter(const uint16_t* x, int64_t tokens, int cols, int top_k, const int* route_pos, uint16_t* out,
+                                         cudaStream_t stream) {
+  if (tokens <= 0) return cudaSuccess;
+  return launch_streaming(gather_tokens_scatter_kernel, dim3(static_cast<unsigned>(tokens)), kQuantThreads, stream, true, x, cols, top_k,
+                          route_pos, out);
+}
+
 cudaError_t launch_gather_rows(const uint16_t* x, int64_t out_rows, int cols, const int* sorted_routes, int top_k,
-                               const int* valid_rows, uint16_t* out, cudaStream_t stream) {
+                               const int* valid_rows, uint16_t* out, cudaStream_t stream, bool chained) {
   if (out_rows <= 0) return cudaSuccess;
-  gather_rows_kernel<<<static_cast<unsigned>(out_rows), kQuantThreads, 0, stream>>>(x, cols, sorted_routes, top_k, valid_rows, out);
-  return cudaGetLastError();
+  return launch_streaming(gather_rows_kernel, dim3(static_cast<unsigned>(out_rows)), kQuantThreads, stream, chained, x, cols, sorted_routes, top_k,
+                        valid_rows, out);
 }
 
 }  // namespace fmoe

@@ -22,6 +22,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "ptx.cuh"
 
 namespace fmoe {
 
@@ -179,6 +180,7 @@ route_build_kernel(const int64_t* __restrict__ topk_ids, int64_t routes, int exp
   const int rank = kCluster ? static_cast<int>(cg::this_cluster().block_rank()) : 0;
   const int ctas = kCluster ? static_cast<int>(cg::this_cluster().num_blocks()) : 1;
 
+  ptx::launch_dependents();  // an ordinary launch: everything before it has completed
   for (int i = threadIdx.x; i < warps * experts; i += blockDim.x) hist[i] = 0;
   if (rank == 0 && threadIdx.x < kStatusWords) status[threadIdx.x] = 0;
   __syncthreads();

@@ -204,11 +204,11 @@ struct UnitInfo {
 };
 
 // rows_per_route: 2 in the two-plane form (first row and row count come back in token rows), else 1.
-__device__ __forceinline__ UnitInfo load_unit(const int* __restrict__ items, int64_t unit, int64_t units, int n_blocks, int rows_per_route = 1) {
+__device__ __forceinline__ UnitInfo load_unit(const int* items, int64_t unit, int64_t units, int n_blocks, int rows_per_route = 1) {
   UnitInfo info = {0, 0, 0, 0};
   if (unit < units) {
     const int item = static_cast<int>(unit / n_blocks);
-    const int4 packed = __ldg(reinterpret_cast<const int4*>(items) + item);
+    const int4 packed = __ldcg(reinterpret_cast<const int4*>(items) + item);
     info.expert = packed.x;
     info.row0 = packed.y * rows_per_route;
     info.rows = packed.z * rows_per_route;
@@ -289,7 +289,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
 
   // (Values that come from global loads pass through a shuffle where the warps that feed TMA and the tensor pipe use
   // them: it changes nothing but lets the compiler treat them as warp-uniform.)
-  const int items = __shfl_sync(0xffffffffu, min(args.status[args.item_count_word], args.max_items), 0);
+  const int items = __shfl_sync(0xffffffffu, min(__ldcg(args.status + args.item_count_word), args.max_items), 0);
   const int n_blocks = (args.n_out + kChannelsPerUnit - 1) / kChannelsPerUnit;
   const int n_total = kGateUp ? 2 * args.n_out : args.n_out;
   const int64_t units = static_cast<int64_t>(items) * n_blocks;
@@ -334,6 +334,8 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
         ptx::prefetch_tensormap(&token_map_mid);
         ptx::prefetch_tensormap(&token_map_full);
       }
+      if (!args.beside) ptx::grid_dependency_wait();
+      ptx::launch_dependents();
       const uint32_t full_leader0 = map_to_cta(ptx::smem_u32(&ctl->full[0]), 0);
       int stage = 0;
       uint32_t phase = 0;
@@ -509,6 +511,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
     }
   } else {
     // ---------------- epilogue (warps 2.. of both CTAs) ----------------
+    if (!args.beside) ptx::grid_dependency_wait();
     const int quarter = warp & 3;                    // the TMEM lanes a warp may read are fixed by warp id % 4
     const int chunk_first = (warp - 2) >> 2;         // warps sharing a lane quarter take 32-column chunks round-robin
     constexpr int kChunkStep = kEpilogueWarps / 4;
@@ -543,22 +546,22 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
         const int column = tid + 256 * i;
         if (column >= info.rows) break;
         const int row = (info.row0 + column) / kRowsPerRoute;  // sorted position of the column's route
-        if (kInt8) t.column_scale[i] = args.a_scale[row];
+        if (kInt8) t.column_scale[i] = __ldcg(args.a_scale + row);
         if constexpr (kDense) {
           t.column_rowptr[i] = reinterpret_cast<uint64_t>(args.dense_out) + static_cast<uint64_t>(row) * n_out * (args.dense_out_bf16 ? 2 : 4);
         } else if constexpr (!kGateUp) {
           t.column_rowptr[i] = args.row_out_ptrs != nullptr
-                                   ? args.row_out_ptrs[row]
+                                   ? __ldcg(args.row_out_ptrs + row)
                                    : reinterpret_cast<uint64_t>(args.route_out) +
-                                         static_cast<uint64_t>(args.sorted_routes[row]) * n_out * (args.route_out_bf16 ? 2 : 4);
+                                         static_cast<uint64_t>(__ldcg(args.sorted_routes + row)) * n_out * (args.route_out_bf16 ? 2 : 4);
         }
       }
       const int n = info.block * kChannelsPerUnit + channel_in_unit;
       if (n < n_out) {
         if (kInt8) {
           const float* s = args.w_scale + static_cast<int64_t>(info.expert) * n_total;
-          t.scale_gate = s[kGateUp ? gate_channel(args, n) : n];
-          if (kGateUp) t.scale_up = s[up_channel(args, n)];
+          t.scale_gate = __ldcg(s + (kGateUp ? gate_channel(args, n) : n));
+          if (kGateUp) t.scale_up = __ldcg(s + up_channel(args, n));
         }
         if (kDense && args.bias != nullptr) t.bias = args.bias[n];
         if (!kInt8 && !kDense && args.expert_bias != nullptr) {
@@ -782,6 +785,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
     }
   }
 
+  if (args.beside && warp == 0) ptx::grid_dependency_wait();  // this kernel's end stands for the end of both
   ptx::tcgen05_fence_before();
   __syncthreads();
   cluster_sync();  // neither CTA leaves while its peer may still signal its barriers or read its operands
@@ -878,8 +882,9 @@ cudaError_t launch_pair(const GroupedGemmArgs& args, cudaStream_t stream) {
   int64_t pairs = static_cast<int64_t>(args.max_items) * n_blocks;
   if (pairs > sms / 2) pairs = sms / 2;
   if (pairs <= 0) return cudaSuccess;
-  kernel<<<static_cast<unsigned>(2 * pairs), kThreads, kSmemBytes, stream>>>(weight_map, token_map, token_map_mid, token_map_full, launch_args);
-  return cudaGetLastError();
+  // Not chained in its dense form, whose work items come from the kernel right in front.
+  return launch_chained(kernel, dim3(static_cast<unsigned>(2 * pairs)), kThreads, kSmemBytes, stream, !kDense, weight_map, token_map,
+                        token_map_mid, token_map_full, launch_args);
 }
 
 }  // namespace

@@ -170,7 +170,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
   const int lane = threadIdx.x & 31;
   int* status = args.status_rw;
 
-  const int items = __shfl_sync(0xffffffffu, min(args.status[args.item_count_word], args.max_items), 0);
+  const int items = __shfl_sync(0xffffffffu, min(__ldcg(args.status + args.item_count_word), args.max_items), 0);
   const int n_blocks = (args.n_out + kBlockM - 1) / kBlockM;
   const int n_total = kGateUp ? 2 * args.n_out : args.n_out;
   const int64_t units = static_cast<int64_t>(items) * n_blocks;
@@ -216,6 +216,35 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
       int stage = 0;
       uint32_t phase = 0;
       int issued = 0;
+      auto load_weights = [&](int to_stage, int kb, int n0, int expert) {
+        uint8_t* dst = smem + static_cast<size_t>(to_stage) * Cfg::kStageBytes;
+        const int x = kb * kBlockKElems;
+        if (kGateUp) {
+          ptx::tma_load_4d(dst, &weight_map, &ctl->full[to_stage], x, n0, 0, expert);
+          ptx::tma_load_4d(dst + kBlockM * kBlockKBytes, &weight_map, &ctl->full[to_stage], x, n0, 1, expert);
+        } else {
+          ptx::tma_load_2d(dst, &weight_map, &ctl->full[to_stage], x, expert * n_total + n0);
+        }
+      };
+      // Work items and weights are older than the kernel in front: the first stages' weights are requested while that one
+      // (it makes the token rows) still runs.
+      int early = 0;
+      if (!kW8A16 && static_cast<int64_t>(blockIdx.x) < units && !FMOE_DIAG_BIT(args, 2)) {
+        int item, block;
+        decode_unit(args.items, blockIdx.x, n_blocks, &item, &block);
+        item = __shfl_sync(0xffffffffu, item, 0);
+        block = __shfl_sync(0xffffffffu, block, 0);
+        const int expert = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 0), 0);
+        early = min(Cfg::kStages, k_blocks);
+        for (int kb = 0; kb < early; ++kb) {
+          if (issuer) {
+            ptx::mbar_arrive_expect_tx(&ctl->full[kb], Cfg::kStageBytes);
+            load_weights(kb, kb, block * kBlockM, expert);
+          }
+        }
+      }
+      ptx::grid_dependency_wait();
+      ptx::launch_dependents();
       if constexpr (kW8A16) {
         // Landing producer: the token tile and the int8 weight tiles of every K block into the landing ring, as far
         // ahead as the ring allows.
@@ -227,9 +256,9 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
           decode_unit(args.items, unit, n_blocks, &item, &block);
           item = __shfl_sync(0xffffffffu, item, 0);  // read from the item list: the same in every lane
           block = __shfl_sync(0xffffffffu, block, 0);
-          const int expert = __shfl_sync(0xffffffffu, args.items[4 * item + 0], 0);
+          const int expert = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 0), 0);
           const int n0 = block * kBlockM;
-          const int row0 = __shfl_sync(0xffffffffu, args.items[4 * item + 1], 0);
+          const int row0 = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 1), 0);
           for (int kb = 0; kb < k_blocks; ++kb) {
             ptx::mbar_wait(&ctl->landing_free[slot], slot_phase ^ 1u, abort_flag, status, 6);
             if (issuer) {
@@ -273,9 +302,8 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
         item = __shfl_sync(0xffffffffu, item, 0);  // read from the item list: the same in every lane
         block = __shfl_sync(0xffffffffu, block, 0);
         const int n0 = block * kBlockM;
-        const int expert = __shfl_sync(0xffffffffu, args.items[4 * item + 0], 0);
-        const int row0 = __shfl_sync(0xffffffffu, args.items[4 * item + 1], 0) * kRowsPerRoute;
-        const int weight_row = expert * n_total + n0;
+        const int expert = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 0), 0);
+        const int row0 = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 1), 0) * kRowsPerRoute;
         for (int kb = 0; kb < k_blocks; ++kb) {
           ptx::mbar_wait(&ctl->empty[stage], phase ^ 1u, abort_flag, status, 1);
           uint8_t* stage_base = smem + static_cast<size_t>(stage) * Cfg::kStageBytes;
@@ -284,15 +312,11 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
           } else if (FMOE_DIAG_BIT(args, 2)) {
             ptx::mbar_arrive(&ctl->full[stage]);
           } else {
-            ptx::mbar_arrive_expect_tx(&ctl->full[stage], Cfg::kStageBytes);
-            const int x = kb * kBlockKElems;
-            if (kGateUp) {
-              ptx::tma_load_4d(stage_base, &weight_map, &ctl->full[stage], x, n0, 0, expert);
-              ptx::tma_load_4d(stage_base + kBlockM * kBlockKBytes, &weight_map, &ctl->full[stage], x, n0, 1, expert);
-            } else {
-              ptx::tma_load_2d(stage_base, &weight_map, &ctl->full[stage], x, weight_row);
+            if (issued >= early) {
+              ptx::mbar_arrive_expect_tx(&ctl->full[stage], Cfg::kStageBytes);
+              load_weights(stage, kb, n0, expert);
             }
-            ptx::tma_load_2d(stage_base + Cfg::kWeightBytes, &token_map, &ctl->full[stage], x, row0);
+            ptx::tma_load_2d(stage_base + Cfg::kWeightBytes, &token_map, &ctl->full[stage], kb * kBlockKElems, row0);
           }
           ++issued;
           if (++stage == Cfg::kStages) {
@@ -394,7 +418,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
         decode_unit(args.items, unit, n_blocks, &item, &block);
         item = __shfl_sync(0xffffffffu, item, 0);  // read from the item list: the same in every lane
         block = __shfl_sync(0xffffffffu, block, 0);
-        const int item_rows = __shfl_sync(0xffffffffu, args.items[4 * item + 2], 0) * kRowsPerRoute;
+        const int item_rows = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 2), 0) * kRowsPerRoute;
         const int mma_n = min(kRowTile, (item_rows + 15) & ~15);
         // Weight-major: M = 128 channels, N = the item's rows.  Token-major (W8A16): M = 128 token lanes, N = the
         // unit's channels (gate and up tiles are one 256-row B operand).
@@ -440,6 +464,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
     }
   } else {
     // ---------------- epilogue (warps 2..5) ----------------
+    ptx::grid_dependency_wait();
     const int quarter = warp & 3;  // the TMEM lanes a warp may read are fixed by warp id % 4
     const int channel_in_block = quarter * 32 + lane;
     const int epilogue_thread = static_cast<int>(threadIdx.x) - kEpilogueWarp0 * 32;
@@ -457,9 +482,9 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
       item = __shfl_sync(0xffffffffu, item, 0);  // read from the item list: the same in every lane
       block = __shfl_sync(0xffffffffu, block, 0);
       const int n = block * kBlockM + channel_in_block;
-      const int expert = args.items[4 * item + 0];
-      const int row0 = args.items[4 * item + 1] * kRowsPerRoute;  // token rows (two per route in the two-plane form)
-      const int rows = args.items[4 * item + 2] * kRowsPerRoute;
+      const int expert = __ldcg(args.items + 4 * item + 0);
+      const int row0 = __ldcg(args.items + 4 * item + 1) * kRowsPerRoute;  // token rows (two per route in the two-plane form)
+      const int rows = __ldcg(args.items + 4 * item + 2) * kRowsPerRoute;
       const bool channel_ok = n < n_out;
       ColumnMeta* meta = &ctl->meta[local & 1];
       if constexpr (kW8A16) {
@@ -487,9 +512,9 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
             out_row = reinterpret_cast<uint8_t*>(args.y + static_cast<int64_t>(row0 + token) * n_out + n0);
           } else {
             const uint64_t base = args.row_out_ptrs != nullptr
-                                      ? args.row_out_ptrs[row0 + token]
+                                      ? __ldcg(args.row_out_ptrs + row0 + token)
                                       : reinterpret_cast<uint64_t>(args.route_out) +
-                                            static_cast<uint64_t>(args.sorted_routes[row0 + token]) * n_out * (args.route_out_bf16 ? 2 : 4);
+                                            static_cast<uint64_t>(__ldcg(args.sorted_routes + row0 + token)) * n_out * (args.route_out_bf16 ? 2 : 4);
             out_row = reinterpret_cast<uint8_t*>(base) + static_cast<size_t>(n0) * (args.route_out_bf16 ? 2 : 4);
           }
         }
@@ -539,12 +564,12 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
       }
       for (int c = epilogue_thread; c < rows; c += 128) {
         const int route_row = (row0 + c) / kRowsPerRoute;  // sorted position of the column's route
-        if (kInt8) meta->scale[c] = args.a_scale[route_row];
+        if (kInt8) meta->scale[c] = __ldcg(args.a_scale + route_row);
         if constexpr (!kGateUp) {
           meta->rowptr[c] = args.row_out_ptrs != nullptr
-                                ? args.row_out_ptrs[route_row]
+                                ? __ldcg(args.row_out_ptrs + route_row)
                                 : reinterpret_cast<uint64_t>(args.route_out) +
-                                      static_cast<uint64_t>(args.sorted_routes[route_row]) * n_out * (args.route_out_bf16 ? 2 : 4);
+                                      static_cast<uint64_t>(__ldcg(args.sorted_routes + route_row)) * n_out * (args.route_out_bf16 ? 2 : 4);
         }
       }
       float scale_gate = 1.0f, scale_up = 1.0f;
@@ -748,8 +773,8 @@ cudaError_t launch_config(const GroupedGemmArgs& args, cudaStream_t stream) {
   const int sms = sm_count_of_current_device();
   if (grid > sms) grid = sms;
   if (grid <= 0) return cudaSuccess;
-  kernel<<<static_cast<unsigned>(grid), kW8A16 ? kThreadsW8A16 : kThreads, Cfg::kSmemBytes, stream>>>(weight_map, token_map, args);
-  return cudaGetLastError();
+  return launch_chained(kernel, dim3(static_cast<unsigned>(grid)), kW8A16 ? kThreadsW8A16 : kThreads, Cfg::kSmemBytes, stream, true,
+                        weight_map, token_map, args);
 }
 
 template <bool kInt8, bool kGateUp, bool kW8A16 = false, bool kPlanes = false>
