@@ -7,6 +7,7 @@ ABI.  Workspaces come from torch's caching allocator and are cached per (device,
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from dataclasses import dataclass
 
@@ -42,7 +43,7 @@ EXPORTS = (
     "fmoe_stage_timer_read", "fmoe_route_build_noalloc", "fmoe_ep_dispatch_workspace_bytes", "fmoe_ep_dispatch_prepare",
     "fmoe_w8a8_expert_rows_forward", "fmoe_bf16_expert_rows_forward", "fmoe_ep_combine_finish",
     "fmoe_i8gemm_dynamic_scaled_mm_pair",
-    "fmoe_router_topk",
+    "fmoe_router_topk", "fmoe_append_shared_route",
     "fmoe_ep_peer_create", "fmoe_ep_peer_handle", "fmoe_ep_peer_connect", "fmoe_ep_peer_destroy", "fmoe_ep_peer_slab_bytes",
     "fmoe_ep_peer_dispatch", "fmoe_ep_peer_experts", "fmoe_ep_peer_combine", "fmoe_ep_peer_read_status",
     "fmoe_ep_peer_slab_address", "fmoe_ep_peer_connect_addresses",
@@ -145,6 +146,7 @@ def _open(path: str) -> ctypes.CDLL:
     lib.fmoe_route_build_noalloc.argtypes = [p, i64, i32, i32, p, p, p, p, p, p]
     lib.fmoe_i8gemm_dynamic_scaled_mm.argtypes = [p, i32, i64, i32, p, p, p, i32, p, i32, p, ctypes.c_size_t, p]
     lib.fmoe_i8gemm_dynamic_scaled_mm_pair.argtypes = [p, i64, i32, p, p, i32, p, p, p, i32, p, p, ctypes.c_size_t, p]
+    lib.fmoe_append_shared_route.argtypes = [p, p, i64, i32, i64, ctypes.c_float, p, p, p]
     lib.fmoe_router_topk.argtypes = [p, p, i64, i32, i32, i32, i32, ctypes.c_float, p, p, p]
     lib.fmoe_ep_peer_create.argtypes = [i32, i32, i64, i32, i32, i32, i32, i32, i32, ctypes.POINTER(ctypes.c_void_p)]
     lib.fmoe_ep_peer_handle.argtypes = [p, p]
@@ -179,14 +181,17 @@ def device_supported(device: int | None = None) -> bool:
     return bool(load().fmoe_device_supported(index))
 
 
-def _ptr(tensor: torch.Tensor | None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if tensor is None else tensor.data_ptr())
+# Plain integers: the argtypes make the pointers.  (A c_void_p object per argument and a torch Stream object per call
+# took a fifth of the host time of a forward.)
+def _ptr(tensor: torch.Tensor | None) -> int | None:
+    return None if tensor is None else tensor.data_ptr()
 
 
-def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
+@functools.lru_cache(maxsize=256)
 def workspace_layout(int8: bool, tokens: int, top_k: int, experts: int, hidden: int, inter: int) -> WorkspaceLayout:
     layout = WorkspaceLayout()
     fn = load().fmoe_w8a8_workspace_layout if int8 else load().fmoe_bf16_workspace_layout
@@ -284,9 +289,9 @@ class StageTimer:
 def _require_cuda(name: str, tensor: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     if not isinstance(tensor, torch.Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")
-    if tensor.device.type != "cuda":
+    if not tensor.is_cuda:
         raise ValueError(f"{name} must be a CUDA tensor (this build has no CPU path)")
-    if tensor.dtype != dtype:
+    if tensor.dtype is not dtype:
         raise TypeError(f"{name} must have dtype {dtype}, got {tensor.dtype}")
     return tensor.contiguous()
 
@@ -325,15 +330,10 @@ def moe_forward(x, w13, w2, topk_weights, topk_ids, *, s13=None, s2=None, numeri
     forced = os.environ.get("FUSED_CPP_MOE_FORCE_TILES")  # "gate_up,down": diagnostic override of the row tiles
     if forced and gate_up_tile == 0 and down_tile == 0:
         gate_up_tile, down_tile = (int(v) for v in forced.split(","))
-    config = Config()
-    config.numerics = numerics
-    config.gemm_impl = gemm_impl
-    config.gate_up_tile = gate_up_tile
-    config.down_tile = down_tile
-    config.swiglu_limit = (10.0 if int8 else 0.0) if swiglu_limit is None else float(swiglu_limit)
-    config.activation = int(activation)
-    config.route_rows_bf16 = 1 if route_rows_bf16 else 0
-    config.w8a16_form = w8a16_form_from_env() if w8a16_form is None else int(w8a16_form)
+    limit = (10.0 if int8 else 0.0) if swiglu_limit is None else float(swiglu_limit)
+    form = w8a16_form_from_env() if w8a16_form is None else int(w8a16_form)
+    config = Config(numerics, gemm_impl, gate_up_tile, down_tile, limit, int(activation), None, None, None, None, None,
+                    1 if route_rows_bf16 else 0, form)
     bias_dtype = torch.float32
     if w13_bias is not None or w2_bias is not None:
         if all(bias is None or bias.dtype == torch.bfloat16 for bias in (w13_bias, w2_bias)):
@@ -508,6 +508,18 @@ def router_topk(logits: torch.Tensor, top_k: int, *, scoring: str = "softmax", s
     ids = torch.empty((tokens, top_k), dtype=torch.int64, device=logits.device)
     check(load().fmoe_router_topk(_ptr(logits), _ptr(bias), tokens, experts, top_k, 1 if scoring == "sigmoid" else 0,
                                   1 if renormalize else 0, float(routed_scaling_factor), _ptr(weights), _ptr(ids), _stream()))
+    return weights, ids
+
+
+def append_shared_route(topk_weights: torch.Tensor, topk_ids: torch.Tensor, shared_expert_id: int, scaling: float):
+    """(fp32 weights * scaling | 1, int64 ids | shared_expert_id), both [T, K + 1], in one launch (fmoe_append_shared_route)."""
+    topk_weights = _require_cuda("topk_weights", topk_weights, torch.float32)
+    topk_ids = _require_cuda("topk_ids", topk_ids, torch.int64)
+    tokens, top_k = topk_ids.shape
+    weights = torch.empty((tokens, top_k + 1), dtype=torch.float32, device=topk_weights.device)
+    ids = torch.empty((tokens, top_k + 1), dtype=torch.int64, device=topk_ids.device)
+    check(load().fmoe_append_shared_route(_ptr(topk_weights), _ptr(topk_ids), tokens, top_k, shared_expert_id, scaling, _ptr(weights),
+                                          _ptr(ids), _stream()))
     return weights, ids
 
 

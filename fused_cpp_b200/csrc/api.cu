@@ -468,10 +468,47 @@ int fmoe_device_supported(int device) {
   return major == 10 ? 1 : 0;
 }
 
+}  // extern "C"
+
+namespace {
+// One status block of page-locked memory per thread that reads one, given back when the thread ends.
+class PinnedWords {
+ public:
+  int* get() {
+    if (!tried_) {
+      tried_ = true;
+      // Another thread may be capturing a graph: this allocation is no part of it.
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      void* memory = nullptr;
+      if (cudaHostAlloc(&memory, sizeof(int) * fmoe::kStatusWords, cudaHostAllocPortable) == cudaSuccess) {
+        words_ = static_cast<int*>(memory);
+      } else {
+        cudaGetLastError();
+      }
+      cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    return words_;
+  }
+  ~PinnedWords() {
+    if (words_ != nullptr) cudaFreeHost(words_);
+  }
+
+ private:
+  int* words_ = nullptr;
+  bool tried_ = false;
+};
+}  // namespace
+
+extern "C" {
+
 int fmoe_read_status(const void* workspace, void* stream, int32_t* error, int32_t* detail) {
   if (workspace == nullptr) return fail(FMOE_ERR_INVALID_ARGUMENT, "workspace is null");
-  int words[fmoe::kStatusWords];
-  cudaError_t result = cudaMemcpyAsync(words, workspace, sizeof(words), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream));
+  // Page-locked: a copy to pageable memory is staged by the driver and costs the call several microseconds more.
+  static thread_local PinnedWords pinned;
+  int fallback[fmoe::kStatusWords];
+  int* const words = pinned.get() != nullptr ? pinned.get() : fallback;
+  cudaError_t result = cudaMemcpyAsync(words, workspace, sizeof(fallback), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream));
   if (result == cudaSuccess) result = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
   if (result != cudaSuccess) return cuda_fail(result, "reading the status block");
   if (error) *error = words[fmoe::kStatusError];
@@ -899,6 +936,22 @@ extern "C" int fmoe_router_topk(const float* logits, const float* selection_bias
                                                      renormalize != 0, routed_scaling_factor, topk_weights, topk_ids,
                                                      static_cast<cudaStream_t>(stream));
   return error == cudaSuccess ? FMOE_OK : cuda_fail(error, "router top-k");
+}
+
+extern "C" int fmoe_append_shared_route(const float* weights, const int64_t* ids, int64_t tokens, int32_t top_k, int64_t shared_id,
+                                        float scaling, float* weights_out, int64_t* ids_out, void* stream) {
+  int status = check_device();
+  if (status != FMOE_OK) return status;
+  if (tokens < 0 || top_k <= 0 || tokens > (int64_t{1} << 30) / (static_cast<int64_t>(top_k) + 1)) {
+    return fail(FMOE_ERR_INVALID_ARGUMENT, "shared route: invalid shape (%lld tokens, top_k %d)", static_cast<long long>(tokens), top_k);
+  }
+  if (tokens == 0) return FMOE_OK;
+  if (weights == nullptr || ids == nullptr || weights_out == nullptr || ids_out == nullptr) {
+    return fail(FMOE_ERR_INVALID_ARGUMENT, "shared route: null pointer");
+  }
+  const cudaError_t error = fmoe::launch_append_shared_route(weights, ids, tokens, top_k, shared_id, scaling, weights_out, ids_out,
+                                                             static_cast<cudaStream_t>(stream));
+  return error == cudaSuccess ? FMOE_OK : cuda_fail(error, "shared route");
 }
 
 /* ---- expert parallelism over peer memory ---------------------------------------------------------- */

@@ -116,6 +116,10 @@ cudaError_t launch_peer_row_ptrs(const int* valid_rows, int64_t capacity, const 
 cudaError_t launch_router_topk(const float* logits, const float* selection_bias, int64_t tokens, int experts, int top_k, int sigmoid,
                                int renormalize, float scaling, float* topk_weights, int64_t* topk_ids, cudaStream_t stream);
 
+// weights_out[t, :] = weights[t, :] * scaling | 1 and ids_out[t, :] = ids[t, :] | shared_id, rows of top_k + 1.
+cudaError_t launch_append_shared_route(const float* weights, const int64_t* ids, int64_t tokens, int top_k, int64_t shared_id, float scaling,
+                                       float* weights_out, int64_t* ids_out, cudaStream_t stream);
+
 // ---- merge.cu
 // W8A8: out[t] = bf16( fma chain over slots of route_out[t*K+slot] * w[t,slot] ).
 // BF16: pairwise tree for K in {2,4,6,8}, chain otherwise.

@@ -120,7 +120,30 @@ router_topk_kernel(const float* __restrict__ logits, const float* __restrict__ s
   }
 }
 
+// The always-active shared expert as one more route per token.  A few hundred KB: launch-bound, so one launch for both
+// arrays (copy, fill, scale, copy and fill as operations of their own kept the host busy for 35 us before the forward).
+__global__ void __launch_bounds__(256)
+append_shared_route_kernel(const float* __restrict__ weights, const int64_t* __restrict__ ids, int64_t count, int top_k, int64_t shared_id,
+                           float scaling, float* __restrict__ weights_out, int64_t* __restrict__ ids_out) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= count) return;
+  const int64_t token = i / (top_k + 1);
+  const int slot = static_cast<int>(i - token * (top_k + 1));
+  const int64_t source = token * top_k + slot;
+  weights_out[i] = slot < top_k ? __fmul_rn(weights[source], scaling) : 1.0f;
+  ids_out[i] = slot < top_k ? ids[source] : shared_id;
+}
+
 }  // namespace
+
+cudaError_t launch_append_shared_route(const float* weights, const int64_t* ids, int64_t tokens, int top_k, int64_t shared_id, float scaling,
+                                       float* weights_out, int64_t* ids_out, cudaStream_t stream) {
+  const int64_t count = tokens * (top_k + 1);
+  if (count <= 0) return cudaSuccess;
+  append_shared_route_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, stream>>>(weights, ids, count, top_k, shared_id, scaling,
+                                                                                           weights_out, ids_out);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_router_topk(const float* logits, const float* selection_bias, int64_t tokens, int experts, int top_k, int sigmoid,
                                int renormalize, float scaling, float* topk_weights, int64_t* topk_ids, cudaStream_t stream) {

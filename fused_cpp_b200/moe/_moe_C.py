@@ -153,7 +153,7 @@ def _check_out(input: torch.Tensor, out: torch.Tensor | None, others) -> None:
 def _tile_from(windows) -> int:
     if windows is None or windows.numel() == 0:
         return 0
-    return int(windows.reshape(-1)[0])
+    return int(windows.item() if windows.numel() == 1 else windows.reshape(-1)[0])
 
 
 def _check_plan_vectors(task_expert_ids, task_core_begins, task_threads, task_dep_offsets, task_deps, plan_version,
@@ -164,9 +164,12 @@ def _check_plan_vectors(task_expert_ids, task_core_begins, task_threads, task_de
     for tensor in (task_core_begins, task_threads, task_min_threads, task_max_threads):
         if tensor.numel() != tasks:
             raise RuntimeError(f"{label} task vectors must have matching lengths")
-    if task_dep_offsets.numel() != tasks + 1 or int(task_dep_offsets[tasks]) != task_deps.numel():
+    # Short vectors (the one-task plan of this package) as lists: a tensor operation on one costs microseconds per call.
+    short = tasks <= 16
+    if task_dep_offsets.numel() != tasks + 1 or (task_dep_offsets.tolist()[tasks] if short else int(task_dep_offsets[tasks])) != task_deps.numel():
         raise RuntimeError(f"{label} dependency offsets are invalid")
-    if task_resize_points.numel() and bool((task_resize_points != 0).any()):
+    points = task_resize_points.numel()
+    if points and (any(task_resize_points.tolist()) if points <= 16 else bool((task_resize_points != 0).any())):
         raise RuntimeError(f"{label} does not support dynamic resize points")
 
 
@@ -188,7 +191,7 @@ def fused_moe_w8a8_tiled_async_plan_v2(
         raise RuntimeError("W8A8 v1 requires weighted TopK merge")
     if early_merge != 0:
         raise RuntimeError("W8A8 v1 requires early_merge=False")
-    if input.dim() != 2 or input.dtype != torch.bfloat16 or input.device.type != "cuda":
+    if input.dim() != 2 or input.dtype != torch.bfloat16 or not input.is_cuda:
         raise RuntimeError("W8A8 input must be a CUDA BF16 [tokens, H] tensor")
     if topk_ids.dim() != 2 or topk_weights.shape != topk_ids.shape or topk_ids.shape[0] != input.shape[0]:
         raise RuntimeError("W8A8 topk tensors must be matching [tokens, top_k]")
@@ -234,12 +237,14 @@ def _check_bias(bias, experts: int, channels: int, name: str, dtype: torch.dtype
         return None
     if bias.dim() != 2 or tuple(bias.shape) != (experts, channels) or not bias.dtype.is_floating_point:
         raise RuntimeError(f"{name} must be a floating [E, N] = [{experts}, {channels}] tensor")
-    return bias.to(device=_device(), dtype=dtype).contiguous()
+    if bias.dtype is not dtype or not bias.is_cuda or bias.device.index != torch.cuda.current_device():
+        bias = bias.to(device=_device(), dtype=dtype)
+    return bias.contiguous()
 
 
 def _bf16_forward(input, w13_packed, w13_k, w13_n, w2_packed, w2_k, w2_n, topk_weights, topk_ids, w13_bias, w2_bias,
                   activation, global_num_experts, skip_weighted, out, gate_up_tile=0, down_tile=0):
-    if input.dim() != 2 or input.dtype != torch.bfloat16 or input.device.type != "cuda":
+    if input.dim() != 2 or input.dtype != torch.bfloat16 or not input.is_cuda:
         raise RuntimeError("input must be a CUDA BF16 [tokens, H] tensor")
     if topk_ids.dim() != 2 or topk_weights.shape != topk_ids.shape or topk_ids.shape[0] != input.shape[0]:
         raise RuntimeError("topk tensors must be matching [tokens, top_k]")
@@ -544,7 +549,7 @@ def fused_moe_w8a16_tiled_async_plan_v2(
     scale multiplies the accumulator."""
     if plan_version != 2:
         raise RuntimeError("W8A16 async plan requires plan_version 2")
-    if input.dim() != 2 or input.dtype != torch.bfloat16 or input.device.type != "cuda":
+    if input.dim() != 2 or input.dtype != torch.bfloat16 or not input.is_cuda:
         raise RuntimeError("W8A16 input must be a CUDA BF16 [tokens, H] tensor")
     if topk_ids.dim() != 2 or topk_weights.shape != topk_ids.shape or topk_ids.shape[0] != input.shape[0]:
         raise RuntimeError("W8A16 topk tensors must be matching [tokens, top_k]")

@@ -14,6 +14,7 @@ from typing import Any, Mapping, Tuple
 
 import torch
 
+from .. import _lib
 from . import _moe_C as _native
 from .plan import AsyncMoEPlanV2, gpu_placeholder_plan
 
@@ -485,6 +486,8 @@ def fused_moe_tiled(input, weights, topk_weights, topk_ids, *, w13_bias=None, w2
 def _combine_with_shared(topk_weights, topk_ids, shared_expert_id: int, scaling: float):
     """Append the shared expert as route K with weight 1 and scale the routed weights (bf16_tiled.py:1007-1013)."""
     tokens, routed_top_k = topk_ids.shape
+    if topk_weights.is_cuda and topk_weights.dtype is torch.float32 and topk_ids.dtype is torch.int64 and topk_ids.is_cuda:
+        return _lib.append_shared_route(topk_weights, topk_ids, shared_expert_id, scaling)
     ids = torch.empty((tokens, routed_top_k + 1), dtype=topk_ids.dtype, device=topk_ids.device)
     weights = torch.empty((tokens, routed_top_k + 1), dtype=topk_weights.dtype, device=topk_weights.device)
     ids[:, :routed_top_k].copy_(topk_ids)

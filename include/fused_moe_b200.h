@@ -329,6 +329,11 @@ FMOE_API int fmoe_router_topk(const float* logits, const float* selection_bias, 
                               int32_t scoring, int32_t renormalize, float routed_scaling_factor, float* topk_weights,
                               int64_t* topk_ids, void* stream);
 
+/* The routing arrays of a layer with one always-active shared expert, rows of top_k + 1: weights_out[t] = weights[t] *
+ * scaling, then 1; ids_out[t] = ids[t], then shared_id. */
+FMOE_API int fmoe_append_shared_route(const float* weights, const int64_t* ids, int64_t tokens, int32_t top_k, int64_t shared_id,
+                                      float scaling, float* weights_out, int64_t* ids_out, void* stream);
+
 /* ---- expert parallelism over peer memory --------------------------------------------------------- */
 
 /* The same sharding as fmoe_ep_dispatch_prepare / fmoe_*_expert_rows_forward / fmoe_ep_combine_finish, with the row
