@@ -166,30 +166,36 @@ __device__ __forceinline__ int quantize_value(float value, float scale_or_invers
   return static_cast<int>(rounded);
 }
 
-// TORCHREF quantisation of four values with the division replaced by a multiplication wherever that cannot change
-// the result.  value * (1/scale) differs from the correctly rounded value / scale by at most a few units in the
-// last place (below 4e-5 in absolute terms for |quotient| <= 128), so the two round to the same integer unless
-// the product lies within 1e-4 of a half-integer; only then the exact division decides.  Bit-identical to
-// quantize_value(TORCHREF).  The conversions are taken out of the common path as well.  The product is clamped
-// first (rint and a clamp at the integers +-127 commute; the order of fminf / fmaxf is quantize_value's, so NaN ends
-// at +127 there too); adding 1.5 * 2^23 rounds it to the nearest integer, ties to even, in the low mantissa bits, so
-// the byte is read out of the sum's bit pattern and subtracting the constant again gives rint(product) for the
-// boundary test: no FRND and no F2I, which issue at a quarter of the FADD rate.  A clamped product is an integer
-// (distance 0) and the exact quotient then rounds to +-127 as well.  One test per four values; the exact division
-// decides all four when any of them is near a boundary.
+__device__ __forceinline__ float max_or_nan(float a, float b) {
+  float result;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(result) : "f"(a), "f"(b));
+  return result;
+}
+
+// TORCHREF quantisation of four values of a row whose scale is that of the row's largest magnitude, with the division
+// replaced by a multiplication wherever that cannot change the result.  value * (1/scale) differs from the correctly rounded
+// value / scale by a few units in the last place (below 2e-5 in absolute terms for |quotient| <= 127.5), so the two round to
+// the same integer unless the product lies within 1e-4 of a half-integer; only then the exact division decides.
+// Bit-identical to quantize_value(TORCHREF).  Adding 1.5 * 2^23 rounds the product (exact inside the fused multiply-add)
+// to the nearest integer, ties to even, in the low mantissa bits: the byte is read out of the sum's bit pattern and
+// subtracting the constant again gives the integer for the boundary test, whose maximum keeps NaN.  No conversion
+// instruction and no clamp: a quotient beyond +-127.5 would need a scale that is not the row's, and what is not finite (a
+// NaN value, an infinite row, a scale whose reciprocal overflows) is a NaN in the test and goes to the exact statement.
+// One test per four values; the exact statement decides all four when any of them asks for it.  Four instructions
+// per value: with the clamp, the product and its distance as separate operations (seven) 65536 rows of 2048 columns took
+// 112 us, 105 us like this.
 __device__ __forceinline__ uint32_t quantize4_torchref_fast(const float* values, float scale, float inverse) {
   constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
   uint32_t bits[4];
   float worst = 0.0f;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float product = fmaxf(fminf(__fmul_rn(values[i], inverse), 127.0f), -127.0f);
-    const float shifted = __fadd_rn(product, kMagic);
+    const float shifted = __fmaf_rn(values[i], inverse, kMagic);
     const float nearest = __fsub_rn(shifted, kMagic);
-    worst = fmaxf(worst, fabsf(__fsub_rn(product, nearest)));
+    worst = max_or_nan(worst, fabsf(__fmaf_rn(values[i], inverse, -nearest)));
     bits[i] = __float_as_uint(shifted);
   }
-  if (worst > 0.4999f) {
+  if (!(worst <= 0.4999f)) {
     uint32_t packed = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {

@@ -37,13 +37,20 @@ __device__ __forceinline__ void unpack8(const uint4& v, float* out) {
   }
 }
 
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t result;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(result) : "r"(a), "r"(b));
+  return result;
+}
+
+// Largest magnitude of eight bf16 values, NaN left out: two values per instruction, exact like the fp32 form.
 __device__ __forceinline__ float amax8(const uint4& v) {
-  float values[8];
-  unpack8(v, values);
-  float m = 0.0f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(values[i]));
-  return m;
+  constexpr uint32_t kMagnitude = 0x7fff7fffu;
+  uint32_t m = max_bf16x2(0u, v.x & kMagnitude);
+  m = max_bf16x2(m, v.y & kMagnitude);
+  m = max_bf16x2(m, v.z & kMagnitude);
+  m = max_bf16x2(m, v.w & kMagnitude);
+  return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u));
 }
 
 // operand: 1/scale (NATIVE) or scale (TORCHREF); inverse: 1/scale, used by the TORCHREF fast path.
