@@ -49,6 +49,7 @@ namespace {
 constexpr int kBlockM = 128;        // output channels per MMA tile (TMEM lanes)
 constexpr int kBlockKBytes = 128;   // bytes of K per pipeline stage = one 128-byte swizzle row
 constexpr int kUmmaKBytes = 32;     // bytes of K per tcgen05.mma
+constexpr int kTokenBox = 16;       // token rows per TMA box: an item loads the rows its MMAs read, not its tile
 constexpr int kThreads = 192;
 constexpr int kEpilogueWarp0 = 2;
 constexpr int kConvertWarp0 = 6;          // W8A16: warps 6.. widen the int8 weight tile to bf16
@@ -235,10 +236,11 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
         item = __shfl_sync(0xffffffffu, item, 0);
         block = __shfl_sync(0xffffffffu, block, 0);
         const int expert = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 0), 0);
+        const int boxes = __shfl_sync(0xffffffffu, (__ldcg(args.items + 4 * item + 2) * kRowsPerRoute + kTokenBox - 1) / kTokenBox, 0);
         early = min(Cfg::kStages, k_blocks);
         for (int kb = 0; kb < early; ++kb) {
           if (issuer) {
-            ptx::mbar_arrive_expect_tx(&ctl->full[kb], Cfg::kStageBytes);
+            ptx::mbar_arrive_expect_tx(&ctl->full[kb], Cfg::kWeightBytes + boxes * kTokenBox * kBlockKBytes);
             load_weights(kb, kb, block * kBlockM, expert);
           }
         }
@@ -304,6 +306,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
         const int n0 = block * kBlockM;
         const int expert = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 0), 0);
         const int row0 = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 1), 0) * kRowsPerRoute;
+        const int boxes = __shfl_sync(0xffffffffu, (__ldcg(args.items + 4 * item + 2) * kRowsPerRoute + kTokenBox - 1) / kTokenBox, 0);
         for (int kb = 0; kb < k_blocks; ++kb) {
           ptx::mbar_wait(&ctl->empty[stage], phase ^ 1u, abort_flag, status, 1);
           uint8_t* stage_base = smem + static_cast<size_t>(stage) * Cfg::kStageBytes;
@@ -313,10 +316,13 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
             ptx::mbar_arrive(&ctl->full[stage]);
           } else {
             if (issued >= early) {
-              ptx::mbar_arrive_expect_tx(&ctl->full[stage], Cfg::kStageBytes);
+              ptx::mbar_arrive_expect_tx(&ctl->full[stage], Cfg::kWeightBytes + boxes * kTokenBox * kBlockKBytes);
               load_weights(stage, kb, n0, expert);
             }
-            ptx::tma_load_2d(stage_base + Cfg::kWeightBytes, &token_map, &ctl->full[stage], kb * kBlockKElems, row0);
+            for (int b = 0; b < boxes; ++b) {
+              ptx::tma_load_2d(stage_base + Cfg::kWeightBytes + b * kTokenBox * kBlockKBytes, &token_map, &ctl->full[stage], kb * kBlockKElems,
+                               row0 + b * kTokenBox);
+            }
           }
           ++issued;
           if (++stage == Cfg::kStages) {
@@ -765,7 +771,7 @@ cudaError_t launch_config(const GroupedGemmArgs& args, cudaStream_t stream) {
                           : kW8A16 ? make_landing_map(&weight_map, args.weights, weight_rows, args.k)
                                    : make_sw128_map(&weight_map, args.weights, kInt8, weight_rows, args.k, kBlockM);
   const uint64_t token_rows = static_cast<uint64_t>(args.total_rows) * (kPlanes ? 2 : 1);
-  if (!weights_ok || !make_sw128_map(&token_map, args.a_rows, kInt8, token_rows, args.k, kRowTile)) {
+  if (!weights_ok || !make_sw128_map(&token_map, args.a_rows, kInt8, token_rows, args.k, kW8A16 ? kRowTile : kTokenBox)) {
     return cudaErrorInvalidValue;
   }
   const int n_blocks = (args.n_out + kBlockM - 1) / kBlockM;
