@@ -74,7 +74,7 @@ struct PairControl {
   uint64_t full[kStages];
   uint64_t empty[kStages];
   uint64_t acc_full[2];
-  uint64_t acc_part[2];   // the blocks of the unit that the next unit's accumulator takes over have been read
+  uint64_t acc_part;      // the blocks of a unit that the next unit's accumulator takes over have been read (units that hand none over skip it)
   uint64_t acc_empty[2];
   uint32_t tmem_base;
   volatile int abort_flag;
@@ -304,9 +304,9 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
     }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(&ctl->acc_full[b], 1);
-      ptx::mbar_init(&ctl->acc_part[b], 2 * kEpilogueWarps);  // the epilogue warps of both CTAs
-      ptx::mbar_init(&ctl->acc_empty[b], 2 * kEpilogueWarps);
+      ptx::mbar_init(&ctl->acc_empty[b], 2 * kEpilogueWarps);  // the epilogue warps of both CTAs
     }
+    ptx::mbar_init(&ctl->acc_part, 2 * kEpilogueWarps);
     ctl->abort_flag = 0;
     ptx::fence_barrier_init();
   }
@@ -343,7 +343,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
       UnitInfo cur = warp_uniform(load_unit(args.items, first_unit, units, n_blocks, kRowsPerRoute));
       int ring_end = 0;
       for (int64_t unit = first_unit; unit < units; unit += unit_stride) {
-        const UnitInfo next = warp_uniform(load_unit(args.items, unit + unit_stride, units, n_blocks, kRowsPerRoute));  // in flight during this unit
+        const UnitInfo next = load_unit(args.items, unit + unit_stride, units, n_blocks, kRowsPerRoute);  // in flight during this unit
         // An MMA of N columns takes its first N/2 token rows from the leader's tile and the other N/2 from the follower's:
         // 16 rows per CTA and block.  One box brings the rows of a one-MMA unit, up to the next box size (a few
         // boxes of exactly its rows move less and take longer: about 512 rows per expert, 16384 tokens, 8087 -> 8216 us);
@@ -353,6 +353,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
         const int tail = slot.blocks - slot.head;
         const int head_row = cur.row0 + slot.head * kBoxTokens * static_cast<int>(cta);
         const int tail_row = cur.row0 + slot.head * 32 + tail * kBoxTokens * static_cast<int>(cta);
+        const CUtensorMap* const one_box = slot.head <= kMidBox ? &token_map_mid : &token_map_full;
         const int loaded = tail > 0 ? slot.blocks : slot.head <= kMidBox ? kMidBox : kFullBox;
         const uint32_t stage_tx = 2u * (kWeightBytes + static_cast<uint32_t>(loaded) * kBoxTokens * kBlockKBytes);
         const int channel0 = cur.block * kChannelsPerUnit + (kChannelsPerUnit / 2) * static_cast<int>(cta);
@@ -391,7 +392,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
               for (; b < blocks; ++b) tma_load_2d_pair(to + b * kBoxTokens * kBlockKBytes, &token_map, bar, x, row + b * kBoxTokens);
             };
             if (tail == 0) {
-              tma_load_2d_pair(tokens, slot.head <= kMidBox ? &token_map_mid : &token_map_full, bar, x, head_row);
+              tma_load_2d_pair(tokens, one_box, bar, x, head_row);
             } else {
               load_tokens(tokens, slot.head, head_row);
               load_tokens(tokens + slot.head * kBoxTokens * kBlockKBytes, tail, tail_row);
@@ -403,7 +404,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
             phase ^= 1u;
           }
         }
-        cur = next;
+        cur = warp_uniform(next);
       }
       if (leader) {
         // Drain: the leader's full barriers count both CTAs' bytes, so this also covers the follower's loads.
@@ -444,6 +445,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
       int local = 0;
       UnitInfo cur = load_unit(args.items, first_unit, units, n_blocks, kRowsPerRoute);
       AccSlot before = {0, 0, 0};
+      uint32_t handovers = 0;
       for (int64_t unit = first_unit; unit < units; unit += unit_stride, ++local) {
         const UnitInfo next = load_unit(args.items, unit + unit_stride, units, n_blocks, kRowsPerRoute);
         const uint32_t buffer = static_cast<uint32_t>(local) & 1u;
@@ -455,17 +457,18 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
         const int tail = __shfl_sync(0xffffffffu, slot.blocks - slot.head, 0);
         const uint32_t idesc_head = __shfl_sync(0xffffffffu, ptx::make_instr_desc(kInt8, 2 * kRowsPerCta, 32 * slot.head), 0);
         const uint32_t idesc_tail = __shfl_sync(0xffffffffu, ptx::make_instr_desc(kInt8, 2 * kRowsPerCta, 32 * tail), 0);
-        // The unit two before this one has left tensor memory, and the one before it the blocks that this one takes over.
-        ptx::mbar_wait(&ctl->acc_empty[buffer], (use & 1u) ^ 1u, abort_flag, status, 12);
-        if (local > 0 && blocks_shared(before, slot) > 0) {
-          ptx::mbar_wait(&ctl->acc_part[buffer ^ 1u], (static_cast<uint32_t>(local - 1) >> 1) & 1u, abort_flag, status, 15);
-        }
-        before = slot;
-        ptx::tcgen05_fence_after();
         const uint32_t acc_head = __shfl_sync(0xffffffffu, tmem_base + 32u * static_cast<uint32_t>(slot.start & (kRingBlocks - 1)), 0);
         const uint32_t acc_tail =
             __shfl_sync(0xffffffffu, tmem_base + 32u * static_cast<uint32_t>((slot.start + slot.head) & (kRingBlocks - 1)), 0);
         const uint32_t tail_step = __shfl_sync(0xffffffffu, kTokenStep + kBlockStep * static_cast<uint32_t>(slot.head), 0);
+        // The unit two before this one has left tensor memory, and the one before it the blocks that this one takes over.
+        ptx::mbar_wait(&ctl->acc_empty[buffer], (use & 1u) ^ 1u, abort_flag, status, 12);
+        if (blocks_shared(before, slot) > 0) {
+          ptx::mbar_wait(&ctl->acc_part, handovers & 1u, abort_flag, status, 15);
+          ++handovers;
+        }
+        before = slot;
+        ptx::tcgen05_fence_after();
         // One loop per form: the usual one carries nothing of the other.
         auto main_loop = [&](auto tail_tag) {
           uint32_t accumulate = 0;
@@ -526,7 +529,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
     // Output channel of this thread inside the unit's channel block.
     const int channel_in_unit = kGateUp ? 64 * static_cast<int>(cta) + 16 * quarter + (lane & 15)
                                         : kRowsPerCta * static_cast<int>(cta) + lane_in_tile;
-    const uint32_t acc_part_leader = map_to_cta(ptx::smem_u32(&ctl->acc_part[0]), 0);
+    const uint32_t acc_part_leader = map_to_cta(ptx::smem_u32(&ctl->acc_part), 0);
     const uint32_t acc_empty_leader = map_to_cta(ptx::smem_u32(&ctl->acc_empty[0]), 0);
     const uint32_t acc_lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t* exp_table = ctl->exp_table;
@@ -640,12 +643,12 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
       // The next unit's accumulator may start on this one's first blocks: they are released as soon as they are read.
       const AccSlot next_slot = place_unit(slot.start + slot.blocks, next.rows);
       const int handed_over = blocks_shared(slot, next_slot);
-      bool part_released = false;
+      bool part_released = handed_over == 0;
       auto release_part = [&]() {
         part_released = true;
         ptx::tcgen05_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(acc_part_leader + 8u * buffer);
+        if (lane == 0) mbar_arrive_cluster(acc_part_leader);
       };
       for (int chunk = chunk_first; chunk < chunks; chunk += kChunkStep) {
         if (!part_released && chunk >= handed_over) release_part();
