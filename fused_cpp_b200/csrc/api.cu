@@ -758,8 +758,8 @@ DenseLayout dense_layout(int64_t rows, int k) {
   return d;
 }
 
-// One or two int8 products over the rows that dense_prologue quantised: up to kDenseMaxRows rows one launch of the
-// split-K kernel, above that one launch of the two-SM kernel (256-row work items) per matrix.
+// One or two int8 products over the rows that dense_prologue quantised: one launch of the split-K kernel where
+// dense_split_pays, else one launch of the two-SM kernel (256-row work items) per matrix.
 // FUSED_CPP_MOE_DENSE_SPLIT=0 keeps the K range of a channel block in one CTA.
 struct DenseProduct {
   const int8_t* w;
@@ -769,9 +769,26 @@ struct DenseProduct {
   void* out;
 };
 
+// Above kDenseMaxRows rows the split-K kernel takes products that would leave the two-SM kernel most of the chip idle: at most
+// 74 tiles of 128 x 128, one for every second SM, over a K range long enough (5120) to pay for the exchange of the parts.
+// Two-SM / split-K kernel, device time per op: 7168 -> 1536 at 129 / 256 / 512 / 768 rows 20.4 / 26.8 / 28.9 / 30.9 us ->
+// 18.4 / 19.4 / 23.3 / 27.0 us; 7168 -> 130 at 200 / 1000 / 4000 rows 28.5 / 36.1 / 58.3 -> 15.8 / 23.9 / 48.2; 16384 -> 4096
+// at 200 rows 45.1 -> 32.3.  Beyond the lines: 4096 -> 3072 at 384 rows 20.4 -> 20.5, 1536 -> 2048 at 129 rows 12.6 -> 16.4,
+// 16384 -> 7168 at 300 rows (168 tiles) 54.8 -> 67.0, 8192 -> 8192 at 150 rows (128 tiles) 23.2 -> 30.1.
+bool dense_split_pays(int64_t rows, int k_padded, const DenseProduct* products, int count, bool split) {
+  if (rows <= fmoe::kDenseMaxRows) return true;
+  if (!split) return false;
+  int64_t tiles = 0;
+  for (int i = 0; i < count; ++i) tiles += (static_cast<int64_t>(products[i].n) + 127) / 128;
+  tiles *= (rows + fmoe::kDenseMaxRows - 1) / fmoe::kDenseMaxRows;
+  return tiles <= 74 && k_padded >= 5120;
+}
+
 cudaError_t dense_gemm(const DenseLayout& d, char* base, int64_t rows, const DenseProduct* products, int count, int out_is_bf16,
                        cudaStream_t stream) {
-  if (rows <= fmoe::kDenseMaxRows) {
+  const char* text = getenv("FUSED_CPP_MOE_DENSE_SPLIT");
+  const bool split = text == nullptr || text[0] != '0';
+  if (dense_split_pays(rows, d.k_padded, products, count, split)) {
     fmoe::DenseGemmArgs args;
     memset(&args, 0, sizeof(args));
     const int8_t* weights[2] = {nullptr, nullptr};
@@ -787,8 +804,7 @@ cudaError_t dense_gemm(const DenseLayout& d, char* base, int64_t rows, const Den
     args.rows = static_cast<int>(rows);
     args.k_padded = d.k_padded;
     args.status = reinterpret_cast<int*>(base + d.status);
-    const char* text = getenv("FUSED_CPP_MOE_DENSE_SPLIT");
-    return fmoe::launch_dense_gemm(args, base + d.xq, weights, text == nullptr || text[0] != '0', stream);
+    return fmoe::launch_dense_gemm(args, base + d.xq, weights, split, stream);
   }
   cudaError_t error = cudaSuccess;
   for (int i = 0; i < count && error == cudaSuccess; ++i) {

@@ -1,4 +1,4 @@
-// Dense W8A8 linear over at most 128 rows: out[row, n] = (acc * row scale) * channel scale (+ bias[n]), acc = Xq * W^T
+// Dense W8A8 linear over few rows, or few channels and a long K range: out[row, n] = (acc * row scale) * channel scale (+ bias[n]), acc = Xq * W^T
 // (csrc/i8gemm.cpp:147-165), for one weight matrix or for two that share the quantised rows (csrc/i8gemm.cpp:454-570).
 //
 // Such a product streams its weights once and does almost nothing else, so what bounds it is HBM if enough SMs ask for
@@ -10,6 +10,8 @@
 //   * The launch is a programmatic dependent of the row quantiser: barriers, tensor memory and the weight tiles of
 //     every pipeline stage (up to 80 KB per CTA, two CTAs per SM) are fetched while the quantiser still runs; only the
 //     token tiles and row scales wait for it.
+//   * More than 128 rows are tiles of 128, a cluster each; the tiles of a channel block are neighbours and share its weights
+//     in L2 (api.cu, dense_split_pays, says when that beats the two-SM kernel).
 //   * Two weight matrices are one launch: the second one's channel blocks follow the first one's.
 // Device time per op in a chain of ops (quantiser included; floor = weights at the copy bandwidth), against a persistent
 // kernel without the cluster (a K split up to 16 rows over an int32 table with atomics) behind a finished quantiser:
@@ -130,7 +132,10 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
   int* status = args.status;
   const int parts = args.parts;
   const int part = static_cast<int>(blockIdx.x) % parts;  // = rank in the cluster
-  const int all_blocks = static_cast<int>(blockIdx.x) / parts;
+  const int unit = static_cast<int>(blockIdx.x) / parts;  // row tiles of a channel block side by side: they share its weights
+  const int all_blocks = unit / args.row_tiles;
+  const int row0 = (unit - all_blocks * args.row_tiles) * kRowTile;
+  const int rows = min(kRowTile, args.rows - row0);  // of this CTA's tile
   const bool second = all_blocks >= args.first_blocks;
   const Side side = {second ? args.w_scale[1] : args.w_scale[0], second ? args.out[1] : args.out[0], second ? args.n[1] : args.n[0], args.out_bf16};
   const int n0 = (all_blocks - (second ? args.first_blocks : 0)) * kBlockM;
@@ -171,7 +176,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
     ptx::grid_dependency_wait();
     for (int i = 0; i < ahead; ++i) {
       if (issuer) {
-        ptx::tma_load_2d(smem + static_cast<size_t>(i) * Cfg::kStageBytes + kWeightBytes, &token_map, &ctl->full[i], (kb_begin + i) * kBlockKBytes, 0);
+        ptx::tma_load_2d(smem + static_cast<size_t>(i) * Cfg::kStageBytes + kWeightBytes, &token_map, &ctl->full[i], (kb_begin + i) * kBlockKBytes, row0);
       }
     }
     int stage = ahead == Cfg::kStages ? 0 : ahead;
@@ -182,7 +187,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
         uint8_t* stage_base = smem + static_cast<size_t>(stage) * Cfg::kStageBytes;
         ptx::mbar_arrive_expect_tx(&ctl->full[stage], Cfg::kStageBytes);
         ptx::tma_load_2d(stage_base, weight_map, &ctl->full[stage], (kb_begin + i) * kBlockKBytes, n0);
-        ptx::tma_load_2d(stage_base + kWeightBytes, &token_map, &ctl->full[stage], (kb_begin + i) * kBlockKBytes, 0);
+        ptx::tma_load_2d(stage_base + kWeightBytes, &token_map, &ctl->full[stage], (kb_begin + i) * kBlockKBytes, row0);
       }
       if (++stage == Cfg::kStages) {
         stage = 0;
@@ -205,7 +210,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     const bool issuer = ptx::elect_one();
-    const uint32_t idesc = ptx::make_instr_desc(true, kBlockM, min(kRowTile, (args.rows + 15) & ~15));
+    const uint32_t idesc = ptx::make_instr_desc(true, kBlockM, (rows + 15) & ~15);
     int stage = 0;
     uint32_t phase = 0;
     for (int i = 0; i < count; ++i) {
@@ -242,12 +247,12 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
       if (!second && args.bias != nullptr) bias = args.bias[n];
     }
     ptx::grid_dependency_wait();  // the row scales come from the quantiser
-    if (thread < args.rows) ctl->row_scale[thread] = args.a_scale[thread];
+    if (thread < rows) ctl->row_scale[thread] = args.a_scale[row0 + thread];
     asm volatile("bar.sync 1, 128;" ::: "memory");
     ptx::mbar_wait(&ctl->acc_full, 0, abort_flag, status, 23);
     ptx::tcgen05_fence_after();
     const uint32_t acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    for (int c0 = 0; c0 < args.rows; c0 += 16) {
+    for (int c0 = 0; c0 < rows; c0 += 16) {
       uint32_t bits[16];
       ptx::tmem_ld_x8(acc + c0, bits);
       ptx::tmem_ld_x8(acc + c0 + 8, bits + 8);
@@ -255,11 +260,11 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int row = c0 + j;
-        if (row >= args.rows) continue;
+        if (row >= rows) continue;
         if (parts > 1) {
           exchange[row * kBlockM + channel] = static_cast<int>(bits[j]);
         } else if (channel_ok) {
-          store_value(side, row, n, static_cast<int>(bits[j]), ctl->row_scale[row], channel_scale, bias);
+          store_value(side, row0 + row, n, static_cast<int>(bits[j]), ctl->row_scale[row], channel_scale, bias);
         }
       }
     }
@@ -280,7 +285,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
       }
       const bool vector_store = side.n % 4 == 0;  // then a lane's four channels all exist or none does
       constexpr int kBatch = 2;  // rows of a warp whose loads are in flight together (a remote load takes most of a microsecond)
-      for (int first = part + parts * (warp - 2); first < args.rows; first += 4 * parts * kBatch) {
+      for (int first = part + parts * (warp - 2); first < rows; first += 4 * parts * kBatch) {
         int4 values[kBatch][kMaxParts];
 #pragma unroll
         for (int b = 0; b < kBatch; ++b) {
@@ -288,13 +293,13 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
 #pragma unroll
           for (int c = 0; c < kMaxParts; ++c) {
             values[b][c] = make_int4(0, 0, 0, 0);
-            if (c < parts && row < args.rows) values[b][c] = load_cluster_int4(mine + static_cast<uint32_t>(row) * (kBlockM * 4), c);
+            if (c < parts && row < rows) values[b][c] = load_cluster_int4(mine + static_cast<uint32_t>(row) * (kBlockM * 4), c);
           }
         }
 #pragma unroll
         for (int b = 0; b < kBatch; ++b) {
           const int row = first + 4 * parts * b;
-          if (row >= args.rows || columns <= 0) continue;
+          if (row >= rows || columns <= 0) continue;
           int4 sum = values[b][0];
 #pragma unroll
           for (int c = 1; c < kMaxParts; ++c) {
@@ -303,7 +308,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
             sum.z += values[b][c].z;
             sum.w += values[b][c].w;
           }
-          store_row4(side, row, n0 + c4, sum, ctl->row_scale[row], scales, biases, columns, vector_store);
+          store_row4(side, row0 + row, n0 + c4, sum, ctl->row_scale[row], scales, biases, columns, vector_store);
         }
       }
     }
@@ -397,7 +402,7 @@ cudaError_t launch_dense(DenseGemmArgs args, const void* a_rows, const int8_t* c
   Residency one_per_sm;
   const cudaError_t error = residency<kRowTile>(&one_per_sm);
   if (error != cudaSuccess) return error;
-  const int blocks = args.first_blocks + (args.n[1] + kBlockM - 1) / kBlockM;
+  const int blocks = (args.first_blocks + (args.n[1] + kBlockM - 1) / kBlockM) * args.row_tiles;
   // As many parts as leave all clusters resident at once, two CTAs per SM if need be, every part at least two K blocks.
   // Device time per op of a chain of ops, parts 1 / 2 / 3 / 4 / 5 / 8, 64 rows: 16384 -> 7168 (56 blocks; clusters of five
   // and more take a second wave) 37 / 31 / 31 / 29.5 / 39 / 38 us; 7168 -> 1536 (12 blocks) 21 / 16 / 14 / 13 / 12 / 11.5 us;
@@ -418,7 +423,8 @@ cudaError_t launch_dense(DenseGemmArgs args, const void* a_rows, const int8_t* c
 
 cudaError_t launch_dense_gemm(const DenseGemmArgs& caller_args, const void* a_rows, const int8_t* const* weights, bool split, cudaStream_t stream) {
   DenseGemmArgs args = caller_args;
-  if (args.rows <= 0 || args.rows > kDenseMaxRows || args.n[0] <= 0 || args.k_padded % 16 != 0) return cudaErrorInvalidValue;
+  if (args.rows <= 0 || args.n[0] <= 0 || args.k_padded % 16 != 0) return cudaErrorInvalidValue;
+  args.row_tiles = (args.rows + kDenseMaxRows - 1) / kDenseMaxRows;
   args.first_blocks = (args.n[0] + kBlockM - 1) / kBlockM;
   args.k_blocks = (args.k_padded + kBlockKBytes - 1) / kBlockKBytes;
   if (args.rows <= 16) return launch_dense<16>(args, a_rows, weights, split, stream);

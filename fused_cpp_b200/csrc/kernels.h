@@ -270,7 +270,7 @@ inline int sm_count_of_current_device() {
 // 2-D K-major tensor [rows, k] with 128-byte-swizzled boxes of {128 bytes of K, box_rows} (umma_gemm.cu).
 bool make_sw128_map(CUtensorMap* map, const void* base, bool int8, uint64_t rows, uint64_t k, uint32_t box_rows);
 
-// ---- dense_gemm.cu: dense W8A8 linear over at most kDenseMaxRows rows, one or two weight matrices in one launch.
+// ---- dense_gemm.cu: dense W8A8 linear over tiles of kDenseMaxRows rows, one or two weight matrices in one launch.
 // Programmatic dependent of the kernel in front of it in the stream (the row quantiser that writes a_rows / a_scale).
 constexpr int kDenseMaxRows = 128;
 struct DenseGemmArgs {
@@ -283,7 +283,7 @@ struct DenseGemmArgs {
   int rows;
   int k_padded;
   int* status;
-  int first_blocks, k_blocks, parts;  // set by the launcher
+  int row_tiles, first_blocks, k_blocks, parts;  // set by the launcher
 };
 cudaError_t launch_dense_gemm(const DenseGemmArgs& args, const void* a_rows, const int8_t* const* weights, bool split, cudaStream_t stream);
 

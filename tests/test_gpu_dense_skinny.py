@@ -22,6 +22,10 @@ def _weight(n, k, generator):
     (33, 1000, 130, torch.float32, torch.float32, True), (64, 4096, 1536, torch.bfloat16, torch.bfloat16, True),
     (65, 777, 300, torch.bfloat16, torch.bfloat16, False), (128, 1536, 4000, torch.bfloat16, torch.bfloat16, True),
     (129, 1536, 300, torch.float32, torch.bfloat16, True), (3, 16384, 136, torch.bfloat16, torch.bfloat16, False),
+    # Above 128 rows with a long K range: row tiles of the split kernel, the last one short, and its limits.
+    (129, 5200, 300, torch.bfloat16, torch.bfloat16, True), (256, 5120, 130, torch.float32, torch.float32, True),
+    (385, 5128, 257, torch.bfloat16, torch.float32, False), (300, 5112, 64, torch.bfloat16, torch.bfloat16, False),
+    (1100, 5120, 1025, torch.bfloat16, torch.bfloat16, True), (1100, 5120, 1000, torch.bfloat16, torch.bfloat16, False),
     (5, 16400, 200, torch.bfloat16, torch.float32, True), (2, 16392, 64, torch.float32, torch.float32, False),
 ])
 def test_product(cuda_device, rows, k, n, x_dtype, out_dtype, with_bias):
@@ -33,7 +37,7 @@ def test_product(cuda_device, rows, k, n, x_dtype, out_dtype, with_bias):
     torch.testing.assert_close(got.cpu(), oracle.i8gemm_dynamic(x, weight, scale, bias, out_dtype), atol=0, rtol=0)
 
 
-@pytest.mark.parametrize("rows,k,first_n,second_n", [(1, 1536, 4000, 72), (40, 512, 130, 129), (128, 300, 64, 700), (200, 512, 300, 130)])
+@pytest.mark.parametrize("rows,k,first_n,second_n", [(1, 1536, 4000, 72), (40, 512, 130, 129), (128, 300, 64, 700), (200, 512, 300, 130), (200, 5136, 130, 260)])
 def test_pair(cuda_device, rows, k, first_n, second_n):
     generator = torch.Generator().manual_seed(rows + k)
     first, second = _weight(first_n, k, generator), _weight(second_n, k, generator)
