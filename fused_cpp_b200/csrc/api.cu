@@ -261,7 +261,12 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
     return fail(FMOE_ERR_INVALID_ARGUMENT, "row tiles must be 16, 32, 64, 128, 256 or 512 = two-SM pairs (got %d, %d)", tile_gu, tile_dn);
   }
   // Tile 512 selects the two-SM kernel, whatever its work items hold.
-  const int pair_item_rows = planes ? fmoe::kPairItemRows / 2 : fmoe::kPairItemRows;  // in routes (two token rows each with planes)
+  // They hold up to 320 token rows where the batch has a work unit for every SM at 256 rows a unit, and 256 where it has not:
+  // there more, smaller units are what keeps SM pairs busy (one expert of 7168 x 2048 over 300 rows, bf16: 111 us as one
+  // item, 82 us as two).
+  const int64_t pair_blocks = (f.inter + 127) / 128 < (f.hidden + 255) / 256 ? (f.inter + 127) / 128 : (f.hidden + 255) / 256;
+  const bool tall_items = (planes ? 2 : 1) * routes / 256 * pair_blocks >= fmoe::sm_count_of_current_device();
+  const int pair_item_rows = (tall_items ? fmoe::kPairItemRows : 256) / (planes ? 2 : 1);  // in routes (two token rows each with planes)
   const int item_rows_gu = tile_gu == fmoe::kPairRowTile ? pair_item_rows : tile_gu;
   const int item_rows_dn = tile_dn == fmoe::kPairRowTile ? pair_item_rows : tile_dn;
 

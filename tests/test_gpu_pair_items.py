@@ -20,7 +20,7 @@ ODD = [289] * 10
 @pytest.mark.parametrize("rows", [MIXED, EVEN, ODD], ids=["mixed", "even", "odd"])
 @pytest.mark.parametrize("kind", ["w8a8", "w8a16", "bf16"])
 def test_against_one_sm_kernel(cuda_device, kind, rows):
-    hidden, inter, experts = 2304, 2048, len(rows)
+    hidden, inter, experts = 4096, 2048, len(rows)
     if kind == "w8a16":
         rows = [(r + 1) // 2 for r in rows]  # two token rows per route
     generator = torch.Generator(device=cuda_device).manual_seed(sum(rows))
