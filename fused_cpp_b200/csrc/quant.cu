@@ -545,15 +545,51 @@ quantize_rows_dense_vec8_kernel(const void* __restrict__ x, int cols, int cols_p
   if (threadIdx.x == 0 && cols_padded > cols) dst[vec8] = make_uint2(0u, 0u);
 }
 
+// bf16 rows by the thousand, or longer than the registers of a CTA hold: a 256-thread CTA reads its row twice, the second
+// time out of L1, and eight of them fit an SM (3000 rows of 7168 columns 19 us, 24 us with the row in registers; of the
+// other kernel's shorter latency nothing is left from four rows per SM on).
+__global__ void __launch_bounds__(kQuantThreads)
+quantize_rows_dense_bf16x8_kernel(const uint16_t* __restrict__ x, int cols, int cols_padded, int8_t* __restrict__ q,
+                                  float* __restrict__ scale_out, DenseItems dense_items) {
+  ptx::launch_dependents();
+  __shared__ float smem[32];
+  if (blockIdx.x == 0) write_dense_items(dense_items);
+  const int64_t row = blockIdx.x;
+  const uint4* src = reinterpret_cast<const uint4*>(x + row * cols);
+  const int vec8 = cols >> 3;
+  float local = 0.0f;
+  for (int v = threadIdx.x; v < vec8; v += kQuantThreads) local = fmaxf(local, amax8(src[v]));
+  const float amax = block_max(local, smem);
+  const float scale = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 1.0f;
+  if (threadIdx.x == 0) scale_out[row] = scale;
+  const float inverse = __fdiv_rn(1.0f, scale);
+  uint2* dst = reinterpret_cast<uint2*>(q + row * cols_padded);
+  const int vec8_padded = cols_padded >> 3;
+  for (int v = threadIdx.x; v < vec8_padded; v += kQuantThreads) {
+    uint2 out = make_uint2(0u, 0u);
+    if (v < vec8) {
+      float values[8];
+      unpack8(src[v], values);
+      out.x = quantize4_torchref_fast(values, scale, inverse);
+      out.y = quantize4_torchref_fast(values + 4, scale, inverse);
+    }
+    dst[v] = out;
+  }
+}
+
 cudaError_t launch_quantize_rows_dense(const void* x, int x_is_bf16, int64_t rows, int cols, int cols_padded, int clamp_low,
                                        int8_t* q, float* scale, int row_tile, int max_items, int* items, int* status,
                                        cudaStream_t stream) {
   if (rows <= 0) return cudaSuccess;
   const DenseItems dense_items = {rows, row_tile, max_items, items, status};
   const int vec8 = cols >> 3;
-  const bool vector_form = cols % 8 == 0 && vec8 <= 1024 * kDenseVectors && cols_padded - cols <= 8 && cols_padded % 8 == 0 &&
-                           (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(q) & 7u) == 0;
-  if (vector_form) {
+  const bool aligned = cols % 8 == 0 && cols_padded - cols <= 8 && cols_padded % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
+                       (reinterpret_cast<uintptr_t>(q) & 7u) == 0;
+  const bool held = vec8 <= 1024 * kDenseVectors;  // a row fits the registers of one CTA
+  if (aligned && x_is_bf16 && (rows > 592 || !held)) {
+    quantize_rows_dense_bf16x8_kernel<<<static_cast<unsigned>(rows), kQuantThreads, 0, stream>>>(static_cast<const uint16_t*>(x), cols,
+                                                                                                cols_padded, q, scale, dense_items);
+  } else if (aligned && held) {
     int threads = 64;
     while (threads * kDenseVectors < vec8) threads *= 2;
     auto kernel = x_is_bf16 ? quantize_rows_dense_vec8_kernel<true> : quantize_rows_dense_vec8_kernel<false>;

@@ -26,6 +26,7 @@ def _weight(n, k, generator):
     (129, 5200, 300, torch.bfloat16, torch.bfloat16, True), (256, 5120, 130, torch.float32, torch.float32, True),
     (385, 5128, 257, torch.bfloat16, torch.float32, False), (300, 5112, 64, torch.bfloat16, torch.bfloat16, False),
     (1100, 5120, 1025, torch.bfloat16, torch.bfloat16, True), (1100, 5120, 1000, torch.bfloat16, torch.bfloat16, False),
+    (592, 264, 130, torch.bfloat16, torch.bfloat16, False), (593, 264, 130, torch.bfloat16, torch.bfloat16, True),
     (5, 16400, 200, torch.bfloat16, torch.float32, True), (2, 16392, 64, torch.float32, torch.float32, False),
 ])
 def test_product(cuda_device, rows, k, n, x_dtype, out_dtype, with_bias):
