@@ -92,7 +92,7 @@ __device__ __forceinline__ void store_value(const Side& side, int row, int n, in
   }
 }
 
-// Four channels of a row, of which `columns` exist; vector_store: the row length is a multiple of four (then all four do).
+// Four channels of a row, of which `columns` exist; vector_store: dense_vector_store holds (then all four do).
 __device__ __forceinline__ void store_row4(const Side& side, int row, int n, int4 acc, float row_scale, const float* scales, const float* biases,
                                            int columns, bool vector_store) {
   const int sums[4] = {acc.x, acc.y, acc.z, acc.w};
@@ -283,7 +283,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
         scales[j] = j < columns ? side.w_scale[n0 + c4 + j] : 1.0f;
         biases[j] = (!second && args.bias != nullptr && j < columns) ? args.bias[n0 + c4 + j] : 0.0f;
       }
-      const bool vector_store = side.n % 4 == 0;  // then a lane's four channels all exist or none does
+      const bool vector_store = (second ? args.vector_store[1] : args.vector_store[0]) != 0;  // a lane's four channels all exist or none does
       constexpr int kBatch = 2;  // rows of a warp whose loads are in flight together (a remote load takes most of a microsecond)
       for (int first = part + parts * (warp - 2); first < rows; first += 4 * parts * kBatch) {
         int4 values[kBatch][kMaxParts];
@@ -427,6 +427,7 @@ cudaError_t launch_dense_gemm(const DenseGemmArgs& caller_args, const void* a_ro
   args.row_tiles = (args.rows + kDenseMaxRows - 1) / kDenseMaxRows;
   args.first_blocks = (args.n[0] + kBlockM - 1) / kBlockM;
   args.k_blocks = (args.k_padded + kBlockKBytes - 1) / kBlockKBytes;
+  for (int i = 0; i < 2; ++i) args.vector_store[i] = dense_vector_store(args.out[i], args.n[i], args.out_bf16 != 0) ? 1 : 0;
   if (args.rows <= 16) return launch_dense<16>(args, a_rows, weights, split, stream);
   if (args.rows <= 32) return launch_dense<32>(args, a_rows, weights, split, stream);
   if (args.rows <= 64) return launch_dense<64>(args, a_rows, weights, split, stream);

@@ -283,8 +283,14 @@ struct DenseGemmArgs {
   int rows;
   int k_padded;
   int* status;
-  int row_tiles, first_blocks, k_blocks, parts;  // set by the launcher
+  int row_tiles, first_blocks, k_blocks, parts, vector_store[2];  // set by the launcher
 };
+// Whether every group of four channels of a dense output, from channel 0 of any row on, may be stored as one vector (8 bytes of
+// bf16, 16 of fp32): the rows keep the alignment of the first one, and that is the caller's, who may pass a view that starts
+// at any element.
+inline bool dense_vector_store(const void* out, int n, bool bf16) {
+  return n % 4 == 0 && reinterpret_cast<uintptr_t>(out) % (bf16 ? 8 : 16) == 0;
+}
 cudaError_t launch_dense_gemm(const DenseGemmArgs& args, const void* a_rows, const int8_t* const* weights, bool split, cudaStream_t stream);
 
 // ---- simt_gemm.cu: CUDA-core grouped GEMM of the diagnostic library only (work items of at most 8 rows)

@@ -46,3 +46,27 @@ def test_pair(cuda_device, rows, k, first_n, second_n):
     got = i8gemm.dynamic_scaled_mm_pair(x.to(cuda_device), i8gemm.prepare(*first), i8gemm.prepare(*second))
     for out, (weight, scale) in zip(got, (first, second)):
         torch.testing.assert_close(out.cpu(), oracle.i8gemm_dynamic(x, weight, scale, None, torch.bfloat16, clamp_low=-127), atol=0, rtol=0)
+
+
+@pytest.mark.parametrize("rows,k,n", [(5, 2048, 1536), (70, 1024, 136), (200, 5120, 512)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("offset", [0, 1, 2, 4, 8])
+def test_output_view_at_any_element(cuda_device, rows, k, n, out_dtype, offset):
+    """The caller's output may start at any element of an allocation (a K split stores vectors only where that is aligned)."""
+    generator = torch.Generator().manual_seed(rows + k)
+    weight, scale = _weight(n, k, generator)
+    x = torch.randn((rows, k), generator=generator).to(torch.bfloat16)
+    packed = i8gemm.prepare(weight, scale)
+    buffer = torch.full((offset + rows * n + 8,), 7.0, dtype=out_dtype, device=cuda_device)
+    out = buffer[offset:offset + rows * n].view(rows, n)
+    i8gemm.i8gemm_dynamic_scaled_mm(out, x.to(cuda_device), packed.packed_weight, packed.weight_scale, None, packed.k, packed.n,
+                                    packed.k_padded, packed.n_padded)
+    assert torch.equal(out.cpu(), oracle.i8gemm_dynamic(x, weight, scale, None, out_dtype))
+    assert bool((buffer[:offset] == 7).all()) and bool((buffer[offset + rows * n:] == 7).all())
+    if out_dtype is torch.bfloat16:
+        other = torch.empty_like(out)
+        i8gemm.i8gemm_dynamic_scaled_mm_pair(out, other, x.to(cuda_device), packed.packed_weight, packed.weight_scale, packed.k,
+                                             packed.n, packed.k_padded, packed.n_padded, packed.packed_weight, packed.weight_scale,
+                                             packed.n, packed.n_padded)
+        assert torch.equal(out, other)
+        assert torch.equal(other.cpu(), oracle.i8gemm_dynamic(x, weight, scale, None, out_dtype, clamp_low=-127))
