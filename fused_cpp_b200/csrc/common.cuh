@@ -154,15 +154,16 @@ __device__ __forceinline__ float row_scale_from_amax(float amax, int numerics) {
   return scale < 1.0e-30f ? 1.0e-30f : scale;
 }
 
-// One activation value -> int8.  `scale_or_inverse` is 1/scale for NATIVE and scale for TORCHREF.
-__device__ __forceinline__ int quantize_value(float value, float scale_or_inverse, int numerics) {
+// One activation value -> int8.  `scale_or_inverse` is 1/scale for NATIVE and scale for TORCHREF; clamp_low: -127, or -128
+// for the single dense product.
+__device__ __forceinline__ int quantize_value(float value, float scale_or_inverse, int numerics, float clamp_low = -127.0f) {
   if (numerics == FMOE_NUMERICS_NATIVE) {
     float scaled = __fmul_rn(value, scale_or_inverse);
     scaled = fmaxf(fminf(scaled, 127.0f), -127.0f);
     return static_cast<int>(roundf(scaled));  // ties away from zero
   }
   float rounded = rintf(__fdiv_rn(value, scale_or_inverse));  // ties to even
-  rounded = fmaxf(fminf(rounded, 127.0f), -127.0f);
+  rounded = fmaxf(fminf(rounded, 127.0f), clamp_low);
   return static_cast<int>(rounded);
 }
 
@@ -179,12 +180,13 @@ __device__ __forceinline__ float max_or_nan(float a, float b) {
 // Bit-identical to quantize_value(TORCHREF).  Adding 1.5 * 2^23 rounds the product (exact inside the fused multiply-add)
 // to the nearest integer, ties to even, in the low mantissa bits: the byte is read out of the sum's bit pattern and
 // subtracting the constant again gives the integer for the boundary test, whose maximum keeps NaN.  No conversion
-// instruction and no clamp: a quotient beyond +-127.5 would need a scale that is not the row's, and what is not finite (a
-// NaN value, an infinite row, a scale whose reciprocal overflows) is a NaN in the test and goes to the exact statement.
+// instruction and no clamp: a quotient beyond +-127.5 needs a scale that is not the row's, or one of so few units of the
+// smallest fp32 number that amax / 127 was rounded by 0.4 % (below 2^-141).  Such a scale's reciprocal overflows, and what is
+// not finite (that, a NaN value, an infinite row) is a NaN or an infinity in the test and goes to the exact statement.
 // One test per four values; the exact statement decides all four when any of them asks for it.  Four instructions
 // per value: with the clamp, the product and its distance as separate operations (seven) 65536 rows of 2048 columns took
 // 112 us, 105 us like this.
-__device__ __forceinline__ uint32_t quantize4_torchref_fast(const float* values, float scale, float inverse) {
+__device__ __forceinline__ uint32_t quantize4_torchref_fast(const float* values, float scale, float inverse, float clamp_low = -127.0f) {
   constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
   uint32_t bits[4];
   float worst = 0.0f;
@@ -199,7 +201,7 @@ __device__ __forceinline__ uint32_t quantize4_torchref_fast(const float* values,
     uint32_t packed = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      packed |= (static_cast<uint32_t>(quantize_value(values[i], scale, FMOE_NUMERICS_TORCHREF)) & 0xffu) << (8 * i);
+      packed |= (static_cast<uint32_t>(quantize_value(values[i], scale, FMOE_NUMERICS_TORCHREF, clamp_low)) & 0xffu) << (8 * i);
     }
     return packed;
   }

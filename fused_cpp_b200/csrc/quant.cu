@@ -494,16 +494,16 @@ cudaError_t launch_quantize_tokens_scatter(const uint16_t* x, int64_t tokens, in
 
 // The same quantiser for rows whose length is a multiple of 8 and at most 16 * 1024: the row is read once, into registers
 // (two groups of eight values per thread: a 512-thread CTA holds a 7168-column row), and the division is replaced as in
-// quantize4_torchref_fast (the statement is the same clamp(rint(x / scale)); with scale = amax / 127 of the same row no
-// quotient rounds below -127, so the lower clamp of -128 some callers ask for never binds).  Latency-bound for a decode
+// quantize4_torchref_fast (the statement is the same clamp(rint(x / scale)); the lower clamp of -128 that the single product
+// asks for binds only in its exact branch, in fp32 rows below 2.3e-41).  Latency-bound for a decode
 // batch: one memory round trip instead of two, and the GEMM behind it fetches weights meanwhile (dense_gemm.cu has the
 // figures of the op); HBM-bound above.
 constexpr int kDenseVectors = 2;
 
 template <bool kBf16>
 __global__ void __launch_bounds__(1024)
-quantize_rows_dense_vec8_kernel(const void* __restrict__ x, int cols, int cols_padded, int8_t* __restrict__ q, float* __restrict__ scale_out,
-                                DenseItems dense_items) {
+quantize_rows_dense_vec8_kernel(const void* __restrict__ x, int cols, int cols_padded, float clamp_low, int8_t* __restrict__ q,
+                                float* __restrict__ scale_out, DenseItems dense_items) {
   ptx::launch_dependents();  // the GEMM behind this kernel may start fetching its weights
   __shared__ float smem[32];
   if (blockIdx.x == 0) write_dense_items(dense_items);
@@ -538,7 +538,7 @@ quantize_rows_dense_vec8_kernel(const void* __restrict__ x, int cols, int cols_p
   for (int i = 0; i < kDenseVectors; ++i) {
     const int v = threadIdx.x + i * blockDim.x;
     if (v < vec8) {
-      dst[v] = make_uint2(quantize4_torchref_fast(values[i], scale, inverse), quantize4_torchref_fast(values[i] + 4, scale, inverse));
+      dst[v] = make_uint2(quantize4_torchref_fast(values[i], scale, inverse, clamp_low), quantize4_torchref_fast(values[i] + 4, scale, inverse, clamp_low));
     }
   }
   // cols_padded is cols or cols + 8 (a multiple of 16).
@@ -547,7 +547,8 @@ quantize_rows_dense_vec8_kernel(const void* __restrict__ x, int cols, int cols_p
 
 // bf16 rows by the thousand, or longer than the registers of a CTA hold: a 256-thread CTA reads its row twice, the second
 // time out of L1, and eight of them fit an SM (3000 rows of 7168 columns 19 us, 24 us with the row in registers; of the
-// other kernel's shorter latency nothing is left from four rows per SM on).
+// other kernel's shorter latency nothing is left from four rows per SM on).  The smallest bf16 number is 2^-133: no scale here
+// is rounded enough for a quotient below -127.5, and the lower clamp does not matter.
 __global__ void __launch_bounds__(kQuantThreads)
 quantize_rows_dense_bf16x8_kernel(const uint16_t* __restrict__ x, int cols, int cols_padded, int8_t* __restrict__ q,
                                   float* __restrict__ scale_out, DenseItems dense_items) {
@@ -593,7 +594,7 @@ cudaError_t launch_quantize_rows_dense(const void* x, int x_is_bf16, int64_t row
     int threads = 64;
     while (threads * kDenseVectors < vec8) threads *= 2;
     auto kernel = x_is_bf16 ? quantize_rows_dense_vec8_kernel<true> : quantize_rows_dense_vec8_kernel<false>;
-    kernel<<<static_cast<unsigned>(rows), threads, 0, stream>>>(x, cols, cols_padded, q, scale, dense_items);
+    kernel<<<static_cast<unsigned>(rows), threads, 0, stream>>>(x, cols, cols_padded, static_cast<float>(clamp_low), q, scale, dense_items);
   } else {
     quantize_rows_dense_kernel<<<static_cast<unsigned>(rows), kQuantThreads, 0, stream>>>(
         x, x_is_bf16, cols, cols_padded, static_cast<float>(clamp_low), q, scale, dense_items);

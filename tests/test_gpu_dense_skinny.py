@@ -70,3 +70,21 @@ def test_output_view_at_any_element(cuda_device, rows, k, n, out_dtype, offset):
                                              packed.n, packed.n_padded)
         assert torch.equal(out, other)
         assert torch.equal(other.cpu(), oracle.i8gemm_dynamic(x, weight, scale, None, out_dtype, clamp_low=-127))
+
+
+@pytest.mark.parametrize("k", [64, 72, 77, 16392], ids=["held", "held_padded", "scalar", "long"])
+@pytest.mark.parametrize("rows", [8, 600])
+def test_rows_of_a_few_smallest_numbers(cuda_device, rows, k):
+    """fp32 rows whose largest magnitude is a few units of the smallest fp32 number: amax / 127 is rounded to whole units, up to
+    15938 units quotients can leave +-127.5, and both clamps bind (-128 below, for the single product)."""
+    generator = torch.Generator().manual_seed(k)
+    units = torch.tensor([190, 63, 254, 100, 64, 1000, 15938, 15939])[torch.arange(rows) % 8].unsqueeze(1)
+    steps = torch.randint(-1000, 1001, (rows, k), generator=generator) * units // 1000
+    steps[:, 0], steps[:, 1] = -units[:, 0], units[:, 0]
+    x = torch.where(steps < 0, (-steps) | -(1 << 31), steps).to(torch.int32).view(torch.float32)
+    assert torch.equal(x.abs().view(torch.int32).amax(dim=1), units[:, 0].to(torch.int32))
+    weight = torch.randint(-127, 128, (40, k), dtype=torch.int8, generator=generator)
+    scale = torch.full((40,), 1e30)
+    got = i8gemm.dynamic_scaled_mm(x.to(cuda_device), i8gemm.prepare(weight, scale), out_dtype=torch.float32)
+    expected = oracle.i8gemm_dynamic(x, weight, scale, None, torch.float32)
+    assert torch.equal(got.cpu(), expected) and bool((expected != 0).any())
