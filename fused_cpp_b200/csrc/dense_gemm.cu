@@ -47,7 +47,7 @@ struct DenseConfig {
   static constexpr int kBudget = kDeep ? 200 * 1024 : 100 * 1024;
   static constexpr int kStages = kBudget / kStageBytes < kMaxStages ? kBudget / kStageBytes : kMaxStages;
   static constexpr int kTmemColumns = kRowTile < 32 ? 32 : kRowTile;
-  static constexpr size_t kSmemBytes = 1024 /*alignment slack*/ + static_cast<size_t>(kStages) * kStageBytes + 1024 /*control block*/;
+  static constexpr size_t kSmemBytes = 1024 /*alignment slack*/ + static_cast<size_t>(kStages) * kStageBytes + 2048 /*control block*/;
   static_assert(kStages * kStageBytes >= kRowTile * kBlockM * 4, "the accumulator exchange reuses the stages");
 };
 
@@ -58,8 +58,10 @@ struct DenseControl {
   uint32_t tmem_base;
   volatile int abort_flag;
   float row_scale[128];
+  alignas(16) float channel_scale[kBlockM];
+  alignas(16) float channel_bias[kBlockM];
 };
-static_assert(sizeof(DenseControl) <= 1024, "control block exceeds its shared-memory reservation");
+static_assert(sizeof(DenseControl) <= 2048, "control block exceeds its shared-memory reservation");
 
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -93,9 +95,11 @@ __device__ __forceinline__ void store_value(const Side& side, int row, int n, in
 }
 
 // Four channels of a row, of which `columns` exist; vector_store: dense_vector_store holds (then all four do).
-__device__ __forceinline__ void store_row4(const Side& side, int row, int n, int4 acc, float row_scale, const float* scales, const float* biases,
+__device__ __forceinline__ void store_row4(const Side& side, int row, int n, int4 acc, float row_scale, float4 scale, float4 bias,
                                            int columns, bool vector_store) {
   const int sums[4] = {acc.x, acc.y, acc.z, acc.w};
+  const float scales[4] = {scale.x, scale.y, scale.z, scale.w};
+  const float biases[4] = {bias.x, bias.y, bias.z, bias.w};
   float out[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) out[j] = __fadd_rn(dequantize(sums[j], row_scale, scales[j], FMOE_NUMERICS_TORCHREF), biases[j]);
@@ -242,10 +246,13 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
   int* exchange = reinterpret_cast<int*>(smem);  // [rows][128 channels], once the stages are done with
   if (warp >= 2) {
     const int thread = static_cast<int>(threadIdx.x) - 64;
+    // Before the wait, hence through L2: a scale or bias that an earlier call read at this address may still lie in L1.
     if (channel_ok) {
-      channel_scale = side.w_scale[n];
-      if (!second && args.bias != nullptr) bias = args.bias[n];
+      channel_scale = __ldcg(side.w_scale + n);
+      if (!second && args.bias != nullptr) bias = __ldcg(args.bias + n);
     }
+    ctl->channel_scale[channel] = channel_scale;
+    ctl->channel_bias[channel] = bias;
     ptx::grid_dependency_wait();  // the row scales come from the quantiser
     if (thread < rows) ctl->row_scale[thread] = args.a_scale[row0 + thread];
     asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -277,12 +284,8 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
       const int c4 = 4 * lane;
       const uint32_t mine = ptx::smem_u32(exchange) + 4u * static_cast<uint32_t>(c4);
       const int columns = side.n - (n0 + c4);  // channels of this lane that exist, if below four
-      float scales[4], biases[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        scales[j] = j < columns ? side.w_scale[n0 + c4 + j] : 1.0f;
-        biases[j] = (!second && args.bias != nullptr && j < columns) ? args.bias[n0 + c4 + j] : 0.0f;
-      }
+      const float4 scales = *reinterpret_cast<const float4*>(ctl->channel_scale + c4);
+      const float4 biases = *reinterpret_cast<const float4*>(ctl->channel_bias + c4);
       const bool vector_store = (second ? args.vector_store[1] : args.vector_store[0]) != 0;  // a lane's four channels all exist or none does
       constexpr int kBatch = 2;  // rows of a warp whose loads are in flight together (a remote load takes most of a microsecond)
       for (int first = part + parts * (warp - 2); first < rows; first += 4 * parts * kBatch) {

@@ -88,3 +88,42 @@ def test_rows_of_a_few_smallest_numbers(cuda_device, rows, k):
     got = i8gemm.dynamic_scaled_mm(x.to(cuda_device), i8gemm.prepare(weight, scale), out_dtype=torch.float32)
     expected = oracle.i8gemm_dynamic(x, weight, scale, None, torch.float32)
     assert torch.equal(got.cpu(), expected) and bool((expected != 0).any())
+
+
+@pytest.mark.parametrize("rows,k,n", [(4, 256, 40000), (4, 2048, 1536), (96, 512, 12000)], ids=["one_part", "split", "row_tile_128"])
+@pytest.mark.parametrize("graph", [False, True], ids=["eager", "graph"])
+def test_scales_and_bias_rewritten_between_calls(cuda_device, rows, k, n, graph):
+    """A weight that is streamed into a fixed buffer: what a call read of it must not be found again by the next one."""
+    generator = torch.Generator().manual_seed(n)
+    x = torch.randn((rows, k), generator=generator).to(torch.bfloat16)
+    rounds = [(_weight(n, k, generator), torch.randn(n, generator=generator)) for _ in range(3)]
+    packed = i8gemm.prepare(*rounds[0][0])
+    bias = rounds[0][1].to(cuda_device)
+    sources = [(i8gemm.prepare(*weight), values.to(cuda_device)) for weight, values in rounds]
+    device_x = x.to(cuda_device)
+
+    def passes():
+        outs = []
+        for source, values in sources:
+            packed.packed_weight.copy_(source.packed_weight)
+            packed.weight_scale.copy_(source.weight_scale)
+            bias.copy_(values)
+            outs.append(i8gemm.dynamic_scaled_mm(device_x, packed, bias=bias, out_dtype=torch.float32))
+        return outs
+
+    expected = [oracle.i8gemm_dynamic(x, *weight, values, torch.float32).to(cuda_device) for weight, values in rounds]
+    outs = passes()
+    if graph:
+        torch.cuda.synchronize()
+        captured = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(captured):
+            outs = passes()
+    for _ in range(6):
+        if graph:
+            captured.replay()
+            captured.replay()
+        else:
+            outs = passes()
+        torch.cuda.synchronize()
+        for out, reference in zip(outs, expected):
+            assert torch.equal(out, reference)
