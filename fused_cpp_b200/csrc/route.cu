@@ -216,6 +216,7 @@ route_build_kernel(const int64_t* __restrict__ topk_ids, int64_t routes, int exp
     totals[e] = running;
   }
   if constexpr (kCluster) {
+    __syncwarp();
     cg::this_cluster().sync();  // totals of every CTA and the cleared status block are visible
     for (int e = threadIdx.x; e < experts; e += blockDim.x) {
       int values[kMaxRouteCluster];
@@ -230,8 +231,10 @@ route_build_kernel(const int64_t* __restrict__ topk_ids, int64_t routes, int exp
       base[e] = before;
       s_counts[e] = all;
     }
-    // This CTA reads no other CTA's totals after this.  (Nothing was written for the others: no release is needed.)
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    // This CTA reads no other CTA's totals after this: the release orders the reads above before the arrival, which lets the
+    // others leave.  (The loop's trip count differs inside a warp, and the barrier wants whole warps.)
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   }
   __syncthreads();
   if (bad_route >= 0) raise_error(status, FMOE_ERR_EXPERT_ID_RANGE, static_cast<int>(bad_route));
@@ -302,7 +305,10 @@ route_build_kernel(const int64_t* __restrict__ topk_ids, int64_t routes, int exp
       row_expert[p] = low;
     }
   }
-  if (kCluster) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // no CTA leaves while another may still read its totals
+  if (kCluster) {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // no CTA leaves while another may still read its totals
+  }
 }
 
 // Work items from given per-expert counts and offsets (rows that already lie in expert order: nothing to sort).

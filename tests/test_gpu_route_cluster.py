@@ -25,6 +25,8 @@ def _covered_rows(items: torch.Tensor, rows_most: int) -> dict:
 
 @pytest.mark.parametrize("tokens,experts,top_k", [
     (1, 1, 1), (1024, 16, 1), (1025, 16, 1), (683, 40, 3), (4097, 33, 2), (9001, 7, 1), (700, 1024, 12), (700, 1025, 12), (300, 2048, 32),
+    # several CTAs with a number of experts that leaves lanes of the last warp out of the loops in front of the cluster barriers
+    (1100, 31, 1), (2100, 257, 4), (16384, 257, 9),
 ])
 def test_lists_and_items(cuda_device, tokens, experts, top_k):
     generator = torch.Generator().manual_seed(tokens + experts)
