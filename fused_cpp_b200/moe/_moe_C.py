@@ -165,11 +165,13 @@ def _check_plan_vectors(task_expert_ids, task_core_begins, task_threads, task_de
         if tensor.numel() != tasks:
             raise RuntimeError(f"{label} task vectors must have matching lengths")
     # Short vectors (the one-task plan of this package) as lists: a tensor operation on one costs microseconds per call.
-    short = tasks <= 16
-    if task_dep_offsets.numel() != tasks + 1 or (task_dep_offsets.tolist()[tasks] if short else int(task_dep_offsets[tasks])) != task_deps.numel():
+    # Tensors of another rank keep the tensor operations: their lists are nested.
+    short = tasks <= 16 and task_dep_offsets.dim() == 1
+    if task_dep_offsets.numel() != tasks + 1 or int(task_dep_offsets.tolist()[tasks] if short else task_dep_offsets[tasks]) != task_deps.numel():
         raise RuntimeError(f"{label} dependency offsets are invalid")
     points = task_resize_points.numel()
-    if points and (any(task_resize_points.tolist()) if points <= 16 else bool((task_resize_points != 0).any())):
+    short = points <= 16 and task_resize_points.dim() == 1
+    if points and (any(task_resize_points.tolist()) if short else bool((task_resize_points != 0).any())):
         raise RuntimeError(f"{label} does not support dynamic resize points")
 
 

@@ -105,6 +105,29 @@ def _w8a8_weights(experts=1, hidden=16, inter=16):
                                                     torch.ones((experts, hidden))))
 
 
+@pytest.mark.parametrize("tasks", [1, 16, 17])
+def test_plan_vectors_of_any_rank(tasks):
+    """The op level takes plan vectors by their element count, whatever their rank."""
+    from fused_cpp_b200.moe import _moe_C
+
+    ones = torch.ones(tasks, dtype=torch.int64)
+    offsets = torch.zeros((tasks + 1, 1), dtype=torch.int64)
+    offsets[tasks] = 3
+    deps = torch.zeros(3, dtype=torch.int64)
+
+    def check(offsets, points):
+        _moe_C._check_plan_vectors(ones, ones, ones, offsets, deps, 2, 0, ones, ones, points, "test")
+
+    for points in (torch.zeros((tasks, 2), dtype=torch.int64), torch.zeros(tasks, dtype=torch.int64), torch.tensor(0), torch.zeros((0, 2))):
+        check(offsets, points)
+        check(offsets.reshape(-1), points)
+    for points in (torch.eye(tasks + 1, dtype=torch.int64), torch.tensor(1), torch.arange(tasks + 1)):
+        with pytest.raises(RuntimeError, match="resize points"):
+            check(offsets, points)
+    with pytest.raises(RuntimeError, match="dependency offsets"):
+        check(offsets + 1, deps)
+
+
 def test_prepared_weight_contract():
     weights = _w8a8_weights()
     assert weights.fused_silu and weights.backend_n_tile == 128 and weights.backend_name == "cuda_sm100_w8a8_tcgen05"
