@@ -476,27 +476,37 @@ int fmoe_device_supported(int device) {
 }  // extern "C"
 
 namespace {
+// For its lifetime, another thread's graph capture is no concern of this thread's allocations: a page-locked allocation or its
+// release is no part of that capture, and would be refused and invalidate it.
+class RelaxedCaptureMode {
+ public:
+  RelaxedCaptureMode() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+  ~RelaxedCaptureMode() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+
+ private:
+  cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
 // One status block of page-locked memory per thread that reads one, given back when the thread ends.
 class PinnedWords {
  public:
   int* get() {
     if (!tried_) {
       tried_ = true;
-      // Another thread may be capturing a graph: this allocation is no part of it.
-      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-      cudaThreadExchangeStreamCaptureMode(&mode);
+      const RelaxedCaptureMode relaxed;
       void* memory = nullptr;
       if (cudaHostAlloc(&memory, sizeof(int) * fmoe::kStatusWords, cudaHostAllocPortable) == cudaSuccess) {
         words_ = static_cast<int*>(memory);
       } else {
         cudaGetLastError();
       }
-      cudaThreadExchangeStreamCaptureMode(&mode);
     }
     return words_;
   }
   ~PinnedWords() {
-    if (words_ != nullptr) cudaFreeHost(words_);
+    if (words_ == nullptr) return;
+    const RelaxedCaptureMode relaxed;
+    cudaFreeHost(words_);
   }
 
  private:
