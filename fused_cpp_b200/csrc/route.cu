@@ -51,8 +51,8 @@ __device__ void build_item_list(int list, int experts, const int* counts, const 
   const int tile = list == 0 ? lists.tile_a : list == 1 ? lists.tile_b : lists.big_tile;
   int* items = list == 0 ? lists.items_a : list == 1 ? lists.items_b : list == 2 ? lists.items_c : lists.items_d;
   // Row tiles are powers of two but for the two-SM kernel's, 5/4 of one (320 token rows): its full height spares an expert a
-  // second pass over its weights for a few rows; longer lists are cut at the power of two, whose accumulators double-buffer
-  // without sharing columns.  About 256 rows per expert (int8, 8192 tokens): 4228 -> 3877 us.  Lists of thousands of rows,
+  // second pass over its weights for a few rows; longer lists are cut at the power of two: two 256-row accumulators
+  // fill tensor memory without sharing columns.  About 256 rows per expert (int8, 8192 tokens): 4228 -> 3877 us.  Lists of thousands of rows,
   // bf16, took 3312 us cut at 256 and 3367 us cut at 320; about 512 rows (int8, 16384 tokens) are the same either way.
   const bool tall = (tile & (tile - 1)) != 0;
   const int cut = tall ? tile / 5 * 4 : tile;

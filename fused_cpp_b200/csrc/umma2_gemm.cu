@@ -30,6 +30,7 @@
 #include <cuda.h>
 #include <stdlib.h>
 
+#include "acc_ring.cuh"
 #include "common.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
@@ -56,9 +57,8 @@ constexpr int kThreads = 64 + kEpilogueThreads;
 constexpr int kStages = 6;
 constexpr int kWeightBytes = kRowsPerCta * kBlockKBytes;                // 16 KB
 constexpr int kStageBytes = kWeightBytes + kTokensPerCta * kBlockKBytes;  // 36 KB
-constexpr int kTmemColumns = 512;                                         // a ring of 32-column blocks (AccSlot)
-constexpr int kRingBlocks = kTmemColumns / 32;
-constexpr int kMmaBlocks = kMmaTokens / 32;
+constexpr int kTmemColumns = 32 * kRingBlocks;                            // a ring of 32-column blocks (acc_ring.cuh)
+static_assert(kMmaBlocks * 32 == kMmaTokens, "the ring's largest MMA");
 constexpr size_t kControlBytes = 9216;
 constexpr size_t kSmemBytes = 1024 + static_cast<size_t>(kStages) * kStageBytes + kControlBytes;
 static_assert(kSmemBytes <= 227 * 1024, "a CTA has 227 KB of shared memory");
@@ -215,41 +215,6 @@ __device__ __forceinline__ UnitInfo load_unit(const int* items, int64_t unit, in
     info.block = static_cast<int>(unit - static_cast<int64_t>(item) * n_blocks);
   }
   return info;
-}
-
-// Where a unit's accumulator lies.  Tensor memory is a ring of sixteen 32-column blocks; a unit of up to 320 rows takes
-// one block per 32 rows, behind the unit before it, so that its main loop runs while that unit's accumulator is still
-// being read: two units of up to 256 rows never share a block, and of two larger ones the second waits only for the
-// blocks it takes over (blocks_shared, barrier acc_part), not for the whole accumulator.
-// Up to 256 rows are one MMA over consecutive columns; above that two MMAs share the staged weight tile, the first over
-// `head` blocks.  Where the ring ends inside the accumulator the split lies there, and each MMA gets at least 64
-// columns (a 32-column MMA takes as long as a 64-column one: it reads the same weight rows).
-struct AccSlot {
-  int start;   // running block number; its place in the ring is start mod 16
-  int blocks;
-  int head;
-};
-
-__device__ __forceinline__ AccSlot place_unit(int start, int rows) {
-  AccSlot slot = {start, (rows + 31) >> 5, 0};
-  const int place = start & (kRingBlocks - 1);
-  const int room = kRingBlocks - place;
-  if (slot.blocks <= kMmaBlocks) {
-    if (slot.blocks > room) slot.start += room;
-    slot.head = slot.blocks;
-  } else if (slot.blocks <= room || room < 2) {
-    if (room < 2) slot.start += room;
-    slot.head = (slot.blocks + 1) >> 1;
-  } else {
-    slot.head = min(room, min(kMmaBlocks, slot.blocks - 2));
-    slot.start += room - slot.head;
-  }
-  return slot;
-}
-
-// Leading blocks of `before` that lie where `slot`, the unit after it, has its accumulator.
-__device__ __forceinline__ int blocks_shared(const AccSlot& before, const AccSlot& slot) {
-  return max(0, slot.start + slot.blocks - kRingBlocks - before.start);
 }
 
 // The same unit with every field taken from lane 0 (all lanes hold the same values already).

@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import random
 import subprocess
 
 import pytest
@@ -31,3 +32,32 @@ def test_dense_vector_store_is_aligned_in_every_row(rules, bf16):
             aligned = all((out + (row * n + channel) * size) % (4 * size) == 0 and channel + 4 <= n
                           for row in range(4) for channel in range(0, n, 4))
             assert rules.dense_vector_store(out, n, bf16) == aligned
+
+
+@pytest.mark.parametrize("sizes", [(1, 320), (65, 256), (257, 320), (1, 32), (256, 256)], ids=str)
+def test_accumulator_ring(rules, sizes):
+    """A unit's MMAs lie on consecutive columns inside tensor memory, and what it takes over from the unit before it is that
+    unit's leading blocks, as many as are counted.  (The unit before that one has been read by then.)"""
+    rng = random.Random(sizes[0])
+    count, ring, worst = 20000, 16, 0
+    rows = [rng.randint(*sizes) for _ in range(count)]
+    slots, shared = (ctypes.c_int * (3 * count))(), (ctypes.c_int * count)()
+    rules.place_units((ctypes.c_int * count)(*rows), count, slots, shared)
+    before: list = []
+    for i, unit_rows in enumerate(rows):
+        start, blocks, head = slots[3 * i:3 * i + 3]
+        tail = blocks - head
+        assert blocks == (unit_rows + 31) // 32 and 0 <= tail
+        for first, length in ((start, head), (start + head, tail)):
+            assert length <= 8 and first % ring + length <= ring
+        assert tail == 0 or (head >= 2 and tail >= 2 and blocks > 8)
+        taken = [block % ring for block in range(start, start + blocks)]
+        assert len(set(taken)) == blocks
+        overlap = [index for index, block in enumerate(before) if block in taken]
+        assert overlap == list(range(shared[i]))
+        worst = max(worst, shared[i])
+        before = taken
+    if sizes[1] <= 256:
+        assert worst <= 7
+    if sizes in ((1, 32), (256, 256)):
+        assert worst == 0
