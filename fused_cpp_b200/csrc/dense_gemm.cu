@@ -21,6 +21,8 @@
 // What is left above the floor is launch and quantiser latency (about 5 us) and, with the rows, the exchange.
 #include <cuda.h>
 
+#include <mutex>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
@@ -345,8 +347,10 @@ cudaError_t configure() {
 
 template <int kRowTile>
 cudaError_t residency(Residency* out) {
+  static std::mutex guard;  // a thread that finds the flag set has to find the table too
   static PerDeviceOnce configured;
   static Residency known[kMaxDevices];
+  const std::lock_guard<std::mutex> lock(guard);
   const int device = current_device_ordinal();
   if (!configured.needed(device)) {
     *out = known[device];
