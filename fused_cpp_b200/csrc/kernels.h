@@ -203,13 +203,15 @@ __device__ __forceinline__ float load_expert_bias(const GroupedGemmArgs& args, i
 // Launch, with `chained` as a programmatic dependent of the kernel before it in the stream.  The kernels of a forward pass
 // behind its first, an ordinary launch, are chained this way, under these rules (griddepcontrol, ptx.cuh):
 //   * every CTA calls grid_dependency_wait before it touches anything that the kernel before it reads or writes;
-//   * it calls launch_dependents (or ends) only after that.  A kernel that has started therefore knows that every kernel
-//     but the one right before it has completed: route lists and work items may be read before the wait by any kernel
-//     that is not the first behind the route build.  What is read before a wait
-//     is read through L2 (__ldcg): only the wait promises that an L1 line left by an earlier call is not found again;
+//   * it calls launch_dependents (or ends) only after that; the one exception is the second grouped GEMM of a split stage
+//     (`beside`), which does both the other way round.  A kernel that has started therefore knows that every kernel but the
+//     one right before it has completed, or, right behind a `beside` kernel, every kernel but that one and the first GEMM of
+//     the stage.  What it may read before its wait is what neither of them writes: weights, scales and biases, and, unless it
+//     is the first behind the route build, route lists and work items.  What is read before a wait is read
+//     through L2 (__ldcg): only the wait promises that an L1 line left by an earlier call is not found again;
 //   * what is read behind a wait is not reached through a const __restrict__ parameter: such loads count as invariant, and
 //     the compiler may move them in front of the wait;
-//   * a kernel that does not need the one before it (the second grouped GEMM of a split stage) waits before it ends.
+//   * a kernel that does not need the one before it (`beside`) waits before it ends.
 // Launch, prologue and the first weight loads of a kernel overlap the end of the one before it: one token of the 256-expert
 // layer 200 -> 181 us, 16 tokens of the 16-expert one 137 -> 119 us.  A kernel whose neighbour in front may be anybody's (the
 // first of a call, a stand-alone quantiser) is not chained.

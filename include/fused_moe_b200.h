@@ -120,7 +120,7 @@ typedef struct fmoe_workspace_layout {
   size_t offsets;        /* int32[E+1] exclusive prefix of counts */
   size_t sorted_routes;  /* int32[T*K] flat route ids t*K+slot grouped by expert, ascending inside an expert */
   size_t row_expert;     /* int32[T*K] expert of each sorted row */
-  size_t items;          /* int32[4*max_items] (expert, first row, rows, reserved) per work item; two lists */
+  size_t items;          /* int32[4*max_items] (expert, first row, rows, group key) per work item; four lists */
   size_t scratch;        /* empty (the route build needs no memory of its own) */
   size_t a_rows;         /* W8A8: int8[T*K,H] quantised token rows; BF16: bf16[T*K,H] gathered rows */
   size_t a_scale;        /* W8A8: fp32[T*K] activation scales */
@@ -286,9 +286,9 @@ FMOE_API int fmoe_ep_combine_finish(const float* returned_rows, const int32_t* s
 
 /* ---- dense W8A8 linear ----------------------------------------------------------------------- */
 
-/* Workspace bytes for the dense calls below (quantised rows, scales, work items, status block, and for at most 16
- * rows the int32 table in which the K-split parts of a product meet; n = the widest N that will use the workspace.
- * A call given less than this for its N runs without the split). */
+/* Workspace bytes for the dense calls below: quantised rows, scales, work items, status block.  n does not matter (a K
+ * split meets in shared memory) and is kept for the ABI.  A call given a smaller workspace is refused with
+ * FMOE_ERR_WORKSPACE. */
 FMOE_API size_t fmoe_i8gemm_workspace_bytes(int64_t rows, int32_t k, int32_t n);
 
 /* out[M,N] = dequant( quant_rows(x[M,K]) @ w^T ) (+ bias): per-row dynamic int8 quantisation
@@ -297,7 +297,8 @@ FMOE_API size_t fmoe_i8gemm_workspace_bytes(int64_t rows, int32_t k, int32_t n);
  * (csrc/i8gemm.cpp:318-452; scalar-fallback arithmetic :384-399, :147-165).
  * w is [N, Kp] int8 with Kp = K rounded up to 16 and the padding zero (what i8gemm_prepare's packed
  * weight is on this backend, csrc/i8gemm.cpp:280-316); w_scale[N] and bias[N] fp32, bias may be NULL;
- * x_is_bf16 / out_is_bf16 select bf16 (else fp32) element types. */
+ * x_is_bf16 / out_is_bf16 select bf16 (else fp32) element types; x and out may start at any element of an allocation
+ * (vector loads and stores are used where their addresses allow it). */
 FMOE_API int fmoe_i8gemm_dynamic_scaled_mm(const void* x, int32_t x_is_bf16, int64_t rows, int32_t k, const int8_t* w,
                                            const float* w_scale, const float* bias, int32_t n, void* out,
                                            int32_t out_is_bf16, void* workspace, size_t workspace_bytes, void* stream);
