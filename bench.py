@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Benchmark of the routed-expert MoE layer (one JSON line on stdout).
+"""Benchmark of the routed-expert MoE layer (one short JSON line on stdout, the report behind it on stderr).
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--workload NAME] [--no-points] [--sweep]
 
@@ -17,7 +17,8 @@ e2e    : the same metric through the public op (fused_cpp_b200.moe.fused_moe_til
 roofline: the gate_up grouped GEMM (the dominant kernel), timed per launch by the library's stage
          timer (CUDA events around that kernel) during the timed steps.
 points : the other benchmark configurations (W8A8 prefill T=8192 uniform and Zipf-routed, BF16 decode, the
-         routed + shared-expert layer at T=16384, the two small-dimension configurations), same measurements.
+         routed + shared-expert layer at T=16384, the two small-dimension configurations), same measurements; one JSON
+         line each on stderr, as are the stage times and the full roofline record of the headline.
 cpu_baseline / --impl reference: the CPU port of the reference arithmetic (oracle/) on all host cores, on the
          same batch.  The reference's native kernels are AArch64-only and cannot run on an x86 host.
 """
@@ -723,6 +724,29 @@ def time_cpu_port(name: str, spec: dict, layer: dict | None, warmup: int, passes
             "passes_timed": timed, "seconds_per_pass": seconds}
 
 
+# What the result line leaves to the report on stderr: one short line is what a reader of the output's end finds whole.
+REPORT_KEYS = ("points", "stage_ms", "layer", "int8_library_peak", "planner_calibration_seconds", "roofline_report", "planner")
+ROOFLINE_KEYS = ("kernel", "bound", "achieved", "peak", "unit", "frac", "traffic")
+
+
+def print_result(line: dict) -> None:
+    """The result as one JSON line on stdout; in front of it, on stderr, the rest as one JSON line per entry (`report`
+    names it, every point is an entry of its own)."""
+    line = dict(line)
+    if line.get("roofline"):
+        line["roofline_report"] = line["roofline"]
+        line["roofline"] = {key: line["roofline"][key] for key in ROOFLINE_KEYS if key in line["roofline"]}
+    if line.get("e2e") and "planner" in line["e2e"]:
+        line["e2e"] = dict(line["e2e"])
+        line["planner"] = line["e2e"].pop("planner")
+    for key in REPORT_KEYS:
+        value = line.pop(key, None)
+        for entry in value if isinstance(value, list) else [value]:
+            if entry:
+                print(json.dumps({"report": key, **entry}), file=sys.stderr, flush=True)
+    print(json.dumps(line), flush=True)
+
+
 def run_reference_arm(args) -> None:
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
@@ -848,7 +872,7 @@ def run_single_gpu(args) -> None:
         "stage_ms": head["stage_ms"], "layer": head["layer"], "launch_mode": head["launch_mode"],
         "eager_ms_per_step": head["eager_ms_per_step"], "points": points,
     }
-    print(json.dumps(line), flush=True)
+    print_result(line)
 
 
 # ---- dense W8A8 linear (the i8gemm op next to the MoE path) -------------------------------------------------
@@ -1121,7 +1145,7 @@ def run_multi_gpu(args) -> None:
         if rank == 0:
             head = lines[0]
             head["points"] = lines[1:]
-            print(json.dumps(head), flush=True)
+            print_result(head)
     finally:
         dist.destroy_process_group()
 
