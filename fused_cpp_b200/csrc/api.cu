@@ -785,7 +785,7 @@ struct DenseProduct {
 };
 
 // Above kDenseMaxRows rows the split-K kernel takes products that would leave the two-SM kernel most of the chip idle: at most
-// 74 tiles of 128 x 128, one for every second SM, over a K range long enough (5120) to pay for the exchange of the parts.
+// one tile of 128 x 128 for every second SM (74 on 148 SMs), over a K range long enough (5120) to pay for the exchange of the parts.
 // Two-SM / split-K kernel, device time per op: 7168 -> 1536 at 129 / 256 / 512 / 768 rows 20.4 / 26.8 / 28.9 / 30.9 us ->
 // 18.4 / 19.4 / 23.3 / 27.0 us; 7168 -> 130 at 200 / 1000 / 4000 rows 28.5 / 36.1 / 58.3 -> 15.8 / 23.9 / 48.2; 16384 -> 4096
 // at 200 rows 45.1 -> 32.3.  Beyond the lines: 4096 -> 3072 at 384 rows 20.4 -> 20.5, 1536 -> 2048 at 129 rows 12.6 -> 16.4,
@@ -796,7 +796,7 @@ bool dense_split_pays(int64_t rows, int k_padded, const DenseProduct* products, 
   int64_t tiles = 0;
   for (int i = 0; i < count; ++i) tiles += (static_cast<int64_t>(products[i].n) + 127) / 128;
   tiles *= (rows + fmoe::kDenseMaxRows - 1) / fmoe::kDenseMaxRows;
-  return tiles <= 74 && k_padded >= 5120;
+  return tiles <= fmoe::sm_count_of_current_device() / 2 && k_padded >= 5120;
 }
 
 cudaError_t dense_gemm(const DenseLayout& d, char* base, int64_t rows, const DenseProduct* products, int count, int out_is_bf16,

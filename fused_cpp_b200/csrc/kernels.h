@@ -199,6 +199,33 @@ __device__ __forceinline__ float load_expert_bias(const GroupedGemmArgs& args, i
 #define FMOE_DIAG_BIT(args, bit) false
 #endif
 
+// Launch set-up that belongs to a device, not to the process: the opt-in to more than 48 KB of dynamic shared
+// memory (a function attribute) and the SM count are remembered per device ordinal.
+constexpr int kMaxDevices = 64;
+inline int current_device_ordinal() {
+  int device = 0;
+  cudaGetDevice(&device);
+  return device;
+}
+struct PerDeviceOnce {
+  bool done[kMaxDevices] = {};
+  // True when `device` still needs its set-up (ordinals beyond the table are set up on every call).
+  bool needed(int device) const { return device < 0 || device >= kMaxDevices || !done[device]; }
+  void mark(int device) {
+    if (device >= 0 && device < kMaxDevices) done[device] = true;
+  }
+};
+inline int sm_count_of_current_device() {
+  static int counts[kMaxDevices] = {};
+  const int device = current_device_ordinal();
+  if (device >= 0 && device < kMaxDevices && counts[device] > 0) return counts[device];
+  int count = 0;
+  cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
+  if (count <= 0) count = 148;
+  if (device >= 0 && device < kMaxDevices) counts[device] = count;
+  return count;
+}
+
 #ifdef __CUDACC__
 // Launch, with `chained` as a programmatic dependent of the kernel before it in the stream.  The kernels of a forward pass
 // behind its first, an ordinary launch, are chained this way, under these rules (griddepcontrol, ptx.cuh):
@@ -234,40 +261,13 @@ inline cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, unsigned
 // The same for the kernels that stream rows with a short-lived CTA per row; the last kernel parameter says whether the
 // launch is chained.  A grid of several waves is not: waiting costs every CTA of it about a microsecond (merge of 65536
 // rows: 302 us, chained 381 us) and hides one launch.
-constexpr uint64_t kChainedBlocks = 148 * 8;
+constexpr uint64_t kChainedBlocksPerSm = 8;
 template <typename... Params, typename... Args>
 inline cudaError_t launch_streaming(void (*kernel)(Params...), dim3 grid, unsigned threads, cudaStream_t stream, bool chained, Args&&... args) {
-  const bool chain = chained && static_cast<uint64_t>(grid.x) * grid.y <= kChainedBlocks;
+  const bool chain = chained && static_cast<uint64_t>(grid.x) * grid.y <= kChainedBlocksPerSm * sm_count_of_current_device();
   return launch_chained(kernel, grid, threads, 0, stream, chain, args..., chain);
 }
 #endif
-
-// Launch set-up that belongs to a device, not to the process: the opt-in to more than 48 KB of dynamic shared
-// memory (a function attribute) and the SM count are remembered per device ordinal.
-constexpr int kMaxDevices = 64;
-inline int current_device_ordinal() {
-  int device = 0;
-  cudaGetDevice(&device);
-  return device;
-}
-struct PerDeviceOnce {
-  bool done[kMaxDevices] = {};
-  // True when `device` still needs its set-up (ordinals beyond the table are set up on every call).
-  bool needed(int device) const { return device < 0 || device >= kMaxDevices || !done[device]; }
-  void mark(int device) {
-    if (device >= 0 && device < kMaxDevices) done[device] = true;
-  }
-};
-inline int sm_count_of_current_device() {
-  static int counts[kMaxDevices] = {};
-  const int device = current_device_ordinal();
-  if (device >= 0 && device < kMaxDevices && counts[device] > 0) return counts[device];
-  int count = 0;
-  cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
-  if (count <= 0) count = 148;
-  if (device >= 0 && device < kMaxDevices) counts[device] = count;
-  return count;
-}
 
 // 2-D K-major tensor [rows, k] with 128-byte-swizzled boxes of {128 bytes of K, box_rows} (umma_gemm.cu).
 bool make_sw128_map(CUtensorMap* map, const void* base, bool int8, uint64_t rows, uint64_t k, uint32_t box_rows);
