@@ -15,9 +15,9 @@
 //   * Two weight matrices are one launch: the second one's channel blocks follow the first one's.
 // Device time per op in a chain of ops (quantiser included; floor = weights at the copy bandwidth), against a persistent
 // kernel without the cluster (a K split up to 16 rows over an int32 table with atomics) behind a finished quantiser:
-//   16384 -> 7168    1 / 64 / 128 rows: 31.9 / 40.5 / 46.5 us -> 23.4 / 29.8 / 36.2 us (floor 18.2 / 18.7 / 19.1)
-//   7168 -> 1536    16 / 64 / 128 rows: 14.4 / 22.2 / 25.6 us ->  8.2 / 11.6 / 16.4 us (floor 1.7 / 1.9 / 2.1)
-//   1536 -> 24576    1 / 64 rows:       15.2 / 19.7 us        -> 10.5 / 15.3 us        (floor 5.9 / 6.4)
+//   16384 -> 7168    1 / 64 / 128 rows: 31.9 / 40.5 / 46.5 us -> 22.4 / 25.9 / 32.0 us (floor 18.2 / 18.7 / 19.1)
+//   7168 -> 1536    16 / 64 / 128 rows: 14.4 / 22.2 / 25.6 us ->  8.0 /  9.5 / 12.8 us (floor 1.7 / 1.9 / 2.1)
+//   1536 -> 24576    1 / 64 rows:       15.2 / 19.7 us        -> 10.4 / 12.9 us        (floor 5.9 / 6.4)
 // What is left above the floor is launch and quantiser latency (about 5 us) and, with the rows, the exchange.
 #include <cuda.h>
 
@@ -59,7 +59,7 @@ struct DenseControl {
   uint64_t acc_full;
   uint32_t tmem_base;
   volatile int abort_flag;
-  float row_scale[128];
+  alignas(16) float row_scale[128];
   alignas(16) float channel_scale[kBlockM];
   alignas(16) float channel_bias[kBlockM];
 };
@@ -86,13 +86,20 @@ struct Side {
   int out_bf16;
 };
 
-__device__ __forceinline__ void store_value(const Side& side, int row, int n, int acc, float row_scale, float channel_scale, float bias) {
-  const float value = __fadd_rn(dequantize(acc, row_scale, channel_scale, FMOE_NUMERICS_TORCHREF), bias);
-  const int64_t index = static_cast<int64_t>(row) * side.n + n;
-  if (side.out_bf16) {
-    static_cast<uint16_t*>(side.out)[index] = f32_to_bf16_bits(value);
-  } else {
-    static_cast<float*>(side.out)[index] = value;
+// Up to sixteen rows of one channel, from row `row` on (`count` of them, all sixteen with kAll): acc[j] belongs to row + j.
+template <typename Out, bool kAll>
+__device__ __forceinline__ void store_column(const Side& side, int row, int n, const uint32_t* acc, int count, const float* row_scale,
+                                             float channel_scale, float bias) {
+  Out* out = static_cast<Out*>(side.out) + static_cast<int64_t>(row) * side.n + n;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if (!kAll && j >= count) break;
+    const float value = __fadd_rn(dequantize(static_cast<int>(acc[j]), row_scale[j], channel_scale, FMOE_NUMERICS_TORCHREF), bias);
+    if constexpr (sizeof(Out) == 2) {
+      out[static_cast<int64_t>(j) * side.n] = f32_to_bf16_bits(value);
+    } else {
+      out[static_cast<int64_t>(j) * side.n] = value;
+    }
   }
 }
 
@@ -261,21 +268,33 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap first_map, const __grid_co
     ptx::mbar_wait(&ctl->acc_full, 0, abort_flag, status, 23);
     ptx::tcgen05_fence_after();
     const uint32_t acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    // Sixteen rows at a time, which form they take decided outside the value loop: with the checks inside it every value waited for
+    // the one before it (128 rows, 64 -> 64: 14.2 -> 9.0 us per op; 7168 -> 129280: 193 -> 172 us; 7168 -> 1536: 17.6 -> 12.8 us).
     for (int c0 = 0; c0 < rows; c0 += 16) {
       uint32_t bits[16];
       ptx::tmem_ld_x8(acc + c0, bits);
       ptx::tmem_ld_x8(acc + c0 + 8, bits + 8);
       ptx::tmem_ld_wait();
+      const int count = rows - c0;
+      const float* const row_scale = ctl->row_scale + c0;
+      if (parts > 1) {
+        // (Rows of the last sixteen that do not exist have room in the stages too.)
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int row = c0 + j;
-        if (row >= rows) continue;
-        if (parts > 1) {
-          exchange[row * kBlockM + channel] = static_cast<int>(bits[j]);
-        } else if (channel_ok) {
-          store_value(side, row0 + row, n, static_cast<int>(bits[j]), ctl->row_scale[row], channel_scale, bias);
+        for (int j = 0; j < 16; ++j) exchange[(c0 + j) * kBlockM + channel] = static_cast<int>(bits[j]);
+      } else if (channel_ok && side.out_bf16) {
+        if (count >= 16) {
+          store_column<uint16_t, true>(side, row0 + c0, n, bits, 16, row_scale, channel_scale, bias);
+        } else {
+          store_column<uint16_t, false>(side, row0 + c0, n, bits, count, row_scale, channel_scale, bias);
+        }
+      } else if (channel_ok) {
+        if (count >= 16) {
+          store_column<float, true>(side, row0 + c0, n, bits, 16, row_scale, channel_scale, bias);
+        } else {
+          store_column<float, false>(side, row0 + c0, n, bits, count, row_scale, channel_scale, bias);
         }
       }
+      __syncwarp();  // the next tensor-memory load wants the whole warp
     }
   }
   if (parts > 1) {
@@ -412,8 +431,8 @@ cudaError_t launch_dense(DenseGemmArgs args, const void* a_rows, const int8_t* c
   const int blocks = (args.first_blocks + (args.n[1] + kBlockM - 1) / kBlockM) * args.row_tiles;
   // As many parts as leave all clusters resident at once, two CTAs per SM if need be, every part at least two K blocks.
   // Device time per op of a chain of ops, parts 1 / 2 / 3 / 4 / 5 / 8, 64 rows: 16384 -> 7168 (56 blocks; clusters of five
-  // and more take a second wave) 37 / 31 / 31 / 29.5 / 39 / 38 us; 7168 -> 1536 (12 blocks) 21 / 16 / 14 / 13 / 12 / 11.5 us;
-  // 1536 -> 24576 (192 blocks) 15.5 / 24 / 30 / 31 / 38 / 56 us.  One CTA per SM with deep stages where that holds them
+  // and more take a second wave) 35 / 28 / 28 / 27 / 29 / 33 us; 7168 -> 1536 (12 blocks) 18.5 / 13.5 / 11.4 / 10.4 / 10.3 / 9.6 us;
+  // 1536 -> 24576 (192 blocks, 12 K blocks) 13 / 19 / 22 / 23 / 27 us.  One CTA per SM with deep stages where that holds them
   // all: 7168 -> 1536 12.2 -> 11.5 us.
   args.parts = 1;
   for (int parts = kMaxParts; split && parts > 1; --parts) {

@@ -28,6 +28,11 @@ def _weight(n, k, generator):
     (1100, 5120, 1025, torch.bfloat16, torch.bfloat16, True), (1100, 5120, 1000, torch.bfloat16, torch.bfloat16, False),
     (592, 264, 130, torch.bfloat16, torch.bfloat16, False), (593, 264, 130, torch.bfloat16, torch.bfloat16, True),
     (5, 16400, 200, torch.bfloat16, torch.float32, True), (2, 16392, 64, torch.float32, torch.float32, False),
+    # One CTA per channel block: whole and short batches of sixteen rows, channels off the block, either output type.
+    (15, 100, 129, torch.bfloat16, torch.bfloat16, True), (31, 128, 257, torch.bfloat16, torch.float32, False),
+    (64, 64, 64, torch.bfloat16, torch.bfloat16, True), (97, 96, 130, torch.float32, torch.float32, True),
+    (127, 128, 200, torch.bfloat16, torch.bfloat16, False), (128, 64, 64, torch.bfloat16, torch.float32, True),
+    (113, 512, 37000, torch.bfloat16, torch.bfloat16, True),
 ])
 def test_product(cuda_device, rows, k, n, x_dtype, out_dtype, with_bias):
     generator = torch.Generator().manual_seed(rows + k + n)
