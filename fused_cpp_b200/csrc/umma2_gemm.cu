@@ -241,6 +241,13 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
   constexpr int kBlockKElems = kBlockKBytes / kElemBytes;
   constexpr int kChannelsPerUnit = kGateUp ? 128 : 256;  // output channels one pair finishes per work unit
   constexpr int kRowsPerRoute = kPlanes ? 2 : 1;
+  // The dense product's items hold at most 256 rows: two accumulators of 256 columns take turns, one MMA per K step, one
+  // column of metadata per thread.  What larger items need is left out (3000 rows, 1536 -> 24576: 106.9 -> 105.9 us; 128 to 600 rows 0.1 to 0.5 us).
+  constexpr bool kTall = !kDense;
+  auto place = [](int start, int rows) {
+    if constexpr (kTall) return place_unit(start, rows);
+    return AccSlot{start, kMmaBlocks, (rows + 31) >> 5};  // a full half of the ring, whatever the unit takes of it
+  };
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -313,9 +320,9 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
         // 16 rows per CTA and block.  One box brings the rows of a one-MMA unit, up to the next box size (a few
         // boxes of exactly its rows move less and take longer: about 512 rows per expert, 16384 tokens, 8087 -> 8216 us);
         // the two halves of a larger unit are laid out by boxes of 64 and 16 rows.
-        const AccSlot slot = place_unit(ring_end, cur.rows);
+        const AccSlot slot = place(ring_end, cur.rows);
         ring_end = slot.start + slot.blocks;
-        const int tail = slot.blocks - slot.head;
+        const int tail = kTall ? slot.blocks - slot.head : 0;
         const int head_row = cur.row0 + slot.head * kBoxTokens * static_cast<int>(cta);
         const int tail_row = cur.row0 + slot.head * 32 + tail * kBoxTokens * static_cast<int>(cta);
         const CUtensorMap* const one_box = slot.head <= kMidBox ? &token_map_mid : &token_map_full;
@@ -418,8 +425,8 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
         // N follows the rows this unit really has (a multiple of 32 for two-SM MMAs).  The row count comes from a global
         // load; the shuffle tells the compiler that every lane holds the same value.
         const int unit_rows = __shfl_sync(0xffffffffu, cur.rows, 0);
-        const AccSlot slot = place_unit(before.start + before.blocks, unit_rows);
-        const int tail = __shfl_sync(0xffffffffu, slot.blocks - slot.head, 0);
+        const AccSlot slot = place(before.start + before.blocks, unit_rows);
+        const int tail = kTall ? __shfl_sync(0xffffffffu, slot.blocks - slot.head, 0) : 0;
         const uint32_t idesc_head = __shfl_sync(0xffffffffu, ptx::make_instr_desc(kInt8, 2 * kRowsPerCta, 32 * slot.head), 0);
         const uint32_t idesc_tail = __shfl_sync(0xffffffffu, ptx::make_instr_desc(kInt8, 2 * kRowsPerCta, 32 * tail), 0);
         const uint32_t acc_head = __shfl_sync(0xffffffffu, tmem_base + 32u * static_cast<uint32_t>(slot.start & (kRingBlocks - 1)), 0);
@@ -428,7 +435,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
         const uint32_t tail_step = __shfl_sync(0xffffffffu, kTokenStep + kBlockStep * static_cast<uint32_t>(slot.head), 0);
         // The unit two before this one has left tensor memory, and the one before it the blocks that this one takes over.
         ptx::mbar_wait(&ctl->acc_empty[buffer], (use & 1u) ^ 1u, abort_flag, status, 12);
-        if (blocks_shared(before, slot) > 0) {
+        if (kTall && blocks_shared(before, slot) > 0) {
           ptx::mbar_wait(&ctl->acc_part, handovers & 1u, abort_flag, status, 15);
           ++handovers;
         }
@@ -465,8 +472,12 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
             }
           }
         };
-        if (tail > 0) {
-          main_loop(TrueTag{});
+        if constexpr (kTall) {
+          if (tail > 0) {
+            main_loop(TrueTag{});
+          } else {
+            main_loop(FalseTag{});
+          }
         } else {
           main_loop(FalseTag{});
         }
@@ -501,8 +512,9 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
 
     // Per-unit values: the column metadata in shared memory and this thread's weight scales in registers.  Both
     // are fetched while the previous unit is being finished.
+    constexpr int kColumns = kTall ? 2 : 1;
     struct ThreadUnit {
-      float column_scale[2];      // of columns `tid` and `tid` + 256
+      float column_scale[2];      // of columns `tid` and `tid` + 256 (the second with kTall)
       uint64_t column_rowptr[2];  // of the same columns: byte address of the output row (down / dense)
       float scale_gate, scale_up, bias;
     };
@@ -510,7 +522,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
       ThreadUnit t = {{0.0f, 0.0f}, {0ull, 0ull}, kInt8 ? 1.0f : 0.0f, kInt8 ? 1.0f : 0.0f, 0.0f};
       if (!valid) return t;
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
+      for (int i = 0; i < kColumns; ++i) {
         const int column = tid + 256 * i;
         if (column >= info.rows) break;
         const int row = (info.row0 + column) / kRowsPerRoute;  // sorted position of the column's route
@@ -577,7 +589,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
     ThreadUnit mine = fetch(cur, first_unit < units);
     auto publish = [&](ColumnMeta* meta, const ThreadUnit& t) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
+      for (int i = 0; i < kColumns; ++i) {
         if (tid >= (i == 0 ? 256 : kMaxTokenRows - 256)) break;
         meta->scale[tid + 256 * i] = t.column_scale[i];
         meta->rowptr[tid + 256 * i] = t.column_rowptr[i];
@@ -587,7 +599,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
     epilogue_bar_sync();
 
     int local = 0;
-    AccSlot slot = place_unit(0, cur.rows);
+    AccSlot slot = place(0, cur.rows);
     for (int64_t unit = first_unit; unit < units; unit += unit_stride, ++local) {
       const uint32_t buffer = static_cast<uint32_t>(local) & 1u;
       const uint32_t use = static_cast<uint32_t>(local) >> 1;
@@ -606,8 +618,8 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
       ptx::mbar_wait(&ctl->acc_full[buffer], use & 1u, abort_flag, status, 14);
       ptx::tcgen05_fence_after();
       // The next unit's accumulator may start on this one's first blocks: they are released as soon as they are read.
-      const AccSlot next_slot = place_unit(slot.start + slot.blocks, next.rows);
-      const int handed_over = blocks_shared(slot, next_slot);
+      const AccSlot next_slot = place(slot.start + slot.blocks, next.rows);
+      const int handed_over = kTall ? blocks_shared(slot, next_slot) : 0;
       bool part_released = handed_over == 0;
       auto release_part = [&]() {
         part_released = true;
