@@ -784,17 +784,24 @@ struct DenseProduct {
   void* out;
 };
 
+// Over 64 rows (stages of 32 KB, three to a CTA) a product with more channel blocks than CTAs are resident at once goes to the
+// two-SM kernel, which is persistent: what a second wave of short-lived CTAs loses in prologues and epilogues is more than that
+// kernel's half-empty token tile.  Split / two-SM kernel, 128 rows: 2048 -> 50000 (391 blocks) 36.1 / 29.5 us, 7168 -> 65536
+// (512) 90.8 / 89.5, 7168 -> 129280 (1010) 176 / 159; 4096 -> 32000 (250 blocks: one wave) 32.1 / 32.8; 64 rows of
+// 7168 -> 129280 153.7 / 152.4, one row 136 / 165.
 // Above kDenseMaxRows rows the split-K kernel takes products that would leave the two-SM kernel most of the chip idle: at most
 // one tile of 128 x 128 for every second SM (74 on 148 SMs), over a K range long enough (5120) to pay for the exchange of the parts.
-// Two-SM / split-K kernel, device time per op: 7168 -> 1536 at 129 / 256 / 512 / 768 rows 20.4 / 26.8 / 28.9 / 30.9 us ->
-// 18.4 / 19.4 / 23.3 / 27.0 us; 7168 -> 130 at 200 / 1000 / 4000 rows 28.5 / 36.1 / 58.3 -> 15.8 / 23.9 / 48.2; 16384 -> 4096
-// at 200 rows 45.1 -> 32.3.  Beyond the lines: 4096 -> 3072 at 384 rows 20.4 -> 20.5, 1536 -> 2048 at 129 rows 12.6 -> 16.4,
-// 16384 -> 7168 at 300 rows (168 tiles) 54.8 -> 67.0, 8192 -> 8192 at 150 rows (128 tiles) 23.2 -> 30.1.
+// Two-SM / split-K kernel, device time per op: 7168 -> 1536 at 129 / 256 / 512 / 768 rows 22.2 / 27.7 / 29.5 / 30.4 us ->
+// 13.9 / 14.9 / 18.6 / 21.7 us; 7168 -> 130 at 200 / 1000 / 4000 rows 28.0 / 35.2 / 47.7 -> 10.7 / 16.9 / 33.0; 16384 -> 4096
+// at 200 rows 46.0 -> 28.4.  Beyond the lines: 16384 -> 7168 at 300 rows (168 tiles) 53.1 -> 61.7, 8192 -> 8192 at 150 rows
+// (128 tiles) 26.9 -> 25.8, 4096 -> 3072 at 384 rows 21.2 -> 15.9, 1536 -> 2048 at 129 rows 12.2 -> 10.9 (the lines were drawn
+// with an epilogue that took those two 20.5 and 16.4 us).
 bool dense_split_pays(int64_t rows, int k_padded, const DenseProduct* products, int count, bool split) {
-  if (rows <= fmoe::kDenseMaxRows) return true;
-  if (!split) return false;
+  if (rows <= 64) return true;
   int64_t tiles = 0;
   for (int i = 0; i < count; ++i) tiles += (static_cast<int64_t>(products[i].n) + 127) / 128;
+  if (rows <= fmoe::kDenseMaxRows) return tiles <= 2 * fmoe::sm_count_of_current_device();
+  if (!split) return false;
   tiles *= (rows + fmoe::kDenseMaxRows - 1) / fmoe::kDenseMaxRows;
   return tiles <= fmoe::sm_count_of_current_device() / 2 && k_padded >= 5120;
 }

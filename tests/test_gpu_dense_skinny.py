@@ -32,7 +32,9 @@ def _weight(n, k, generator):
     (15, 100, 129, torch.bfloat16, torch.bfloat16, True), (31, 128, 257, torch.bfloat16, torch.float32, False),
     (64, 64, 64, torch.bfloat16, torch.bfloat16, True), (97, 96, 130, torch.float32, torch.float32, True),
     (127, 128, 200, torch.bfloat16, torch.bfloat16, False), (128, 64, 64, torch.bfloat16, torch.float32, True),
-    (113, 512, 37000, torch.bfloat16, torch.bfloat16, True),
+    # More channel blocks than resident CTAs: the two-SM kernel over 64 rows.
+    (113, 512, 37000, torch.bfloat16, torch.bfloat16, True), (65, 264, 38017, torch.float32, torch.float32, True),
+    (128, 128, 40000, torch.bfloat16, torch.bfloat16, False), (64, 128, 40000, torch.bfloat16, torch.bfloat16, True),
 ])
 def test_product(cuda_device, rows, k, n, x_dtype, out_dtype, with_bias):
     generator = torch.Generator().manual_seed(rows + k + n)
@@ -43,7 +45,7 @@ def test_product(cuda_device, rows, k, n, x_dtype, out_dtype, with_bias):
     torch.testing.assert_close(got.cpu(), oracle.i8gemm_dynamic(x, weight, scale, bias, out_dtype), atol=0, rtol=0)
 
 
-@pytest.mark.parametrize("rows,k,first_n,second_n", [(1, 1536, 4000, 72), (40, 512, 130, 129), (128, 300, 64, 700), (200, 512, 300, 130), (200, 5136, 130, 260)])
+@pytest.mark.parametrize("rows,k,first_n,second_n", [(1, 1536, 4000, 72), (40, 512, 130, 129), (128, 300, 64, 700), (100, 144, 30000, 9000), (200, 512, 300, 130), (200, 5136, 130, 260)])
 def test_pair(cuda_device, rows, k, first_n, second_n):
     generator = torch.Generator().manual_seed(rows + k)
     first, second = _weight(first_n, k, generator), _weight(second_n, k, generator)
