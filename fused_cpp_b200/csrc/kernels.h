@@ -228,7 +228,7 @@ inline int sm_count_of_current_device() {
 
 #ifdef __CUDACC__
 // Launch, with `chained` as a programmatic dependent of the kernel before it in the stream.  The kernels of a forward pass
-// behind its first, an ordinary launch, are chained this way, under these rules (griddepcontrol, ptx.cuh):
+// (and the GEMM of a dense product) behind its first, an ordinary launch, are chained this way, under these rules (griddepcontrol, ptx.cuh):
 //   * every CTA calls grid_dependency_wait before it touches anything that the kernel before it reads or writes;
 //   * it calls launch_dependents (or ends) only after that; the one exception is the second grouped GEMM of a split stage
 //     (`beside`), which does both the other way round.  A kernel that has started therefore knows that every kernel but the

@@ -97,28 +97,31 @@ def test_rows_of_a_few_smallest_numbers(cuda_device, rows, k):
     assert torch.equal(got.cpu(), expected) and bool((expected != 0).any())
 
 
-@pytest.mark.parametrize("rows,k,n", [(4, 256, 40000), (4, 2048, 1536), (96, 512, 12000)], ids=["one_part", "split", "row_tile_128"])
+@pytest.mark.parametrize("rows,k,n", [(4, 256, 40000), (4, 2048, 1536), (96, 512, 12000), (700, 512, 1536), (128, 128, 40000)],
+                         ids=["one_part", "split", "row_tile_128", "two_sm", "two_sm_wide"])
 @pytest.mark.parametrize("graph", [False, True], ids=["eager", "graph"])
-def test_scales_and_bias_rewritten_between_calls(cuda_device, rows, k, n, graph):
-    """A weight that is streamed into a fixed buffer: what a call read of it must not be found again by the next one."""
+def test_buffers_rewritten_between_calls(cuda_device, rows, k, n, graph):
+    """Rows and a weight that are streamed into fixed buffers: what a call read of them must not be found again by the next."""
     generator = torch.Generator().manual_seed(n)
-    x = torch.randn((rows, k), generator=generator).to(torch.bfloat16)
     rounds = [(_weight(n, k, generator), torch.randn(n, generator=generator)) for _ in range(3)]
+    rows_of = [torch.randn((rows, k), generator=generator).to(torch.bfloat16) for _ in rounds]
     packed = i8gemm.prepare(*rounds[0][0])
     bias = rounds[0][1].to(cuda_device)
-    sources = [(i8gemm.prepare(*weight), values.to(cuda_device)) for weight, values in rounds]
-    device_x = x.to(cuda_device)
+    sources = [(i8gemm.prepare(*weight), values.to(cuda_device), x.to(cuda_device)) for (weight, values), x in zip(rounds, rows_of)]
+    device_x = torch.empty_like(sources[0][2])
 
     def passes():
         outs = []
-        for source, values in sources:
+        for source, values, x in sources:
+            device_x.copy_(x)
             packed.packed_weight.copy_(source.packed_weight)
             packed.weight_scale.copy_(source.weight_scale)
             bias.copy_(values)
             outs.append(i8gemm.dynamic_scaled_mm(device_x, packed, bias=bias, out_dtype=torch.float32))
         return outs
 
-    expected = [oracle.i8gemm_dynamic(x, *weight, values, torch.float32).to(cuda_device) for weight, values in rounds]
+    expected = [oracle.i8gemm_dynamic(x, *weight, values, torch.float32).to(cuda_device)
+                for (weight, values), x in zip(rounds, rows_of)]
     outs = passes()
     if graph:
         torch.cuda.synchronize()
