@@ -12,6 +12,10 @@
 #include "diag.h"
 #endif
 
+namespace fmoe {
+thread_local int threshold_sms = 148;
+}
+
 namespace {
 
 thread_local char g_error[512] = "";
@@ -40,6 +44,7 @@ int check_device() {
     return fail(FMOE_ERR_UNSUPPORTED_DEVICE, "device %d is not a compute capability 10.x GPU; this library has no other path", device);
   }
   checked_device = device;
+  fmoe::threshold_sms = fmoe::sm_count_of_current_device();
   return FMOE_OK;
 }
 
@@ -800,10 +805,10 @@ bool dense_split_pays(int64_t rows, int k_padded, const DenseProduct* products, 
   if (rows <= 64) return true;
   int64_t tiles = 0;
   for (int i = 0; i < count; ++i) tiles += (static_cast<int64_t>(products[i].n) + 127) / 128;
-  if (rows <= fmoe::kDenseMaxRows) return tiles <= 2 * fmoe::sm_count_of_current_device();
+  if (rows <= fmoe::kDenseMaxRows) return tiles <= 2 * fmoe::threshold_sms;
   if (!split) return false;
   tiles *= (rows + fmoe::kDenseMaxRows - 1) / fmoe::kDenseMaxRows;
-  return tiles <= fmoe::sm_count_of_current_device() / 2 && k_padded >= 5120;
+  return tiles <= fmoe::threshold_sms / 2 && k_padded >= 5120;
 }
 
 cudaError_t dense_gemm(const DenseLayout& d, char* base, int64_t rows, const DenseProduct* products, int count, int out_is_bf16,

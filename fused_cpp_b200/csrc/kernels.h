@@ -226,6 +226,10 @@ inline int sm_count_of_current_device() {
   return count;
 }
 
+// SMs of the device that the calling thread last entered the library on, for rules that choose between kernels: a stale value
+// costs time and nothing else, and reading it costs no runtime call (0.1 us each, of 22 us of host time for a short dense call).
+extern thread_local int threshold_sms;
+
 #ifdef __CUDACC__
 // Launch, with `chained` as a programmatic dependent of the kernel before it in the stream.  The kernels of a forward pass
 // (and the GEMM of a dense product) behind its first, an ordinary launch, are chained this way, under these rules (griddepcontrol, ptx.cuh):
@@ -264,7 +268,7 @@ inline cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, unsigned
 constexpr uint64_t kChainedBlocksPerSm = 8;
 template <typename... Params, typename... Args>
 inline cudaError_t launch_streaming(void (*kernel)(Params...), dim3 grid, unsigned threads, cudaStream_t stream, bool chained, Args&&... args) {
-  const bool chain = chained && static_cast<uint64_t>(grid.x) * grid.y <= kChainedBlocksPerSm * sm_count_of_current_device();
+  const bool chain = chained && static_cast<uint64_t>(grid.x) * grid.y <= kChainedBlocksPerSm * threshold_sms;
   return launch_chained(kernel, grid, threads, 0, stream, chain, args..., chain);
 }
 #endif

@@ -456,7 +456,7 @@ cudaError_t launch_quantize_rows(const uint16_t* x, int64_t out_rows, int cols, 
   const unsigned warp_blocks = static_cast<unsigned>((out_rows + kQuantThreads / 32 - 1) / (kQuantThreads / 32));
   // A few rows (decode): one CTA per row spreads a row over 256 threads, where one warp per row would walk its 64
   // values per lane alone on an SM (10.7 us against the other kernel's ~5 us for 8 rows of 2048 columns).
-  const bool few_rows = out_rows <= kFewRowsPerSm * sm_count_of_current_device();
+  const bool few_rows = out_rows <= kFewRowsPerSm * threshold_sms;
   if (few_rows) {
     return launch_streaming(quantize_rows_kernel, dim3(static_cast<unsigned>(out_rows)), kQuantThreads, stream, chained, x, cols, sorted_routes,
                           top_k, valid_rows, numerics, weight_mode, q, scale);
@@ -588,7 +588,7 @@ cudaError_t launch_quantize_rows_dense(const void* x, int x_is_bf16, int64_t row
   const bool aligned = cols % 8 == 0 && cols_padded - cols <= 8 && cols_padded % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
                        (reinterpret_cast<uintptr_t>(q) & 7u) == 0;
   const bool held = vec8 <= 1024 * kDenseVectors;  // a row fits the registers of one CTA
-  if (aligned && x_is_bf16 && (rows > kFewRowsPerSm * sm_count_of_current_device() || !held)) {
+  if (aligned && x_is_bf16 && (rows > kFewRowsPerSm * threshold_sms || !held)) {
     quantize_rows_dense_bf16x8_kernel<<<static_cast<unsigned>(rows), kQuantThreads, 0, stream>>>(static_cast<const uint16_t*>(x), cols,
                                                                                                 cols_padded, q, scale, dense_items);
   } else if (aligned && held) {
