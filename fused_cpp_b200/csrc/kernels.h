@@ -227,7 +227,7 @@ inline int sm_count_of_current_device() {
 }
 
 // SMs of the device that the calling thread last entered the library on, for rules that choose between kernels: a stale value
-// costs time and nothing else, and reading it costs no runtime call (0.1 us each, of 22 us of host time for a short dense call).
+// costs time and nothing else, and reading it costs no runtime call.
 extern thread_local int threshold_sms;
 
 #ifdef __CUDACC__
