@@ -22,7 +22,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(OUT_DIR, "libfused_moe_b200.so")
 DIAG_LIB = os.path.join(OUT_DIR, "libfused_moe_b200_diag.so")
-SOURCES = ["api.cu", "route.cu", "quant.cu", "merge.cu", "umma_gemm.cu", "umma2_gemm.cu", "dense_gemm.cu", "ep.cu", "router.cu"]
+SOURCES = ["api.cu", "route.cu", "front.cu", "quant.cu", "merge.cu", "umma_gemm.cu", "umma2_gemm.cu", "dense_gemm.cu", "ep.cu", "router.cu"]
 DIAG_ONLY_SOURCES = ["simt_gemm.cu", "probe.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

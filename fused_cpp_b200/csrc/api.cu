@@ -306,6 +306,7 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   mark(0);
   cudaError_t error = cudaSuccess;
   uint64_t* row_out_ptrs = nullptr;
+  const bool front = !f.rows_mode && umma && fmoe::front_pays(f.tokens, f.top_k, f.experts);
   if (peer) {
     // The rows arrived in expert order: only the work items and the output addresses remain to be made.
     error = cudaMemsetAsync(status_block, 0, sizeof(int) * fmoe::kStatusWords, stream);
@@ -316,6 +317,12 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
                                        f.hidden * (f.peer_rows_bf16 ? 2 : 4), row_out_ptrs, f.peer_world, f.peer_routes_max,
                                        f.peer_scrap_row, status_block, stream);
     if (error != cudaSuccess) return cuda_fail(error, "peer output addresses");
+  } else if (front) {
+    error = fmoe::launch_front(planes ? fmoe::FrontRows::kPlanes : f.int8 ? fmoe::FrontRows::kInt8 : fmoe::FrontRows::kBf16, f.topk_ids, f.tokens,
+                               f.top_k, f.experts, lists, status_block, counts, offsets, sorted_routes, row_expert,
+                               reinterpret_cast<int*>(base + layout.route_pos), static_cast<const uint16_t*>(f.x), f.hidden, cfg.numerics,
+                               base + layout.a_rows, a_scale, stream);
+    if (error != cudaSuccess) return cuda_fail(error, "route build and token rows");
   } else {
     error = fmoe::launch_route_build(f.topk_ids, routes, f.experts, lists, status_block, counts, offsets, sorted_routes, row_expert, stream,
                                      reinterpret_cast<int*>(base + layout.route_pos));
@@ -329,6 +336,8 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   if (peer) {
     gemm_rows = f.x;  // already sorted, already quantised
     gemm_row_scale = f.rows_scale;
+  } else if (front) {
+    // made with the routes
   } else if (f.rows_mode && f.int8) {
     // int8 rows travel as H bytes: gather them as H/2 16-bit words, then their scales.
     error = fmoe::launch_gather_rows(static_cast<const uint16_t*>(f.x), routes, f.hidden / 2, sorted_routes, 1, valid_rows,
@@ -376,6 +385,7 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   gu.route_out = nullptr;
   gu.dump_acc = cfg.dump_acc1;
   gu.total_rows = routes;
+  gu.items_late = front ? 1 : 0;
   gu.row_tile = (planes && tile_gu != fmoe::kPairRowTile) ? 2 * tile_gu : tile_gu;
   const bool int8_gemm = f.int8 || planes;
 #ifdef FMOE_DIAG
@@ -387,6 +397,7 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
     fmoe::GroupedGemmArgs big = gu;
     big.items = items_gu_big;
     big.item_count_word = fmoe::kStatusItemsC;
+    big.items_late = 0;
     big.beside = 1;
     big.row_tile = fmoe::kPairRowTile;
     error = fmoe::launch_umma_grouped_gemm(big, int8_gemm, true, stream);
@@ -419,6 +430,7 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   dn.k = f.inter;
   dn.n_out = f.hidden;
   dn.y = nullptr;
+  dn.items_late = 0;
   dn.route_out = route_out;
   dn.row_out_ptrs = row_out_ptrs;
   // bf16 route rows: the peer-memory return in its compact form, or the single-GPU compact mode of fmoe_config.

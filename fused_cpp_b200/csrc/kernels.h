@@ -36,6 +36,14 @@ cudaError_t launch_route_build(const int64_t* topk_ids, int64_t routes, int expe
 cudaError_t launch_items_from_counts(int experts, const int* counts, const int* offsets, const ItemLists& lists, int* status,
                                      cudaStream_t stream);
 
+// ---- front.cu: the route build and the token rows of a small batch (front_pays) in one launch.  rows_out takes what the
+// kernels of quant.cu write: int8 rows + scales, bf16 rows, or two int8 planes per route + scales.
+enum class FrontRows { kInt8, kBf16, kPlanes };
+bool front_pays(int64_t tokens, int top_k, int experts);
+cudaError_t launch_front(FrontRows rows, const int64_t* topk_ids, int64_t tokens, int top_k, int experts, const ItemLists& lists, int* status,
+                         int* counts, int* offsets, int* sorted_routes, int* row_expert, int* route_pos, const uint16_t* x, int cols,
+                         int numerics, void* rows_out, float* scale_out, cudaStream_t stream);
+
 // ---- quant.cu
 // Quantise rows of a bf16 matrix to int8 with one fp32 scale per row.  When `sorted_routes` is
 // non-null, output row p reads source row sorted_routes[p] / top_k (gather by token).
@@ -175,6 +183,8 @@ struct GroupedGemmArgs {
   // Two-SM kernel: the kernel in front is the one-SM launch of the same stage (the thin experts' items), which waited for all
   // that this one reads and writes other rows: no wait before the work, SM pairs are taken as they fall free, one at the end.
   int beside;
+  // The kernel in front is the one that makes the work items (front.cu): they are read behind the wait, not in front of it.
+  int items_late;
   int gate_up_one_box;       // two-SM gate_up: the weight rows of a stage arrive as one 16 KB TMA box (set by the launcher)
   int route_out_bf16;        // the result rows are stored as bf16 (2 bytes per channel, rows 2 * n_out bytes apart) instead of fp32
   // Diagnostic build only (compiled with -DFMOE_DIAG, the separate libfused_moe_b200_diag.so; the product library

@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
+#include "row_quant.cuh"
 
 namespace fmoe {
 
@@ -16,54 +17,6 @@ namespace {
 
 constexpr int kQuantThreads = 256;
 constexpr int kFewRowsPerSm = 4;  // up to so many rows per SM latency counts, above it throughput
-
-__device__ __forceinline__ float block_max(float value, float* smem) {
-  value = warp_max(value);
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  if (lane == 0) smem[warp] = value;
-  __syncthreads();
-  float result = lane < (blockDim.x >> 5) ? smem[lane] : 0.0f;
-  result = warp_max(result);
-  __syncthreads();
-  return result;
-}
-
-__device__ __forceinline__ void unpack8(const uint4& v, float* out) {
-  const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    out[2 * i] = __uint_as_float(words[i] << 16);
-    out[2 * i + 1] = __uint_as_float(words[i] & 0xffff0000u);
-  }
-}
-
-__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
-  uint32_t result;
-  asm("max.bf16x2 %0, %1, %2;" : "=r"(result) : "r"(a), "r"(b));
-  return result;
-}
-
-// Largest magnitude of eight bf16 values, NaN left out: two values per instruction, exact like the fp32 form.
-__device__ __forceinline__ float amax8(const uint4& v) {
-  constexpr uint32_t kMagnitude = 0x7fff7fffu;
-  uint32_t m = max_bf16x2(0u, v.x & kMagnitude);
-  m = max_bf16x2(m, v.y & kMagnitude);
-  m = max_bf16x2(m, v.z & kMagnitude);
-  m = max_bf16x2(m, v.w & kMagnitude);
-  return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u));
-}
-
-// operand: 1/scale (NATIVE) or scale (TORCHREF); inverse: 1/scale, used by the TORCHREF fast path.
-__device__ __forceinline__ uint32_t pack4(const float* values, float operand, float inverse, int numerics) {
-  if (numerics == FMOE_NUMERICS_TORCHREF) return quantize4_torchref_fast(values, operand, inverse);
-  uint32_t packed = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    packed |= (static_cast<uint32_t>(quantize_value(values[i], operand, numerics)) & 0xffu) << (8 * i);
-  }
-  return packed;
-}
 
 // cols % 16 == 0.  One CTA per output row.
 __global__ void __launch_bounds__(kQuantThreads)
@@ -242,18 +195,7 @@ split_rows_planes_kernel(const uint16_t* x, int cols, const int* sorted_routes, 
     float values[16];
     unpack8(src[2 * v], values);
     unpack8(src[2 * v + 1], values + 8);
-    uint32_t high[4] = {0, 0, 0, 0};
-    uint32_t low[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int fixed = plane_fixed_point(values[i], scale);
-      const int low_part = ((fixed + 128) & 255) - 128;
-      const int high_part = (fixed - low_part) >> 8;  // fixed - low_part is a multiple of 256
-      high[i >> 2] |= (static_cast<uint32_t>(high_part) & 0xffu) << (8 * (i & 3));
-      low[i >> 2] |= (static_cast<uint32_t>(low_part) & 0xffu) << (8 * (i & 3));
-    }
-    high_row[v] = make_uint4(high[0], high[1], high[2], high[3]);
-    low_row[v] = make_uint4(low[0], low[1], low[2], low[3]);
+    split16_planes(values, scale, high_row + v, low_row + v);
   }
 }
 
@@ -284,18 +226,8 @@ split_tokens_scatter_planes_kernel(const uint16_t* x, int cols, int top_k, const
     float values[16];
     unpack8(__ldcg(src + 2 * v), values);
     unpack8(__ldcg(src + 2 * v + 1), values + 8);
-    uint32_t high[4] = {0, 0, 0, 0};
-    uint32_t low[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int fixed = plane_fixed_point(values[i], scale);
-      const int low_part = ((fixed + 128) & 255) - 128;
-      const int high_part = (fixed - low_part) >> 8;
-      high[i >> 2] |= (static_cast<uint32_t>(high_part) & 0xffu) << (8 * (i & 3));
-      low[i >> 2] |= (static_cast<uint32_t>(low_part) & 0xffu) << (8 * (i & 3));
-    }
-    const uint4 high_vector = make_uint4(high[0], high[1], high[2], high[3]);
-    const uint4 low_vector = make_uint4(low[0], low[1], low[2], low[3]);
+    uint4 high_vector, low_vector;
+    split16_planes(values, scale, &high_vector, &low_vector);
     for (int slot = 0; slot < top_k; ++slot) {
       const int64_t position = positions[slot];
       if (position >= 0) {
@@ -309,7 +241,7 @@ split_tokens_scatter_planes_kernel(const uint16_t* x, int cols, int top_k, const
 // Dense linear: arbitrary cols, fp32 or bf16 source, zero-padded to cols_padded, clamp to [-128,127]
 // (single GEMM) or [-127,127] (paired GEMMs) with division and ties-to-even (csrc/i8gemm.cpp:384-399, :492-506).
 // Status block and work items of the dense GEMM that follows (one "expert", row tiles of row_tile rows; the group key
-// of decode_unit in the fourth word), written by block 0 of the quantiser so that the op needs no launches of its own
+// of a list entry in the fourth word), written by block 0 of the quantiser so that the op needs no launches of its own
 // for them.  Every status word is written: the block starts out in an unknown state.
 struct DenseItems {
   int64_t rows;

@@ -262,6 +262,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
   // (Values that come from global loads pass through a shuffle where the warps that feed TMA and the tensor pipe use
   // them: it changes nothing but lets the compiler treat them as warp-uniform.)
   auto count_items = [&]() { return __shfl_sync(0xffffffffu, min(__ldcg(args.status + args.item_count_word), args.max_items), 0); };
+  if (args.items_late) ptx::grid_dependency_wait();
   int items = kDense ? 0 : count_items();
   const int n_blocks = (args.n_out + kChannelsPerUnit - 1) / kChannelsPerUnit;
   const int n_total = kGateUp ? 2 * args.n_out : args.n_out;

@@ -145,6 +145,39 @@ __device__ __forceinline__ void widen_int8x4(uint32_t word, uint32_t* low_pair, 
   *high_pair = __byte_perm(__float_as_uint(f2), __float_as_uint(f3), 0x7632);
 }
 
+// A work unit's item and its 128-channel block.
+struct ItemUnit {
+  int expert, row0, rows, block;
+};
+
+// Work unit -> (work item, channel block).  Items are sorted by (expert, row tile); units are ordered so that,
+// inside one expert, the row tiles of a channel block are adjacent: CTAs that run side by side then read the
+// same weight tile at the same time and the second read is served by L2 instead of HBM.  The fourth word of an item packs
+// the first item of its expert (20 bits) and that expert's tile count.  `guess`: the entry of item unit / n_blocks, which is
+// the unit's own where the expert has one item.
+__device__ __forceinline__ ItemUnit resolve_unit(const int* items, int64_t unit, int n_blocks, int4 guess) {
+  const int first = guess.w & 0xfffff;
+  const int tiles = guess.w >> 20;
+  const int local = static_cast<int>(unit - static_cast<int64_t>(first) * n_blocks);
+  if (tiles == 1) return ItemUnit{guess.x, guess.y, guess.z, local};
+  const int4 own = __ldcg(reinterpret_cast<const int4*>(items) + first + local % tiles);
+  return ItemUnit{own.x, own.y, own.z, local / tiles};
+}
+
+__device__ __forceinline__ int4 guess_item(const int* items, int64_t unit, int n_blocks) {
+  return __ldcg(reinterpret_cast<const int4*>(items) + unit / n_blocks);
+}
+
+// The same with every field taken from lane 0 (all lanes hold the same values already), for the warps that feed TMA and
+// the tensor pipe (ptx::elect_one).
+__device__ __forceinline__ ItemUnit warp_uniform(ItemUnit unit) {
+  unit.expert = __shfl_sync(0xffffffffu, unit.expert, 0);
+  unit.row0 = __shfl_sync(0xffffffffu, unit.row0, 0);
+  unit.rows = __shfl_sync(0xffffffffu, unit.rows, 0);
+  unit.block = __shfl_sync(0xffffffffu, unit.block, 0);
+  return unit;
+}
+
 // kPlanes (an instance of the int8 kernel; W8A16 in its fixed-point form): every activation row arrives as two int8
 // rows, row 2p = the high plane and row 2p + 1 = the low plane of the row's 16-bit fixed-point values
 // X = 256 * high + low, so a work item of r routes has 2r token rows and its accumulator columns come in pairs:
@@ -165,16 +198,14 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   SmemControl* ctl = reinterpret_cast<SmemControl*>(smem + static_cast<size_t>(Cfg::kOperandBytes));
 
-  // Warp index, item count and (below) the tensor-memory base pass through a shuffle: the same values, but known to the
+  // Warp index, unit count and (below) the tensor-memory base pass through a shuffle: the same values, but known to the
   // compiler as warp-uniform, which the warps that feed TMA and the tensor pipe need (ptx::elect_one).
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   int* status = args.status_rw;
 
-  const int items = __shfl_sync(0xffffffffu, min(__ldcg(args.status + args.item_count_word), args.max_items), 0);
   const int n_blocks = (args.n_out + kBlockM - 1) / kBlockM;
   const int n_total = kGateUp ? 2 * args.n_out : args.n_out;
-  const int64_t units = static_cast<int64_t>(items) * n_blocks;
   const int k_blocks = (args.k + kBlockKElems - 1) / kBlockKElems;
 
   if (threadIdx.x == 0) {
@@ -205,6 +236,21 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
   volatile int* abort_flag = &ctl->abort_flag;
 
+  if (args.items_late) ptx::grid_dependency_wait();
+  // The count and the list entry of this CTA's first unit are read side by side; the entry counts only if the unit exists
+  // (the grid has no more CTAs than the longest list has units, so it lies inside the list's memory).
+  const int item_count = __ldcg(args.status + args.item_count_word);
+  const int4 first_guess = guess_item(args.items, blockIdx.x, n_blocks);
+  const int64_t units = static_cast<int64_t>(__shfl_sync(0xffffffffu, min(item_count, args.max_items), 0)) * n_blocks;
+  const int64_t unit_step = gridDim.x;
+  ItemUnit cur = {0, 0, 0, 0};
+  if (static_cast<int64_t>(blockIdx.x) < units) cur = resolve_unit(args.items, blockIdx.x, n_blocks, first_guess);
+  // The unit after `unit`: its load is in flight while the warps work on this one.
+  auto load_next = [&](int64_t unit) {
+    if (unit + unit_step >= units) return ItemUnit{0, 0, 0, 0};
+    return resolve_unit(args.items, unit + unit_step, n_blocks, guess_item(args.items, unit + unit_step, n_blocks));
+  };
+
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     // The whole warp walks the loops; one elected lane issues the loads.
@@ -230,18 +276,14 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
       // Work items and weights are older than the kernel in front: the first stages' weights are requested while that one
       // (it makes the token rows) still runs.
       int early = 0;
-      if (!kW8A16 && static_cast<int64_t>(blockIdx.x) < units && !FMOE_DIAG_BIT(args, 2)) {
-        int item, block;
-        decode_unit(args.items, blockIdx.x, n_blocks, &item, &block);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        block = __shfl_sync(0xffffffffu, block, 0);
-        const int expert = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 0), 0);
-        const int boxes = __shfl_sync(0xffffffffu, (__ldcg(args.items + 4 * item + 2) * kRowsPerRoute + kTokenBox - 1) / kTokenBox, 0);
+      if (!kW8A16 && !args.items_late && static_cast<int64_t>(blockIdx.x) < units && !FMOE_DIAG_BIT(args, 2)) {
+        const ItemUnit first = warp_uniform(cur);
+        const int boxes = (first.rows * kRowsPerRoute + kTokenBox - 1) / kTokenBox;
         early = min(Cfg::kStages, k_blocks);
         for (int kb = 0; kb < early; ++kb) {
           if (issuer) {
             ptx::mbar_arrive_expect_tx(&ctl->full[kb], Cfg::kWeightBytes + boxes * kTokenBox * kBlockKBytes);
-            load_weights(kb, kb, block * kBlockM, expert);
+            load_weights(kb, kb, first.block * kBlockM, first.expert);
           }
         }
       }
@@ -253,14 +295,12 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
         int slot = 0;
         uint32_t slot_phase = 0;
         int landed_issued = 0;
-        for (int64_t unit = blockIdx.x; unit < units; unit += gridDim.x) {
-          int item, block;
-          decode_unit(args.items, unit, n_blocks, &item, &block);
-          item = __shfl_sync(0xffffffffu, item, 0);  // read from the item list: the same in every lane
-          block = __shfl_sync(0xffffffffu, block, 0);
-          const int expert = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 0), 0);
-          const int n0 = block * kBlockM;
-          const int row0 = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 1), 0);
+        for (int64_t unit = blockIdx.x; unit < units; unit += unit_step) {
+          const ItemUnit now = warp_uniform(cur);
+          cur = load_next(unit);
+          const int expert = now.expert;
+          const int n0 = now.block * kBlockM;
+          const int row0 = now.row0;
           for (int kb = 0; kb < k_blocks; ++kb) {
             ptx::mbar_wait(&ctl->landing_free[slot], slot_phase ^ 1u, abort_flag, status, 6);
             if (issuer) {
@@ -298,15 +338,13 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
           }
         }
       }
-      for (int64_t unit = blockIdx.x; !kW8A16 && unit < units; unit += gridDim.x) {
-        int item, block;
-        decode_unit(args.items, unit, n_blocks, &item, &block);
-        item = __shfl_sync(0xffffffffu, item, 0);  // read from the item list: the same in every lane
-        block = __shfl_sync(0xffffffffu, block, 0);
-        const int n0 = block * kBlockM;
-        const int expert = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 0), 0);
-        const int row0 = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 1), 0) * kRowsPerRoute;
-        const int boxes = __shfl_sync(0xffffffffu, (__ldcg(args.items + 4 * item + 2) * kRowsPerRoute + kTokenBox - 1) / kTokenBox, 0);
+      for (int64_t unit = blockIdx.x; !kW8A16 && unit < units; unit += unit_step) {
+        const ItemUnit now = warp_uniform(cur);
+        cur = load_next(unit);
+        const int n0 = now.block * kBlockM;
+        const int expert = now.expert;
+        const int row0 = now.row0 * kRowsPerRoute;
+        const int boxes = (now.rows * kRowsPerRoute + kTokenBox - 1) / kTokenBox;
         for (int kb = 0; kb < k_blocks; ++kb) {
           ptx::mbar_wait(&ctl->empty[stage], phase ^ 1u, abort_flag, status, 1);
           uint8_t* stage_base = smem + static_cast<size_t>(stage) * Cfg::kStageBytes;
@@ -357,7 +395,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
     constexpr int kUnits = Cfg::kWeightTiles * kBlockM * 4;  // 16-byte units of the int8 tile
     int stage = 0, slot = 0;
     uint32_t phase = 0, slot_phase = 0;
-    for (int64_t unit = blockIdx.x; unit < units; unit += gridDim.x) {
+    for (int64_t unit = blockIdx.x; unit < units; unit += unit_step) {
       for (int kb = 0; kb < k_blocks; ++kb) {
         ptx::mbar_wait(&ctl->empty[stage], phase ^ 1u, abort_flag, status, 1);
         uint8_t* stage_base = smem + static_cast<size_t>(stage) * Cfg::kStageBytes;
@@ -415,16 +453,13 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
       uint32_t phase = 0;
       int slot = 0;  // W8A16: landing slot of the K block (its token tile is the MMA's B operand)
       int local = 0;
-      for (int64_t unit = blockIdx.x; unit < units; unit += gridDim.x, ++local) {
+      for (int64_t unit = blockIdx.x; unit < units; unit += unit_step, ++local) {
         const int buffer = local % Cfg::kAccBuffers;
         const uint32_t use = static_cast<uint32_t>(local / Cfg::kAccBuffers);
         // The MMA's N follows the rows this unit really has (multiple of 16): a tail item of a few rows costs a
         // few columns of tensor-core time, not a full tile.  Unused accumulator columns are never read.
-        int item, block;
-        decode_unit(args.items, unit, n_blocks, &item, &block);
-        item = __shfl_sync(0xffffffffu, item, 0);  // read from the item list: the same in every lane
-        block = __shfl_sync(0xffffffffu, block, 0);
-        const int item_rows = __shfl_sync(0xffffffffu, __ldcg(args.items + 4 * item + 2), 0) * kRowsPerRoute;
+        const int item_rows = __shfl_sync(0xffffffffu, cur.rows, 0) * kRowsPerRoute;
+        cur = load_next(unit);
         const int mma_n = min(kRowTile, (item_rows + 15) & ~15);
         // Weight-major: M = 128 channels, N = the item's rows.  Token-major (W8A16): M = 128 token lanes, N = the
         // unit's channels (gate and up tiles are one 256-row B operand).
@@ -480,17 +515,15 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
     const int activation = args.activation;
     uint32_t* const dump = kPlanes ? nullptr : static_cast<uint32_t*>(args.dump_acc);  // the dump holds one row per route
     int local = 0;
-    for (int64_t unit = blockIdx.x; unit < units; unit += gridDim.x, ++local) {
+    for (int64_t unit = blockIdx.x; unit < units; unit += unit_step, ++local) {
       const int buffer = local % Cfg::kAccBuffers;
       const uint32_t use = static_cast<uint32_t>(local / Cfg::kAccBuffers);
-      int item, block;
-      decode_unit(args.items, unit, n_blocks, &item, &block);
-      item = __shfl_sync(0xffffffffu, item, 0);  // read from the item list: the same in every lane
-      block = __shfl_sync(0xffffffffu, block, 0);
+      const int block = cur.block;
+      const int expert = cur.expert;
+      const int row0 = cur.row0 * kRowsPerRoute;  // token rows (two per route in the two-plane form)
+      const int rows = cur.rows * kRowsPerRoute;
+      cur = load_next(unit);
       const int n = block * kBlockM + channel_in_block;
-      const int expert = __ldcg(args.items + 4 * item + 0);
-      const int row0 = __ldcg(args.items + 4 * item + 1) * kRowsPerRoute;  // token rows (two per route in the two-plane form)
-      const int rows = __ldcg(args.items + 4 * item + 2) * kRowsPerRoute;
       const bool channel_ok = n < n_out;
       ColumnMeta* meta = &ctl->meta[local & 1];
       if constexpr (kW8A16) {
