@@ -649,22 +649,23 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
           // channel: the gate lane finishes the first route of the four columns, the up lane the second, each receiving
           // the other's two plane values of that route.
           const float* scale = meta->scale + col0;
+          with_activation<false>(activation, [&](auto act) {
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const uint32_t first = __shfl_xor_sync(0xffffffffu, low ? v[4 * q + 2] : v[4 * q], 16);
-            const uint32_t second = __shfl_xor_sync(0xffffffffu, low ? v[4 * q + 3] : v[4 * q + 1], 16);
-            const int column = col0 + 4 * q + (low ? 0 : 2);  // plane row of this lane's route inside the item
-            if (column >= rows || !channel_ok) continue;
-            const int gate_high = static_cast<int>(low ? v[4 * q] : first);
-            const int gate_low = static_cast<int>(low ? v[4 * q + 1] : second);
-            const int up_high = static_cast<int>(low ? first : v[4 * q + 2]);
-            const int up_low = static_cast<int>(low ? second : v[4 * q + 3]);
-            const float a = scale[4 * q + (low ? 0 : 2)];
-            const float gate = dequantize_planes(gate_high, gate_low, a, mine.scale_gate);
-            const float up = dequantize_planes(up_high, up_low, a, mine.scale_up);
-            args.y[static_cast<int64_t>((row0 + column) >> 1) * n_out + n] =
-                activation == FMOE_ACT_SILU ? swiglu_to_bf16_with(gate, up, limit, exp_table) : other_activation_to_bf16(activation, gate, up);
-          }
+            for (int q = 0; q < 8; ++q) {
+              const uint32_t first = __shfl_xor_sync(0xffffffffu, low ? v[4 * q + 2] : v[4 * q], 16);
+              const uint32_t second = __shfl_xor_sync(0xffffffffu, low ? v[4 * q + 3] : v[4 * q + 1], 16);
+              const int column = col0 + 4 * q + (low ? 0 : 2);  // plane row of this lane's route inside the item
+              if (column >= rows || !channel_ok) continue;
+              const int gate_high = static_cast<int>(low ? v[4 * q] : first);
+              const int gate_low = static_cast<int>(low ? v[4 * q + 1] : second);
+              const int up_high = static_cast<int>(low ? first : v[4 * q + 2]);
+              const int up_low = static_cast<int>(low ? second : v[4 * q + 3]);
+              const float a = scale[4 * q + (low ? 0 : 2)];
+              const float gate = dequantize_planes(gate_high, gate_low, a, mine.scale_gate);
+              const float up = dequantize_planes(up_high, up_low, a, mine.scale_up);
+              args.y[static_cast<int64_t>((row0 + column) >> 1) * n_out + n] = gated_to_bf16(act, gate, up, limit, exp_table);
+            }
+          });
         } else if constexpr (kPlanes) {
           // down: adjacent columns are the two planes of one route; the route's output row address is staged per column.
           const bool bf16_out = args.route_out_bf16 != 0;
@@ -690,32 +691,32 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
           const float4* scale4 = reinterpret_cast<const float4*>(meta->scale + col0);
           auto body = [&](auto fast_tag, auto native_tag) {
             constexpr bool kFast = decltype(fast_tag)::value;
+            with_activation<kInt8>(activation, [&](auto act) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const float4 s4 = scale4[q];  // the scales of columns 4q .. 4q+3 (one broadcast load)
+              for (int q = 0; q < 8; ++q) {
+                const float4 s4 = scale4[q];  // the scales of columns 4q .. 4q+3 (one broadcast load)
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const int p = 2 * q + h;
-                const uint32_t received = __shfl_xor_sync(0xffffffffu, low ? v[2 * p + 1] : v[2 * p], 16);
-                const uint32_t gate_bits = low ? v[2 * p] : received;
-                const uint32_t up_bits = low ? received : v[2 * p + 1];
-                const float a = h == 0 ? (low ? s4.x : s4.y) : (low ? s4.z : s4.w);
-                if constexpr (!kFast) {
-                  const int column = col0 + 2 * p + (low ? 0 : 1);
-                  if (column >= rows || !channel_ok) continue;
-                  if (dump != nullptr) {
-                    uint32_t* out = dump + static_cast<int64_t>(row0 + column) * n_total;
-                    out[n] = gate_bits;
-                    out[n + n_out] = up_bits;
+                for (int h = 0; h < 2; ++h) {
+                  const int p = 2 * q + h;
+                  const uint32_t received = __shfl_xor_sync(0xffffffffu, low ? v[2 * p + 1] : v[2 * p], 16);
+                  const uint32_t gate_bits = low ? v[2 * p] : received;
+                  const uint32_t up_bits = low ? received : v[2 * p + 1];
+                  const float a = h == 0 ? (low ? s4.x : s4.y) : (low ? s4.z : s4.w);
+                  if constexpr (!kFast) {
+                    const int column = col0 + 2 * p + (low ? 0 : 1);
+                    if (column >= rows || !channel_ok) continue;
+                    if (dump != nullptr) {
+                      uint32_t* out = dump + static_cast<int64_t>(row0 + column) * n_total;
+                      out[n] = gate_bits;
+                      out[n + n_out] = up_bits;
+                    }
                   }
+                  const float gate = to_float(native_tag, gate_bits, a, mine.scale_gate);
+                  const float up = to_float(native_tag, up_bits, a, mine.scale_up);
+                  out0[static_cast<uint32_t>(p) * pair_stride] = gated_to_bf16(act, gate, up, limit, exp_table);
                 }
-                const float gate = to_float(native_tag, gate_bits, a, mine.scale_gate);
-                const float up = to_float(native_tag, up_bits, a, mine.scale_up);
-                out0[static_cast<uint32_t>(p) * pair_stride] =
-                    (kInt8 || activation == FMOE_ACT_SILU) ? swiglu_to_bf16_with(gate, up, limit, exp_table)
-                                                           : other_activation_to_bf16(activation, gate, up);
               }
-            }
+            });
           };
           dispatch(fast, body);
         } else {

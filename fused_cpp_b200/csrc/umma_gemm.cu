@@ -17,14 +17,14 @@
 // gate_up issues two MMAs per K step (gate rows n and up rows I+n against the same token tile) so
 // that each epilogue thread holds the gate and the up value of the same (token, channel).
 //
-// CTA = 6 warps, persistent over work units (work item x 128-channel block), round-robin:
+// CTA = 10 warps, persistent over work units (work item x 128-channel block), round-robin:
 //   warp 0      TMA producer: per K block of 128 bytes, one or two weight tiles + the token tile;
 //   warp 1      allocates TMEM, issues tcgen05.mma (one thread), commits to the stage's "empty"
 //               barrier and, per work unit, to the accumulator's "full" barrier;
-//   warps 2..5  epilogue: tcgen05.ld their 32-lane TMEM quarter, apply the epilogue, store.
+//   warps 2..9  epilogue: tcgen05.ld their 32-lane TMEM quarter, apply the epilogue, store.
 // W8A16 (int8 weights, bf16 activations; the reference's fused_moe_w8a16_* ops, csrc/moe/arm/common/
 // fused_moe_bf16_tiled.cpp:4916-5000, 8740-8760): the weight tile arrives as int8 (half the HBM bytes of bf16) in a
-// landing area of the stage, eight more warps (6..13) widen it to bf16 -- exact, |q| <= 128 -- into the 128-byte
+// landing area of the stage, eight more warps (6..13, behind four of the epilogue) widen it to bf16 -- exact, |q| <= 128 -- into the 128-byte
 // swizzled operand tile the kind::f16 MMA reads, and the epilogue multiplies by the per-output-channel scale in
 // fp32.  This instance runs TOKEN-MAJOR: the token tile is the A operand (M = 128 lanes = token rows, of which the
 // item's rows are real) and the widened weight tile the B operand (N = 256 = 128 gate + 128 up channels, or 128 for
@@ -50,8 +50,13 @@ constexpr int kBlockM = 128;        // output channels per MMA tile (TMEM lanes)
 constexpr int kBlockKBytes = 128;   // bytes of K per pipeline stage = one 128-byte swizzle row
 constexpr int kUmmaKBytes = 32;     // bytes of K per tcgen05.mma
 constexpr int kTokenBox = 16;       // token rows per TMA box: an item loads the rows its MMAs read, not its tile
-constexpr int kThreads = 192;
+// Epilogue warps: two per tensor-memory lane quarter, which take 8-column chunks in turn.  With one, the epilogue behind
+// the last unit of a short launch is twice as long, and units of 64 rows and more wait for it: int8 weights with 16-bit
+// activations, 1000 tokens of the 256-expert layer (planes) 2054 -> 2028 us, 64 tokens (int8) 1489 -> 1476 (W8A16's widening form keeps one: its eight converter warps need the issue slots).
 constexpr int kEpilogueWarp0 = 2;
+constexpr int kEpilogueWarps = 8;
+constexpr int kEpilogueWarpsW8A16 = 4;
+constexpr int kThreads = 64 + kEpilogueWarps * 32;
 constexpr int kConvertWarp0 = 6;          // W8A16: warps 6.. widen the int8 weight tile to bf16
 #ifndef FMOE_W8A16_CONVERT_WARPS
 #define FMOE_W8A16_CONVERT_WARPS 8
@@ -60,7 +65,7 @@ constexpr int kConvertWarp0 = 6;          // W8A16: warps 6.. widen the int8 wei
 #define FMOE_W8A16_STAGES 2
 #endif
 constexpr int kConvertWarps = FMOE_W8A16_CONVERT_WARPS;
-constexpr int kThreadsW8A16 = kThreads + kConvertWarps * 32;
+constexpr int kThreadsW8A16 = 64 + kEpilogueWarpsW8A16 * 32 + kConvertWarps * 32;
 constexpr int kLandingRowBytes = 64;      // W8A16: one K block = 64 weights = 64 int8 bytes per channel row
 constexpr int kSmemBudget = 216 * 1024;  // operand stages; with the control block and alignment slack 224 KB of the 227 KB a CTA may have
 
@@ -190,6 +195,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
   static_assert(!kW8A16 || !kInt8, "W8A16 is an instance of the bf16 grouped kernel");
   static_assert(!kPlanes || (kInt8 && !kW8A16), "the two-plane form is an instance of the int8 grouped kernel");
   constexpr int kRowsPerRoute = kPlanes ? 2 : 1;
+  constexpr int kEpiWarps = kW8A16 ? kEpilogueWarpsW8A16 : kEpilogueWarps;
   using Cfg = TileConfig<kGateUp, kRowTile, kW8A16>;
   constexpr int kElemBytes = kInt8 ? 1 : 2;
   constexpr int kBlockKElems = kBlockKBytes / kElemBytes;
@@ -220,7 +226,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
     }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(&ctl->acc_full[b], 1);
-      ptx::mbar_init(&ctl->acc_empty[b], 4);
+      ptx::mbar_init(&ctl->acc_empty[b], kEpiWarps);
     }
     ctl->abort_flag = 0;
     ptx::fence_barrier_init();
@@ -504,7 +510,7 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
       }
     }
   } else {
-    // ---------------- epilogue (warps 2..5) ----------------
+    // ---------------- epilogue (warps 2 .. 1 + kEpiWarps) ----------------
     ptx::grid_dependency_wait();
     const int quarter = warp & 3;  // the TMEM lanes a warp may read are fixed by warp id % 4
     const int channel_in_block = quarter * 32 + lane;
@@ -557,51 +563,52 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
             out_row = reinterpret_cast<uint8_t*>(base) + static_cast<size_t>(n0) * (args.route_out_bf16 ? 2 : 4);
           }
         }
-        for (int c0 = 0; warp_has_rows && c0 < channels; c0 += 8) {
-          uint32_t gate_bits[8];
-          uint32_t up_bits[8];
-          ptx::tmem_ld_x8(acc + c0, gate_bits);
-          if (kGateUp) ptx::tmem_ld_x8(acc + kBlockM + c0, up_bits);
-          ptx::tmem_ld_wait();
-          if (!row_ok) continue;
-          if constexpr (kGateUp) {
-            uint32_t packed[4];
-#pragma unroll
-            for (int j = 0; j < 8; j += 2) {
-              uint16_t pair[2];
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const float gate = __fmul_rn(__uint_as_float(gate_bits[j + h]), meta->scale[c0 + j + h]);
-                const float up = __fmul_rn(__uint_as_float(up_bits[j + h]), meta->scale[kBlockM + c0 + j + h]);
-                pair[h] = activation == FMOE_ACT_SILU ? swiglu_to_bf16_with(gate, up, limit, ctl->exp_table)
-                                                      : other_activation_to_bf16(activation, gate, up);
-              }
-              packed[j >> 1] = static_cast<uint32_t>(pair[0]) | (static_cast<uint32_t>(pair[1]) << 16);
-            }
-            *reinterpret_cast<uint4*>(out_row + c0 * 2) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-          } else {
-            float values[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) values[j] = __fmul_rn(__uint_as_float(gate_bits[j]), meta->scale[c0 + j]);
-            if (args.route_out_bf16) {
+        with_activation<!kGateUp>(activation, [&](auto act) {
+          for (int c0 = 0; warp_has_rows && c0 < channels; c0 += 8) {
+            uint32_t gate_bits[8];
+            uint32_t up_bits[8];
+            ptx::tmem_ld_x8(acc + c0, gate_bits);
+            if (kGateUp) ptx::tmem_ld_x8(acc + kBlockM + c0, up_bits);
+            ptx::tmem_ld_wait();
+            if (!row_ok) continue;
+            if constexpr (kGateUp) {
               uint32_t packed[4];
 #pragma unroll
               for (int j = 0; j < 8; j += 2) {
-                packed[j >> 1] = static_cast<uint32_t>(f32_to_bf16_bits(values[j])) | (static_cast<uint32_t>(f32_to_bf16_bits(values[j + 1])) << 16);
+                uint16_t pair[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                  const float gate = __fmul_rn(__uint_as_float(gate_bits[j + h]), meta->scale[c0 + j + h]);
+                  const float up = __fmul_rn(__uint_as_float(up_bits[j + h]), meta->scale[kBlockM + c0 + j + h]);
+                  pair[h] = gated_to_bf16(act, gate, up, limit, ctl->exp_table);
+                }
+                packed[j >> 1] = static_cast<uint32_t>(pair[0]) | (static_cast<uint32_t>(pair[1]) << 16);
               }
               *reinterpret_cast<uint4*>(out_row + c0 * 2) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
             } else {
-              *reinterpret_cast<float4*>(out_row + c0 * 4) = make_float4(values[0], values[1], values[2], values[3]);
-              *reinterpret_cast<float4*>(out_row + c0 * 4 + 16) = make_float4(values[4], values[5], values[6], values[7]);
+              float values[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) values[j] = __fmul_rn(__uint_as_float(gate_bits[j]), meta->scale[c0 + j]);
+              if (args.route_out_bf16) {
+                uint32_t packed[4];
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) {
+                  packed[j >> 1] = static_cast<uint32_t>(f32_to_bf16_bits(values[j])) | (static_cast<uint32_t>(f32_to_bf16_bits(values[j + 1])) << 16);
+                }
+                *reinterpret_cast<uint4*>(out_row + c0 * 2) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+              } else {
+                *reinterpret_cast<float4*>(out_row + c0 * 4) = make_float4(values[0], values[1], values[2], values[3]);
+                *reinterpret_cast<float4*>(out_row + c0 * 4 + 16) = make_float4(values[4], values[5], values[6], values[7]);
+              }
             }
           }
-        }
+        });
         ptx::tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&ctl->acc_empty[buffer]);
         continue;
       }
-      for (int c = epilogue_thread; c < rows; c += 128) {
+      for (int c = epilogue_thread; c < rows; c += kEpiWarps * 32) {
         const int route_row = (row0 + c) / kRowsPerRoute;  // sorted position of the column's route
         if (kInt8) meta->scale[c] = __ldcg(args.a_scale + route_row);
         if constexpr (!kGateUp) {
@@ -623,31 +630,69 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
         bias_gate = load_expert_bias(args, first + (kGateUp ? gate_channel(args, n) : n));
         if (kGateUp) bias_up = load_expert_bias(args, first + up_channel(args, n));
       }
-      asm volatile("bar.sync 1, 128;" ::: "memory");  // metadata visible to the four epilogue warps
+      asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");  // metadata visible to the epilogue warps
       ptx::mbar_wait(&ctl->acc_full[buffer], use & 1u, abort_flag, status, 4);
       ptx::tcgen05_fence_after();
       const uint32_t acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buffer * Cfg::kAccColumns);
-      for (int c0 = 0; c0 < (FMOE_DIAG_BIT(args, 1) ? 0 : rows); c0 += 8) {
-        uint32_t gate_bits[8];
-        uint32_t up_bits[8];
-        ptx::tmem_ld_x8(acc + c0, gate_bits);
-        if (kGateUp) ptx::tmem_ld_x8(acc + kRowTile + c0, up_bits);
-        ptx::tmem_ld_wait();
-        if (channel_ok) {
+      with_activation<!kGateUp || (kInt8 && !kPlanes)>(activation, [&](auto act) {
+        for (int c0 = 8 * ((warp - kEpilogueWarp0) >> 2); c0 < (FMOE_DIAG_BIT(args, 1) ? 0 : rows); c0 += 8 * (kEpiWarps / 4)) {
+          uint32_t gate_bits[8];
+          uint32_t up_bits[8];
+          ptx::tmem_ld_x8(acc + c0, gate_bits);
+          if (kGateUp) ptx::tmem_ld_x8(acc + kRowTile + c0, up_bits);
+          ptx::tmem_ld_wait();
+          if (channel_ok) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            if constexpr (kPlanes) {
-              // Columns (j, j + 1) = (high, low) plane of one route; rows is even, so the pair is complete.
-              if ((j & 1) == 0 && c0 + j < rows) {
-                const float a = meta->scale[c0 + j];
+            for (int j = 0; j < 8; ++j) {
+              if constexpr (kPlanes) {
+                // Columns (j, j + 1) = (high, low) plane of one route; rows is even, so the pair is complete.
+                if ((j & 1) == 0 && c0 + j < rows) {
+                  const float a = meta->scale[c0 + j];
+                  if constexpr (kGateUp) {
+                    const float gate = dequantize_planes(static_cast<int>(gate_bits[j]), static_cast<int>(gate_bits[j + 1]), a, scale_gate);
+                    const float up = dequantize_planes(static_cast<int>(up_bits[j]), static_cast<int>(up_bits[j + 1]), a, scale_up);
+                    args.y[static_cast<int64_t>((row0 + c0 + j) >> 1) * n_out + n] = gated_to_bf16(act, gate, up, limit, ctl->exp_table);
+                  } else {
+                    const float value = dequantize_planes(static_cast<int>(gate_bits[j]), static_cast<int>(gate_bits[j + 1]), a, scale_gate);
+                    const uint64_t rowptr = meta->rowptr[c0 + j];
+                    if (args.route_out_bf16) {
+                      reinterpret_cast<uint16_t*>(rowptr)[n] = f32_to_bf16_bits(value);
+                    } else {
+                      reinterpret_cast<float*>(rowptr)[n] = value;
+                    }
+                  }
+                }
+                continue;
+              }
+              if (c0 + j < rows) {
+                if (dump != nullptr) {
+                  uint32_t* out = dump + static_cast<int64_t>(row0 + c0 + j) * n_total;
+                  out[n] = gate_bits[j];
+                  if (kGateUp) out[n + n_out] = up_bits[j];
+                }
                 if constexpr (kGateUp) {
-                  const float gate = dequantize_planes(static_cast<int>(gate_bits[j]), static_cast<int>(gate_bits[j + 1]), a, scale_gate);
-                  const float up = dequantize_planes(static_cast<int>(up_bits[j]), static_cast<int>(up_bits[j + 1]), a, scale_up);
-                  args.y[static_cast<int64_t>((row0 + c0 + j) >> 1) * n_out + n] =
-                      activation == FMOE_ACT_SILU ? swiglu_to_bf16_with(gate, up, limit, ctl->exp_table)
-                                                  : other_activation_to_bf16(activation, gate, up);
+                  float gate, up;
+                  if constexpr (kInt8) {
+                    const float a = meta->scale[c0 + j];
+                    gate = dequantize(static_cast<int>(gate_bits[j]), a, scale_gate, numerics);
+                    up = dequantize(static_cast<int>(up_bits[j]), a, scale_up, numerics);
+                  } else if constexpr (kW8A16) {
+                    gate = __fmul_rn(__uint_as_float(gate_bits[j]), scale_gate);
+                    up = __fmul_rn(__uint_as_float(up_bits[j]), scale_up);
+                  } else {
+                    gate = __fadd_rn(__uint_as_float(gate_bits[j]), bias_gate);
+                    up = __fadd_rn(__uint_as_float(up_bits[j]), bias_up);
+                  }
+                  args.y[static_cast<int64_t>(row0 + c0 + j) * n_out + n] = gated_to_bf16(act, gate, up, limit, ctl->exp_table);
                 } else {
-                  const float value = dequantize_planes(static_cast<int>(gate_bits[j]), static_cast<int>(gate_bits[j + 1]), a, scale_gate);
+                  float value;
+                  if constexpr (kInt8) {
+                    value = dequantize(static_cast<int>(gate_bits[j]), meta->scale[c0 + j], scale_gate, numerics);
+                  } else if constexpr (kW8A16) {
+                    value = __fmul_rn(__uint_as_float(gate_bits[j]), scale_gate);
+                  } else {
+                    value = __fadd_rn(__uint_as_float(gate_bits[j]), bias_gate);
+                  }
                   const uint64_t rowptr = meta->rowptr[c0 + j];
                   if (args.route_out_bf16) {
                     reinterpret_cast<uint16_t*>(rowptr)[n] = f32_to_bf16_bits(value);
@@ -656,50 +701,10 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
                   }
                 }
               }
-              continue;
-            }
-            if (c0 + j < rows) {
-              if (dump != nullptr) {
-                uint32_t* out = dump + static_cast<int64_t>(row0 + c0 + j) * n_total;
-                out[n] = gate_bits[j];
-                if (kGateUp) out[n + n_out] = up_bits[j];
-              }
-              if constexpr (kGateUp) {
-                float gate, up;
-                if constexpr (kInt8) {
-                  const float a = meta->scale[c0 + j];
-                  gate = dequantize(static_cast<int>(gate_bits[j]), a, scale_gate, numerics);
-                  up = dequantize(static_cast<int>(up_bits[j]), a, scale_up, numerics);
-                } else if constexpr (kW8A16) {
-                  gate = __fmul_rn(__uint_as_float(gate_bits[j]), scale_gate);
-                  up = __fmul_rn(__uint_as_float(up_bits[j]), scale_up);
-                } else {
-                  gate = __fadd_rn(__uint_as_float(gate_bits[j]), bias_gate);
-                  up = __fadd_rn(__uint_as_float(up_bits[j]), bias_up);
-                }
-                args.y[static_cast<int64_t>(row0 + c0 + j) * n_out + n] =
-                    (kInt8 || activation == FMOE_ACT_SILU) ? swiglu_to_bf16_with(gate, up, limit, ctl->exp_table)
-                                                           : other_activation_to_bf16(activation, gate, up);
-              } else {
-                float value;
-                if constexpr (kInt8) {
-                  value = dequantize(static_cast<int>(gate_bits[j]), meta->scale[c0 + j], scale_gate, numerics);
-                } else if constexpr (kW8A16) {
-                  value = __fmul_rn(__uint_as_float(gate_bits[j]), scale_gate);
-                } else {
-                  value = __fadd_rn(__uint_as_float(gate_bits[j]), bias_gate);
-                }
-                const uint64_t rowptr = meta->rowptr[c0 + j];
-                if (args.route_out_bf16) {
-                  reinterpret_cast<uint16_t*>(rowptr)[n] = f32_to_bf16_bits(value);
-                } else {
-                  reinterpret_cast<float*>(rowptr)[n] = value;
-                }
-              }
             }
           }
         }
-      }
+      });
       ptx::tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&ctl->acc_empty[buffer]);
