@@ -52,7 +52,8 @@ constexpr int kUmmaKBytes = 32;     // bytes of K per tcgen05.mma
 constexpr int kTokenBox = 16;       // token rows per TMA box: an item loads the rows its MMAs read, not its tile
 // Epilogue warps: two per tensor-memory lane quarter, which take 8-column chunks in turn.  With one, the epilogue behind
 // the last unit of a short launch is twice as long, and units of 64 rows and more wait for it: int8 weights with 16-bit
-// activations, 1000 tokens of the 256-expert layer (planes) 2054 -> 2028 us, 64 tokens (int8) 1489 -> 1476 (W8A16's widening form keeps one: its eight converter warps need the issue slots).
+// activations, 1000 tokens of the 256-expert layer (planes) 2054 -> 2028 us (W8A16's widening form keeps one:
+// its eight converter warps need the issue slots).
 constexpr int kEpilogueWarp0 = 2;
 constexpr int kEpilogueWarps = 8;
 constexpr int kEpilogueWarpsW8A16 = 4;
