@@ -932,6 +932,15 @@ int fmoe_i8gemm_dynamic_scaled_mm_pair(const void* x_bf16, int64_t rows, int32_t
 }
 
 #ifdef FMOE_DIAG
+int fmoe_diag_quotient_check(uint32_t seed, int32_t numerators, void* mismatches, void* stream) {
+  const int status = check_device();
+  if (status != FMOE_OK) return status;
+  if (numerators <= 0 || mismatches == nullptr) return fail(FMOE_ERR_INVALID_ARGUMENT, "quotient check: nothing to do");
+  const cudaError_t error =
+      fmoe::launch_quotient_check(seed, numerators, static_cast<unsigned long long*>(mismatches), static_cast<cudaStream_t>(stream));
+  return error == cudaSuccess ? FMOE_OK : cuda_fail(error, "quotient check");
+}
+
 int fmoe_probe_mma_rate(int32_t int8, int32_t n, int32_t iterations, int32_t mode, float* tera_ops_per_s) {
   int status = check_device();
   if (status != FMOE_OK) return status;

@@ -8,6 +8,7 @@
 //   bf16 store         csrc/moe/arm/i8mm_w8a8/kernels.cpp:194-198
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -53,14 +54,31 @@ __device__ __constant__ const uint32_t kExp2Table[64] = {
     0x3feac0c7u, 0x3fed4f30u, 0x3fefe4bau, 0x3ff28177u, 0x3ff5257du, 0x3ff7d0dfu, 0x3ffa83b3u, 0x3ffd3e0cu,
 };
 
+// Approximate reciprocal (within one unit in the last place), the seed of quotient_fast.
+__device__ __forceinline__ float reciprocal_seed(float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  return r;
+}
+
+// n / d rounded to nearest for d in [1, 2^40] and |n| in [2^-60, 2^60]: a Newton step makes the seed the correctly rounded
+// reciprocal, and by Markstein's theorem (P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990) a quotient that is corrected once by its exact remainder times that reciprocal is
+// the correctly rounded one; in these ranges no step over- or underflows.  __fdiv_rn gives the same bits but tests its operands
+// and branches, which keeps the compiler from overlapping the elements of an unrolled loop.
+// (tests/test_gpu_quotient.py compares the two for every mantissa of d.)
+__device__ __forceinline__ float quotient_fast(float n, float d) {
+  const float seed = reciprocal_seed(d);
+  const float r = __fmaf_rn(seed, __fmaf_rn(-d, seed, 1.0f), seed);
+  const float q = __fmul_rn(n, r);
+  return __fmaf_rn(__fmaf_rn(-d, q, n), r, q);
+}
+
 // exp(-gate) with the reference's FEXPA evaluator: range reduction to multiples of 1/64 in the
 // exponent, a table significand and a degree-2 correction.  `table` is kExp2Table or a copy of it in
 // shared memory: lanes index it with different values, which the constant cache serialises (one
 // address per pass) while shared memory serves 32 banks at once.
-__device__ __forceinline__ float expneg_with(float gate, const uint32_t* table) {
-  float x = -gate;
-  x = fminf(x, 87.0f);
-  x = fmaxf(x, -87.0f);
+__device__ __forceinline__ float expneg_clamped(float x, const uint32_t* table) {
   const float encoded = __fmaf_rn(x, 1.4426950216293335f, 196735.0f);
   const float k = __fsub_rn(encoded, 196735.0f);
   float residual = __fmaf_rn(-k, 0.693145751953125f, x);
@@ -70,6 +88,13 @@ __device__ __forceinline__ float expneg_with(float gate, const uint32_t* table) 
   const float scale = __uint_as_float(scale_bits);
   const float polynomial = __fmaf_rn(residual, 0.5000003576278687f, 1.000003695487976f);
   return __fmaf_rn(scale, __fmul_rn(polynomial, residual), scale);
+}
+
+__device__ __forceinline__ float expneg_with(float gate, const uint32_t* table) {
+  float x = -gate;
+  x = fminf(x, 87.0f);
+  x = fmaxf(x, -87.0f);
+  return expneg_clamped(x, table);
 }
 
 __device__ __forceinline__ float expneg(float gate) { return expneg_with(gate, kExp2Table); }
@@ -82,6 +107,37 @@ __device__ __forceinline__ uint16_t swiglu_to_bf16_with(float gate, float up, fl
   }
   const float value = __fdiv_rn(__fmul_rn(gate, up), __fadd_rn(expneg_with(gate, table), 1.0f));
   return f32_to_bf16_bits(value);
+}
+
+// swiglu_to_bf16_with for N elements, the same bits.  Where every gate lies in [-27, 80] (no clamp of the exponent, and
+// 1 + exp(-gate) below 2^40) and every product in the range of quotient_fast, no element has a branch and the N chains
+// overlap; what lies outside, zeros, infinities and NaN among it, sends all N through the plain statement.
+template <int N>
+__device__ __forceinline__ void swiglu_group(const float (&gate)[N], const float (&up)[N], float limit, const uint32_t* table,
+                                             uint16_t (&out)[N]) {
+  constexpr uint32_t kSmallest = 0x21800000u;          // 2^-60
+  constexpr uint32_t kRange = 0x5d800000u - kSmallest;  // up to 2^60
+  const float clamp = limit > 0.0f ? limit : __int_as_float(0x7f800000);
+  float product[N], denominator[N];
+  uint32_t worst = 0;
+  float lowest = 0.0f, highest = 0.0f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float g = fminf(gate[i], clamp);
+    const float u = fmaxf(fminf(up[i], clamp), -clamp);
+    product[i] = __fmul_rn(g, u);
+    denominator[i] = __fadd_rn(expneg_clamped(-g, table), 1.0f);
+    worst = max(worst, (__float_as_uint(product[i]) & 0x7fffffffu) - kSmallest);
+    lowest = fminf(lowest, g);
+    highest = fmaxf(highest, g);
+  }
+  if (worst <= kRange && lowest >= -27.0f && highest <= 80.0f) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) out[i] = __bfloat16_as_ushort(__float2bfloat16_rn(quotient_fast(product[i], denominator[i])));
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) out[i] = swiglu_to_bf16_with(gate[i], up[i], limit, table);
+  }
 }
 
 // The other gated activations of the reference's BF16 op (csrc/moe/arm/common/fused_moe_bf16_tiled.cpp:1911-1936,
@@ -123,6 +179,18 @@ __device__ __forceinline__ uint16_t gated_to_bf16(Tag, float gate, float up, flo
     up = fmaxf(fminf(up, 7.0f), -7.0f);
     const float glu = gate / (1.0f + expf(-1.702f * gate));
     return f32_to_bf16_bits((up + 1.0f) * glu);
+  }
+}
+
+// N elements of either kind.
+template <typename Tag, int N>
+__device__ __forceinline__ void gated_group(Tag act, const float (&gate)[N], const float (&up)[N], float limit, const uint32_t* table,
+                                            uint16_t (&out)[N]) {
+  if constexpr (Tag::value == FMOE_ACT_SILU) {
+    swiglu_group(gate, up, limit, table, out);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) out[i] = gated_to_bf16(act, gate[i], up[i], limit, table);
   }
 }
 

@@ -193,7 +193,35 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128, 1) mma_rate_pai
   }
 }
 
+// quotient_fast against __fdiv_rn: one thread per mantissa of d; numerators are the two ends and the middle of a binade and
+// random ones, exponents random inside the ranges of quotient_fast.
+__global__ void quotient_check_kernel(uint32_t seed, int numerators, unsigned long long* mismatches) {
+  const uint32_t mantissa = blockIdx.x * blockDim.x + threadIdx.x;
+  if (mantissa >= (1u << 23)) return;
+  uint32_t state = seed ^ (mantissa * 2654435761u);
+  auto next = [&]() {
+    state ^= state << 13;
+    state ^= state >> 17;
+    state ^= state << 5;
+    return state;
+  };
+  if (state == 0) state = 1;
+  unsigned long long wrong = 0;
+  for (int i = 0; i < numerators; ++i) {
+    const float d = __uint_as_float(((127u + next() % 40u) << 23) | mantissa);
+    const uint32_t numerator = i == 0 ? 0u : i == 1 ? 0x7fffffu : i == 2 ? 0x400000u : i == 3 ? mantissa : next() & 0x7fffffu;
+    const float n = __uint_as_float((next() & 0x80000000u) | ((67u + next() % 120u) << 23) | numerator);
+    if (__float_as_uint(quotient_fast(n, d)) != __float_as_uint(__fdiv_rn(n, d))) ++wrong;
+  }
+  if (wrong != 0) atomicAdd(mismatches, wrong);
+}
+
 }  // namespace
+
+cudaError_t launch_quotient_check(uint32_t seed, int numerators, unsigned long long* mismatches, cudaStream_t stream) {
+  quotient_check_kernel<<<(1 << 23) / 256, 256, 0, stream>>>(seed, numerators, mismatches);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_mma_rate_probe(bool int8, int n, int iterations, int mode, int blocks, int* status, cudaStream_t stream) {
   const size_t smem = 1024 + 16384 + 32768;

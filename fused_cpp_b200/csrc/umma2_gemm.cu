@@ -666,20 +666,27 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
           // the other's two plane values of that route.
           const float* scale = meta->scale + col0;
           with_activation<false>(activation, [&](auto act) {
+            float gate[8], up[8];
+            uint16_t result[8];
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
               const uint32_t first = __shfl_xor_sync(0xffffffffu, low ? v[4 * q + 2] : v[4 * q], 16);
               const uint32_t second = __shfl_xor_sync(0xffffffffu, low ? v[4 * q + 3] : v[4 * q + 1], 16);
-              const int column = col0 + 4 * q + (low ? 0 : 2);  // plane row of this lane's route inside the item
-              if (column >= rows || !channel_ok) continue;
+              const int column = 4 * q + (low ? 0 : 2);  // plane row of this lane's route inside the chunk
               const int gate_high = static_cast<int>(low ? v[4 * q] : first);
               const int gate_low = static_cast<int>(low ? v[4 * q + 1] : second);
               const int up_high = static_cast<int>(low ? first : v[4 * q + 2]);
               const int up_low = static_cast<int>(low ? second : v[4 * q + 3]);
-              const float a = scale[4 * q + (low ? 0 : 2)];
-              const float gate = dequantize_planes(gate_high, gate_low, a, mine.scale_gate);
-              const float up = dequantize_planes(up_high, up_low, a, mine.scale_up);
-              args.y[static_cast<int64_t>((row0 + column) >> 1) * n_out + n] = gated_to_bf16(act, gate, up, limit, exp_table);
+              const float a = scale[column];
+              gate[q] = dequantize_planes(gate_high, gate_low, a, mine.scale_gate);
+              up[q] = dequantize_planes(up_high, up_low, a, mine.scale_up);
+              if (col0 + column >= rows) gate[q] = up[q] = 1.0f;  // no row: nothing that could send the group to its slow branch
+            }
+            gated_group(act, gate, up, limit, exp_table, result);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const int column = col0 + 4 * q + (low ? 0 : 2);
+              if (column < rows && channel_ok) args.y[static_cast<int64_t>((row0 + column) >> 1) * n_out + n] = result[q];
             }
           });
         } else if constexpr (kPlanes) {
@@ -709,27 +716,35 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
             constexpr bool kFast = decltype(fast_tag)::value;
             with_activation<kInt8>(activation, [&](auto act) {
 #pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                const float4 s4 = scale4[q];  // the scales of columns 4q .. 4q+3 (one broadcast load)
+              for (int group = 0; group < 2; ++group) {  // sixteen columns, eight elements of this thread
+                float gate[8], up[8];
+                uint16_t result[8];
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                  const int p = 2 * q + h;
+                for (int i = 0; i < 8; ++i) {
+                  const int p = 8 * group + i;
+                  const float4 s4 = scale4[p >> 1];  // the scales of four columns (one broadcast load)
                   const uint32_t received = __shfl_xor_sync(0xffffffffu, low ? v[2 * p + 1] : v[2 * p], 16);
                   const uint32_t gate_bits = low ? v[2 * p] : received;
                   const uint32_t up_bits = low ? received : v[2 * p + 1];
-                  const float a = h == 0 ? (low ? s4.x : s4.y) : (low ? s4.z : s4.w);
+                  const float a = (p & 1) == 0 ? (low ? s4.x : s4.y) : (low ? s4.z : s4.w);
+                  gate[i] = to_float(native_tag, gate_bits, a, mine.scale_gate);
+                  up[i] = to_float(native_tag, up_bits, a, mine.scale_up);
                   if constexpr (!kFast) {
                     const int column = col0 + 2 * p + (low ? 0 : 1);
-                    if (column >= rows || !channel_ok) continue;
-                    if (dump != nullptr) {
+                    if (column >= rows || !channel_ok) {
+                      gate[i] = up[i] = 1.0f;  // no element: nothing that could send the group to its slow branch
+                    } else if (dump != nullptr) {
                       uint32_t* out = dump + static_cast<int64_t>(row0 + column) * n_total;
                       out[n] = gate_bits;
                       out[n + n_out] = up_bits;
                     }
                   }
-                  const float gate = to_float(native_tag, gate_bits, a, mine.scale_gate);
-                  const float up = to_float(native_tag, up_bits, a, mine.scale_up);
-                  out0[static_cast<uint32_t>(p) * pair_stride] = gated_to_bf16(act, gate, up, limit, exp_table);
+                }
+                gated_group(act, gate, up, limit, exp_table, result);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  const int p = 8 * group + i;
+                  if (kFast || (col0 + 2 * p + (low ? 0 : 1) < rows && channel_ok)) out0[static_cast<uint32_t>(p) * pair_stride] = result[i];
                 }
               }
             });

@@ -573,18 +573,17 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
             ptx::tmem_ld_wait();
             if (!row_ok) continue;
             if constexpr (kGateUp) {
+              float gate[8], up[8];
+              uint16_t result[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                gate[j] = __fmul_rn(__uint_as_float(gate_bits[j]), meta->scale[c0 + j]);
+                up[j] = __fmul_rn(__uint_as_float(up_bits[j]), meta->scale[kBlockM + c0 + j]);
+              }
+              gated_group(act, gate, up, limit, ctl->exp_table, result);
               uint32_t packed[4];
 #pragma unroll
-              for (int j = 0; j < 8; j += 2) {
-                uint16_t pair[2];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                  const float gate = __fmul_rn(__uint_as_float(gate_bits[j + h]), meta->scale[c0 + j + h]);
-                  const float up = __fmul_rn(__uint_as_float(up_bits[j + h]), meta->scale[kBlockM + c0 + j + h]);
-                  pair[h] = gated_to_bf16(act, gate, up, limit, ctl->exp_table);
-                }
-                packed[j >> 1] = static_cast<uint32_t>(pair[0]) | (static_cast<uint32_t>(pair[1]) << 16);
-              }
+              for (int j = 0; j < 8; j += 2) packed[j >> 1] = static_cast<uint32_t>(result[j]) | (static_cast<uint32_t>(result[j + 1]) << 16);
               *reinterpret_cast<uint4*>(out_row + c0 * 2) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
             } else {
               float values[8];
@@ -642,65 +641,61 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
           ptx::tmem_ld_x8(acc + c0, gate_bits);
           if (kGateUp) ptx::tmem_ld_x8(acc + kRowTile + c0, up_bits);
           ptx::tmem_ld_wait();
-          if (channel_ok) {
+          if (!channel_ok) continue;
+          if (dump != nullptr) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
+              if (c0 + j >= rows) break;
+              uint32_t* out = dump + static_cast<int64_t>(row0 + c0 + j) * n_total;
+              out[n] = gate_bits[j];
+              if (kGateUp) out[n + n_out] = up_bits[j];
+            }
+          }
+          // kPlanes: columns (j, j + 1) = (high, low) plane of one route; rows is even, so the pair is complete.
+          if constexpr (kGateUp) {
+            constexpr int kElements = 8 / kRowsPerRoute;
+            float gate[kElements], up[kElements];
+            uint16_t result[kElements];
+#pragma unroll
+            for (int i = 0; i < kElements; ++i) {
+              const int j = i * kRowsPerRoute;
               if constexpr (kPlanes) {
-                // Columns (j, j + 1) = (high, low) plane of one route; rows is even, so the pair is complete.
-                if ((j & 1) == 0 && c0 + j < rows) {
-                  const float a = meta->scale[c0 + j];
-                  if constexpr (kGateUp) {
-                    const float gate = dequantize_planes(static_cast<int>(gate_bits[j]), static_cast<int>(gate_bits[j + 1]), a, scale_gate);
-                    const float up = dequantize_planes(static_cast<int>(up_bits[j]), static_cast<int>(up_bits[j + 1]), a, scale_up);
-                    args.y[static_cast<int64_t>((row0 + c0 + j) >> 1) * n_out + n] = gated_to_bf16(act, gate, up, limit, ctl->exp_table);
-                  } else {
-                    const float value = dequantize_planes(static_cast<int>(gate_bits[j]), static_cast<int>(gate_bits[j + 1]), a, scale_gate);
-                    const uint64_t rowptr = meta->rowptr[c0 + j];
-                    if (args.route_out_bf16) {
-                      reinterpret_cast<uint16_t*>(rowptr)[n] = f32_to_bf16_bits(value);
-                    } else {
-                      reinterpret_cast<float*>(rowptr)[n] = value;
-                    }
-                  }
-                }
-                continue;
+                const float a = meta->scale[c0 + j];
+                gate[i] = dequantize_planes(static_cast<int>(gate_bits[j]), static_cast<int>(gate_bits[j + 1]), a, scale_gate);
+                up[i] = dequantize_planes(static_cast<int>(up_bits[j]), static_cast<int>(up_bits[j + 1]), a, scale_up);
+              } else if constexpr (kInt8) {
+                const float a = meta->scale[c0 + j];
+                gate[i] = dequantize(static_cast<int>(gate_bits[j]), a, scale_gate, numerics);
+                up[i] = dequantize(static_cast<int>(up_bits[j]), a, scale_up, numerics);
+              } else {
+                gate[i] = __fadd_rn(__uint_as_float(gate_bits[j]), bias_gate);
+                up[i] = __fadd_rn(__uint_as_float(up_bits[j]), bias_up);
               }
-              if (c0 + j < rows) {
-                if (dump != nullptr) {
-                  uint32_t* out = dump + static_cast<int64_t>(row0 + c0 + j) * n_total;
-                  out[n] = gate_bits[j];
-                  if (kGateUp) out[n + n_out] = up_bits[j];
-                }
-                if constexpr (kGateUp) {
-                  float gate, up;
-                  if constexpr (kInt8) {
-                    const float a = meta->scale[c0 + j];
-                    gate = dequantize(static_cast<int>(gate_bits[j]), a, scale_gate, numerics);
-                    up = dequantize(static_cast<int>(up_bits[j]), a, scale_up, numerics);
-                  } else if constexpr (kW8A16) {
-                    gate = __fmul_rn(__uint_as_float(gate_bits[j]), scale_gate);
-                    up = __fmul_rn(__uint_as_float(up_bits[j]), scale_up);
-                  } else {
-                    gate = __fadd_rn(__uint_as_float(gate_bits[j]), bias_gate);
-                    up = __fadd_rn(__uint_as_float(up_bits[j]), bias_up);
-                  }
-                  args.y[static_cast<int64_t>(row0 + c0 + j) * n_out + n] = gated_to_bf16(act, gate, up, limit, ctl->exp_table);
-                } else {
-                  float value;
-                  if constexpr (kInt8) {
-                    value = dequantize(static_cast<int>(gate_bits[j]), meta->scale[c0 + j], scale_gate, numerics);
-                  } else if constexpr (kW8A16) {
-                    value = __fmul_rn(__uint_as_float(gate_bits[j]), scale_gate);
-                  } else {
-                    value = __fadd_rn(__uint_as_float(gate_bits[j]), bias_gate);
-                  }
-                  const uint64_t rowptr = meta->rowptr[c0 + j];
-                  if (args.route_out_bf16) {
-                    reinterpret_cast<uint16_t*>(rowptr)[n] = f32_to_bf16_bits(value);
-                  } else {
-                    reinterpret_cast<float*>(rowptr)[n] = value;
-                  }
-                }
+              if (c0 + j >= rows) gate[i] = up[i] = 1.0f;  // no row: nothing that could send the group to its slow branch
+            }
+            gated_group(act, gate, up, limit, ctl->exp_table, result);
+#pragma unroll
+            for (int i = 0; i < kElements; ++i) {
+              const int j = i * kRowsPerRoute;
+              if (c0 + j < rows) args.y[static_cast<int64_t>((row0 + c0 + j) / kRowsPerRoute) * n_out + n] = result[i];
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; j += kRowsPerRoute) {
+              if (c0 + j >= rows) break;
+              float value;
+              if constexpr (kPlanes) {
+                value = dequantize_planes(static_cast<int>(gate_bits[j]), static_cast<int>(gate_bits[j + 1]), meta->scale[c0 + j], scale_gate);
+              } else if constexpr (kInt8) {
+                value = dequantize(static_cast<int>(gate_bits[j]), meta->scale[c0 + j], scale_gate, numerics);
+              } else {
+                value = __fadd_rn(__uint_as_float(gate_bits[j]), bias_gate);
+              }
+              const uint64_t rowptr = meta->rowptr[c0 + j];
+              if (args.route_out_bf16) {
+                reinterpret_cast<uint16_t*>(rowptr)[n] = f32_to_bf16_bits(value);
+              } else {
+                reinterpret_cast<float*>(rowptr)[n] = value;
               }
             }
           }
