@@ -29,6 +29,9 @@ GEMM_UMMA = 2
 ACTIVATION_SILU = 0
 ACTIVATION_GELU = 2
 ACTIVATION_SWIGLUOAI = 3
+PATH_W8A8 = 0
+PATH_BF16 = 1
+PATH_W8A16 = 2
 W13_INTERLEAVED = 0x100  # or-ed into the activation: gate and up rows of w13 alternate
 BIAS_BF16 = 0x200        # or-ed into the activation: w13_bias / w2_bias are bf16
 
@@ -36,7 +39,7 @@ LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libf
 DIAG_LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libfused_moe_b200_diag.so")
 
 EXPORTS = (
-    "fmoe_abi_version", "fmoe_last_error", "fmoe_device_supported", "fmoe_read_status",
+    "fmoe_abi_version", "fmoe_last_error", "fmoe_device_supported", "fmoe_read_status", "fmoe_forward_checked",
     "fmoe_w8a8_workspace_layout", "fmoe_w8a8_forward", "fmoe_quantize_weight_rows", "fmoe_quantize_rows",
     "fmoe_bf16_workspace_layout", "fmoe_bf16_forward", "fmoe_w8a16_forward", "fmoe_i8gemm_workspace_bytes", "fmoe_i8gemm_dynamic_scaled_mm",
     "fmoe_stage_timer_create", "fmoe_stage_timer_destroy", "fmoe_stage_timer_reset", "fmoe_stage_timer_calls",
@@ -55,10 +58,30 @@ W8A16_FIXED_POINT = 0
 W8A16_BF16_ACTIVATIONS = 1
 
 
+class Switch:
+    """An environment variable that every call looks up.  os.environ.get raises and catches a KeyError inside for a name that
+    is not set, over a microsecond, and a forward asks for six; the mapping's own table answers in a twentieth of that, and
+    changes to os.environ still count from the next call on."""
+
+    def __init__(self, name: str, default: str):
+        self.name, self.key, self.default = name, os.fsencode(name), default
+
+    def get(self) -> str:
+        try:
+            value = os.environ._data.get(self.key)
+        except AttributeError:  # not CPython's mapping
+            return os.environ.get(self.name, self.default)
+        return self.default if value is None else os.fsdecode(value)
+
+
+_FORM_SWITCH = Switch("FUSED_CPP_MOE_W8A16_FORM", "fixed")
+_TILES_SWITCH = Switch("FUSED_CPP_MOE_FORCE_TILES", "")
+
+
 def w8a16_form_from_env() -> int:
     """FUSED_CPP_MOE_W8A16_FORM: "fixed" (default; activations as 16-bit fixed point on the int8 tensor cores) or "bf16"
     (activations stay bf16, weights widened on the SM)."""
-    value = os.environ.get("FUSED_CPP_MOE_W8A16_FORM", "fixed").strip().lower()
+    value = _FORM_SWITCH.get().strip().lower()
     if value in ("fixed", "fixed_point", "0", ""):
         return W8A16_FIXED_POINT
     if value in ("bf16", "bf16_activations", "1"):
@@ -129,6 +152,8 @@ def _open(path: str) -> ctypes.CDLL:
     lib.fmoe_bf16_forward.argtypes = [p, p, p, p, p, i64, i32, i32, i32, i32, ctypes.POINTER(Config), p, p,
                                       ctypes.c_size_t, p]
     lib.fmoe_w8a16_forward.argtypes = lib.fmoe_w8a8_forward.argtypes
+    lib.fmoe_forward_checked.argtypes = [i32, p, p, p, p, p, p, p, i64, i32, i32, i32, i32, ctypes.POINTER(Config), p, p, ctypes.c_size_t, p,
+                                         ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_int32)]
     lib.fmoe_quantize_weight_rows.argtypes = [p, i64, i32, p, p, p]
     lib.fmoe_quantize_rows.argtypes = [p, i64, i32, i32, p, p, p]
     lib.fmoe_stage_timer_create.argtypes = [i32, ctypes.POINTER(ctypes.c_void_p)]
@@ -203,7 +228,7 @@ _WORKSPACES: dict[tuple[int, int], torch.Tensor] = {}
 
 
 def get_workspace(nbytes: int, device: torch.device) -> torch.Tensor:
-    """A cached uint8 workspace of at least nbytes (grown geometrically, one per device).
+    """A cached uint8 workspace of at least nbytes, 256-byte aligned (grown geometrically, one per device).
 
     Like the reference's per-thread RuntimeScratch (csrc/moe/arm/i8mm_w8a8/kernels.cpp:177-182) it is
     reused across calls, so calls on one device must be serialised by the caller (one stream).
@@ -213,10 +238,11 @@ def get_workspace(nbytes: int, device: torch.device) -> torch.Tensor:
     if current is None or current.numel() < nbytes:
         size = max(nbytes, 0 if current is None else int(current.numel() * 1.5))
         _WORKSPACES.pop(key, None)
-        current = torch.empty(size + 256, dtype=torch.uint8, device=device)
+        buffer = torch.empty(size + 256, dtype=torch.uint8, device=device)
+        offset = (-buffer.data_ptr()) % 256
+        current = buffer[offset:offset + size]
         _WORKSPACES[key] = current
-    offset = (-current.data_ptr()) % 256
-    return current[offset:offset + nbytes]
+    return current
 
 
 @dataclass
@@ -226,6 +252,7 @@ class ForwardResult:
     layout: WorkspaceLayout
     acc1: torch.Tensor | None = None
     acc2: torch.Tensor | None = None
+    checked: tuple[int, int] | None = None  # (error, detail) of a call that waited for its kernels
 
     def region(self, name: str, dtype: torch.dtype, shape) -> torch.Tensor:
         count = 1
@@ -236,6 +263,8 @@ class ForwardResult:
         return self.workspace[begin:begin + nbytes].view(dtype).reshape(shape)
 
     def status(self) -> tuple[int, int]:
+        if self.checked is not None:
+            return self.checked
         error, detail = ctypes.c_int32(0), ctypes.c_int32(0)
         check(load().fmoe_read_status(_ptr(self.workspace), _stream(), ctypes.byref(error), ctypes.byref(detail)))
         return error.value, detail.value
@@ -286,6 +315,11 @@ class StageTimer:
             pass
 
 
+def as_dtype(tensor: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """tensor.to(dtype).contiguous(), without the two calls where the tensor is that already."""
+    return tensor if tensor.dtype is dtype and tensor.is_contiguous() else tensor.to(dtype).contiguous()
+
+
 def _require_cuda(name: str, tensor: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     if not isinstance(tensor, torch.Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")
@@ -293,7 +327,7 @@ def _require_cuda(name: str, tensor: torch.Tensor, dtype: torch.dtype) -> torch.
         raise ValueError(f"{name} must be a CUDA tensor (this build has no CPU path)")
     if tensor.dtype is not dtype:
         raise TypeError(f"{name} must have dtype {dtype}, got {tensor.dtype}")
-    return tensor.contiguous()
+    return tensor if tensor.is_contiguous() else tensor.contiguous()
 
 
 def moe_forward(x, w13, w2, topk_weights, topk_ids, *, s13=None, s2=None, numerics: int = NUMERICS_TORCHREF,
@@ -301,11 +335,13 @@ def moe_forward(x, w13, w2, topk_weights, topk_ids, *, s13=None, s2=None, numeri
                 out: torch.Tensor | None = None, dump: bool = False, workspace: torch.Tensor | None = None,
                 stage_timer: "StageTimer | None" = None, diagnostic: bool = False, activation: int = ACTIVATION_SILU,
                 w13_bias: torch.Tensor | None = None, w2_bias: torch.Tensor | None = None, w8a16: bool = False,
-                route_rows_bf16: bool = False, w8a16_form: int | None = None) -> ForwardResult:
+                route_rows_bf16: bool = False, w8a16_form: int | None = None, wait: bool = False) -> ForwardResult:
     """One routed-expert MoE forward through the C ABI.  int8 weights (with s13/s2) select W8A8, or, with
     w8a16=True, the W8A16 path (16-bit activations; w8a16_form picks W8A16_FIXED_POINT, the default, or
     W8A16_BF16_ACTIVATIONS; None reads FUSED_CPP_MOE_W8A16_FORM = "fixed" | "bf16").
-    diagnostic=True (or gemm_impl=GEMM_SIMT) runs the call in the diagnostic library instead of the product one."""
+    diagnostic=True (or gemm_impl=GEMM_SIMT) runs the call in the diagnostic library instead of the product one.
+    wait=True waits for the kernels and brings their status along (fmoe_forward_checked), for a caller that would read it
+    next anyway; the other form enqueues and returns."""
     quantised_weights = w13.dtype == torch.int8
     if w8a16 and not quantised_weights:
         raise TypeError("w8a16 needs int8 weights with s13 / s2")
@@ -327,7 +363,7 @@ def moe_forward(x, w13, w2, topk_weights, topk_ids, *, s13=None, s2=None, numeri
     layout = workspace_layout(int8, tokens, top_k, experts, hidden, inter)
     if workspace is None:
         workspace = get_workspace(layout.total_bytes, x.device)
-    forced = os.environ.get("FUSED_CPP_MOE_FORCE_TILES")  # "gate_up,down": diagnostic override of the row tiles
+    forced = _TILES_SWITCH.get()  # "gate_up,down": diagnostic override of the row tiles
     if forced and gate_up_tile == 0 and down_tile == 0:
         gate_up_tile, down_tile = (int(v) for v in forced.split(","))
     limit = (10.0 if int8 else 0.0) if swiglu_limit is None else float(swiglu_limit)
@@ -360,7 +396,15 @@ def moe_forward(x, w13, w2, topk_weights, topk_ids, *, s13=None, s2=None, numeri
         config.dump_acc2 = acc2.data_ptr()
     # The CUDA-core cross-check and the stage switches exist only in the diagnostic library.
     lib = load_diag() if (gemm_impl == GEMM_SIMT or diagnostic) else load()
-    if quantised_weights:
+    checked = None
+    if wait:
+        error, detail = ctypes.c_int32(0), ctypes.c_int32(0)
+        code = lib.fmoe_forward_checked(PATH_W8A16 if w8a16 else PATH_W8A8 if int8 else PATH_BF16, _ptr(x), _ptr(w13), _ptr(s13), _ptr(w2),
+                                        _ptr(s2), _ptr(topk_weights), _ptr(topk_ids), tokens, top_k, experts, hidden, inter,
+                                        ctypes.byref(config), _ptr(out), _ptr(workspace), workspace.numel(), _stream(),
+                                        ctypes.byref(error), ctypes.byref(detail))
+        checked = (error.value, detail.value)
+    elif quantised_weights:
         entry = lib.fmoe_w8a16_forward if w8a16 else lib.fmoe_w8a8_forward
         code = entry(_ptr(x), _ptr(w13), _ptr(s13), _ptr(w2), _ptr(s2), _ptr(topk_weights), _ptr(topk_ids),
                      tokens, top_k, experts, hidden, inter, ctypes.byref(config), _ptr(out),
@@ -370,7 +414,7 @@ def moe_forward(x, w13, w2, topk_weights, topk_ids, *, s13=None, s2=None, numeri
                                      experts, hidden, inter, ctypes.byref(config), _ptr(out), _ptr(workspace),
                                      workspace.numel(), _stream())
     check(code, lib)
-    return ForwardResult(out=out, workspace=workspace, layout=layout, acc1=acc1, acc2=acc2)
+    return ForwardResult(out=out, workspace=workspace, layout=layout, acc1=acc1, acc2=acc2, checked=checked)
 
 
 def quantize_rows(x: torch.Tensor, numerics: int = NUMERICS_TORCHREF, weight_mode: bool = False):

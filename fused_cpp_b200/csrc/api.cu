@@ -157,6 +157,7 @@ struct Forward {
   int peer_world = 0;
   int64_t peer_routes_max = 0;
   void* peer_scrap_row = nullptr;
+  const int* status_mirror = nullptr;  // page-locked host words that take the first error too
 };
 
 int run_forward(const Forward& f, const fmoe_config* config, void* out, void* workspace, size_t workspace_bytes, void* stream_ptr) {
@@ -321,11 +322,11 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
     error = fmoe::launch_front(planes ? fmoe::FrontRows::kPlanes : f.int8 ? fmoe::FrontRows::kInt8 : fmoe::FrontRows::kBf16, f.topk_ids, f.tokens,
                                f.top_k, f.experts, lists, status_block, counts, offsets, sorted_routes, row_expert,
                                reinterpret_cast<int*>(base + layout.route_pos), static_cast<const uint16_t*>(f.x), f.hidden, cfg.numerics,
-                               base + layout.a_rows, a_scale, stream);
+                               base + layout.a_rows, a_scale, stream, f.status_mirror);
     if (error != cudaSuccess) return cuda_fail(error, "route build and token rows");
   } else {
     error = fmoe::launch_route_build(f.topk_ids, routes, f.experts, lists, status_block, counts, offsets, sorted_routes, row_expert, stream,
-                                     reinterpret_cast<int*>(base + layout.route_pos));
+                                     reinterpret_cast<int*>(base + layout.route_pos), f.status_mirror);
     if (error != cudaSuccess) return cuda_fail(error, "route build");
   }
   mark(FMOE_STAGE_ROUTE + 1);
@@ -512,7 +513,7 @@ class PinnedWords {
       tried_ = true;
       const RelaxedCaptureMode relaxed;
       void* memory = nullptr;
-      if (cudaHostAlloc(&memory, sizeof(int) * fmoe::kStatusWords, cudaHostAllocPortable) == cudaSuccess) {
+      if (cudaHostAlloc(&memory, sizeof(int) * fmoe::kStatusWords, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
         words_ = static_cast<int*>(memory);
       } else {
         cudaGetLastError();
@@ -530,19 +531,14 @@ class PinnedWords {
   int* words_ = nullptr;
   bool tried_ = false;
 };
-}  // namespace
 
-extern "C" {
-
-int fmoe_read_status(const void* workspace, void* stream, int32_t* error, int32_t* detail) {
-  if (workspace == nullptr) return fail(FMOE_ERR_INVALID_ARGUMENT, "workspace is null");
-  // Page-locked: a copy to pageable memory is staged by the driver and costs the call several microseconds more.
+int* pinned_status_words() {
   static thread_local PinnedWords pinned;
-  int fallback[fmoe::kStatusWords];
-  int* const words = pinned.get() != nullptr ? pinned.get() : fallback;
-  cudaError_t result = cudaMemcpyAsync(words, workspace, sizeof(fallback), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream));
-  if (result == cudaSuccess) result = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
-  if (result != cudaSuccess) return cuda_fail(result, "reading the status block");
+  return pinned.get();
+}
+
+// The error and its argument out of a status block, with the thread's error text set.
+void report_status(const int* words, int32_t* error, int32_t* detail) {
   if (error) *error = words[fmoe::kStatusError];
   if (detail) *detail = words[fmoe::kStatusDetail];
   if (words[fmoe::kStatusError] == FMOE_ERR_EXPERT_ID_RANGE) {
@@ -558,6 +554,21 @@ int fmoe_read_status(const void* workspace, void* stream, int32_t* error, int32_
            -words[fmoe::kStatusDetail]);
     }
   }
+}
+}  // namespace
+
+extern "C" {
+
+int fmoe_read_status(const void* workspace, void* stream, int32_t* error, int32_t* detail) {
+  if (workspace == nullptr) return fail(FMOE_ERR_INVALID_ARGUMENT, "workspace is null");
+  // Page-locked: a copy to pageable memory is staged by the driver and costs the call several microseconds more.
+  int fallback[fmoe::kStatusWords];
+  int* const pinned = pinned_status_words();
+  int* const words = pinned != nullptr ? pinned : fallback;
+  cudaError_t result = cudaMemcpyAsync(words, workspace, sizeof(fallback), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream));
+  if (result == cudaSuccess) result = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
+  if (result != cudaSuccess) return cuda_fail(result, "reading the status block");
+  report_status(words, error, detail);
   return FMOE_OK;
 }
 
@@ -640,6 +651,35 @@ int fmoe_w8a16_forward(const void* x, const int8_t* w13, const float* s13, const
   if (config != nullptr && config->gemm_impl == FMOE_GEMM_SIMT) return fail(FMOE_ERR_INVALID_ARGUMENT, "W8A16 runs on the tensor-core GEMM only");
 #endif
   return run_forward(f, config, out, workspace, workspace_bytes, stream);
+}
+
+int fmoe_forward_checked(int32_t path, const void* x, const void* w13, const float* s13, const void* w2, const float* s2,
+                         const float* topk_weights, const int64_t* topk_ids, int64_t tokens, int32_t top_k, int32_t experts,
+                         int32_t hidden, int32_t inter, const fmoe_config* config, void* out, void* workspace, size_t workspace_bytes,
+                         void* stream, int32_t* error, int32_t* detail) {
+  if (path != FMOE_PATH_W8A8 && path != FMOE_PATH_BF16 && path != FMOE_PATH_W8A16) return fail(FMOE_ERR_INVALID_ARGUMENT, "unknown path %d", path);
+  if (error != nullptr) *error = FMOE_OK;
+  if (detail != nullptr) *detail = 0;
+  Forward f{path == FMOE_PATH_W8A8, x, w13, s13, w2, s2, topk_weights, topk_ids, tokens, top_k, experts, hidden, inter};
+  f.w8a16 = path == FMOE_PATH_W8A16;
+#ifdef FMOE_DIAG
+  if (f.w8a16 && config != nullptr && config->gemm_impl == FMOE_GEMM_SIMT) return fail(FMOE_ERR_INVALID_ARGUMENT, "W8A16 runs on the tensor-core GEMM only");
+#endif
+  // The kernels store an error, if there is one, into these host words themselves: nothing is copied back after the last of
+  // them (16 tokens of the 16-expert layer: the copy and the gaps around it took 7 of 90 us).  The words are this thread's,
+  // and no call leaves before its kernels have ended.
+  int* const words = pinned_status_words();
+  if (words != nullptr) memset(words, 0, sizeof(int) * fmoe::kStatusWords);
+  f.status_mirror = words;
+  const int code = run_forward(f, config, out, workspace, workspace_bytes, stream);
+  if (tokens == 0 && code == FMOE_OK) return code;
+  if (words == nullptr) return code == FMOE_OK ? fmoe_read_status(workspace, stream, error, detail) : code;
+  if (code != FMOE_OK && code != FMOE_ERR_CUDA) return code;  // refused: nothing was launched
+  const cudaError_t result = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
+  if (code != FMOE_OK) return code;
+  if (result != cudaSuccess) return cuda_fail(result, "waiting for the forward");
+  report_status(words, error, detail);
+  return FMOE_OK;
 }
 
 int fmoe_w8a8_expert_rows_forward(const int8_t* rows_q, const float* rows_scale, const int64_t* rows_expert, int64_t rows,

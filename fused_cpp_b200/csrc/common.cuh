@@ -26,11 +26,26 @@ enum StatusWord : int {
   kStatusItemsB = 5,     // work items of the second list (down GEMM)
   kStatusItemsC = 6,     // split mode: gate_up work items of the experts with many rows (two-SM kernel)
   kStatusItemsD = 7,     // split mode: down work items of those experts
+  kStatusMirror = 10,    // two words: address of page-locked host words that take the first error too (0 = none)
   kStatusWords = 16,
 };
 
-__device__ __forceinline__ void raise_error(int* status, int code, int detail) {
-  if (atomicCAS(status + kStatusError, 0, code) == 0) status[kStatusDetail] = detail;
+__device__ __forceinline__ void raise_error(int* status, int code, int detail, int wait_site = 0) {
+  if (atomicCAS(status + kStatusError, 0, code) != 0) return;
+  status[kStatusDetail] = detail;
+  status[kStatusWaitSite] = wait_site;
+  int* const mirror = *reinterpret_cast<int* volatile*>(status + kStatusMirror);
+  if (mirror == nullptr) return;
+  mirror[kStatusDetail] = detail;
+  mirror[kStatusWaitSite] = wait_site;
+  __threadfence_system();
+  *reinterpret_cast<volatile int*>(mirror + kStatusError) = code;
+}
+
+// Word `index` of a cleared status block.
+__device__ __forceinline__ int cleared_status_word(int index, const int* mirror) {
+  const uint64_t address = reinterpret_cast<uint64_t>(mirror);
+  return index == kStatusMirror ? static_cast<int>(address) : index == kStatusMirror + 1 ? static_cast<int>(address >> 32) : 0;
 }
 
 __device__ __forceinline__ float bf16_bits_to_f32(uint16_t bits) { return __uint_as_float(static_cast<uint32_t>(bits) << 16); }

@@ -32,6 +32,7 @@ struct RouteArgs {
   int experts, warps;
   int64_t run;
   ItemLists lists;
+  const int* mirror;
   int *status, *counts, *offsets, *sorted_routes, *row_expert, *route_pos;
 };
 
@@ -43,8 +44,8 @@ front_kernel(RouteArgs route, const uint16_t* x, int cols, int top_k, int numeri
   extern __shared__ int route_smem[];
   ptx::launch_dependents();  // an ordinary launch: everything before it has completed
   if (blockIdx.x == 0) {
-    route_build<false>(route_smem, route.topk_ids, route.routes, route.experts, route.warps, route.run, route.lists, route.status, route.counts,
-                       route.offsets, route.sorted_routes, route.row_expert, route.route_pos);
+    route_build<false>(route_smem, route.topk_ids, route.routes, route.experts, route.warps, route.run, route.lists, route.status, route.mirror,
+                       route.counts, route.offsets, route.sorted_routes, route.row_expert, route.route_pos);
     return;
   }
   __shared__ float warp_amax[kFrontWarps];
@@ -149,12 +150,12 @@ bool front_pays(int64_t tokens, int top_k, int experts) {
 
 cudaError_t launch_front(FrontRows rows, const int64_t* topk_ids, int64_t tokens, int top_k, int experts, const ItemLists& lists, int* status,
                          int* counts, int* offsets, int* sorted_routes, int* row_expert, int* route_pos, const uint16_t* x, int cols,
-                         int numerics, void* rows_out, float* scale_out, cudaStream_t stream) {
+                         int numerics, void* rows_out, float* scale_out, cudaStream_t stream, const int* mirror) {
   const int64_t routes = tokens * top_k;
   const int64_t used = (routes + 31) / 32;
   const int warps = static_cast<int>(used < kFrontWarps ? used : kFrontWarps);
   const int64_t run = 32 * ((used + warps - 1) / warps);
-  const RouteArgs route = {topk_ids, routes, experts, warps, run, lists, status, counts, offsets, sorted_routes, row_expert, route_pos};
+  const RouteArgs route = {topk_ids, routes, experts, warps, run, lists, mirror, status, counts, offsets, sorted_routes, row_expert, route_pos};
   const size_t smem = route_smem_bytes(warps, experts, false);
   auto kernel = rows == FrontRows::kInt8    ? front_kernel<FrontRows::kInt8>
                 : rows == FrontRows::kBf16 ? front_kernel<FrontRows::kBf16>

@@ -28,9 +28,11 @@ struct ItemLists {
   int* items_d;
 };
 inline ItemLists no_item_lists() { return ItemLists{16, 16, nullptr, nullptr, 0, 0, 0, nullptr, nullptr}; }
-// One launch; clears the status block, then raises FMOE_ERR_EXPERT_ID_RANGE in it for ids outside [0, experts).
+// One launch; clears the status block (mirror: page-locked host words that take the first error of the call as well, or null),
+// then raises FMOE_ERR_EXPERT_ID_RANGE in it for ids outside [0, experts).
 cudaError_t launch_route_build(const int64_t* topk_ids, int64_t routes, int experts, const ItemLists& lists, int* status, int* counts,
-                               int* offsets, int* sorted_routes, int* row_expert, cudaStream_t stream, int* route_pos = nullptr);
+                               int* offsets, int* sorted_routes, int* row_expert, cudaStream_t stream, int* route_pos = nullptr,
+                               const int* mirror = nullptr);
 
 // Work items from per-expert counts / offsets of rows that are already in expert order.
 cudaError_t launch_items_from_counts(int experts, const int* counts, const int* offsets, const ItemLists& lists, int* status,
@@ -42,7 +44,7 @@ enum class FrontRows { kInt8, kBf16, kPlanes };
 bool front_pays(int64_t tokens, int top_k, int experts);
 cudaError_t launch_front(FrontRows rows, const int64_t* topk_ids, int64_t tokens, int top_k, int experts, const ItemLists& lists, int* status,
                          int* counts, int* offsets, int* sorted_routes, int* row_expert, int* route_pos, const uint16_t* x, int cols,
-                         int numerics, void* rows_out, float* scale_out, cudaStream_t stream);
+                         int numerics, void* rows_out, float* scale_out, cudaStream_t stream, const int* mirror);
 
 // ---- quant.cu
 // Quantise rows of a bf16 matrix to int8 with one fp32 scale per row.  When `sorted_routes` is

@@ -97,10 +97,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     if (*abort_flag) return false;
     if (global_timer_ns() - start > kWaitLimitNs) {
       *abort_flag = 1;
-      if (atomicCAS(status + kStatusError, 0, FMOE_ERR_DEVICE_WAIT) == 0) {
-        status[kStatusDetail] = static_cast<int>(blockIdx.x);
-        status[kStatusWaitSite] = site;
-      }
+      raise_error(status, FMOE_ERR_DEVICE_WAIT, static_cast<int>(blockIdx.x), site);
       return false;
     }
   }
@@ -118,10 +115,7 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, v
     if (*abort_flag) return false;
     if (global_timer_ns() - start > kWaitLimitNs) {
       *abort_flag = 1;
-      if (atomicCAS(status + kStatusError, 0, FMOE_ERR_DEVICE_WAIT) == 0) {
-        status[kStatusDetail] = static_cast<int>(blockIdx.x);
-        status[kStatusWaitSite] = site;
-      }
+      raise_error(status, FMOE_ERR_DEVICE_WAIT, static_cast<int>(blockIdx.x), site);
       return false;
     }
   }

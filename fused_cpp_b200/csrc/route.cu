@@ -36,10 +36,11 @@ constexpr int kHistogramInts = 32 * 1024;   // shared-memory histogram rows: 32 
 template <bool kCluster>
 __global__ void __launch_bounds__(kRouteThreads)
 route_build_kernel(const int64_t* __restrict__ topk_ids, int64_t routes, int experts, int warps, int64_t run, ItemLists lists, int* status,
-                   int* counts, int* offsets, int* sorted_routes, int* row_expert, int* route_pos) {
+                   const int* mirror, int* counts, int* offsets, int* sorted_routes, int* row_expert, int* route_pos) {
   extern __shared__ int route_smem[];
   ptx::launch_dependents();  // an ordinary launch: everything before it has completed
-  route_build<kCluster>(route_smem, topk_ids, routes, experts, warps, run, lists, status, counts, offsets, sorted_routes, row_expert, route_pos);
+  route_build<kCluster>(route_smem, topk_ids, routes, experts, warps, run, lists, status, mirror, counts, offsets, sorted_routes, row_expert,
+                        route_pos);
 }
 
 // Work items from given per-expert counts and offsets (rows that already lie in expert order: nothing to sort).
@@ -52,7 +53,7 @@ items_from_counts_kernel(int experts, const int* __restrict__ counts, const int*
 
 // The status block is cleared by the build.
 cudaError_t launch_route_build(const int64_t* topk_ids, int64_t routes, int experts, const ItemLists& lists, int* status, int* counts,
-                               int* offsets, int* sorted_routes, int* row_expert, cudaStream_t stream, int* route_pos) {
+                               int* offsets, int* sorted_routes, int* row_expert, cudaStream_t stream, int* route_pos, const int* mirror) {
   static_assert(kMaxExperts * 16 <= kHistogramInts, "the histogram rows of kMaxExperts experts need at least 16 warps");
   int64_t ctas = 1;
   while (ctas < kMaxRouteCluster && ctas * kRoutesPerCta < routes) ctas *= 2;
@@ -78,8 +79,8 @@ cudaError_t launch_route_build(const int64_t* topk_ids, int64_t routes, int expe
     configured.mark(device);
   }
   if (ctas == 1) {
-    route_build_kernel<false><<<1, threads, smem, stream>>>(topk_ids, routes, experts, warps, run, lists, status, counts, offsets, sorted_routes,
-                                                            row_expert, route_pos);
+    route_build_kernel<false><<<1, threads, smem, stream>>>(topk_ids, routes, experts, warps, run, lists, status, mirror, counts, offsets,
+                                                            sorted_routes, row_expert, route_pos);
     return cudaGetLastError();
   }
   cudaLaunchConfig_t config = {};
@@ -94,7 +95,7 @@ cudaError_t launch_route_build(const int64_t* topk_ids, int64_t routes, int expe
   attribute.val.clusterDim.z = 1;
   config.attrs = &attribute;
   config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, route_build_kernel<true>, topk_ids, routes, experts, warps, run, lists, status, counts, offsets,
+  return cudaLaunchKernelEx(&config, route_build_kernel<true>, topk_ids, routes, experts, warps, run, lists, status, mirror, counts, offsets,
                             sorted_routes, row_expert, route_pos);
 }
 

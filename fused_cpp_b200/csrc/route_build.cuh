@@ -146,8 +146,8 @@ __device__ __forceinline__ unsigned lanes_with_same(int id, int bits) {
 // Called by every thread of the CTA (kCluster: of every CTA of the cluster).
 template <bool kCluster>
 __device__ __forceinline__ void route_build(int* route_smem, const int64_t* topk_ids, int64_t routes, int experts, int warps, int64_t run,
-                                            const ItemLists& lists, int* status, int* counts, int* offsets, int* sorted_routes,
-                                            int* row_expert, int* route_pos) {
+                                            const ItemLists& lists, int* status, const int* mirror, int* counts, int* offsets,
+                                            int* sorted_routes, int* row_expert, int* route_pos) {
   namespace cg = cooperative_groups;
   int* hist = route_smem;
   int* s_counts = hist + warps * experts;  // routes per expert
@@ -161,7 +161,7 @@ __device__ __forceinline__ void route_build(int* route_smem, const int64_t* topk
   const int ctas = kCluster ? static_cast<int>(cg::this_cluster().num_blocks()) : 1;
 
   for (int i = threadIdx.x; i < warps * experts; i += blockDim.x) hist[i] = 0;
-  if (rank == 0 && threadIdx.x < kStatusWords) status[threadIdx.x] = 0;
+  if (rank == 0 && threadIdx.x < kStatusWords) status[threadIdx.x] = cleared_status_word(threadIdx.x, mirror);
   __syncthreads();
 
   const int64_t begin = (static_cast<int64_t>(rank) * warps + warp) * run;

@@ -24,6 +24,11 @@ BACKEND_NAME = "cuda_sm100_tcgen05"
 BACKEND_N_TILE = 128
 W8A8_BACKEND_NAME = "cuda_sm100_w8a8_tcgen05"
 
+_NUMERICS_SWITCH = _lib.Switch("FUSED_CPP_MOE_W8A8_NUMERICS", "torchref")
+_IMPL_SWITCH = _lib.Switch("FUSED_CPP_MOE_GEMM_IMPL", "auto")
+_ROUTE_SWITCH = _lib.Switch("FUSED_CPP_MOE_W2_BF16_ROUTE", "0")
+_SYNC_SWITCH = _lib.Switch("FUSED_CPP_MOE_SYNC_CHECK", "1")
+
 
 def _device() -> torch.device:
     if not torch.cuda.is_available():
@@ -32,7 +37,7 @@ def _device() -> torch.device:
 
 
 def _numerics() -> int:
-    value = os.environ.get("FUSED_CPP_MOE_W8A8_NUMERICS", "torchref").strip().lower()
+    value = _NUMERICS_SWITCH.get().strip().lower()
     if value in ("torchref", "0", ""):
         return _lib.NUMERICS_TORCHREF
     if value in ("native", "1"):
@@ -41,7 +46,7 @@ def _numerics() -> int:
 
 
 def _gemm_impl() -> int:
-    value = os.environ.get("FUSED_CPP_MOE_GEMM_IMPL", "auto").strip().lower()
+    value = _IMPL_SWITCH.get().strip().lower()
     table = {"auto": _lib.GEMM_AUTO, "simt": _lib.GEMM_SIMT, "umma": _lib.GEMM_UMMA}
     if value not in table:
         raise ValueError("FUSED_CPP_MOE_GEMM_IMPL must be auto, simt or umma")
@@ -52,11 +57,11 @@ def _route_rows_bf16() -> bool:
     """The reference's opt-in for bf16 route storage, FUSED_CPP_MOE_W2_BF16_ROUTE=1 (default off,
     csrc/moe/arm/common/fused_moe_bf16_tiled.cpp:1016-1019): here it selects the compact route rows of every path
     (fmoe_config.route_rows_bf16): half the bytes of the largest intermediate, output to tolerance instead of bit for bit."""
-    return os.environ.get("FUSED_CPP_MOE_W2_BF16_ROUTE", "0") not in ("", "0")
+    return _ROUTE_SWITCH.get() not in ("", "0")
 
 
 def _sync_check() -> bool:
-    return os.environ.get("FUSED_CPP_MOE_SYNC_CHECK", "1") != "0"
+    return _SYNC_SWITCH.get() != "0"
 
 
 def fused_moe_bf16_tiled_available_backends() -> list[str]:
@@ -150,6 +155,11 @@ def _check_out(input: torch.Tensor, out: torch.Tensor | None, others) -> None:
             raise RuntimeError("out must not alias the input, weights or top-k tensors")
 
 
+def _as_shape(tensor: torch.Tensor, shape: tuple) -> torch.Tensor:
+    """reshape, which costs two microseconds where there is nothing to do."""
+    return tensor if tensor.shape == shape else tensor.reshape(shape)
+
+
 def _tile_from(windows) -> int:
     if windows is None or windows.numel() == 0:
         return 0
@@ -209,13 +219,13 @@ def fused_moe_w8a8_tiled_async_plan_v2(
     if tuple(w13_scales.shape) != (experts, w13_n) or tuple(w2_scales.shape) != (experts, w2_n):
         raise RuntimeError("W8A8 scale shapes are invalid")
     _check_out(input, out, (input, w13_packed, w2_packed, topk_weights, topk_ids))
-    w13 = w13_packed.reshape(experts, w13_n, w13_k)
-    w2 = w2_packed.reshape(experts, w2_n, w2_k)
+    w13 = _as_shape(w13_packed, (experts, w13_n, w13_k))
+    w2 = _as_shape(w2_packed, (experts, w2_n, w2_k))
     result = _lib.moe_forward(input, w13, w2, topk_weights, topk_ids, s13=w13_scales, s2=w2_scales, numerics=_numerics(),
                               gemm_impl=_gemm_impl(), gate_up_tile=_tile_from(task_w13_window_tiles),
                               down_tile=_tile_from(task_w2_window_tiles), swiglu_limit=float(swiglu_limit), out=out,
-                              route_rows_bf16=_route_rows_bf16())
-    if _sync_check():
+                              route_rows_bf16=_route_rows_bf16(), wait=_sync_check())
+    if result.checked is not None:
         result.raise_for_status()
     if out is not None:
         out._version  # noqa: B018  (written in place by the kernels; torch tracks no version bump for raw pointers)
@@ -265,8 +275,8 @@ def _bf16_forward(input, w13_packed, w13_k, w13_n, w2_packed, w2_k, w2_n, topk_w
     bias_dtype = torch.bfloat16 if all(b is None or b.dtype == torch.bfloat16 for b in (w13_bias, w2_bias)) else torch.float32
     w13_bias = _check_bias(w13_bias, experts, w13_n, "w13_bias", bias_dtype)
     w2_bias = _check_bias(w2_bias, experts, w2_n, "w2_bias", bias_dtype)
-    w13 = w13_packed.reshape(experts, w13_n, w13_k)
-    w2 = w2_packed.reshape(experts, w2_n, w2_k)
+    w13 = _as_shape(w13_packed, (experts, w13_n, w13_k))
+    w2 = _as_shape(w2_packed, (experts, w2_n, w2_k))
     # The reference narrows the valid id range to [0, global_num_experts) and raises on ids beyond it
     # (fused_moe_bf16_tiled.cpp:6439-6458): the route build sees only that many experts, so such ids are reported as
     # out of range instead of being routed to the trailing prepared experts.
@@ -275,13 +285,13 @@ def _bf16_forward(input, w13_packed, w13_k, w13_n, w2_packed, w2_k, w2_n, topk_w
         w13, w2 = w13[:experts], w2[:experts]
         w13_bias = None if w13_bias is None else w13_bias[:experts]
         w2_bias = None if w2_bias is None else w2_bias[:experts]
-    weights = topk_weights.to(torch.float32)
+    weights = _lib.as_dtype(topk_weights, torch.float32)
     if skip_weighted:
         weights = torch.ones_like(weights)
-    result = _lib.moe_forward(input, w13, w2, weights, topk_ids.to(torch.int64), gemm_impl=_gemm_impl(), gate_up_tile=gate_up_tile,
+    result = _lib.moe_forward(input, w13, w2, weights, _lib.as_dtype(topk_ids, torch.int64), gemm_impl=_gemm_impl(), gate_up_tile=gate_up_tile,
                               down_tile=down_tile, swiglu_limit=limit, out=out, activation=activation_id, w13_bias=w13_bias,
-                              w2_bias=w2_bias, route_rows_bf16=_route_rows_bf16())
-    if _sync_check():
+                              w2_bias=w2_bias, route_rows_bf16=_route_rows_bf16(), wait=_sync_check())
+    if result.checked is not None:
         result.raise_for_status()
     return result.out
 
@@ -570,18 +580,18 @@ def fused_moe_w8a16_tiled_async_plan_v2(
         raise RuntimeError("silu_poly_degree must be 4, 5 or 6")
     _check_out(input, out, (input, w13_packed, w2_packed, topk_weights, topk_ids))
     activation_id, limit = _native_activation(activation)
-    w13 = w13_packed.reshape(experts, w13_N, w13_K)
-    w2 = w2_packed.reshape(experts, w2_N, w2_K)
+    w13 = _as_shape(w13_packed, (experts, w13_N, w13_K))
+    w2 = _as_shape(w2_packed, (experts, w2_N, w2_K))
     s13, s2 = w13_scales, w2_scales
     if global_num_experts != -1 and global_num_experts < experts:
         experts = int(global_num_experts)
         w13, w2, s13, s2 = w13[:experts], w2[:experts], s13[:experts], s2[:experts]
-    weights = topk_weights.to(torch.float32)
+    weights = _lib.as_dtype(topk_weights, torch.float32)
     if skip_weighted:
         weights = torch.ones_like(weights)
-    result = _lib.moe_forward(input, w13, w2, weights, topk_ids.to(torch.int64), s13=s13.contiguous(), s2=s2.contiguous(), w8a16=True,
+    result = _lib.moe_forward(input, w13, w2, weights, _lib.as_dtype(topk_ids, torch.int64), s13=s13.contiguous(), s2=s2.contiguous(), w8a16=True,
                               gate_up_tile=_tile_from(task_w13_window_tiles), down_tile=_tile_from(task_w2_window_tiles),
-                              swiglu_limit=limit, out=out, activation=activation_id, route_rows_bf16=_route_rows_bf16())
-    if _sync_check():
+                              swiglu_limit=limit, out=out, activation=activation_id, route_rows_bf16=_route_rows_bf16(), wait=_sync_check())
+    if result.checked is not None:
         result.raise_for_status()
     return result.out

@@ -283,7 +283,7 @@ def fused_moe_bf16_tiled_async_plan(input, weights, topk_weights, topk_ids, plan
     materialized = plan if isinstance(plan, AsyncMoEPlanV2) else AsyncMoEPlanV2.from_dict(plan)
     result = _fused_moe_bf16_tiled_async_plan_v2_impl(
         input.contiguous(), weights.w13[0], weights.w13[1], weights.w13[2], weights.w2[0], weights.w2[1], weights.w2[2],
-        topk_weights.to(torch.float32).contiguous(), topk_ids.to(torch.int64).contiguous(), *_plan_args(materialized),
+        _lib.as_dtype(topk_weights, torch.float32), _lib.as_dtype(topk_ids, torch.int64), *_plan_args(materialized),
         w13_bias, w2_bias, materialized.num_threads, _native_activation_name(activation, weights, swiglu_limit), int(global_num_experts),
         bool(skip_weighted), bool(weights.fused_silu), int(silu_poly_degree), int(weights.gemm_backend),
         int(weights.backend_n_tile), out, materialized.native_early_merge)
@@ -313,7 +313,7 @@ def fused_moe_bf16_tiled(input, weights, topk_weights, topk_ids, *, w13_bias=Non
                                                    swiglu_limit=swiglu_limit, out=out)
     result = _fused_moe_bf16_tiled_impl(
         input.contiguous(), weights.w13[0], weights.w13[1], weights.w13[2], weights.w2[0], weights.w2[1], weights.w2[2],
-        topk_weights.to(torch.float32).contiguous(), topk_ids.to(torch.int64).contiguous(), w13_bias, w2_bias, int(num_threads),
+        _lib.as_dtype(topk_weights, torch.float32), _lib.as_dtype(topk_ids, torch.int64), w13_bias, w2_bias, int(num_threads),
         _native_activation_name(activation, weights, swiglu_limit), int(global_num_experts), bool(skip_weighted), bool(weights.fused_silu),
         int(silu_poly_degree), int(weights.gemm_backend), int(weights.backend_n_tile), out)
     return out if out is not None else result
@@ -429,7 +429,7 @@ def fused_moe_w8a8_tiled_async_plan(input, weights, topk_weights, topk_ids, plan
     materialized = plan if isinstance(plan, AsyncMoEPlanV2) else AsyncMoEPlanV2.from_dict(plan)
     result = _fused_moe_w8a8_async_plan_v2_impl(
         input.contiguous(), weights.w13[0], weights.w13[1], weights.w13[2], weights.w13[3], weights.w2[0], weights.w2[1],
-        weights.w2[2], weights.w2[3], topk_weights.to(torch.float32).contiguous(), topk_ids.to(torch.int64).contiguous(),
+        weights.w2[2], weights.w2[3], _lib.as_dtype(topk_weights, torch.float32), _lib.as_dtype(topk_ids, torch.int64),
         *_plan_args(materialized), materialized.num_threads, "silu", int(global_num_experts), bool(skip_weighted),
         int(weights.backend_n_tile), out, 0, float(swiglu_limit))
     return out if out is not None else result

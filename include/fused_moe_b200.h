@@ -145,6 +145,18 @@ FMOE_API int fmoe_device_supported(int device);
  * device-detected error, *detail its argument (e.g. the offending flat route id). */
 FMOE_API int fmoe_read_status(const void* workspace, void* stream, int32_t* error, int32_t* detail);
 
+/* fmoe_w8a8_forward, fmoe_bf16_forward (s13 = s2 = NULL) or fmoe_w8a16_forward, then what fmoe_read_status says of the
+ * call: waits for `stream`, like that function, but copies nothing back (the kernels store an error into host memory of the
+ * library themselves).  Not for a stream under capture. */
+#define FMOE_PATH_W8A8 0
+#define FMOE_PATH_BF16 1
+#define FMOE_PATH_W8A16 2
+FMOE_API int fmoe_forward_checked(int32_t path, const void* x, const void* w13, const float* s13, const void* w2,
+                                  const float* s2, const float* topk_weights, const int64_t* topk_ids, int64_t tokens,
+                                  int32_t top_k, int32_t experts, int32_t hidden, int32_t inter, const fmoe_config* config,
+                                  void* out, void* workspace, size_t workspace_bytes, void* stream, int32_t* error,
+                                  int32_t* detail);
+
 /* ---- per-stage timing ------------------------------------------------------------------------ */
 
 /* Stages of one forward call, in launch order.  With a stage timer in fmoe_config the forward records
