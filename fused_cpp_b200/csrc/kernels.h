@@ -246,11 +246,12 @@ extern thread_local int threshold_sms;
 // Launch, with `chained` as a programmatic dependent of the kernel before it in the stream.  The kernels of a forward pass
 // (and the GEMM of a dense product) behind its first, an ordinary launch, are chained this way, under these rules (griddepcontrol, ptx.cuh):
 //   * every CTA calls grid_dependency_wait before it touches anything that the kernel before it reads or writes;
-//   * it calls launch_dependents (or ends) only after that; the one exception is the second grouped GEMM of a split stage
-//     (`beside`), which does both the other way round.  A kernel that has started therefore knows that every kernel but the
-//     one right before it has completed, or, right behind a `beside` kernel, every kernel but that one and the first GEMM of
-//     the stage.  What it may read before its wait is what neither of them writes: weights, scales and biases, and, unless it
-//     is the first behind the route build, route lists and work items.  What is read before a wait is read
+//   * it calls launch_dependents (or ends) only after that; the exceptions are the second grouped GEMM of a split stage
+//     (`beside`) and the intermediate's quantiser for few rows (quantize_rows_held_kernel), which do both the other way round.
+//     A kernel that has started therefore knows that every kernel but the one right before it has completed, or, right behind
+//     a `beside` kernel, every kernel but that one and the first GEMM of the stage, or, right behind that quantiser, every
+//     kernel but it and the gate_up stage.  What it may read before its wait is what none of them writes: weights, scales and
+//     biases, and, unless it is the first behind the route build, route lists and work items.  What is read before a wait is read
 //     through L2 (__ldcg): only the wait promises that an L1 line left by an earlier call is not found again;
 //   * what is read behind a wait is not reached through a const __restrict__ parameter: such loads count as invariant, and
 //     the compiler may move them in front of the wait;

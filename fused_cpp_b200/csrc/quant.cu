@@ -124,6 +124,72 @@ quantize_rows_warp_kernel(const uint16_t* x, int64_t out_rows, int cols, const i
   }
 }
 
+// The intermediate of a small batch, one CTA per row of at most 256 * 8 * kVectors columns (a multiple of 16): between two GEMMs
+// nothing but this kernel's latency counts, so the row is read once, beside the row count, and held in registers, one barrier
+// lies between the maximum and the store, and the GEMM behind it is let in before the wait: its CTAs take the SMs that
+// gate_up leaves, and the first weights are on their way while the last rows are still computed.  One token of the 256-expert
+// layer: down's first MMA 8.0 us after gate_up's end with the two-pass kernel and the launch behind the wait, 6.1 us like this
+// (of 126 us; 16 tokens of the 16-expert one 71.5 -> 70.3).
+// kPlanes: two int8 rows per route (split16_planes).
+template <bool kPlanes, int kVectors>
+__global__ void __launch_bounds__(kQuantThreads)
+quantize_rows_held_kernel(const uint16_t* x, int cols, const int* valid_rows, int numerics, int8_t* __restrict__ q, float* __restrict__ scale_out,
+                          bool chained) {
+  __shared__ float warp_amax[kQuantThreads / 32];
+  if (chained) {
+    ptx::launch_dependents();
+    ptx::grid_dependency_wait();
+  }
+  const int64_t row = blockIdx.x;
+  const int rows = __ldcg(valid_rows);
+  const uint4* src = reinterpret_cast<const uint4*>(x + row * cols);
+  const int vec8 = cols >> 3;
+  uint4 held[kVectors];
+  float local = 0.0f;
+#pragma unroll
+  for (int i = 0; i < kVectors; ++i) {
+    const int v = threadIdx.x + i * kQuantThreads;
+    held[i] = v < vec8 ? __ldcg(src + v) : make_uint4(0, 0, 0, 0);
+  }
+  if (row >= rows) return;  // rows of dropped (out-of-range) routes
+#pragma unroll
+  for (int i = 0; i < kVectors; ++i) local = fmaxf(local, amax8(held[i]));
+  local = warp_max(local);
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) warp_amax[threadIdx.x >> 5] = local;
+  __syncthreads();
+  const float amax = warp_max(warp_amax[lane & (kQuantThreads / 32 - 1)]);
+  const float scale = kPlanes ? plane_row_scale(amax) : row_scale_from_amax(amax, numerics);
+  if (threadIdx.x == 0) scale_out[row] = scale;
+  const float operand = quantize_operand(scale, numerics);
+  const float inverse = __fdiv_rn(1.0f, scale);
+#pragma unroll
+  for (int i = 0; i < kVectors; ++i) {
+    const int v = threadIdx.x + i * kQuantThreads;
+    if (v >= vec8) break;
+    float values[8];
+    unpack8(held[i], values);
+    if constexpr (kPlanes) {
+      uint2 high, low;
+      split8_planes(values, scale, &high, &low);
+      reinterpret_cast<uint2*>(q + 2 * row * cols)[v] = high;
+      reinterpret_cast<uint2*>(q + (2 * row + 1) * cols)[v] = low;
+    } else {
+      reinterpret_cast<uint2*>(q + row * cols)[v] = make_uint2(pack4(values, operand, inverse, numerics), pack4(values + 4, operand, inverse, numerics));
+    }
+  }
+}
+
+constexpr int kHeldColumns = kQuantThreads * 8;  // per vector of a thread
+
+template <bool kPlanes>
+cudaError_t launch_held(const uint16_t* x, int64_t rows, int cols, const int* valid_rows, int numerics, int8_t* q, float* scale, cudaStream_t stream) {
+  auto kernel = cols <= kHeldColumns ? quantize_rows_held_kernel<kPlanes, 1>
+                : cols <= 2 * kHeldColumns ? quantize_rows_held_kernel<kPlanes, 2>
+                                           : quantize_rows_held_kernel<kPlanes, 4>;
+  return launch_streaming(kernel, dim3(static_cast<unsigned>(rows)), kQuantThreads, stream, true, x, cols, valid_rows, numerics, q, scale);
+}
+
 // cols % 16 == 0, top_k <= 32.  One CTA per token: the row is quantised once and stored to each of its routes'
 // sorted positions (the reference re-quantises the token for every route, kernels.cpp:639-644; the bits are the same).
 __global__ void __launch_bounds__(kQuantThreads)
@@ -389,6 +455,9 @@ cudaError_t launch_quantize_rows(const uint16_t* x, int64_t out_rows, int cols, 
   // A few rows (decode): one CTA per row spreads a row over 256 threads, where one warp per row would walk its 64
   // values per lane alone on an SM (10.7 us against the other kernel's ~5 us for 8 rows of 2048 columns).
   const bool few_rows = out_rows <= kFewRowsPerSm * threshold_sms;
+  if (few_rows && chained && sorted_routes == nullptr && valid_rows != nullptr && weight_mode == 0 && cols <= 4 * kHeldColumns) {
+    return launch_held<false>(x, out_rows, cols, valid_rows, numerics, q, scale, stream);
+  }
   if (few_rows) {
     return launch_streaming(quantize_rows_kernel, dim3(static_cast<unsigned>(out_rows)), kQuantThreads, stream, chained, x, cols, sorted_routes,
                           top_k, valid_rows, numerics, weight_mode, q, scale);
@@ -407,6 +476,9 @@ cudaError_t launch_quantize_rows(const uint16_t* x, int64_t out_rows, int cols, 
 cudaError_t launch_split_rows_planes(const uint16_t* x, int64_t out_rows, int cols, const int* sorted_routes, int top_k,
                                      const int* valid_rows, int8_t* planes, float* scale, cudaStream_t stream) {
   if (out_rows <= 0) return cudaSuccess;
+  if (out_rows <= kFewRowsPerSm * threshold_sms && sorted_routes == nullptr && valid_rows != nullptr && cols <= 4 * kHeldColumns) {
+    return launch_held<true>(x, out_rows, cols, valid_rows, FMOE_NUMERICS_TORCHREF, planes, scale, stream);
+  }
   return launch_streaming(split_rows_planes_kernel, dim3(static_cast<unsigned>(out_rows)), kQuantThreads, stream, true, x, cols, sorted_routes,
                         top_k, valid_rows, planes, scale);
 }

@@ -55,20 +55,29 @@ __device__ __forceinline__ uint32_t pack4(const float* values, float operand, fl
   return packed;
 }
 
-// 16 values of a row -> 16 bytes of its high and 16 of its low plane (W8A16 in its fixed-point form).
-__device__ __forceinline__ void split16_planes(const float* values, float scale, uint4* high_vector, uint4* low_vector) {
-  uint32_t high[4] = {0, 0, 0, 0};
-  uint32_t low[4] = {0, 0, 0, 0};
+// Eight values of a row -> eight bytes of its high and eight of its low plane (W8A16 in its fixed-point form).
+__device__ __forceinline__ void split8_planes(const float* values, float scale, uint2* high_vector, uint2* low_vector) {
+  uint32_t high[2] = {0, 0};
+  uint32_t low[2] = {0, 0};
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
+  for (int i = 0; i < 8; ++i) {
     const int fixed = plane_fixed_point(values[i], scale);
     const int low_part = ((fixed + 128) & 255) - 128;
     const int high_part = (fixed - low_part) >> 8;  // fixed - low_part is a multiple of 256
     high[i >> 2] |= (static_cast<uint32_t>(high_part) & 0xffu) << (8 * (i & 3));
     low[i >> 2] |= (static_cast<uint32_t>(low_part) & 0xffu) << (8 * (i & 3));
   }
-  *high_vector = make_uint4(high[0], high[1], high[2], high[3]);
-  *low_vector = make_uint4(low[0], low[1], low[2], low[3]);
+  *high_vector = make_uint2(high[0], high[1]);
+  *low_vector = make_uint2(low[0], low[1]);
+}
+
+// The same for 16 values.
+__device__ __forceinline__ void split16_planes(const float* values, float scale, uint4* high_vector, uint4* low_vector) {
+  uint2 high[2], low[2];
+  split8_planes(values, scale, &high[0], &low[0]);
+  split8_planes(values + 8, scale, &high[1], &low[1]);
+  *high_vector = make_uint4(high[0].x, high[0].y, high[1].x, high[1].y);
+  *low_vector = make_uint4(low[0].x, low[0].y, low[1].x, low[1].y);
 }
 
 }  // namespace
