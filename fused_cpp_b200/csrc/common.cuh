@@ -263,6 +263,24 @@ __device__ __forceinline__ float max_or_nan(float a, float b) {
   return result;
 }
 
+// Four values by the exact statement.
+__device__ __forceinline__ uint32_t quantize4_torchref_exact(float v0, float v1, float v2, float v3, float scale, float clamp_low) {
+  const float values[4] = {v0, v1, v2, v3};
+  uint32_t packed = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    packed |= (static_cast<uint32_t>(quantize_value(values[i], scale, FMOE_NUMERICS_TORCHREF, clamp_low)) & 0xffu) << (8 * i);
+  }
+  return packed;
+}
+
+// The same out of line.  A row kernel runs for a few microseconds and fetches its instructions cold; four divisions at each of its
+// unrolled groups, which it hardly ever enters, were most of its code (4072 rows of 2048 columns, a warp each, start to end
+// behind the wait: 13.7 us with them, 6 to 7 us without; 509 Zipf tokens 430.7 -> 427.4 us).
+static __device__ __noinline__ uint32_t quantize4_torchref_call(float v0, float v1, float v2, float v3, float scale, float clamp_low) {
+  return quantize4_torchref_exact(v0, v1, v2, v3, scale, clamp_low);
+}
+
 // TORCHREF quantisation of four values of a row whose scale is that of the row's largest magnitude, with the division
 // replaced by a multiplication wherever that cannot change the result.  value * (1/scale) differs from the correctly rounded
 // value / scale by a few units in the last place (below 2e-5 in absolute terms for |quotient| <= 127.5), so the two round to
@@ -276,6 +294,9 @@ __device__ __forceinline__ float max_or_nan(float a, float b) {
 // One test per four values; the exact statement decides all four when any of them asks for it.  Four instructions
 // per value: with the clamp, the product and its distance as separate operations (seven) 65536 rows of 2048 columns took
 // 112 us, 105 us like this.
+// kCall: the exact statement as a call, for kernels with many groups (the dense quantiser has two or four: 28.5 us for the op
+// at 64 rows, 28.6 with a call).
+template <bool kCall = true>
 __device__ __forceinline__ uint32_t quantize4_torchref_fast(const float* values, float scale, float inverse, float clamp_low = -127.0f) {
   constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
   uint32_t bits[4];
@@ -288,12 +309,8 @@ __device__ __forceinline__ uint32_t quantize4_torchref_fast(const float* values,
     bits[i] = __float_as_uint(shifted);
   }
   if (!(worst <= 0.4999f)) {
-    uint32_t packed = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      packed |= (static_cast<uint32_t>(quantize_value(values[i], scale, FMOE_NUMERICS_TORCHREF, clamp_low)) & 0xffu) << (8 * i);
-    }
-    return packed;
+    if constexpr (kCall) return quantize4_torchref_call(values[0], values[1], values[2], values[3], scale, clamp_low);
+    return quantize4_torchref_exact(values[0], values[1], values[2], values[3], scale, clamp_low);
   }
   // Low byte of each sum = the integer in two's complement.
   return __byte_perm(__byte_perm(bits[0], bits[1], 0x0040), __byte_perm(bits[2], bits[3], 0x0040), 0x5410);

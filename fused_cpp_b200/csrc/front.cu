@@ -106,40 +106,37 @@ front_kernel(RouteArgs route, const uint16_t* x, int cols, int top_k, int numeri
     inverse = __fdiv_rn(1.0f, scale);
     if (threadIdx.x < top_k && slot_ids[threadIdx.x] >= 0) scale_out[positions[threadIdx.x]] = scale;
   }
-  for (int v = threadIdx.x; v < vec16; v += kFrontThreads) {
-    if (v >= kFrontThreads) {
-      held[0] = src[2 * v];
-      held[1] = src[2 * v + 1];
-    }
-    uint4 first = held[0], second = held[1];  // bf16: the row as it is
-    if constexpr (kRows != FrontRows::kBf16) {
-      float values[16];
-      unpack8(held[0], values);
-      unpack8(held[1], values + 8);
+  with_numerics(kRows == FrontRows::kInt8 ? numerics : FMOE_NUMERICS_TORCHREF, [&](auto tag) {
+    for (int v = threadIdx.x; v < vec16; v += kFrontThreads) {
+      if (v >= kFrontThreads) {
+        held[0] = src[2 * v];
+        held[1] = src[2 * v + 1];
+      }
+      uint4 first = held[0], second = held[1];  // bf16: the row as it is
       if constexpr (kRows == FrontRows::kPlanes) {
+        float values[16];
+        unpack8(held[0], values);
+        unpack8(held[1], values + 8);
         split16_planes(values, scale, &first, &second);
-      } else {
-        first.x = pack4(values, operand, inverse, numerics);
-        first.y = pack4(values + 4, operand, inverse, numerics);
-        first.z = pack4(values + 8, operand, inverse, numerics);
-        first.w = pack4(values + 12, operand, inverse, numerics);
+      } else if constexpr (kRows == FrontRows::kInt8) {
+        first = pack16(tag, held[0], held[1], operand, inverse);
+      }
+      for (int slot = 0; slot < top_k; ++slot) {
+        if (slot_ids[slot] < 0) continue;  // dropped by the route build, which reports it
+        const int64_t position = positions[slot];
+        if constexpr (kRows == FrontRows::kInt8) {
+          reinterpret_cast<uint4*>(static_cast<int8_t*>(rows_out) + position * cols)[v] = first;
+        } else if constexpr (kRows == FrontRows::kPlanes) {
+          reinterpret_cast<uint4*>(static_cast<int8_t*>(rows_out) + 2 * position * cols)[v] = first;
+          reinterpret_cast<uint4*>(static_cast<int8_t*>(rows_out) + (2 * position + 1) * cols)[v] = second;
+        } else {
+          uint4* dst = reinterpret_cast<uint4*>(static_cast<uint16_t*>(rows_out) + position * cols) + 2 * v;
+          dst[0] = first;
+          dst[1] = second;
+        }
       }
     }
-    for (int slot = 0; slot < top_k; ++slot) {
-      if (slot_ids[slot] < 0) continue;  // dropped by the route build, which reports it
-      const int64_t position = positions[slot];
-      if constexpr (kRows == FrontRows::kInt8) {
-        reinterpret_cast<uint4*>(static_cast<int8_t*>(rows_out) + position * cols)[v] = first;
-      } else if constexpr (kRows == FrontRows::kPlanes) {
-        reinterpret_cast<uint4*>(static_cast<int8_t*>(rows_out) + 2 * position * cols)[v] = first;
-        reinterpret_cast<uint4*>(static_cast<int8_t*>(rows_out) + (2 * position + 1) * cols)[v] = second;
-      } else {
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<uint16_t*>(rows_out) + position * cols) + 2 * v;
-        dst[0] = first;
-        dst[1] = second;
-      }
-    }
-  }
+  });
 }
 
 }  // namespace

@@ -51,17 +51,9 @@ quantize_rows_kernel(const uint16_t* x, int cols, const int* sorted_routes, int 
   const float operand = quantize_operand(scale, mode);
   const float inverse = __fdiv_rn(1.0f, scale);
   uint4* dst = reinterpret_cast<uint4*>(q + row * cols);
-  for (int v = threadIdx.x; v < vec16; v += kQuantThreads) {
-    float values[16];
-    unpack8(src[2 * v], values);
-    unpack8(src[2 * v + 1], values + 8);
-    uint4 out;
-    out.x = pack4(values, operand, inverse, mode);
-    out.y = pack4(values + 4, operand, inverse, mode);
-    out.z = pack4(values + 8, operand, inverse, mode);
-    out.w = pack4(values + 12, operand, inverse, mode);
-    dst[v] = out;
-  }
+  with_numerics(mode, [&](auto tag) {
+    for (int v = threadIdx.x; v < vec16; v += kQuantThreads) dst[v] = pack16(tag, src[2 * v], src[2 * v + 1], operand, inverse);
+  });
 }
 
 // Same work, one warp per output row, for rows of at most 32 * 16 * kVectors columns: the row is read once
@@ -73,8 +65,8 @@ quantize_rows_warp_kernel(const uint16_t* x, int64_t out_rows, int cols, const i
                           const int* valid_rows, int numerics, int weight_mode, int8_t* __restrict__ q,
                           float* __restrict__ scale_out, bool chained) {
   if (chained) {
+    ptx::launch_dependents();  // ahead of the wait, as in quantize_rows_held_kernel
     ptx::grid_dependency_wait();
-    ptx::launch_dependents();
   }
   const int lane = threadIdx.x & 31;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * (kQuantThreads / 32) + (threadIdx.x >> 5);
@@ -107,21 +99,13 @@ quantize_rows_warp_kernel(const uint16_t* x, int64_t out_rows, int cols, const i
   const float operand = quantize_operand(scale, mode);
   const float inverse = __fdiv_rn(1.0f, scale);
   uint4* dst = reinterpret_cast<uint4*>(q + row * cols);
+  with_numerics(mode, [&](auto tag) {
 #pragma unroll
-  for (int i = 0; i < kVectors; ++i) {
-    const int v = lane + 32 * i;
-    if (v < vec16) {
-      float values[16];
-      unpack8(held[i][0], values);
-      unpack8(held[i][1], values + 8);
-      uint4 out;
-      out.x = pack4(values, operand, inverse, mode);
-      out.y = pack4(values + 4, operand, inverse, mode);
-      out.z = pack4(values + 8, operand, inverse, mode);
-      out.w = pack4(values + 12, operand, inverse, mode);
-      dst[v] = out;
+    for (int i = 0; i < kVectors; ++i) {
+      const int v = lane + 32 * i;
+      if (v < vec16) dst[v] = pack16(tag, held[i][0], held[i][1], operand, inverse);
     }
-  }
+  });
 }
 
 // The intermediate of a small batch, one CTA per row of at most 256 * 8 * kVectors columns (a multiple of 16): between two GEMMs
@@ -163,21 +147,23 @@ quantize_rows_held_kernel(const uint16_t* x, int cols, const int* valid_rows, in
   if (threadIdx.x == 0) scale_out[row] = scale;
   const float operand = quantize_operand(scale, numerics);
   const float inverse = __fdiv_rn(1.0f, scale);
+  with_numerics(numerics, [&](auto tag) {
 #pragma unroll
-  for (int i = 0; i < kVectors; ++i) {
-    const int v = threadIdx.x + i * kQuantThreads;
-    if (v >= vec8) break;
-    float values[8];
-    unpack8(held[i], values);
-    if constexpr (kPlanes) {
-      uint2 high, low;
-      split8_planes(values, scale, &high, &low);
-      reinterpret_cast<uint2*>(q + 2 * row * cols)[v] = high;
-      reinterpret_cast<uint2*>(q + (2 * row + 1) * cols)[v] = low;
-    } else {
-      reinterpret_cast<uint2*>(q + row * cols)[v] = make_uint2(pack4(values, operand, inverse, numerics), pack4(values + 4, operand, inverse, numerics));
+    for (int i = 0; i < kVectors; ++i) {
+      const int v = threadIdx.x + i * kQuantThreads;
+      if (v >= vec8) break;
+      float values[8];
+      unpack8(held[i], values);
+      if constexpr (kPlanes) {
+        uint2 high, low;
+        split8_planes(values, scale, &high, &low);
+        reinterpret_cast<uint2*>(q + 2 * row * cols)[v] = high;
+        reinterpret_cast<uint2*>(q + (2 * row + 1) * cols)[v] = low;
+      } else {
+        reinterpret_cast<uint2*>(q + row * cols)[v] = make_uint2(pack4(tag, values, operand, inverse), pack4(tag, values + 4, operand, inverse));
+      }
     }
-  }
+  });
 }
 
 constexpr int kHeldColumns = kQuantThreads * 8;  // per vector of a thread
@@ -215,20 +201,15 @@ quantize_tokens_scatter_kernel(const uint16_t* x, int cols, int top_k, const int
   if (threadIdx.x < top_k && positions[threadIdx.x] >= 0) scale_out[positions[threadIdx.x]] = scale;
   const float operand = quantize_operand(scale, numerics);
   const float inverse = __fdiv_rn(1.0f, scale);
-  for (int v = threadIdx.x; v < vec16; v += kQuantThreads) {
-    float values[16];
-    unpack8(__ldcg(src + 2 * v), values);
-    unpack8(__ldcg(src + 2 * v + 1), values + 8);
-    uint4 out;
-    out.x = pack4(values, operand, inverse, numerics);
-    out.y = pack4(values + 4, operand, inverse, numerics);
-    out.z = pack4(values + 8, operand, inverse, numerics);
-    out.w = pack4(values + 12, operand, inverse, numerics);
-    for (int slot = 0; slot < top_k; ++slot) {
-      const int position = positions[slot];
-      if (position >= 0) reinterpret_cast<uint4*>(q + static_cast<int64_t>(position) * cols)[v] = out;
+  with_numerics(numerics, [&](auto tag) {
+    for (int v = threadIdx.x; v < vec16; v += kQuantThreads) {
+      const uint4 out = pack16(tag, __ldcg(src + 2 * v), __ldcg(src + 2 * v + 1), operand, inverse);
+      for (int slot = 0; slot < top_k; ++slot) {
+        const int position = positions[slot];
+        if (position >= 0) reinterpret_cast<uint4*>(q + static_cast<int64_t>(position) * cols)[v] = out;
+      }
     }
-  }
+  });
 }
 
 // W8A16 in its fixed-point form.  cols % 16 == 0.  One CTA per route row p (gathered by token when sorted_routes is
@@ -239,8 +220,8 @@ split_rows_planes_kernel(const uint16_t* x, int cols, const int* sorted_routes, 
                          const int* valid_rows, int8_t* __restrict__ planes, float* __restrict__ scale_out, bool chained) {
   __shared__ float smem[32];
   if (chained) {
+    ptx::launch_dependents();  // ahead of the wait, as in quantize_rows_held_kernel
     ptx::grid_dependency_wait();
-    ptx::launch_dependents();
   }
   const int64_t row = blockIdx.x;
   if (valid_rows && row >= __ldcg(valid_rows)) return;
@@ -543,7 +524,7 @@ quantize_rows_dense_vec8_kernel(const void* __restrict__ x, int cols, int cols_p
   for (int i = 0; i < kDenseVectors; ++i) {
     const int v = threadIdx.x + i * blockDim.x;
     if (v < vec8) {
-      dst[v] = make_uint2(quantize4_torchref_fast(values[i], scale, inverse, clamp_low), quantize4_torchref_fast(values[i] + 4, scale, inverse, clamp_low));
+      dst[v] = make_uint2(quantize4_torchref_fast<false>(values[i], scale, inverse, clamp_low), quantize4_torchref_fast<false>(values[i] + 4, scale, inverse, clamp_low));
     }
   }
   // cols_padded is cols or cols + 8 (a multiple of 16).
@@ -576,8 +557,8 @@ quantize_rows_dense_bf16x8_kernel(const uint16_t* __restrict__ x, int cols, int 
     if (v < vec8) {
       float values[8];
       unpack8(src[v], values);
-      out.x = quantize4_torchref_fast(values, scale, inverse);
-      out.y = quantize4_torchref_fast(values + 4, scale, inverse);
+      out.x = quantize4_torchref_fast<false>(values, scale, inverse);
+      out.y = quantize4_torchref_fast<false>(values + 4, scale, inverse);
     }
     dst[v] = out;
   }

@@ -44,15 +44,40 @@ __device__ __forceinline__ float amax8(const uint4& v) {
   return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u));
 }
 
+template <int kNumerics>
+struct NumericsTag {
+  static constexpr int value = kNumerics;
+};
+
+// Calls body(NumericsTag): one instance of a row loop per arithmetic statement, side by side instead of a choice per group.
+template <typename Body>
+__device__ __forceinline__ void with_numerics(int numerics, Body&& body) {
+  if (numerics == FMOE_NUMERICS_TORCHREF) {
+    body(NumericsTag<FMOE_NUMERICS_TORCHREF>{});
+  } else {
+    body(NumericsTag<FMOE_NUMERICS_NATIVE>{});
+  }
+}
+
 // operand: 1/scale (NATIVE) or scale (TORCHREF); inverse: 1/scale, used by the TORCHREF fast path.
-__device__ __forceinline__ uint32_t pack4(const float* values, float operand, float inverse, int numerics) {
-  if (numerics == FMOE_NUMERICS_TORCHREF) return quantize4_torchref_fast(values, operand, inverse);
+template <typename Tag>
+__device__ __forceinline__ uint32_t pack4(Tag, const float* values, float operand, float inverse) {
+  if constexpr (Tag::value == FMOE_NUMERICS_TORCHREF) return quantize4_torchref_fast(values, operand, inverse);
   uint32_t packed = 0;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    packed |= (static_cast<uint32_t>(quantize_value(values[i], operand, numerics)) & 0xffu) << (8 * i);
+    packed |= (static_cast<uint32_t>(quantize_value(values[i], operand, Tag::value)) & 0xffu) << (8 * i);
   }
   return packed;
+}
+
+template <typename Tag>
+__device__ __forceinline__ uint4 pack16(Tag tag, const uint4& first, const uint4& second, float operand, float inverse) {
+  float values[16];
+  unpack8(first, values);
+  unpack8(second, values + 8);
+  return make_uint4(pack4(tag, values, operand, inverse), pack4(tag, values + 4, operand, inverse), pack4(tag, values + 8, operand, inverse),
+                    pack4(tag, values + 12, operand, inverse));
 }
 
 // Eight values of a row -> eight bytes of its high and eight of its low plane (W8A16 in its fixed-point form).
