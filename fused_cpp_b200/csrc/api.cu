@@ -370,6 +370,7 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   gu.status = status_block;
   gu.status_rw = status_block;
   gu.item_count_word = fmoe::kStatusItems;
+  gu.tallest_word = fmoe::kStatusTallestA;
   gu.max_items = max_items;
   gu.sorted_routes = sorted_routes;
   gu.experts = f.experts;
@@ -398,6 +399,7 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
     fmoe::GroupedGemmArgs big = gu;
     big.items = items_gu_big;
     big.item_count_word = fmoe::kStatusItemsC;
+    big.tallest_word = fmoe::kStatusTallestC;
     big.items_late = 0;
     big.beside = 1;
     big.row_tile = fmoe::kPairRowTile;
@@ -428,6 +430,7 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
   dn.expert_bias = cfg.w2_bias;
   dn.items = items_dn;
   dn.item_count_word = fmoe::kStatusItemsB;
+  dn.tallest_word = fmoe::kStatusTallestB;
   dn.k = f.inter;
   dn.n_out = f.hidden;
   dn.y = nullptr;
@@ -448,6 +451,7 @@ int run_forward(const Forward& f, const fmoe_config* config, void* out, void* wo
     fmoe::GroupedGemmArgs big = dn;
     big.items = items_dn_big;
     big.item_count_word = fmoe::kStatusItemsD;
+    big.tallest_word = fmoe::kStatusTallestD;
     big.beside = 1;
     big.row_tile = fmoe::kPairRowTile;
     error = fmoe::launch_umma_grouped_gemm(big, int8_gemm, false, stream);

@@ -26,7 +26,11 @@ enum StatusWord : int {
   kStatusItemsB = 5,     // work items of the second list (down GEMM)
   kStatusItemsC = 6,     // split mode: gate_up work items of the experts with many rows (two-SM kernel)
   kStatusItemsD = 7,     // split mode: down work items of those experts
+  kStatusTallestC = 8,   // rows of the largest work item of lists C, D and (below) A, B
+  kStatusTallestD = 9,
   kStatusMirror = 10,    // two words: address of page-locked host words that take the first error too (0 = none)
+  kStatusTallestA = 12,
+  kStatusTallestB = 13,
   kStatusWords = 16,
 };
 

@@ -148,7 +148,8 @@ struct GroupedGemmArgs {
   const float* w_scale;      // [E, N_total] (int8) or null
   const int* items;          // (expert, first row, rows, 0) per work item
   const int* status;         // status block: item counts are read from it
-  int item_count_word;       // kStatusItems or kStatusItemsB
+  int item_count_word;       // kStatusItems .. kStatusItemsD
+  int tallest_word;          // kStatusTallestA .. kStatusTallestD: rows of the list's largest item
   int max_items;
   const int* sorted_routes;  // down GEMM: flat route id of each sorted row
   int experts;

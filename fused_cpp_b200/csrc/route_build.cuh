@@ -40,6 +40,7 @@ __device__ void build_item_list(int list, int experts, const int* counts, const 
   auto tiles_of = [&](int rows) { return tall && rows > cut && rows <= tile ? 1 : (rows + cut - 1) >> shift; };
   int carry = 0;
   int active = 0;
+  int tallest = 0;
   constexpr int kBatch = 8;  // groups of 32 experts whose scans are interleaved: a scan is a chain of dependent shuffles
   for (int base = 0; base < experts; base += 32 * kBatch) {
     int count[kBatch], inclusive[kBatch];
@@ -75,6 +76,7 @@ __device__ void build_item_list(int list, int experts, const int* counts, const 
         const int even = ((count[i] + tiles - 1) / tiles + step - 1) & ~(step - 1);
         if (even <= tile && (tiles - 1) * even < count[i]) rows_per = even;
       }
+      tallest = max(tallest, min(rows_per, count[i]));
       for (int t = 0; t < tiles && first + t < max_items; ++t) {
         // Group key for the unit order of the grouped GEMM: first item of this expert and its tile count, so that the
         // row tiles of one (expert, channel block) are consecutive work units (see resolve_unit in umma_gemm.cu).
@@ -83,7 +85,9 @@ __device__ void build_item_list(int list, int experts, const int* counts, const 
       }
     }
   }
+  for (int offset = 16; offset > 0; offset >>= 1) tallest = max(tallest, __shfl_xor_sync(0xffffffffu, tallest, offset));
   if (lane == 0) {
+    status[list == 0 ? kStatusTallestA : list == 1 ? kStatusTallestB : list == 2 ? kStatusTallestC : kStatusTallestD] = tallest;
     status[word] = carry < max_items ? carry : max_items;
     if (list == 0) status[kStatusActive] = active;
   }
