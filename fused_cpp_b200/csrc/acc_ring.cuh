@@ -51,4 +51,12 @@ FMOE_HOST_DEVICE int blocks_shared(const AccSlot& before, const AccSlot& slot) {
   return shared > 0 ? shared : 0;
 }
 
+// A warp of the epilogue reads every other chunk (block) of a unit, `chunks` of them in all; its next one is `next_chunk`.  Whether
+// it is past the blocks that the next unit takes over, and so owes their barrier its arrival.  A unit's chunks are its blocks, and
+// blocks_shared is never more than those; but a unit whose accumulator is not read at all (the diagnostic library's switch,
+// chunks = 0) hands its blocks over too, and the barrier counts every warp once a handover.
+FMOE_HOST_DEVICE bool handed_over_read(int next_chunk, int handed_over, int chunks) {
+  return next_chunk >= handed_over || next_chunk >= chunks;
+}
+
 }  // namespace fmoe

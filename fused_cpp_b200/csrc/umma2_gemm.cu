@@ -652,7 +652,7 @@ umma_pair_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, co
       bool part_held = handed_over > 0;
       bool all_held = true;
       auto release = [&](int next_chunk) {
-        const bool part = part_held && next_chunk >= handed_over;
+        const bool part = part_held && handed_over_read(next_chunk, handed_over, chunks);
         const bool all = all_held && next_chunk >= chunks;
         if (!part && !all) return;
         ptx::tcgen05_fence_before();

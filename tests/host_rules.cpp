@@ -18,3 +18,21 @@ extern "C" void place_units(const int* rows, int count, int* slots, int* shared)
     before = slot;
   }
 }
+
+// Arrivals of one epilogue warp (chunks first, first + step, ...) on the handover barrier of a unit, in the order of the kernel's
+// epilogue; *early counts those in front of a load of a handed-over block.
+extern "C" int handover_arrivals(int first, int step, int handed_over, int chunks, int* early) {
+  bool held = handed_over > 0;
+  int arrivals = 0;
+  auto release = [&](int next_chunk) {
+    if (!held || !fmoe::handed_over_read(next_chunk, handed_over, chunks)) return;
+    held = false;
+    ++arrivals;
+  };
+  release(first);
+  for (int chunk = first; chunk < chunks; chunk += step) {
+    if (!held && chunk < handed_over) ++*early;
+    release(chunk + step);
+  }
+  return arrivals;
+}

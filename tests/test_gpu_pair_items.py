@@ -48,3 +48,16 @@ def test_against_one_sm_kernel(cuda_device, kind, rows):
         assert float(error) <= 4e-3
     else:
         assert torch.equal(result.out.view(torch.int16), reference.view(torch.int16))
+
+
+def test_ends_without_an_epilogue(cuda_device, monkeypatch):
+    """The diagnostic library's switch for an epilogue that reads nothing: units still hand their accumulators on."""
+    hidden, inter, experts = 4096, 2048, len(MIXED)
+    ids = torch.repeat_interleave(torch.arange(experts, device=cuda_device), torch.tensor(MIXED, device=cuda_device)).reshape(-1, 1)
+    x = torch.zeros((ids.shape[0], hidden), dtype=torch.bfloat16, device=cuda_device)
+    w13 = torch.zeros((experts, 2 * inter, hidden), dtype=torch.int8, device=cuda_device)
+    w2 = torch.zeros((experts, hidden, inter), dtype=torch.int8, device=cuda_device)
+    monkeypatch.setenv("FUSED_CPP_MOE_GEMM_DIAG", "1")
+    result = _lib.moe_forward(x, w13, w2, torch.ones(ids.shape, device=cuda_device), ids, gate_up_tile=512, down_tile=512, diagnostic=True,
+                              s13=torch.ones((experts, 2 * inter), device=cuda_device), s2=torch.ones((experts, hidden), device=cuda_device))
+    assert result.status() == (_lib.OK, 0)

@@ -61,3 +61,15 @@ def test_accumulator_ring(rules, sizes):
         assert worst <= 7
     if sizes in ((1, 32), (256, 256)):
         assert worst == 0
+
+
+@pytest.mark.parametrize("read", [True, False], ids=["read", "not read"])
+def test_every_warp_hands_blocks_over_once(rules, read):
+    """Also where the epilogue is switched off and a unit has no chunks to read."""
+    for blocks in range(1, 11):
+        for handed_over in range(0, blocks + 1):
+            for first, step in ((0, 1), (0, 2), (1, 2)):
+                early = ctypes.c_int(0)
+                arrivals = rules.handover_arrivals(first, step, handed_over, blocks if read else 0, ctypes.byref(early))
+                assert arrivals == (1 if handed_over else 0), (blocks, handed_over, first, step)
+                assert early.value == 0
