@@ -190,9 +190,13 @@ def _open(path: str) -> ctypes.CDLL:
     return lib
 
 
+def _error_text(lib: ctypes.CDLL) -> str:
+    return lib.fmoe_last_error().decode("utf-8", "replace")
+
+
 def check(code: int, lib: ctypes.CDLL | None = None) -> None:
     if code != OK:
-        message = (lib or load()).fmoe_last_error().decode("utf-8", "replace")
+        message = _error_text(lib or load())
         error_type = ValueError if code == ERR_INVALID_ARGUMENT else FusedMoEError
         if error_type is ValueError:
             raise ValueError(message)
@@ -253,6 +257,7 @@ class ForwardResult:
     acc1: torch.Tensor | None = None
     acc2: torch.Tensor | None = None
     checked: tuple[int, int] | None = None  # (error, detail) of a call that waited for its kernels
+    checked_text: str = ""                  # its error text, taken when it returned: the thread's text is the next call's then
 
     def region(self, name: str, dtype: torch.dtype, shape) -> torch.Tensor:
         count = 1
@@ -280,7 +285,7 @@ class ForwardResult:
         if error == ERR_EXPERT_ID_RANGE:
             raise FusedMoEError(error, f"topk expert id is out of range (flat route {detail})")
         if error != OK:
-            raise FusedMoEError(error, load().fmoe_last_error().decode("utf-8", "replace"))
+            raise FusedMoEError(error, _error_text(load()) if self.checked is None else self.checked_text)
 
 
 class StageTimer:
@@ -414,7 +419,8 @@ def moe_forward(x, w13, w2, topk_weights, topk_ids, *, s13=None, s2=None, numeri
                                      experts, hidden, inter, ctypes.byref(config), _ptr(out), _ptr(workspace),
                                      workspace.numel(), _stream())
     check(code, lib)
-    return ForwardResult(out=out, workspace=workspace, layout=layout, acc1=acc1, acc2=acc2, checked=checked)
+    text = _error_text(lib) if checked is not None and checked[0] != OK else ""
+    return ForwardResult(out=out, workspace=workspace, layout=layout, acc1=acc1, acc2=acc2, checked=checked, checked_text=text)
 
 
 def quantize_rows(x: torch.Tensor, numerics: int = NUMERICS_TORCHREF, weight_mode: bool = False):
