@@ -58,6 +58,16 @@ W8A16_FIXED_POINT = 0
 W8A16_BF16_ACTIVATIONS = 1
 
 
+def _table_of_bytes(environ) -> bool:
+    """Whether environ keeps its variables the way Switch reads them: a dict of encoded names and values, `_data`."""
+    table = getattr(environ, "_data", None)
+    return type(table) is dict and all(table.get(os.fsencode(name)) == os.fsencode(value) for name, value in environ.items())
+
+
+# The mapping type that was found to do so.  `_data` is private to the interpreter, so any other type is asked through `get`.
+_KNOWN_ENVIRON = type(os.environ) if os.environ and _table_of_bytes(os.environ) else None
+
+
 class Switch:
     """An environment variable that every call looks up.  os.environ.get raises and catches a KeyError inside for a name that
     is not set, over a microsecond, and a forward asks for six; the mapping's own table answers in a twentieth of that, and
@@ -67,10 +77,10 @@ class Switch:
         self.name, self.key, self.default = name, os.fsencode(name), default
 
     def get(self) -> str:
-        try:
-            value = os.environ._data.get(self.key)
-        except AttributeError:  # not CPython's mapping
-            return os.environ.get(self.name, self.default)
+        environ = os.environ
+        if type(environ) is not _KNOWN_ENVIRON:
+            return environ.get(self.name, self.default)
+        value = environ._data.get(self.key)
         return self.default if value is None else os.fsdecode(value)
 
 
