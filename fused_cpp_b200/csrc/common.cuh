@@ -80,15 +80,22 @@ __device__ __forceinline__ float reciprocal_seed(float d) {
   return r;
 }
 
-// n / d rounded to nearest for d in [1, 2^40] and |n| in [2^-60, 2^60]: a Newton step makes the seed the correctly rounded
-// reciprocal, and by Markstein's theorem (P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", IBM J. Res. Dev. 34, 1990) a quotient that is corrected once by its exact remainder times that reciprocal is
-// the correctly rounded one; in these ranges no step over- or underflows.  __fdiv_rn gives the same bits but tests its operands
+// 1 / d rounded to nearest for d in [1, 2^40]: one Newton step on the seed.  (That it is the correctly rounded one is what
+// quotient_fast rests on; with a seed one unit high the step would miss it at 32 mantissas.  tests/test_gpu_quotient.py compares it with
+// __frcp_rn for every mantissa.)
+__device__ __forceinline__ float reciprocal_fast(float d) {
+  const float seed = reciprocal_seed(d);
+  return __fmaf_rn(seed, __fmaf_rn(-d, seed, 1.0f), seed);
+}
+
+// n / d rounded to nearest for d in [1, 2^40] and |n| in [2^-60, 2^60]: by Markstein's theorem (P. W. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990) a quotient by the correctly rounded
+// reciprocal that is corrected once by its exact remainder times that reciprocal is the correctly rounded one; in these ranges
+// no step over- or underflows.  __fdiv_rn gives the same bits but tests its operands
 // and branches, which keeps the compiler from overlapping the elements of an unrolled loop.
 // (tests/test_gpu_quotient.py compares the two for every mantissa of d.)
 __device__ __forceinline__ float quotient_fast(float n, float d) {
-  const float seed = reciprocal_seed(d);
-  const float r = __fmaf_rn(seed, __fmaf_rn(-d, seed, 1.0f), seed);
+  const float r = reciprocal_fast(d);
   const float q = __fmul_rn(n, r);
   return __fmaf_rn(__fmaf_rn(-d, q, n), r, q);
 }

@@ -21,7 +21,7 @@ extern "C" {
  * timed launches.  Allocates a few bytes and synchronises. */
 FMOE_API int fmoe_probe_mma_rate(int32_t int8, int32_t n, int32_t iterations, int32_t mode, float* tera_ops_per_s);
 
-/* The quotient of the SwiGLU epilogues against the compiler's division: every mantissa of the divisor, `numerators` each;
+/* The reciprocal and the quotient of the SwiGLU epilogues against the compiler's: every mantissa of the divisor, `numerators` each;
  * *mismatches (device memory, 8 bytes) is added to. */
 FMOE_API int fmoe_diag_quotient_check(uint32_t seed, int32_t numerators, void* mismatches, void* stream);
 

@@ -327,7 +327,8 @@ constexpr int kPairItemRows = 320;  // token rows of a work item at most (umma2_
 cudaError_t launch_umma_pair_grouped_gemm(const GroupedGemmArgs& args, bool int8, bool gate_up, cudaStream_t stream);
 
 // ---- probe.cu (diagnostic library only)
-// Adds to *mismatches how often quotient_fast differs from __fdiv_rn: every mantissa of the divisor, `numerators` each.
+// Adds to *mismatches how often reciprocal_fast differs from __frcp_rn and quotient_fast from __fdiv_rn: every mantissa of the
+// divisor, `numerators` each.
 cudaError_t launch_quotient_check(uint32_t seed, int numerators, unsigned long long* mismatches, cudaStream_t stream);
 // tcgen05.mma issue-rate probe (128 x n x 32-byte MMAs back to back on every CTA)
 cudaError_t launch_mma_rate_probe(bool int8, int n, int iterations, int mode, int blocks, int* status, cudaStream_t stream);

@@ -193,8 +193,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128, 1) mma_rate_pai
   }
 }
 
-// quotient_fast against __fdiv_rn: one thread per mantissa of d; numerators are the two ends and the middle of a binade and
-// random ones, exponents random inside the ranges of quotient_fast.
+// reciprocal_fast against __frcp_rn and quotient_fast against __fdiv_rn: one thread per mantissa of d; numerators are the two ends
+// and the middle of a binade, the divisor's mantissa, one that a reciprocal off by a unit would show, and random ones; exponents
+// random inside the ranges of quotient_fast.
 __global__ void quotient_check_kernel(uint32_t seed, int numerators, unsigned long long* mismatches) {
   const uint32_t mantissa = blockIdx.x * blockDim.x + threadIdx.x;
   if (mantissa >= (1u << 23)) return;
@@ -209,8 +210,9 @@ __global__ void quotient_check_kernel(uint32_t seed, int numerators, unsigned lo
   unsigned long long wrong = 0;
   for (int i = 0; i < numerators; ++i) {
     const float d = __uint_as_float(((127u + next() % 40u) << 23) | mantissa);
-    const uint32_t numerator = i == 0 ? 0u : i == 1 ? 0x7fffffu : i == 2 ? 0x400000u : i == 3 ? mantissa : next() & 0x7fffffu;
+    const uint32_t numerator = i == 0 ? 0u : i == 1 ? 0x7fffffu : i == 2 ? 0x400000u : i == 3 ? mantissa : i == 4 ? 0x555553u : next() & 0x7fffffu;
     const float n = __uint_as_float((next() & 0x80000000u) | ((67u + next() % 120u) << 23) | numerator);
+    if (__float_as_uint(reciprocal_fast(d)) != __float_as_uint(__frcp_rn(d))) ++wrong;
     if (__float_as_uint(quotient_fast(n, d)) != __float_as_uint(__fdiv_rn(n, d))) ++wrong;
   }
   if (wrong != 0) atomicAdd(mismatches, wrong);

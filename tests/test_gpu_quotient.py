@@ -1,5 +1,5 @@
-"""The branch-free quotient of the SwiGLU epilogues: the compiler's division bit for bit, and the plain statement outside
-its ranges."""
+"""The branch-free quotient of the SwiGLU epilogues: the compiler's reciprocal and division bit for bit, and the plain statement
+outside its ranges."""
 import ctypes
 
 import pytest
