@@ -6,8 +6,12 @@
 // route is the number of valid routes with a smaller expert id plus that of earlier routes with the same one, a few hundred
 // comparisons per slot that hide behind the load of the row.  CTA 0 is the route build of route.cu, the others one token
 // each; the GEMM behind it reads its work items behind its wait (GroupedGemmArgs::items_late).  Against the two launches, whole
-// forwards with the status read: one token of the 256-expert layer with its router 153.9 -> 148.9 us, 16 tokens of the
-// 16-expert one (int8) 99.3 -> 93.6, 200 tokens of it (bf16) 126.2 -> 121.9; 64 tokens of the 256-expert layer 1516 -> 1502.
+// forwards with the status read, cold L2: one token of the 16-expert layer (int8) 49.7 -> 48.2 us, 16 tokens 62.8 -> 60.9, 100 and
+// 200 tokens the same within the spread; bf16 52.1 -> 49.8, 77.6 -> 73.9, 89.6 -> 86.8, 93.9 -> 91.0; one token of the 256-expert layer
+// 105.9 -> 104.8.  Most of that is a launch less for the host.  On the device alone (captured, no status read) it gains for the
+// 256-expert layer (one token 87.3 -> 86.5) and W8A16 (16 tokens 38.5 -> 37.7), and costs small int8 layers the weights
+// that gate_up fetched while the rows were quantised: 16 experts, 1 / 16 / 65 / 200 tokens 24.8 -> 26.9, 37.8 -> 38.8, 45.9 -> 49.7,
+// 50.9 -> 52.8 us (bf16 65 tokens 65.7 -> 67.2).
 // The reference's order of work is csrc/moe/arm/i8mm_w8a8/kernels.cpp:583-592 and :639-644.
 #include "common.cuh"
 #include "kernels.h"
@@ -23,7 +27,10 @@ constexpr int kFrontThreads = 512;
 constexpr int kFrontWarps = kFrontThreads / 32;
 constexpr int kFrontMaxRoutes = 1024;   // two rounds of comparisons per thread, one CTA of route build
 constexpr int kFrontMaxExperts = 512;   // histogram rows of kFrontWarps warps stay below the 48 KB every launch may have
-constexpr int kFrontTokensPerSm = 4;    // a CTA per token: all resident at once
+// A CTA per token; two of them fit an SM (62 registers a thread), so from 2 * SMs tokens on they run in two waves.  That is still
+// faster than two launches: device time of a captured forward with one route per token, int8, 512 experts of 2048 x 256, 443 tokens
+// 120.4 -> 116.8 us, 592 tokens 138.3 -> 134.9; 16 experts of 2048 x 1024 47.7 -> 46.5 (300 tokens), 51.0 -> 50.9 (592).
+constexpr int kFrontTokensPerSm = 4;
 constexpr int kMaxTopK = 32;
 
 struct RouteArgs {

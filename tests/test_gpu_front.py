@@ -64,3 +64,31 @@ def test_bf16_rows(tokens, top_k, experts, hidden):
     order, _, rows, _ = _rows(result, tokens, top_k, hidden, experts, torch.bfloat16)
     assert torch.equal(order.cpu().long(), torch.argsort(ids.reshape(-1), stable=True))
     assert torch.equal(rows, x[(order // top_k).long()])
+
+
+@pytest.mark.parametrize("tokens,hidden", [(297, 256), (592, 1040), (593, 256)])  # a second wave of CTAs; four tokens per SM of 148 and one more
+def test_many_tokens_of_one_route(tokens, hidden):
+    test_int8_rows_and_routes(tokens, 1, 16, hidden, _lib.NUMERICS_TORCHREF)
+
+
+@pytest.mark.parametrize("tokens,top_k,experts,hidden", [(1, 1, 2, 16), (3, 2, 2, 8208), (37, 4, 16, 272), (129, 8, 9, 144), (297, 3, 5, 48)])
+def test_plane_rows(tokens, top_k, experts, hidden):
+    """Two int8 rows per route: 256 * high + low is the row's value in units of its largest magnitude / 32512, ties to even."""
+    generator = torch.Generator().manual_seed(tokens)
+    x = torch.randn((tokens, hidden), generator=generator).to(torch.bfloat16)
+    x[tokens // 2] = 0
+    ids = torch.stack([torch.randperm(experts, generator=generator)[:top_k] for _ in range(tokens)])
+    inter = hidden + 16  # wider than the rows: the planes of the intermediate have a region of their own
+    w13 = torch.zeros((experts, 2 * inter, hidden), dtype=torch.int8, device="cuda")
+    w2 = torch.zeros((experts, hidden, inter), dtype=torch.int8, device="cuda")
+    result = _lib.moe_forward(x.cuda(), w13, w2, torch.ones((tokens, top_k), device="cuda"), ids.cuda(), w8a16=True, w8a16_form=_lib.W8A16_FIXED_POINT,
+                              s13=torch.ones((experts, 2 * inter), device="cuda"), s2=torch.ones((experts, hidden), device="cuda"))
+    result.raise_for_status()
+    order, _, planes, scales = _rows(result, tokens, top_k, 2 * hidden, experts, torch.int8)
+    assert torch.equal(order.cpu().long(), torch.argsort(ids.reshape(-1), stable=True))
+    rows = x.float()[(order.cpu() // top_k).long()]
+    amax = rows.abs().amax(dim=1)
+    scale = torch.where(amax > 0, amax / 32512.0, torch.ones(()))
+    assert torch.equal(scales.cpu(), scale)
+    high, low = planes.cpu().view(-1, 2, hidden).to(torch.int32).unbind(1)
+    assert torch.equal((256 * high + low).float(), torch.round(rows / scale[:, None]).clamp(-32512, 32512))
