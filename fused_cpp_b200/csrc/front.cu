@@ -5,13 +5,10 @@
 // learn those positions.  With at most kFrontMaxRoutes routes a token's CTA counts them itself: the sorted position of a
 // route is the number of valid routes with a smaller expert id plus that of earlier routes with the same one, a few hundred
 // comparisons per slot that hide behind the load of the row.  CTA 0 is the route build of route.cu, the others one token
-// each; the GEMM behind it reads its work items behind its wait (GroupedGemmArgs::items_late).  Against the two launches, whole
-// forwards with the status read, cold L2: one token of the 16-expert layer (int8) 49.7 -> 48.2 us, 16 tokens 62.8 -> 60.9, 100 and
-// 200 tokens the same within the spread; bf16 52.1 -> 49.8, 77.6 -> 73.9, 89.6 -> 86.8, 93.9 -> 91.0; one token of the 256-expert layer
-// 105.9 -> 104.8.  Most of that is a launch less for the host.  On the device alone (captured, no status read) it gains for the
-// 256-expert layer (one token 87.3 -> 86.5) and W8A16 (16 tokens 38.5 -> 37.7), and costs small int8 layers the weights
-// that gate_up fetched while the rows were quantised: 16 experts, 1 / 16 / 65 / 200 tokens 24.8 -> 26.9, 37.8 -> 38.8, 45.9 -> 49.7,
-// 50.9 -> 52.8 us (bf16 65 tokens 65.7 -> 67.2).
+// each; the GEMM behind it reads its work items behind its wait (GroupedGemmArgs::items_late).  Against the two launches, device time
+// of a captured forward: 16 experts of 2048 x 1024, int8, 1 / 16 / 65 / 200 tokens 25.3 -> 23.2, 38.2 -> 37.0, 45.9 -> 44.1, 51.1 -> 48.7 us,
+// bf16 200 tokens 72.7 -> 70.6, W8A16 16 tokens 37.9 -> 36.2; one token of the 256-expert layer 87.1 -> 84.3.  Eager with the status read, where a
+// launch less for the host counts too: int8 1 and 16 tokens 50.2 -> 48.0, 63.4 -> 61.5, bf16 200 tokens 94.6 -> 91.2.
 // The reference's order of work is csrc/moe/arm/i8mm_w8a8/kernels.cpp:583-592 and :639-644.
 #include "common.cuh"
 #include "kernels.h"
@@ -27,10 +24,11 @@ constexpr int kFrontThreads = 512;
 constexpr int kFrontWarps = kFrontThreads / 32;
 constexpr int kFrontMaxRoutes = 1024;   // two rounds of comparisons per thread, one CTA of route build
 constexpr int kFrontMaxExperts = 512;   // histogram rows of kFrontWarps warps stay below the 48 KB every launch may have
-// A CTA per token; two of them fit an SM (62 registers a thread), so from 2 * SMs tokens on they run in two waves.  That is still
-// faster than two launches: device time of a captured forward with one route per token, int8, 512 experts of 2048 x 256, 443 tokens
-// 120.4 -> 116.8 us, 592 tokens 138.3 -> 134.9; 16 experts of 2048 x 1024 47.7 -> 46.5 (300 tokens), 51.0 -> 50.9 (592).
+// A CTA per token; two of them fit an SM, so from 2 * SMs tokens on they run in two waves.  That is still faster than two launches (one
+// route per token, captured: 512 experts of 2048 x 256, int8, 443 and 592 tokens 120.9 -> 117.8 us, 138.5 -> 136.0; 16 experts of
+// 2048 x 1024 47.9 -> 46.2 at 300 tokens, 51.3 -> 50.9 at 592).
 constexpr int kFrontTokensPerSm = 4;
+constexpr int kFrontCtasPerSm = 2;
 constexpr int kMaxTopK = 32;
 
 struct RouteArgs {
@@ -41,15 +39,20 @@ struct RouteArgs {
   ItemLists lists;
   const int* mirror;
   int *status, *counts, *offsets, *sorted_routes, *row_expert, *route_pos;
+  bool one_wave;  // every CTA of the launch is resident at once
 };
 
 // cols % 16 == 0, top_k <= 32.  The bits are those of route_build_kernel and of quantize_tokens_scatter_kernel,
 // split_tokens_scatter_planes_kernel or gather_tokens_scatter_kernel.
 template <FrontRows kRows>
-__global__ void __launch_bounds__(kFrontThreads)
+__global__ void __launch_bounds__(kFrontThreads, kFrontCtasPerSm)
 front_kernel(RouteArgs route, const uint16_t* x, int cols, int top_k, int numerics, void* rows_out, float* scale_out) {
   extern __shared__ int route_smem[];
-  ptx::launch_dependents();  // an ordinary launch: everything before it has completed
+  // (An ordinary launch: everything before it has completed.)  The GEMM behind may start once every CTA has let it in.  A CTA of a
+  // single wave does so when its row is read and its positions are counted: with the GEMM's CTAs beside them from the start the 16-expert
+  // int8 layer takes 49.2 instead of 44.1 us at 65 tokens, 26.7 instead of 23.2 at one.  With two waves the second one's start comes late by
+  // itself, and it lets the GEMM in at once (500 tokens of two routes, bf16, 97.5 -> 91.3 us).
+  if (!route.one_wave || blockIdx.x == 0) ptx::launch_dependents();
   if (blockIdx.x == 0) {
     route_build<false>(route_smem, route.topk_ids, route.routes, route.experts, route.warps, route.run, route.lists, route.status, route.mirror,
                        route.counts, route.offsets, route.sorted_routes, route.row_expert, route.route_pos);
@@ -113,6 +116,7 @@ front_kernel(RouteArgs route, const uint16_t* x, int cols, int top_k, int numeri
     inverse = __fdiv_rn(1.0f, scale);
     if (threadIdx.x < top_k && slot_ids[threadIdx.x] >= 0) scale_out[positions[threadIdx.x]] = scale;
   }
+  ptx::launch_dependents();
   with_numerics(kRows == FrontRows::kInt8 ? numerics : FMOE_NUMERICS_TORCHREF, [&](auto tag) {
     for (int v = threadIdx.x; v < vec16; v += kFrontThreads) {
       if (v >= kFrontThreads) {
@@ -159,7 +163,8 @@ cudaError_t launch_front(FrontRows rows, const int64_t* topk_ids, int64_t tokens
   const int64_t used = (routes + 31) / 32;
   const int warps = static_cast<int>(used < kFrontWarps ? used : kFrontWarps);
   const int64_t run = 32 * ((used + warps - 1) / warps);
-  const RouteArgs route = {topk_ids, routes, experts, warps, run, lists, mirror, status, counts, offsets, sorted_routes, row_expert, route_pos};
+  const RouteArgs route = {topk_ids, routes, experts, warps, run, lists, mirror, status, counts, offsets, sorted_routes, row_expert, route_pos,
+                           tokens + 1 <= static_cast<int64_t>(kFrontCtasPerSm) * threshold_sms};
   const size_t smem = route_smem_bytes(warps, experts, false);
   auto kernel = rows == FrontRows::kInt8    ? front_kernel<FrontRows::kInt8>
                 : rows == FrontRows::kBf16 ? front_kernel<FrontRows::kBf16>
