@@ -248,7 +248,9 @@ extern thread_local int threshold_sms;
 // (and the GEMM of a dense product) behind its first, an ordinary launch, are chained this way, under these rules (griddepcontrol, ptx.cuh):
 //   * every CTA calls grid_dependency_wait before it touches anything that the kernel before it reads or writes;
 //   * it calls launch_dependents (or ends) only after that; the exceptions are the second grouped GEMM of a split stage
-//     (`beside`) and the quantisers of the intermediate (quant.cu: held, warp and planes kernels), which do both the other way round.
+//     (`beside`) and the quantisers of the intermediate (quant.cu: held, warp and planes kernels), which do both the other way
+//     round.  (The two-pass kernel keeps the rule and has not been measured without: int8 rows of more than 2048 columns above
+//     four rows per SM, of more than 8192 up to there.)
 //     A kernel that has started therefore knows that every kernel but the one right before it has completed, or, right behind
 //     a `beside` kernel, every kernel but that one and the first GEMM of the stage, or, right behind that quantiser, every
 //     kernel but it and the gate_up stage.  What it may read before its wait is what none of them writes: weights, scales and

@@ -252,7 +252,8 @@ umma_grouped_gemm_kernel(const __grid_constant__ CUtensorMap weight_map, const _
   const int64_t unit_step = gridDim.x;
   ItemUnit cur = {0, 0, 0, 0};
   if (static_cast<int64_t>(blockIdx.x) < units) cur = resolve_unit(args.items, blockIdx.x, n_blocks, first_guess);
-  // The unit after `unit`: its load is in flight while the warps work on this one.
+  // The unit after `unit`, looked up ahead of the work on this one.  Its entry is waited for here, an L2 round trip: it says whether
+  // its expert has other items, and then which of them to read.
   auto load_next = [&](int64_t unit) {
     if (unit + unit_step >= units) return ItemUnit{0, 0, 0, 0};
     return resolve_unit(args.items, unit + unit_step, n_blocks, guess_item(args.items, unit + unit_step, n_blocks));
