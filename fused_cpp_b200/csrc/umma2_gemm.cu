@@ -57,7 +57,8 @@ constexpr int kThreads = 64 + kEpilogueThreads;
 // Pipeline stages: a stage holds a CTA's weight rows and the token rows of the list's largest item.  Up to 128 rows per item (64
 // per CTA) that is 24 KB instead of 36 and nine stages instead of six: with about a hundred rows per expert the weights'
 // stream bounds the kernel, and half as many of their bytes again are on the way (256-expert layer, 2500 tokens int8 2266 ->
-// 2203 us, 2048 tokens bf16 3888 -> 3835).
+// 2203 us, 2048 tokens bf16 3888 -> 3835).  One longer item puts the whole list back on six stages: with uniform routing over 256
+// experts a mean of a hundred rows has one about every second time, a mean of 110 nearly always.
 constexpr int kStages = 6;
 constexpr int kShortStages = 9;
 constexpr int kShortTokens = 64;
@@ -111,7 +112,8 @@ __device__ __forceinline__ void cluster_sync() {
 // stands in front of it) and publishes nothing that lies in memory, so it carries no cluster-wide release: that one waits
 // until every store of the warp has reached L2, which in the epilogue are the result rows of the unit before (256-expert layer,
 // 8192 tokens, int8, one pass after a pause: gate_up 1860 -> 1620 us, down 1015 -> 908, together with the release in front of
-// the element loop; a steady loop is held by the power limit and gains 1.6 %; 2048 tokens of the 20-expert layer 374 -> 359).
+// the element loop; a steady loop is held by the power limit and gains 2 %, which is the spread of two runs; 2048 tokens of the
+// 20-expert layer 374 -> 359).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_address) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
 }
