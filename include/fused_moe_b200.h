@@ -162,10 +162,10 @@ FMOE_API int fmoe_forward_checked(int32_t path, const void* x, const void* w13, 
 /* Stages of one forward call, in launch order.  With a stage timer in fmoe_config the forward records
  * a CUDA event on its stream before the first stage and after every stage; this is the GPU form of
  * the reference's FUSED_CPP_MOE_STAGE_TIMING report (csrc/moe/arm/common/fused_moe_bf16_tiled.cpp:6756-6762). */
-#define FMOE_STAGE_ROUTE 0      /* route build (3 kernels) */
-#define FMOE_STAGE_QUANT_IN 1   /* activation quantise + gather (W8A8) / gather (BF16) */
+#define FMOE_STAGE_ROUTE 0      /* route build; for small batches the token rows too, in the same kernel */
+#define FMOE_STAGE_QUANT_IN 1   /* activation quantise + gather (W8A8, W8A16) / gather (BF16); empty where the route stage made the rows */
 #define FMOE_STAGE_GATE_UP 2    /* grouped gate_up GEMM + SwiGLU epilogue */
-#define FMOE_STAGE_QUANT_MID 3  /* intermediate requantise (W8A8; empty for BF16) */
+#define FMOE_STAGE_QUANT_MID 3  /* intermediate requantise (W8A8, W8A16; empty for BF16) */
 #define FMOE_STAGE_DOWN 4       /* grouped down GEMM + dequant/un-permute epilogue */
 #define FMOE_STAGE_MERGE 5      /* top-k merge */
 #define FMOE_STAGES 6
